@@ -6,6 +6,10 @@
 // row's result does not depend on how many rows the launch holds, on the tile
 // shape chosen, or on which expert group the row fell into.
 //
+// Three kernels share that arithmetic: gemm_stream_kernel (few rows: the weights are
+// streamed once), gemm_tile_kernel (many rows: register tiles) and gemm_rows_kernel (any
+// size and alignment).  launch() says which takes what.
+//
 // Grouped use (routed experts; reference python/freetoken/moe/fused.py:267-337,
 // python/freetoken/kernel/triton/fused_moe.py:156-302): rows are sorted by
 // expert, group_offsets[g]..group_offsets[g+1] are expert g's rows, W holds one
@@ -15,6 +19,7 @@
 // The SwiGLU epilogue reads W as [gate rows 0..N-1 ; up rows N..2N-1] and
 // stores act(gate)*up (python/freetoken/kernel/triton/activation.py:96-107).
 #include "common.cuh"
+#include "mma_utils.cuh"
 
 namespace ft {
 
@@ -44,9 +49,48 @@ __device__ __forceinline__ float glu_act(float g, float u, int act, float alpha,
   return (g / (1.f + expf(-alpha * g))) * (u + 1.f);
 }
 
+// Warp 0 writes {group, first row, rows} of row tile blockIdx.x (rows 0: nothing to do): the groups' tile
+// counts are summed 32 groups at a time.
+template <int BM>
+__device__ __forceinline__ void find_tile(const GemmArgs& a, int* info) {
+  if (threadIdx.x >= 32) return;
+  if (!a.group_offsets) {
+    if (threadIdx.x == 0) {
+      info[0] = 0;
+      info[1] = blockIdx.x * BM;
+      info[2] = min(BM, a.M - (int)blockIdx.x * BM);
+    }
+    return;
+  }
+  const int tile = blockIdx.x, lane = threadIdx.x;
+  int before = 0;
+  for (int g0 = 0; g0 < a.G; g0 += 32) {
+    const int g = g0 + lane;
+    const int begin = g < a.G ? a.group_offsets[g] : 0, end = g < a.G ? a.group_offsets[g + 1] : 0;
+    const int nt = (end - begin + BM - 1) / BM;
+    int upto = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int first = before + upto - nt;
+    const bool mine = tile >= first && tile < first + nt;
+    if (mine) {
+      info[0] = g;
+      info[1] = begin + (tile - first) * BM;
+      info[2] = min(BM, end - info[1]);
+    }
+    if (__any_sync(0xffffffffu, mine)) return;
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  if (lane == 0) info[2] = 0;
+}
+
 constexpr int BN = 64;
 constexpr int BK = 32;
 
+// Any K, any alignment.
 template <typename AT, typename WT, typename OT, int BM, bool GLU>
 __global__ void __launch_bounds__(256) gemm_rows_kernel(GemmArgs a) {
   constexpr int TM = BM / 16, TN = BN / 16;
@@ -54,29 +98,8 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(GemmArgs a) {
   __shared__ float Ws[BN][BK + 1];
   __shared__ float Us[GLU ? BN : 1][BK + 1];
   __shared__ int tile_info[3];  // group, first row, rows
-  if (threadIdx.x == 0) {
-    int group = 0, row0 = 0, rows = 0;
-    if (!a.group_offsets) {
-      row0 = blockIdx.x * BM;
-      rows = min(BM, a.M - row0);
-    } else {
-      int tile = blockIdx.x;
-      for (int g = 0; g < a.G; ++g) {
-        const int begin = a.group_offsets[g], end = a.group_offsets[g + 1];
-        const int nt = (end - begin + BM - 1) / BM;
-        if (tile < nt) {
-          group = g;
-          row0 = begin + tile * BM;
-          rows = min(BM, end - row0);
-          break;
-        }
-        tile -= nt;
-      }
-    }
-    tile_info[0] = group;
-    tile_info[1] = row0;
-    tile_info[2] = rows;
-  }
+  pdl_wait();
+  find_tile<BM>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
   if (rows <= 0) return;
@@ -155,10 +178,6 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(GemmArgs a) {
   }
 }
 
-// Dense product for many rows: the same arithmetic (every output element is
-// one thread's fma chain over ascending k, so results are bit-identical to
-// gemm_rows_kernel) with 16-byte global loads, k-major shared tiles and
-// 128-bit shared loads.  Needs K % 32 == 0 and 16-byte aligned rows.
 __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
   const float4 a = *reinterpret_cast<const float4*>(p);
   const float4 b = *reinterpret_cast<const float4*>(p + 4);
@@ -174,91 +193,287 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
     v[2 * i + 1] = f.y;
   }
 }
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+// Two fused multiply-adds in one instruction; each half rounds like fmaf.
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long x, unsigned long long y) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
 
-template <typename AT, typename WT, typename OT>
-__global__ void __launch_bounds__(256) gemm_dense_kernel(GemmArgs a) {
-  constexpr int TBM = 64, TBN = 64, TBK = 32;
-  __shared__ __align__(16) float As[TBK][TBM + 4];
-  __shared__ __align__(16) float Ws[TBK][TBN + 4];
-  const int row0 = blockIdx.x * TBM, n0 = blockIdx.y * TBN;
+template <typename OT, bool GLU>
+__device__ __forceinline__ void store_out(const GemmArgs& a, OT* C, int crow, int n, float v, float up) {
+  if (GLU) v = glu_act(v, up, a.act, a.act_alpha, a.act_limit);
+  if (a.row_scale) v *= a.row_scale[crow];
+  C[(size_t)crow * a.ldc + n] = from_float<OT>(v);
+}
+
+// Few rows: the launch is bound by the weights it streams and, below that, by the one chain of K fused
+// multiply-adds an output is (4 cycles each: 4.3 us for K = 2048).  A lane owns a column, a warp R of the
+// block's MR rows; weights and rows come through STREAM_STAGES cp.async stages of STREAM_K values of k, so
+// that a block keeps three stages in flight and no thread's load waits for its arithmetic.  (The plain kernel
+// loads a 32-wide k tile, waits, multiplies and waits again: 53 products of two rows, K = 2048, N = 2048 .. 32768, took
+// 13,350 us and take 1,014.)  Weight rows are padded by 16 bytes: a quarter warp's 16-byte reads touch all banks.
+constexpr int STREAM_K = 128;
+constexpr int STREAM_STAGES = 4;
+constexpr int STREAM_COLS = 32;
+
+template <typename AT, typename WT, int MR, bool GLU>
+constexpr size_t stream_smem() {
+  return (size_t)STREAM_STAGES * ((GLU ? 2 : 1) * STREAM_COLS * (STREAM_K * sizeof(WT) + 16) + MR * STREAM_K * sizeof(AT));
+}
+
+template <typename AT, typename WT, typename OT, int MR, bool GLU>
+__global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(GemmArgs a) {
+  constexpr int WARPS = MR < 8 ? MR : 8, R = MR / WARPS, THREADS = 32 * WARPS;
+  constexpr int HALVES = GLU ? 2 : 1, WROWS = HALVES * STREAM_COLS;
+  constexpr int WROW = STREAM_K * sizeof(WT) + 16, AROW = STREAM_K * sizeof(AT);
+  constexpr int WPIECES = STREAM_K * sizeof(WT) / 16, APIECES = AROW / 16;       // 16-byte pieces of a row
+  constexpr int STAGE = WROWS * WROW + MR * AROW;
+  extern __shared__ __align__(16) unsigned char stream_sm[];
+  __shared__ int tile_info[3];
+  pdl_wait();
+  find_tile<MR>(a, tile_info);
+  __syncthreads();
+  const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
+  if (rows <= 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n0 = blockIdx.y * STREAM_COLS;
   const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
-  const WT* W = (const WT*)a.W + (size_t)blockIdx.z * a.w_batch_stride;
+  const WT* W = (const WT*)a.W + (size_t)group * a.w_group_stride + (size_t)blockIdx.z * a.w_batch_stride;
+
+  auto fetch = [&](int stage, int k0) {        // rows and columns beyond the last repeat it; k stops at K
+    unsigned char* to = stream_sm + stage * STAGE;
+    for (int i = threadIdx.x; i < WROWS * WPIECES; i += THREADS) {
+      const int n = i / WPIECES, piece = i % WPIECES, k = k0 + piece * (16 / (int)sizeof(WT));
+      const int col = min(n0 + n % STREAM_COLS, a.N - 1) + (n / STREAM_COLS) * a.N;
+      if (k < a.K) cp_async16(to + n * WROW + piece * 16, W + (size_t)col * a.K + k);
+    }
+    to += WROWS * WROW;
+    for (int i = threadIdx.x; i < MR * APIECES; i += THREADS) {
+      const int r = i / APIECES, piece = i % APIECES, k = k0 + piece * (16 / (int)sizeof(AT));
+      const int at = row0 + min(r, rows - 1);
+      const int src = a.a_rows ? a.a_rows[at] : at;
+      if (k < a.K) cp_async16(to + r * AROW + piece * 16, A + (size_t)src * a.lda + k);
+    }
+  };
+
+  float acc[HALVES][R];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[h][r] = 0.f;
+#pragma unroll
+  for (int s = 0; s < STREAM_STAGES - 1; ++s) {
+    if (s * STREAM_K < a.K) fetch(s, s * STREAM_K);
+    cp_async_commit();
+  }
+  int stage = 0;
+  for (int k0 = 0; k0 < a.K; k0 += STREAM_K) {
+    cp_async_wait<STREAM_STAGES - 2>();
+    __syncthreads();                           // this stage has landed for all; the one before it is free
+    const int ahead = k0 + (STREAM_STAGES - 1) * STREAM_K;
+    if (ahead < a.K) fetch((stage + STREAM_STAGES - 1) % STREAM_STAGES, ahead);
+    cp_async_commit();
+    const unsigned char* from = stream_sm + stage * STAGE;
+    const WT* ws = reinterpret_cast<const WT*>(from + lane * WROW);
+    const WT* us = reinterpret_cast<const WT*>(from + (STREAM_COLS + lane) * WROW);
+    const AT* as = reinterpret_cast<const AT*>(from + WROWS * WROW) + warp * R * STREAM_K;
+    auto eight = [&](int kk) {
+      float w[HALVES][8], x[8];
+      load8(ws + kk, w[0]);
+      if constexpr (GLU) load8(us + kk, w[HALVES - 1]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        load8(as + r * STREAM_K + kk, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int h = 0; h < HALVES; ++h) acc[h][r] = fmaf(x[i], w[h][i], acc[h][r]);
+      }
+    };
+    if (k0 + STREAM_K <= a.K) {
+#pragma unroll
+      for (int kk = 0; kk < STREAM_K; kk += 8) eight(kk);
+    } else {
+      for (int kk = 0; kk < a.K - k0; kk += 8) eight(kk);
+    }
+    stage = (stage + 1) % STREAM_STAGES;
+  }
+  cp_async_wait<0>();
+  OT* C = (OT*)a.C + (size_t)blockIdx.z * a.c_batch_stride;
+  const int n = n0 + lane;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int at = warp * R + r;
+    if (at < rows && n < a.N)
+      store_out<OT, GLU>(a, C, a.c_rows ? a.c_rows[row0 + at] : row0 + at, n, acc[0][r], acc[HALVES - 1][r]);
+  }
+}
+
+// Many rows: bound by the multiply-adds (72 TFLOP/s of them on this chip) and by what shared memory returns to
+// registers, 128 bytes a cycle whatever is broadcast (12 cycles a warp and k here, for 8 of arithmetic).  A block
+// takes 64 rows by 128 weight rows (GLU: 64 gate rows and the 64 up rows of the same features), a thread 4 rows by
+// 4 + 4 columns: three 16-byte shared loads feed 32 multiply-adds, issued two at a time.  The next 16 values of
+// k are fetched into registers while these are multiplied, and two shared buffers leave one barrier a step.
+// Measured: 342 x 3072 x 2048 in 126 us (64 x 64 tiles of 4 x 4 a thread, without the paired multiply-adds: 161),
+// gate_up + GLU of 684 rows over 8 experts, 2 x 2688 x 2048, in 571 us (the plain kernel: 1,124).  Tried and
+// slower at these sizes: 8 x 8 outputs a thread (545 and 158 us a launch, but 1,573 instead of 1,860 us for 2048 x
+// 4096 x 4096), 32 rows a block (158 us), two tiles of k ahead in registers (175 us).
+template <typename AT, typename WT, typename OT, bool GLU>
+__global__ void __launch_bounds__(256) gemm_tile_kernel(GemmArgs a) {
+  constexpr int TBM = 64, TBN = 128, TBK = 16, HALF = 64;
+  __shared__ __align__(16) float As[2][TBK][TBM + 4];
+  __shared__ __align__(16) float Ws[2][TBK][TBN + 4];
+  __shared__ int tile_info[3];
+  pdl_wait();
+  find_tile<TBM>(a, tile_info);
+  __syncthreads();
+  const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
+  if (rows <= 0) return;
+  const int n0 = blockIdx.y * (GLU ? HALF : TBN);
+  const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
+  const WT* W = (const WT*)a.W + (size_t)group * a.w_group_stride + (size_t)blockIdx.z * a.w_batch_stride;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 8;      // this thread loads row lr, k lk..lk+7
-  const bool a_ok = row0 + lr < a.M, w_ok = n0 + lr < a.N;
-  const AT* ap = A + (size_t)(a_ok ? row0 + lr : 0) * a.lda + lk;
-  const WT* wp = W + (size_t)(w_ok ? n0 + lr : 0) * a.K + lk;
-  float acc[4][4];
+  // this thread loads k ak .. ak + 3 of row ar and k wk .. wk + 7 of weight row wr; rows beyond the last repeat it
+  const int ar = threadIdx.x >> 2, ak = (threadIdx.x & 3) * 4, wr = threadIdx.x >> 1, wk = (threadIdx.x & 1) * 8;
+  const int at = row0 + min(ar, rows - 1);
+  const AT* ap = A + (size_t)(a.a_rows ? a.a_rows[at] : at) * a.lda + ak;
+  const int col = GLU ? min(n0 + (wr & (HALF - 1)), a.N - 1) + (wr >= HALF ? a.N : 0) : min(n0 + wr, a.N - 1);
+  const WT* wp = W + (size_t)col * a.K + wk;
+  unsigned long long acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  float av[8], wv[8];
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  float av[4], wv[8];
+  auto put = [&](int b) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) av[i] = wv[i] = 0.f;
-  if (a_ok) load8(ap, av);
-  if (w_ok) load8(wp, wv);
-  for (int k0 = 0; k0 < a.K; k0 += TBK) {
+    for (int i = 0; i < 4; ++i) As[b][ak + i][ar] = av[i];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      As[lk + i][lr] = av[i];
-      Ws[lk + i][lr] = wv[i];
-    }
-    __syncthreads();
-    if (k0 + TBK < a.K) {            // next tile's loads fly while this one is multiplied
-      if (a_ok) load8(ap + k0 + TBK, av);
-      if (w_ok) load8(wp + k0 + TBK, wv);
+    for (int i = 0; i < 8; ++i) Ws[b][wk + i][wr] = wv[i];
+  };
+  load4(ap, av);
+  load8(wp, wv);
+  put(0);
+  __syncthreads();
+  int b = 0;
+  for (int k0 = 0; k0 < a.K; k0 += TBK, b ^= 1) {
+    const bool more = k0 + TBK < a.K;
+    if (more) {
+      load4(ap + k0 + TBK, av);
+      load8(wp + k0 + TBK, wv);
     }
 #pragma unroll
     for (int kk = 0; kk < TBK; ++kk) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 w4 = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
-      const float ar[4] = {a4.x, a4.y, a4.z, a4.w}, wr[4] = {w4.x, w4.y, w4.z, w4.w};
+      const float4 x4 = *reinterpret_cast<const float4*>(&As[b][kk][ty * 4]);
+      const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][tx * 4]);
+      const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][HALF + tx * 4]);
+      const float xs[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+      for (int i = 0; i < 4; ++i) {
+        const unsigned long long x2 = pack2(xs[i], xs[i]);
+        fma2(acc[i][0], x2, w0.x);
+        fma2(acc[i][1], x2, w0.y);
+        fma2(acc[i][2], x2, w1.x);
+        fma2(acc[i][3], x2, w1.y);
+      }
     }
+    if (more) put(b ^ 1);
     __syncthreads();
   }
   OT* C = (OT*)a.C + (size_t)blockIdx.z * a.c_batch_stride;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = row0 + ty * 4 + i;
-    if (r >= a.M) continue;
+    const int r = ty * 4 + i;
+    if (r >= rows) continue;
+    const int crow = a.c_rows ? a.c_rows[row0 + r] : row0 + r;
+    float v[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < a.N) C[(size_t)r * a.ldc + n] = from_float<OT>(acc[i][j]);
+      const float2 f = unpack2(acc[i][j]);
+      v[2 * j] = f.x;
+      v[2 * j + 1] = f.y;
+    }
+#pragma unroll
+    for (int j = 0; j < (GLU ? 4 : 8); ++j) {
+      const int n = n0 + tx * 4 + (j & 3) + (j >= 4 ? HALF : 0);
+      if (n < a.N) store_out<OT, GLU>(a, C, crow, n, v[j], v[(j & 3) + 4]);
     }
   }
 }
 
-template <typename AT, typename WT, typename OT>
-int launch(const GemmArgs& a, int glu, int max_tiles_hint, cudaStream_t stream) {
-  const bool plain = !glu && !a.group_offsets && !a.a_rows && !a.c_rows && !a.row_scale;
-  const int a_align = sizeof(AT) == 2 ? 7 : 3, w_align = sizeof(WT) == 2 ? 7 : 3;
-  if (plain && a.M >= 64 && !(a.K & 31) && !(a.lda & a_align) && !(a.K & w_align) &&
-      !(a.a_batch_stride & a_align) && !(a.w_batch_stride & w_align) &&
-      !((uintptr_t)a.A & 15) && !((uintptr_t)a.W & 15)) {
-    dim3 grid((a.M + 63) / 64, (a.N + 63) / 64, a.batch);
-    gemm_dense_kernel<AT, WT, OT><<<grid, 256, 0, stream>>>(a);
-    return FT_OK;
+template <typename AT, typename WT, typename OT, int MR, bool GLU>
+int launch_stream(const GemmArgs& a, cudaStream_t stream) {
+  constexpr size_t smem = stream_smem<AT, WT, MR, GLU>();
+  const auto kernel = gemm_stream_kernel<AT, WT, OT, MR, GLU>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
   }
+  const int tiles = a.group_offsets ? a.M / MR + min(a.G, a.M) : (a.M + MR - 1) / MR;
+  const dim3 grid(tiles, (a.N + STREAM_COLS - 1) / STREAM_COLS, a.batch);
+  const cudaError_t e = launch_pdl(kernel, grid, dim3(32 * (MR < 8 ? MR : 8)), smem, stream, a);
+  return e == cudaSuccess ? FT_OK : (int)e;
+}
+
+template <typename AT, typename WT, typename OT, bool GLU>
+int launch_kind(const GemmArgs& a, cudaStream_t stream) {
   const int per_group = a.group_offsets ? a.M / max(a.G, 1) : a.M;
+  const int a_align = sizeof(AT) == 2 ? 7 : 3, w_align = sizeof(WT) == 2 ? 7 : 3;
+  const bool pieces = !(a.K & 7) && !(a.lda & a_align) && !(a.a_batch_stride & a_align) &&
+                      !(a.w_batch_stride & w_align) && !(a.w_group_stride & w_align) && !((uintptr_t)a.A & 15) &&
+                      !((uintptr_t)a.W & 15);
+  if (pieces) {
+    // Register tiles from 32 rows a group on, where they give half of the SMs a block; below that, and for few
+    // columns (a router's), the weights are streamed by many small blocks (342 rows of 8 columns: 24 instead of 99 us).
+    const int cols = (a.N + (GLU ? 63 : 127)) / (GLU ? 64 : 128);
+    if (!(a.K & 15) && per_group >= 32 && (a.M + 63) / 64 * (long long)cols * a.batch >= 64) {
+      const dim3 grid(a.group_offsets ? a.M / 64 + min(a.G, a.M) : (a.M + 63) / 64, cols, a.batch);
+      const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(256), 0, stream, a);
+      return e == cudaSuccess ? FT_OK : (int)e;
+    }
+    // rows a block: about twice a group's mean, so that most busy groups are read once
+    const int want = a.group_offsets ? 2 * ((a.M + a.G - 1) / a.G) : a.M;
+    if (want <= 1) return launch_stream<AT, WT, OT, 1, GLU>(a, stream);
+    if (want <= 2) return launch_stream<AT, WT, OT, 2, GLU>(a, stream);
+    if (want <= 4) return launch_stream<AT, WT, OT, 4, GLU>(a, stream);
+    if (want <= 8) return launch_stream<AT, WT, OT, 8, GLU>(a, stream);
+    return launch_stream<AT, WT, OT, 16, GLU>(a, stream);
+  }
   const bool big = per_group >= 32;
   const int bm = big ? 64 : 16;
   const int tiles = (a.M + bm - 1) / bm + (a.group_offsets ? a.G : 0);
-  dim3 grid(tiles, (a.N + BN - 1) / BN, a.batch);
-  (void)max_tiles_hint;
-  if (big) {
-    if (glu) gemm_rows_kernel<AT, WT, OT, 64, true><<<grid, 256, 0, stream>>>(a);
-    else gemm_rows_kernel<AT, WT, OT, 64, false><<<grid, 256, 0, stream>>>(a);
-  } else {
-    if (glu) gemm_rows_kernel<AT, WT, OT, 16, true><<<grid, 256, 0, stream>>>(a);
-    else gemm_rows_kernel<AT, WT, OT, 16, false><<<grid, 256, 0, stream>>>(a);
-  }
-  return FT_OK;
+  const dim3 grid(tiles, (a.N + BN - 1) / BN, a.batch);
+  const cudaError_t e = big ? launch_pdl(gemm_rows_kernel<AT, WT, OT, 64, GLU>, grid, dim3(256), 0, stream, a)
+                            : launch_pdl(gemm_rows_kernel<AT, WT, OT, 16, GLU>, grid, dim3(256), 0, stream, a);
+  return e == cudaSuccess ? FT_OK : (int)e;
+}
+
+template <typename AT, typename WT, typename OT>
+int launch(const GemmArgs& a, int glu, cudaStream_t stream) {
+  return glu ? launch_kind<AT, WT, OT, true>(a, stream) : launch_kind<AT, WT, OT, false>(a, stream);
 }
 
 }  // namespace ft
@@ -285,11 +500,11 @@ extern "C" int ft_gemm_rows(const void* A, int a_dtype, long long lda, const voi
   const int key = a_dtype * 100 + w_dtype * 10 + c_dtype;
   int rc;
   switch (key) {
-    case 0: rc = launch<float, float, float>(a, glu, 0, stream); break;
-    case 10: rc = launch<float, __nv_bfloat16, float>(a, glu, 0, stream); break;
-    case 111: rc = launch<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(a, glu, 0, stream); break;
-    case 110: rc = launch<__nv_bfloat16, __nv_bfloat16, float>(a, glu, 0, stream); break;
-    case 100: rc = launch<__nv_bfloat16, float, float>(a, glu, 0, stream); break;
+    case 0: rc = launch<float, float, float>(a, glu, stream); break;
+    case 10: rc = launch<float, __nv_bfloat16, float>(a, glu, stream); break;
+    case 111: rc = launch<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(a, glu, stream); break;
+    case 110: rc = launch<__nv_bfloat16, __nv_bfloat16, float>(a, glu, stream); break;
+    case 100: rc = launch<__nv_bfloat16, float, float>(a, glu, stream); break;
     default: return FT_ERR_DTYPE;
   }
   if (rc != FT_OK) return rc;
@@ -310,11 +525,11 @@ extern "C" int ft_gemm_heads(const void* A, int a_dtype, long long lda, long lon
   const int key = a_dtype * 100 + w_dtype * 10 + c_dtype;
   int rc;
   switch (key) {
-    case 0: rc = launch<float, float, float>(a, 0, 0, stream); break;
-    case 10: rc = launch<float, __nv_bfloat16, float>(a, 0, 0, stream); break;
-    case 111: rc = launch<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(a, 0, 0, stream); break;
-    case 110: rc = launch<__nv_bfloat16, __nv_bfloat16, float>(a, 0, 0, stream); break;
-    case 100: rc = launch<__nv_bfloat16, float, float>(a, 0, 0, stream); break;
+    case 0: rc = launch<float, float, float>(a, 0, stream); break;
+    case 10: rc = launch<float, __nv_bfloat16, float>(a, 0, stream); break;
+    case 111: rc = launch<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(a, 0, stream); break;
+    case 110: rc = launch<__nv_bfloat16, __nv_bfloat16, float>(a, 0, stream); break;
+    case 100: rc = launch<__nv_bfloat16, float, float>(a, 0, stream); break;
     default: return FT_ERR_DTYPE;
   }
   if (rc != FT_OK) return rc;
