@@ -16,7 +16,12 @@
 // of its own chunk: floor(j / chunk) == floor(pos / chunk)), scores capped
 // as cap * tanh(s / cap), and a sink - a score without key or value that enters
 // the softmax's denominator only, fixed (sink_mode 1) or one per query head (2).
+//
+// Two kernels with the same arithmetic.  attn_shared_kernel brings a chunk's keys and values into shared
+// memory once for all the (token, head) rows of a block that read them; attn_paged_kernel reads them from
+// global memory row by row (head sizes above 256, rows that are no multiple of 16 bytes).
 #include "common.cuh"
+#include "mma_utils.cuh"
 
 namespace ft {
 
@@ -116,6 +121,174 @@ __global__ void __launch_bounds__(128) attn_paged_kernel(AttnArgs a) {
   }
 }
 
+// A block's eight warps are (token, query head) rows of one KV head: `tokens` tokens by `heads` heads.  The
+// rows of one request walk the chunks together: every chunk is fetched once by all threads (cp.async, 16-byte
+// pieces, the next chunk on its way while this one is used), and a warp leaves out the chunks that its own
+// token does not see, so its arithmetic is attn_paged_kernel's, operation by operation.  That kernel is bound
+// by latency: a lane reads its key's row from global memory value by value.
+// Measured (16 heads of 128 on 4 KV heads, float32): two prompts of 214 and 128 tokens in 70 us, a token behind
+// each in 25; four launches of the one and sixteen of the other took 4,552 us and take 686.
+constexpr int SHARED_WARPS = 8;
+
+__device__ __forceinline__ void piece_of(const float* p, float (&v)[4]) {
+  const float4 f = *reinterpret_cast<const float4*>(p);
+  v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+__device__ __forceinline__ void piece_of(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+
+template <typename AT, bool EXACT>
+__global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs a, int T, int tokens, int heads) {
+  constexpr int MAXD = 8, PIECE = 16 / sizeof(AT), CHUNK = 32;
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ int row_seg[SHARED_WARPS], row_lo[SHARED_WARPS], row_pos[SHARED_WARPS];
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int d = a.d, group = a.nq / a.nkv, slices = (group + heads - 1) / heads;
+  const int krow = d * sizeof(AT) + 16, vrow = d * sizeof(AT);       // padded key rows: no bank conflicts
+  const int stage_bytes = CHUNK * (krow + vrow);
+  float* qv = reinterpret_cast<float*>(sm + 2 * stage_bytes) + warp * d;
+  const int kvh = blockIdx.y / slices, in_group = (blockIdx.y % slices) * heads + warp % heads;
+  const int r = blockIdx.x * tokens + warp / heads;
+  const bool live = r < T && warp / heads < tokens && in_group < group;
+  const int h = kvh * group + in_group;
+  int t = 0, pos = -1, lo = 0;
+  if (live) {
+    t = a.rows ? a.rows[r] : r;
+    pos = a.token_pos[t];
+    lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
+    const AT* q = (const AT*)a.q + ((size_t)t * a.nq + h) * d;
+    for (int i = lane; i < d; i += 32) qv[i] = to_float(q[i]);
+  }
+  if (lane == 0) {
+    row_seg[warp] = live ? a.token_seg[t] : -1;
+    row_lo[warp] = lo;
+    row_pos[warp] = pos;
+  }
+  __syncthreads();
+
+  float acc[MAXD];
+#pragma unroll
+  for (int c = 0; c < MAXD; ++c) acc[c] = 0.f;
+  float m = -INFINITY, l = 0.f;
+  const AT* kbase = (const AT*)a.kv_pages + (size_t)kvh * a.P * d;
+  const AT* vbase = kbase + a.kv_stride;
+
+  unsigned todo = 0;
+  for (int w = 0; w < SHARED_WARPS; ++w) todo |= row_seg[w] >= 0 ? 1u << w : 0u;
+  while (todo) {                               // one request after the other (mostly there is one)
+    const int seg = row_seg[__ffs(todo) - 1];
+    int first = INT_MAX, last = -1;
+    for (int w = 0; w < SHARED_WARPS; ++w) {
+      if (row_seg[w] != seg) continue;
+      todo &= ~(1u << w);
+      first = min(first, row_lo[w]);
+      last = max(last, row_pos[w]);
+    }
+    const int* table = a.block_table + (size_t)seg * a.table_width;
+    auto fetch = [&](int stage, int c0) {      // keys outside first .. last are never read: those repeat one of them
+      unsigned char* ks = sm + stage * stage_bytes;
+      unsigned char* vs = ks + CHUNK * krow;
+      const int pieces = d / PIECE;
+      for (int i = threadIdx.x; i < CHUNK * pieces; i += 32 * SHARED_WARPS) {
+        const int jj = i / pieces, piece = i % pieces;
+        const int j = min(max(c0 + jj, first), last);
+        const size_t at = (size_t)table[j / a.P] * a.page_stride + (size_t)(j % a.P) * d + piece * PIECE;
+        cp_async16(ks + jj * krow + piece * 16, kbase + at);
+        cp_async16(vs + jj * vrow + piece * 16, vbase + at);
+      }
+    };
+    const int begin = first / CHUNK * CHUNK;
+    fetch(0, begin);
+    cp_async_commit();
+    int stage = 0;
+    for (int c0 = begin; c0 <= last; c0 += CHUNK, stage ^= 1) {
+      if (c0 + CHUNK <= last) fetch(stage ^ 1, c0 + CHUNK);
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncthreads();
+      if (row_seg[warp] == seg && c0 <= pos && c0 + CHUNK > lo) {
+        const unsigned char* ks = sm + stage * stage_bytes;
+        const AT* kr = reinterpret_cast<const AT*>(ks + lane * krow);
+        const AT* vs = reinterpret_cast<const AT*>(ks + CHUNK * krow);
+        const int j = c0 + lane;
+        const bool valid = j >= lo && j <= pos;
+        float dot = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < d; i += PIECE) {
+          float kv[PIECE];
+          piece_of(kr + i, kv);
+#pragma unroll
+          for (int e = 0; e < PIECE; ++e) dot = fmaf(qv[i + e], kv[e], dot);
+        }
+        float s = -INFINITY;
+        if (valid) {
+          s = dot * a.scale;
+          if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+        }
+        const float m_new = fmaxf(m, warp_max(s));
+        const float p = valid ? (EXACT ? expf(s - m_new) : __expf(s - m_new)) : 0.f;
+        const float alpha = (m == -INFINITY) ? 0.f : (EXACT ? expf(m - m_new) : __expf(m - m_new));
+        l = l * alpha + warp_sum(p);
+        m = m_new;
+#pragma unroll
+        for (int c = 0; c < MAXD; ++c) acc[c] *= alpha;
+        const int jj_lo = max(lo - c0, 0), jj_hi = min(pos - c0, CHUNK - 1);
+#pragma unroll 4
+        for (int jj = jj_lo; jj <= jj_hi; ++jj) {
+          const float pj = __shfl_sync(0xffffffffu, p, jj);
+#pragma unroll
+          for (int c = 0; c < MAXD; ++c) {
+            const int i = lane + 32 * c;
+            if (i < d) acc[c] = fmaf(pj, to_float(vs[jj * d + i]), acc[c]);
+          }
+        }
+      }
+      __syncthreads();                         // the stage may be written again
+    }
+    cp_async_wait<0>();
+  }
+  if (!live) return;
+  if (a.sink_mode) {
+    const float sk = a.sink_mode == 2 ? a.sink[h] : a.sink_value;
+    const float m_new = fmaxf(m, sk);
+    const float alpha = EXACT ? expf(m - m_new) : __expf(m - m_new);
+    l = l * alpha + (EXACT ? expf(sk - m_new) : __expf(sk - m_new));
+#pragma unroll
+    for (int c = 0; c < MAXD; ++c) acc[c] *= alpha;
+  }
+  AT* o = (AT*)a.out + ((size_t)t * a.nq + h) * d;
+  const float inv = 1.f / l;
+#pragma unroll
+  for (int c = 0; c < MAXD; ++c) {
+    const int i = lane + 32 * c;
+    if (i < d) o[i] = from_float<AT>(acc[c] * inv);
+  }
+}
+
+template <typename AT, bool EXACT>
+static int launch_shared(const AttnArgs& a, int T, cudaStream_t stream) {
+  const size_t smem = 2 * (size_t)32 * (2 * a.d * sizeof(AT) + 16) + (size_t)SHARED_WARPS * a.d * sizeof(float);
+  const auto kernel = attn_shared_kernel<AT, EXACT>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const int group = a.nq / a.nkv, heads = min(group, SHARED_WARPS), slices = (group + heads - 1) / heads;
+  // a token a block while that leaves SMs without one; otherwise neighbouring tokens share the chunks
+  const int tokens = (long long)T * a.nkv * slices <= 2 * 148 ? 1 : SHARED_WARPS / heads;
+  const cudaError_t le = launch_pdl(kernel, dim3((T + tokens - 1) / tokens, a.nkv * slices), dim3(32 * SHARED_WARPS),
+                                    smem, stream, a, T, tokens, heads);
+  return le == cudaSuccess ? FT_OK : (int)le;
+}
+
 }  // namespace ft
 
 using namespace ft;
@@ -135,7 +308,13 @@ extern "C" int ft_attn_paged_simt(const void* q, void* out, const void* kv_pages
   dim3 grid(T, (nq + 3) / 4);
   const size_t smem = 4 * (size_t)d * sizeof(float);
   if (dtype != FT_DTYPE_F32 && dtype != FT_DTYPE_BF16) return FT_ERR_DTYPE;
-  if (d <= 256) {
+  const int in_piece = dtype == FT_DTYPE_F32 ? 3 : 7;              // 16-byte pieces along a row, from its start
+  if (d <= 256 && !(d & in_piece) && !(page_stride & in_piece) && !(kv_stride & in_piece) && !((uintptr_t)kv_pages & 15) &&
+      (long long)nkv * nq <= 65535) {
+    const int rc = dtype == FT_DTYPE_F32 ? launch_shared<float, true>(a, T, stream)
+                                         : launch_shared<__nv_bfloat16, false>(a, T, stream);
+    if (rc != FT_OK) return rc;
+  } else if (d <= 256) {
     if (dtype == FT_DTYPE_F32) attn_paged_kernel<float, true, 8><<<grid, 128, smem, stream>>>(a);
     else attn_paged_kernel<__nv_bfloat16, false, 8><<<grid, 128, smem, stream>>>(a);
   } else if (d <= 512) {        // a latent that is wider than any head
