@@ -691,10 +691,10 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         raise KernelError("ssd_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * state_dim * head_dim:
         raise KernelError("ssd_scan: a state row must hold heads * state_dim * head_dim values")
-    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i")
+    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i")
     _check(f(_ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
              _ptr(state), state.stride(0), _ptr(y), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim,
-             state_dim, groups, seg_slot.numel(), code(xbc.dtype), _stream()), "ssd_scan")
+             state_dim, groups, seg_slot.numel(), T, code(xbc.dtype), _stream()), "ssd_scan")
 
 
 def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
@@ -721,10 +721,10 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bi
         raise KernelError("delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i")
+    f = _fn("recurrent", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), _ptr(decay), beta.stride(0), _ptr(dt_bias), _ptr(a_log),
              _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), code(qkv.dtype),
+             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, code(qkv.dtype),
              _stream()), "delta_scan")
 
 
@@ -751,10 +751,10 @@ def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tenso
         raise KernelError("channel_delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("channel_delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i")
+    f = _fn("recurrent", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(decay), decay.stride(0), _ptr(dt_bias),
              _ptr(a_log), _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), code(qkv.dtype), _stream()),
+             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, code(qkv.dtype), _stream()),
            "channel_delta_scan")
 
 
@@ -780,10 +780,10 @@ def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[tor
         raise KernelError("retention_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("retention_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_retention_scan", "p q p p i p p q p p p i i i f i i")
+    f = _fn("recurrent", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(decay), _ptr(cos_sin), rot, _ptr(seg_pos0), _ptr(state), state.stride(0),
              _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim, key_dim, float(k_scale),
-             seg_slot.numel(), code(qkv.dtype), _stream()), "retention_scan")
+             seg_slot.numel(), T, code(qkv.dtype), _stream()), "retention_scan")
 
 
 def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: torch.Tensor, token_seg: torch.Tensor,

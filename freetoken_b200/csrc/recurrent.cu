@@ -20,7 +20,9 @@
 // products are one warp reduction; a block's four warps share the tokens of a
 // chunk, which all threads stage into shared memory together.  Which WC a launch
 // takes depends on the step's shape, never on a token's place in it, and the
-// operations on a column are the same for every WC.
+// operations on a column are the same for every WC.  Launches in which some segment
+// has several tokens take kernels with 16 lanes a column that perform the same
+// operations (see there).
 #include "common.cuh"
 
 namespace ft {
@@ -686,6 +688,514 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   }
 }
 
+// ------------------------------------------------- segments of several tokens
+// A prompt portion's tokens are a chain, and the kernels above spend a microsecond and more on four of them: 32
+// lanes a column, five shuffle stages for the unit vectors, five for the column sums, a broadcast.  Here a column
+// belongs to 16 lanes; lane l keeps rows l + 32 e and l + 16 + 32 e of CPL columns, sums them in two chains (what
+// lanes l and l + 16 sum above) and adds the two, so that four shuffle stages remain and every sum has the bits of
+// the kernels above: which of the two a launch takes does not show in the results.  What does not wait for the
+// state (unit vectors, gates, rotations, k . q) is done while a chunk is staged, a warp a token; what nothing waits
+// for (the read-outs) is added over the lanes once a chunk, for its eight tokens together.  q and k rows lie in
+// shared memory in the lanes' order, so that a lane reads its rows in 16-byte pieces.  Four warps work and four stage (the staging's chain of
+// sums, roots and exponentials is as long as eight tokens' work), with two more chunks on their way in registers.
+// A chain of eight tokens is bound by its own latency, many segments by issue slots.  Measured, before and now
+// (us): one segment of 2,048 tokens, 16 heads of 128 x 128: delta rule 1,037 -> 347, with a decay per channel 1,469
+// -> 575, retention 904 -> 338; 32 heads of 64 x 128 of the state space 579 -> 203.  Four segments of 640 .. 1,335
+// tokens, 32 heads (64): 1,364 -> 750, 1,665 -> 1,049, 1,257 -> 598, 709 -> 427.
+constexpr int SEQ_WARPS = 4;
+constexpr int SEQ_THREADS = 64 * SEQ_WARPS;           // as many warps stage as work
+constexpr int SEQ_CHUNK = 8;
+constexpr int SEQ_PER_WARP = SEQ_CHUNK / SEQ_WARPS;    // tokens a staging warp takes of a chunk
+
+// place of row n in a staged row: lane n & 15 holds its rows one behind the other, in pieces of four (two)
+template <int NPL>
+__device__ __forceinline__ int seq_place(int n) {
+  const int l = n & 15, i = ((n >> 4) & 1) + 2 * (n >> 5);
+  return NPL == 1 ? 2 * l + i : (i >> 2) * 64 + 4 * l + (i & 3);
+}
+template <int NPL>
+__device__ __forceinline__ void seq_row(const float* row, int l, float (&v)[2 * NPL]) {
+  if constexpr (NPL == 1) {
+    const float2 f = *reinterpret_cast<const float2*>(row + 2 * l);
+    v[0] = f.x; v[1] = f.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 2 * NPL; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(row + 16 * i + 4 * l);
+      v[i] = f.x; v[i + 1] = f.y; v[i + 2] = f.z; v[i + 3] = f.w;
+    }
+  }
+}
+// part[t] of the 16 lanes of a column summed: lane l ends with token l >> 1
+__device__ __forceinline__ void seq_totals(float (&part)[SEQ_CHUNK], int l) {
+  int mask = 8;
+#pragma unroll
+  for (int w = SEQ_CHUNK / 2; w >= 1; w >>= 1) {
+    const bool upper = l & mask;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float send = upper ? part[i] : part[i + w];
+      const float keep = upper ? part[i + w] : part[i];
+      part[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+    }
+    mask >>= 1;
+  }
+  part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+}
+// the columns of row n that a lane owns
+template <int NPL, int CPL>
+__device__ __forceinline__ void seq_load_state(const float* st, int rows, int P, int col, int l, bool vec,
+                                               float (&S)[2 * NPL][CPL]) {
+#pragma unroll
+  for (int i = 0; i < 2 * NPL; ++i) {
+    const int n = l + 16 * i;
+    if (n < rows) load_cols<CPL>(st + (size_t)n * P + col, S[i], P - col, vec);
+    else {
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) S[i][c] = 0.f;
+    }
+  }
+}
+template <int NPL, int CPL>
+__device__ __forceinline__ void seq_store_state(float* st, int rows, int P, int col, int l, bool vec,
+                                                const float (&S)[2 * NPL][CPL]) {
+#pragma unroll
+  for (int i = 0; i < 2 * NPL; ++i) {
+    const int n = l + 16 * i;
+    if (n < rows) store_cols<CPL>(st + (size_t)n * P + col, S[i], P - col, vec);
+  }
+}
+
+constexpr int seq_buffer(int npl, int cpl, int rows) {           // floats of one buffer: rows of 32 npl, columns, gates
+  return SEQ_CHUNK * (rows * 32 * npl + 2 * SEQ_WARPS * cpl + 4);
+}
+
+// The three modes of delta_scan_kernel.
+template <typename AT, int NPL, int CPL, int MODE>
+__global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel(DeltaArgs a) {
+  constexpr int R = 2 * NPL, DP = 32 * NPL, COLS = 2 * SEQ_WARPS * CPL;
+  constexpr int PER = seq_buffer(NPL, CPL, MODE == 1 ? 3 : 2);
+  constexpr int VR = (SEQ_CHUNK * COLS + 32 * SEQ_WARPS - 1) / (32 * SEQ_WARPS);
+  extern __shared__ __align__(16) float sm[];
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % SEQ_WARPS, l = lane & 15;
+  const bool stages = threadIdx.x >= 32 * SEQ_WARPS;
+  const int head = blockIdx.y, seg = blockIdx.z;
+  const int D = a.D, P = a.P;
+  const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1];
+  if (q1 <= q0) return;
+  const int g = head / (a.heads / a.G);
+  const int width = a.heads * P;
+  const int col0 = blockIdx.x * COLS, cb = (2 * warp + (lane >> 4)) * CPL, col = col0 + cb;
+  float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * D * P;
+  const float rate = MODE == 2 ? 0.f : -expf(a.A_log[head]);
+  const float bias = MODE == 1 ? 0.f : a.dt_bias[head];          // MODE 2: the head's constant decay
+  const AT* qkv = (const AT*)a.qkv;
+  const int half = MODE == 2 ? a.rot_dims >> 1 : 0;
+  const int pos0 = MODE == 2 && half ? a.seg_pos0[seg] : 0;
+  float ch_bias[NPL];
+  if constexpr (MODE == 1) {
+#pragma unroll
+    for (int e = 0; e < NPL; ++e) {
+      const int n = lane + 32 * e;
+      ch_bias[e] = n < D ? a.dt_bias[(size_t)head * D + n] : 0.f;
+    }
+  }
+  struct Staged {
+    AT q[SEQ_PER_WARP][NPL], k[SEQ_PER_WARP][NPL], v[VR], beta[SEQ_PER_WARP], decay[SEQ_PER_WARP];
+    float g[MODE == 1 ? SEQ_PER_WARP : 1][NPL], c[MODE == 2 ? SEQ_PER_WARP : 1][NPL], s[MODE == 2 ? SEQ_PER_WARP : 1][NPL];
+  } even, odd;
+  auto fetch = [&](int t0, Staged& x) {
+    const int nt = min(SEQ_CHUNK, q1 - t0);                      // may be 0 or less: nothing is read
+#pragma unroll
+    for (int j = 0; j < SEQ_PER_WARP; ++j) {
+      const int tt = warp + SEQ_WARPS * j;
+      const size_t t = t0 + tt;
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        const int n = lane + 32 * e;
+        const bool in = tt < nt && n < D;
+        const AT* row = qkv + t * a.ld + (size_t)g * D + n;
+        x.q[j][e] = in ? row[0] : from_float<AT>(0.f);
+        x.k[j][e] = in ? row[(size_t)a.G * D] : from_float<AT>(0.f);
+        if constexpr (MODE == 1) x.g[j][e] = in ? a.decay_rows[t * a.ld_decay + (size_t)head * D + n] : 0.f;
+        if constexpr (MODE == 2) {
+          if (in && n < 2 * half) {
+            const float* cs = a.cos_sin + (size_t)(pos0 + t0 + tt - q0) * a.rot_dims + (n < half ? n : n - half);
+            x.c[j][e] = cs[0];
+            x.s[j][e] = cs[half];
+          }
+        }
+      }
+      if (MODE != 2 && tt < nt) {
+        const size_t at = t * a.ld_gate + head;
+        x.beta[j] = ((const AT*)a.beta)[at];
+        if constexpr (MODE == 0) x.decay[j] = ((const AT*)a.decay)[at];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < VR; ++r) {
+      const int i = threadIdx.x % (32 * SEQ_WARPS) + 32 * SEQ_WARPS * r, tt = i / COLS, c = i % COLS;
+      x.v[r] = (tt < nt && col0 + c < P)
+                   ? qkv[(size_t)(t0 + tt) * a.ld + 2 * (size_t)a.G * D + (size_t)head * P + col0 + c]
+                   : from_float<AT>(0.f);
+    }
+  };
+  auto put = [&](float* buf, const Staged& x) {
+    float* qs = buf;
+    float* ks = qs + SEQ_CHUNK * DP;
+    float* gs = ks + SEQ_CHUNK * DP;                             // MODE 1
+    float* vs = gs + (MODE == 1 ? SEQ_CHUNK * DP : 0);
+    float4* gates = reinterpret_cast<float4*>(vs + SEQ_CHUNK * COLS);      // write strength, decay, k . q
+    float kq[SEQ_PER_WARP];
+#pragma unroll
+    for (int j = 0; j < SEQ_PER_WARP; ++j) {
+      const int tt = warp + SEQ_WARPS * j;
+      float qv[NPL], kv[NPL], unit[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        qv[e] = to_float(x.q[j][e]);
+        kv[e] = to_float(x.k[j][e]);
+      }
+      if constexpr (MODE == 2) {
+        if (half) {                                              // a pair's two values meet in the token's own rows
+          float* qr = qs + tt * DP;
+          float* kr = ks + tt * DP;
+#pragma unroll
+          for (int e = 0; e < NPL; ++e) {
+            qr[lane + 32 * e] = qv[e];
+            kr[lane + 32 * e] = kv[e];
+          }
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < NPL; ++e) {
+            const int n = lane + 32 * e;
+            if (n < 2 * half) {                                  // rounded as delta_scan_kernel rounds
+              const float c = x.c[j][e], sn = x.s[j][e];
+              const int other = n < half ? n + half : n - half;
+              const float qo = qr[other], ko = kr[other];
+              qv[e] = n < half ? __fmaf_rn(qv[e], c, -__fmul_rn(qo, sn)) : __fmaf_rn(qo, sn, __fmul_rn(qv[e], c));
+              kv[e] = n < half ? __fmaf_rn(kv[e], c, -__fmul_rn(ko, sn)) : __fmaf_rn(ko, sn, __fmul_rn(kv[e], c));
+            }
+          }
+          __syncwarp();
+        }
+#pragma unroll
+        for (int e = 0; e < NPL; ++e) kv[e] *= a.q_scale;
+      }
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        unit[0] = fmaf(qv[e], qv[e], unit[0]);
+        unit[1] = fmaf(kv[e], kv[e], unit[1]);
+        unit[2] = fmaf(qv[e], kv[e], unit[2]);
+      }
+      warp_sum_multi<4>(unit);                                   // lane n holds value n >> 3
+      if constexpr (MODE == 2) {
+        kq[j] = __shfl_sync(0xffffffffu, unit[0], 16);
+      } else {
+        const float iq = a.q_scale / sqrtf(__shfl_sync(0xffffffffu, unit[0], 0) + a.unit_eps);
+        const float ik = 1.f / sqrtf(__shfl_sync(0xffffffffu, unit[0], 8) + a.unit_eps);
+        kq[j] = __shfl_sync(0xffffffffu, unit[0], 16) * iq * ik;
+#pragma unroll
+        for (int e = 0; e < NPL; ++e) {
+          qv[e] *= iq;
+          kv[e] *= ik;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        const int n = lane + 32 * e, at = tt * DP + seq_place<NPL>(n);
+        qs[at] = qv[e];
+        ks[at] = kv[e];
+        if constexpr (MODE == 1) gs[at] = n < D ? expf(rate * softplus_f(x.g[j][e] + ch_bias[e])) : 1.f;
+      }
+    }
+    if (lane < SEQ_PER_WARP) {                                   // a lane a token
+      float beta = 1.f, decay = bias, product = kq[0];
+      if constexpr (MODE != 2) {
+        AT raw_beta = x.beta[0], raw_decay = x.decay[0];
+#pragma unroll
+        for (int j = 1; j < SEQ_PER_WARP; ++j)
+          if (lane == j) { raw_beta = x.beta[j]; raw_decay = x.decay[j]; }
+        beta = 1.f / (1.f + expf(-to_float(raw_beta)));
+        decay = MODE == 1 ? 1.f : expf(rate * softplus_f(to_float(raw_decay) + bias));
+      }
+#pragma unroll
+      for (int j = 1; j < SEQ_PER_WARP; ++j)
+        if (lane == j) product = kq[j];
+      gates[warp + SEQ_WARPS * lane] = make_float4(beta, decay, product, 0.f);
+    }
+#pragma unroll
+    for (int r = 0; r < VR; ++r) {
+      const int i = threadIdx.x % (32 * SEQ_WARPS) + 32 * SEQ_WARPS * r;
+      if (i < SEQ_CHUNK * COLS) vs[i] = to_float(x.v[r]);
+    }
+  };
+
+  if (stages) {
+    // two chunks on their way in registers; a buffer is filled while the other one is worked through
+    fetch(q0, even);
+    fetch(q0 + SEQ_CHUNK, odd);
+    put(sm, even);
+    fetch(q0 + 2 * SEQ_CHUNK, even);
+    __syncthreads();
+    for (int t0 = q0; t0 < q1; t0 += 2 * SEQ_CHUNK) {
+      if (t0 + SEQ_CHUNK < q1) put(sm + PER, odd);
+      fetch(t0 + 3 * SEQ_CHUNK, odd);
+      __syncthreads();
+      if (t0 + SEQ_CHUNK >= q1) break;
+      if (t0 + 2 * SEQ_CHUNK < q1) put(sm, even);
+      fetch(t0 + 4 * SEQ_CHUNK, even);
+      __syncthreads();
+    }
+    return;
+  }
+  float S[R][CPL];
+  seq_load_state<NPL, CPL>(st, D, P, col, l, a.vec, S);
+  auto chunk = [&](int t0, int turn) {
+    const int nt = min(SEQ_CHUNK, q1 - t0);
+    const float* qs = sm + turn * PER;
+    const float* ks = qs + SEQ_CHUNK * DP;
+    const float* gs = ks + SEQ_CHUNK * DP;
+    float* vs = sm + turn * PER + (MODE == 1 ? 3 : 2) * SEQ_CHUNK * DP;
+    const float4* gates = reinterpret_cast<const float4*>(vs + SEQ_CHUNK * COLS);
+    float part[CPL][SEQ_CHUNK];
+    auto token = [&](int tt) {
+      float q[R], k[R], v[CPL];
+      seq_row<NPL>(qs + tt * DP, l, q);
+      seq_row<NPL>(ks + tt * DP, l, k);
+      const float4 gate = gates[tt];
+      if constexpr (MODE == 1) {
+        float gn[R];
+        seq_row<NPL>(gs + tt * DP, l, gn);
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) S[i][c] *= gn[i];
+      }
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) v[c] = vs[tt * COLS + cb + c];
+      float u[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        float b0 = 0.f, b1 = 0.f;
+        if constexpr (MODE != 2) {
+          float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+          for (int i = 0; i < R; i += 2) {
+            a0 = fmaf(S[i][c], k[i], a0);
+            a1 = fmaf(S[i + 1][c], k[i + 1], a1);
+          }
+          u[c] = a0 + a1;
+        }
+#pragma unroll
+        for (int i = 0; i < R; i += 2) {
+          b0 = fmaf(S[i][c], q[i], b0);
+          b1 = fmaf(S[i + 1][c], q[i + 1], b1);
+        }
+        part[c][tt] = b0 + b1;
+      }
+      if constexpr (MODE == 2) {
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) u[c] = v[c];
+      } else {
+#pragma unroll
+        for (int mask = 8; mask >= 1; mask >>= 1)
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) u[c] += __shfl_xor_sync(0xffffffffu, u[c], mask);
+        // the decayed state answers k with decay * (S^T k); the token writes u along k
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          u[c] = gate.x * (v[c] - gate.y * u[c]);
+          if (l == 0) vs[tt * COLS + cb + c] = u[c];             // for the read-out, by lanes of this column only
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) S[i][c] = fmaf(k[i], u[c], MODE == 1 ? S[i][c] : gate.y * S[i][c]);
+    };
+    if (nt == SEQ_CHUNK) {
+#pragma unroll
+      for (int tt = 0; tt < SEQ_CHUNK; ++tt) token(tt);
+    } else {
+#pragma unroll
+      for (int tt = 0; tt < SEQ_CHUNK; ++tt) {
+        if (tt < nt) token(tt);
+        else {
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) part[c][tt] = 0.f;
+        }
+      }
+    }
+    __syncwarp();
+    const int tok = l >> 1;
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      seq_totals(part[c], l);
+      if (!(l & 1) && tok < nt && col + c < P) {
+        // the read-out already contains the token's own write: decay * (S^T q) + (k . q) u
+        const float4 gate = gates[tok];
+        a.o[(size_t)(t0 + tok) * width + (size_t)head * P + col + c] =
+            fmaf(gate.z, vs[tok * COLS + cb + c], MODE == 1 ? part[c][0] : gate.y * part[c][0]);
+      }
+    }
+    __syncthreads();
+  };
+  __syncthreads();
+  int turn = 0;
+  for (int t0 = q0; t0 < q1; t0 += SEQ_CHUNK, turn ^= 1) chunk(t0, turn);
+  seq_store_state<NPL, CPL>(st, D, P, col, l, a.vec, S);
+}
+
+// The same for the selective state space (ssd_scan_kernel).
+template <typename AT, int NPL, int CPL>
+__global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) ssd_seq_kernel(SsdArgs a) {
+  constexpr int R = 2 * NPL, DP = 32 * NPL, COLS = 2 * SEQ_WARPS * CPL;
+  constexpr int PER = seq_buffer(NPL, CPL, 2);
+  constexpr int XR = (SEQ_CHUNK * COLS + 32 * SEQ_WARPS - 1) / (32 * SEQ_WARPS);
+  extern __shared__ __align__(16) float sm[];
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % SEQ_WARPS, l = lane & 15;
+  const bool stages = threadIdx.x >= 32 * SEQ_WARPS;
+  const int head = blockIdx.y, seg = blockIdx.z;
+  const int N = a.N, P = a.P;
+  const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1];
+  if (q1 <= q0) return;
+  const int g = head / (a.heads / a.G);
+  const int inner = a.heads * P;
+  const int col0 = blockIdx.x * COLS, cb = (2 * warp + (lane >> 4)) * CPL, col = col0 + cb;
+  float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * N * P;
+  const float rate = -expf(a.A_log[head]), bias = a.dt_bias[head], skip = a.D[head];
+  const AT* xbc = (const AT*)a.xbc;
+  struct Staged {
+    AT b[SEQ_PER_WARP][NPL], c[SEQ_PER_WARP][NPL], x[XR], dt[SEQ_PER_WARP];
+  } even, odd;
+  auto fetch = [&](int t0, Staged& x) {
+    const int nt = min(SEQ_CHUNK, q1 - t0);
+#pragma unroll
+    for (int j = 0; j < SEQ_PER_WARP; ++j) {
+      const int tt = warp + SEQ_WARPS * j;
+      const size_t t = t0 + tt;
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        const int n = lane + 32 * e;
+        const bool in = tt < nt && n < N;
+        const AT* row = xbc + t * a.ld + inner + (size_t)g * N + n;
+        x.b[j][e] = in ? row[0] : from_float<AT>(0.f);
+        x.c[j][e] = in ? row[(size_t)a.G * N] : from_float<AT>(0.f);
+      }
+      if (tt < nt) x.dt[j] = ((const AT*)a.dt)[t * a.ld_dt + head];
+    }
+#pragma unroll
+    for (int r = 0; r < XR; ++r) {
+      const int i = threadIdx.x % (32 * SEQ_WARPS) + 32 * SEQ_WARPS * r, tt = i / COLS, c = i % COLS;
+      x.x[r] = (tt < nt && col0 + c < P) ? xbc[(size_t)(t0 + tt) * a.ld + (size_t)head * P + col0 + c] : from_float<AT>(0.f);
+    }
+  };
+  auto put = [&](float* buf, const Staged& x) {
+    float* bs = buf;
+    float* cs = bs + SEQ_CHUNK * DP;
+    float* xs = cs + SEQ_CHUNK * DP;
+    float4* gates = reinterpret_cast<float4*>(xs + SEQ_CHUNK * COLS);      // step, decay
+#pragma unroll
+    for (int j = 0; j < SEQ_PER_WARP; ++j) {
+      const int tt = warp + SEQ_WARPS * j;
+#pragma unroll
+      for (int e = 0; e < NPL; ++e) {
+        const int at = tt * DP + seq_place<NPL>(lane + 32 * e);
+        bs[at] = to_float(x.b[j][e]);
+        cs[at] = to_float(x.c[j][e]);
+      }
+    }
+    if (lane < SEQ_PER_WARP) {                                   // a lane a token
+      AT raw = x.dt[0];
+#pragma unroll
+      for (int j = 1; j < SEQ_PER_WARP; ++j)
+        if (lane == j) raw = x.dt[j];
+      const float step = softplus_f(to_float(raw) + bias);
+      gates[warp + SEQ_WARPS * lane] = make_float4(step, expf(rate * step), 0.f, 0.f);
+    }
+#pragma unroll
+    for (int r = 0; r < XR; ++r) {
+      const int i = threadIdx.x % (32 * SEQ_WARPS) + 32 * SEQ_WARPS * r;
+      if (i < SEQ_CHUNK * COLS) xs[i] = to_float(x.x[r]);
+    }
+  };
+  if (stages) {
+    // two chunks on their way in registers; a buffer is filled while the other one is worked through
+    fetch(q0, even);
+    fetch(q0 + SEQ_CHUNK, odd);
+    put(sm, even);
+    fetch(q0 + 2 * SEQ_CHUNK, even);
+    __syncthreads();
+    for (int t0 = q0; t0 < q1; t0 += 2 * SEQ_CHUNK) {
+      if (t0 + SEQ_CHUNK < q1) put(sm + PER, odd);
+      fetch(t0 + 3 * SEQ_CHUNK, odd);
+      __syncthreads();
+      if (t0 + SEQ_CHUNK >= q1) break;
+      if (t0 + 2 * SEQ_CHUNK < q1) put(sm, even);
+      fetch(t0 + 4 * SEQ_CHUNK, even);
+      __syncthreads();
+    }
+    return;
+  }
+  float S[R][CPL];
+  seq_load_state<NPL, CPL>(st, N, P, col, l, a.vec, S);
+  auto chunk = [&](int t0, int turn) {
+    const int nt = min(SEQ_CHUNK, q1 - t0);
+    const float* bs = sm + turn * PER;
+    const float* cs = bs + SEQ_CHUNK * DP;
+    const float* xs = cs + SEQ_CHUNK * DP;
+    const float4* gates = reinterpret_cast<const float4*>(xs + SEQ_CHUNK * COLS);
+    float part[CPL][SEQ_CHUNK];
+    auto token = [&](int tt) {
+      float b[R], c[R];
+      seq_row<NPL>(bs + tt * DP, l, b);
+      seq_row<NPL>(cs + tt * DP, l, c);
+      const float4 gate = gates[tt];
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) {
+        const float in = gate.x * xs[tt * COLS + cb + j];
+        float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; i += 2) {
+          S[i][j] = fmaf(gate.y, S[i][j], in * b[i]);
+          p0 = fmaf(S[i][j], c[i], p0);
+          S[i + 1][j] = fmaf(gate.y, S[i + 1][j], in * b[i + 1]);
+          p1 = fmaf(S[i + 1][j], c[i + 1], p1);
+        }
+        part[j][tt] = p0 + p1;
+      }
+    };
+    if (nt == SEQ_CHUNK) {
+#pragma unroll
+      for (int tt = 0; tt < SEQ_CHUNK; ++tt) token(tt);
+    } else {
+#pragma unroll
+      for (int tt = 0; tt < SEQ_CHUNK; ++tt) {
+        if (tt < nt) token(tt);
+        else {
+#pragma unroll
+          for (int j = 0; j < CPL; ++j) part[j][tt] = 0.f;
+        }
+      }
+    }
+    const int tok = l >> 1;
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) {
+      seq_totals(part[j], l);
+      if (!(l & 1) && tok < nt && col + j < P)
+        a.y[(size_t)(t0 + tok) * inner + (size_t)head * P + col + j] = part[j][0] + skip * xs[tok * COLS + cb + j];
+    }
+    __syncthreads();
+  };
+  __syncthreads();
+  int turn = 0;
+  for (int t0 = q0; t0 < q1; t0 += SEQ_CHUNK, turn ^= 1) chunk(t0, turn);
+  seq_store_state<NPL, CPL>(st, N, P, col, l, a.vec, S);
+}
+
 // A few segments of a long prompt leave most SMs without a block when a warp owns 8 columns:
 // then a warp owns 2 and four times as many blocks share the work.
 #ifndef NARROW_WC
@@ -721,17 +1231,72 @@ static int launch_delta(DeltaArgs a, int S, cudaStream_t stream) {
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
+// Columns a lane of the kernels for several tokens a segment.  Four need fewer shared loads and less staging a
+// column, two leave twice as many blocks: measured, two win while the columns of a launch (heads, segments) fill
+// the chip once (4,096: delta 499 against 594 us for 2,048 tokens), four from there on (16,384: 911 against 750).
+static int seq_columns(int P, int heads, int S) { return (long long)P * heads * S <= 5000 ? 2 : 4; }
+
+template <typename AT, int NPL, int CPL, int MODE>
+static int launch_delta_seq(DeltaArgs a, int S, cudaStream_t stream) {
+  constexpr size_t smem = 2 * seq_buffer(NPL, CPL, MODE == 1 ? 3 : 2) * sizeof(float);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(delta_seq_kernel<AT, NPL, CPL, MODE>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  a.vec = !(a.P % CPL) && !(a.slot_stride % 4) && !((uintptr_t)a.state & 15) && !((size_t)a.D * a.P % CPL);
+  constexpr int COLS = 2 * SEQ_WARPS * CPL;
+  const dim3 grid((a.P + COLS - 1) / COLS, a.heads, S);
+  const cudaError_t e = launch_pdl(delta_seq_kernel<AT, NPL, CPL, MODE>, grid, dim3(SEQ_THREADS), smem, stream, a);
+  return e == cudaSuccess ? FT_OK : (int)e;
+}
+template <typename AT, int NPL, int MODE>
+static int launch_delta_seq(const DeltaArgs& a, int S, cudaStream_t stream) {
+  if constexpr (NPL == 8) return launch_delta_seq<AT, NPL, 1, MODE>(a, S, stream);
+  else if (sizeof(AT) == 4 || seq_columns(a.P, a.heads, S) == 2) return launch_delta_seq<AT, NPL, 2, MODE>(a, S, stream);
+  else if constexpr (sizeof(AT) == 2) return launch_delta_seq<AT, NPL, 4, MODE>(a, S, stream);
+  return FT_ERR_DTYPE;
+}
+template <typename AT, int NPL, int CPL>
+static int launch_ssd_seq(SsdArgs a, int S, cudaStream_t stream) {
+  constexpr size_t smem = 2 * seq_buffer(NPL, CPL, 2) * sizeof(float);
+  static_assert(smem <= 48 * 1024, "no opt-in needed");
+  a.vec = !(a.P % CPL) && !(a.slot_stride % 4) && !((uintptr_t)a.state & 15) && !((size_t)a.N * a.P % CPL);
+  constexpr int COLS = 2 * SEQ_WARPS * CPL;
+  const dim3 grid((a.P + COLS - 1) / COLS, a.heads, S);
+  const cudaError_t e = launch_pdl(ssd_seq_kernel<AT, NPL, CPL>, grid, dim3(SEQ_THREADS), smem, stream, a);
+  return e == cudaSuccess ? FT_OK : (int)e;
+}
+template <typename AT, int NPL>
+static int launch_ssd_seq(const SsdArgs& a, int S, cudaStream_t stream) {
+  if constexpr (NPL == 8) return launch_ssd_seq<AT, NPL, 1>(a, S, stream);
+  else if (sizeof(AT) == 4 || seq_columns(a.P, a.heads, S) == 2) return launch_ssd_seq<AT, NPL, 2>(a, S, stream);
+  else if constexpr (sizeof(AT) == 2) return launch_ssd_seq<AT, NPL, 4>(a, S, stream);
+  return FT_ERR_DTYPE;
+}
+
+// T tokens in S segments: one token each (decode) is bound by the states' traffic, which the kernels with 32
+// lanes a column read and write in wider pieces; any segment of more takes the others.
 template <int MODE>
-static int dispatch_delta(DeltaArgs a, int S, int dtype, cudaStream_t stream) {
+static int dispatch_delta(DeltaArgs a, int S, int T, int dtype, cudaStream_t stream) {
   int rc = FT_OK;
   const int D = a.D;
   const bool narrow = narrow_warps(a.P, a.heads, S);
-  FT_DISPATCH(dtype, AT, {
-    if (D <= 32) rc = narrow ? launch_delta<AT, 1, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 1, 8, MODE>(a, S, stream);
-    else if (D <= 64) rc = narrow ? launch_delta<AT, 2, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 2, 8, MODE>(a, S, stream);
-    else if (D <= 128) rc = narrow ? launch_delta<AT, 4, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 4, 8, MODE>(a, S, stream);
-    else rc = narrow ? launch_delta<AT, 8, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 8, 8, MODE>(a, S, stream);
-  });
+  if (T > S) {
+    FT_DISPATCH(dtype, AT, {
+      if (D <= 32) rc = launch_delta_seq<AT, 1, MODE>(a, S, stream);
+      else if (D <= 64) rc = launch_delta_seq<AT, 2, MODE>(a, S, stream);
+      else if (D <= 128) rc = launch_delta_seq<AT, 4, MODE>(a, S, stream);
+      else rc = launch_delta_seq<AT, 8, MODE>(a, S, stream);
+    });
+  } else {
+    FT_DISPATCH(dtype, AT, {
+      if (D <= 32) rc = narrow ? launch_delta<AT, 1, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 1, 8, MODE>(a, S, stream);
+      else if (D <= 64) rc = narrow ? launch_delta<AT, 2, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 2, 8, MODE>(a, S, stream);
+      else if (D <= 128) rc = narrow ? launch_delta<AT, 4, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 4, 8, MODE>(a, S, stream);
+      else rc = narrow ? launch_delta<AT, 8, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 8, 8, MODE>(a, S, stream);
+    });
+  }
   if (rc != FT_OK) return rc;
   FT_LAUNCH_CHECK();
   return FT_OK;
@@ -780,18 +1345,27 @@ int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const f
 int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, const float* dt_bias,
                 const float* A_log, const float* D, float* state, long long slot_stride, float* y,
                 const int* seg_slot, const int* seg_q_start, int heads, int P, int N, int G, int S,
-                int dtype, cudaStream_t stream) {
+                int T, int dtype, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || N <= 0 || N > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   SsdArgs a{xbc, dt, dt_bias, A_log, D, state, y, seg_slot, seg_q_start, ld, ld_dt, slot_stride, heads, P, N, G, 0};
   int rc = FT_OK;
   const bool narrow = narrow_warps(P, heads, S);
-  FT_DISPATCH(dtype, AT, {
-    if (N <= 32) rc = narrow ? launch_ssd<AT, 1, NARROW_WC>(a, S, stream) : launch_ssd<AT, 1, 8>(a, S, stream);
-    else if (N <= 64) rc = narrow ? launch_ssd<AT, 2, NARROW_WC>(a, S, stream) : launch_ssd<AT, 2, 8>(a, S, stream);
-    else if (N <= 128) rc = narrow ? launch_ssd<AT, 4, NARROW_WC>(a, S, stream) : launch_ssd<AT, 4, 8>(a, S, stream);
-    else rc = narrow ? launch_ssd<AT, 8, NARROW_WC>(a, S, stream) : launch_ssd<AT, 8, 8>(a, S, stream);
-  });
+  if (T > S) {                                          // see dispatch_delta
+    FT_DISPATCH(dtype, AT, {
+      if (N <= 32) rc = launch_ssd_seq<AT, 1>(a, S, stream);
+      else if (N <= 64) rc = launch_ssd_seq<AT, 2>(a, S, stream);
+      else if (N <= 128) rc = launch_ssd_seq<AT, 4>(a, S, stream);
+      else rc = launch_ssd_seq<AT, 8>(a, S, stream);
+    });
+  } else {
+    FT_DISPATCH(dtype, AT, {
+      if (N <= 32) rc = narrow ? launch_ssd<AT, 1, NARROW_WC>(a, S, stream) : launch_ssd<AT, 1, 8>(a, S, stream);
+      else if (N <= 64) rc = narrow ? launch_ssd<AT, 2, NARROW_WC>(a, S, stream) : launch_ssd<AT, 2, 8>(a, S, stream);
+      else if (N <= 128) rc = narrow ? launch_ssd<AT, 4, NARROW_WC>(a, S, stream) : launch_ssd<AT, 4, 8>(a, S, stream);
+      else rc = narrow ? launch_ssd<AT, 8, NARROW_WC>(a, S, stream) : launch_ssd<AT, 8, 8>(a, S, stream);
+    });
+  }
   if (rc != FT_OK) return rc;
   FT_LAUNCH_CHECK();
   return FT_OK;
@@ -800,12 +1374,12 @@ int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, 
 int ft_delta_scan(const void* qkv, long long ld, const void* beta, const void* decay, long long ld_gate,
                   const float* dt_bias, const float* A_log, float* state, long long slot_stride, float* o,
                   const int* seg_slot, const int* seg_q_start, int heads, int P, int D, int G, float unit_eps,
-                  float q_scale, int S, int dtype, cudaStream_t stream) {
+                  float q_scale, int S, int T, int dtype, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   DeltaArgs a{qkv, beta, decay, dt_bias, A_log, state, o, seg_slot, seg_q_start, ld, ld_gate, slot_stride,
               heads, P, D, G, unit_eps, q_scale, 0, nullptr, 0, nullptr, nullptr, 0};
-  return dispatch_delta<0>(a, S, dtype, stream);
+  return dispatch_delta<0>(a, S, T, dtype, stream);
 }
 
 // The delta rule with a decay per key channel: `decay` is float32 [T, ld_decay] (channel n of head
@@ -813,27 +1387,27 @@ int ft_delta_scan(const void* qkv, long long ld, const void* beta, const void* d
 int ft_channel_delta_scan(const void* qkv, long long ld, const void* beta, long long ld_gate, const float* decay,
                           long long ld_decay, const float* dt_bias, const float* A_log, float* state,
                           long long slot_stride, float* o, const int* seg_slot, const int* seg_q_start, int heads,
-                          int P, int D, int G, float unit_eps, float q_scale, int S, int dtype,
+                          int P, int D, int G, float unit_eps, float q_scale, int S, int T, int dtype,
                           cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   DeltaArgs a{qkv, beta, nullptr, dt_bias, A_log, state, o, seg_slot, seg_q_start, ld, ld_gate, slot_stride,
               heads, P, D, G, unit_eps, q_scale, 0, decay, ld_decay, nullptr, nullptr, 0};
-  return dispatch_delta<1>(a, S, dtype, stream);
+  return dispatch_delta<1>(a, S, T, dtype, stream);
 }
 
 // Retention: rows of `qkv` are q (heads * D) | k (heads * D) | v (heads * P); `decay` [heads] float32 holds
 // each head's constant factor; cos_sin [positions, rot_dims] (rot_dims 0: nothing turns).
 int ft_retention_scan(const void* qkv, long long ld, const float* decay, const float* cos_sin, int rot_dims,
                       const int* seg_pos0, float* state, long long slot_stride, float* o, const int* seg_slot,
-                      const int* seg_q_start, int heads, int P, int D, float k_scale, int S, int dtype,
+                      const int* seg_q_start, int heads, int P, int D, float k_scale, int S, int T, int dtype,
                       cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || rot_dims < 0 || (rot_dims & 1) || rot_dims > D)
     return FT_ERR_SHAPE;
   DeltaArgs a{qkv, nullptr, nullptr, decay, nullptr, state, o, seg_slot, seg_q_start, ld, 0, slot_stride,
               heads, P, D, heads, 0.f, k_scale, 0, nullptr, 0, cos_sin, seg_pos0, cos_sin ? rot_dims : 0};
-  return dispatch_delta<2>(a, S, dtype, stream);
+  return dispatch_delta<2>(a, S, T, dtype, stream);
 }
 
 }  // extern "C"

@@ -1,0 +1,74 @@
+"""The scans of the recurrent mixers: a launch of several tokens takes
+other kernels than a launch of one token a segment, and gives the same bits."""
+
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, DT, ops, rnd
+
+pytestmark = pytest.mark.gpu
+
+# heads, value size, key size, tokens a segment, groups: remainders of chunks of 8, of lanes' columns and rows;
+# the last two fill the chip (four columns a lane)
+SIZES = [(4, 10, 12, [9], 2), (2, 36, 40, [3, 1, 17], 1), (4, 64, 64, [16, 7], 2), (3, 28, 20, [33], 3),
+         (2, 130, 200, [12, 5], 1), (1, 7, 129, [8], 1), (8, 16, 32, [1, 2, 25], 4), (2, 8, 256, [10], 2),
+         (32, 64, 96, [11, 8, 3], 1), (40, 130, 33, [9], 40)]
+
+
+def _segments(lens):
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    return (torch.arange(len(lens), dtype=torch.int32, device=DEV) + 1,
+            torch.tensor(starts, dtype=torch.int32, device=DEV))
+
+
+def _token_by_token(lens, launch):
+    """``launch(token rows, slots, starts)`` for the first token of every segment, then the second ..."""
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    for t in range(max(lens)):
+        live = [i for i, n in enumerate(lens) if t < n]
+        rows = torch.tensor([starts[i] + t for i in live], device=DEV)
+        launch(rows, torch.tensor([i + 1 for i in live], dtype=torch.int32, device=DEV),
+               torch.arange(len(live) + 1, dtype=torch.int32, device=DEV), t)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("kind", ["delta", "channel_delta", "retention", "ssd"])
+@pytest.mark.parametrize("H,P,D,lens,G", SIZES)
+def test_scans_agree_bitwise(dtype, kind, H, P, D, lens, G):
+    T, dt, o = sum(lens), DT[dtype], ops()
+    slot, starts = _segments(lens)
+    a_log, bias = rnd(H, seed=3, scale=0.5) - 1, rnd(H, seed=4, scale=0.5) - 1
+    gates = rnd(T, 2 * H, dtype=dt, seed=2)
+    first = rnd(len(lens) + 2, H * D * P + 5, seed=5, scale=0.1)
+    if kind == "ssd":
+        x, skip = rnd(T, H * P + 2 * G * D, dtype=dt, seed=1), rnd(H, seed=6)
+        call = lambda state, y, rows, s, q, t: o.ssd_scan(x[rows], gates[rows][:, :H], bias, a_log, skip, state, y, s, q,
+                                                          H, P, D, G)
+    elif kind == "retention":
+        x, decay = rnd(T, 2 * H * D + H * P, dtype=dt, seed=1), torch.linspace(0.9, 0.999, H, device=DEV)
+        rot = 2 * (D // 4)
+        turn = rnd(64, rot, seed=7) if rot else None
+        call = lambda state, y, rows, s, q, t: o.retention_scan(x[rows], decay, turn, torch.full_like(s, t), state, y, s,
+                                                                q, H, D, P, D ** -0.5)
+    else:
+        x = rnd(T, 2 * G * D + H * P, dtype=dt, seed=1)
+        per_channel = rnd(T, H * D, seed=8), rnd(H * D, seed=9, scale=0.5) - 1
+        if kind == "delta":
+            call = lambda state, y, rows, s, q, t: o.delta_scan(
+                x[rows], gates[rows][:, :H], gates[rows][:, H:], bias, a_log, state, y, s, q, H, G, D, P, 1e-6, D ** -0.5)
+        else:
+            call = lambda state, y, rows, s, q, t: o.channel_delta_scan(
+                x[rows], gates[rows][:, :H], per_channel[0][rows], per_channel[1], a_log, state, y, s, q, H, G, D, P, 1e-6,
+                D ** -0.5)
+    whole, y = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+    call(whole, y, torch.arange(T, device=DEV), slot, starts, 0)
+    steps, want = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+
+    def launch(rows, s, q, t):
+        out = torch.empty(rows.numel(), H * P, device=DEV)
+        call(steps, out, rows, s, q, t)
+        want[rows] = out
+    _token_by_token(lens, launch)
+    assert torch.equal(y, want) and torch.equal(whole, steps)
