@@ -664,7 +664,7 @@ def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Op
     for name, t in (("token_seg", token_seg), ("seg_slot", seg_slot), ("seg_q_start", seg_q_start)):
         _need(t, name, torch.int32)
     global LAUNCHES
-    LAUNCHES += 1 if taps > 1 else 0
+    LAUNCHES += 1 if taps > 1 and (T != seg_slot.numel() or taps > 8) else 0      # a kernel for the slots' new contents
     f = _fn("recurrent", "ft_conv_silu", "p q p q p p p q p p p i i i i i i")
     _check(f(_ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(weight), _ptr(bias), _ptr(state),
              state.stride(0), _ptr(token_seg), _ptr(seg_slot), _ptr(seg_q_start), C, taps, T,

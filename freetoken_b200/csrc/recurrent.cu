@@ -162,6 +162,60 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T) {
   }
 }
 
+// As many segments as tokens, that is, one token each (decode): a thread owns a segment's channel (or two) with the
+// inputs before it in registers, and leaves the last taps - 1 in the slot itself: one launch instead of two, and no
+// value read twice.  (One row of 6,144 channels: 2.6 us instead of 2.8 + 2.4.)  It walks whatever tokens the segment has.
+template <typename AT, int CPT>
+__global__ void __launch_bounds__(128) conv_step_kernel(ConvArgs a) {
+  pdl_wait();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * CPT, seg = blockIdx.x;
+  if (c >= a.C) return;
+  const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1], K = a.taps - 1;
+  if (q1 <= q0) return;
+  const AT* x = (const AT*)a.x;
+  float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + c;
+  float w[CPT][CONV_MAX_TAPS], win[CPT][CONV_MAX_TAPS], bias[CPT];
+#pragma unroll
+  for (int u = 0; u < CPT; ++u) {
+    bias[u] = a.bias ? a.bias[c + u] : 0.f;
+#pragma unroll
+    for (int j = 0; j < CONV_MAX_TAPS; ++j) {
+      w[u][j] = j <= K ? a.w[(size_t)(c + u) * a.taps + j] : 0.f;
+      if (j < K) win[u][j] = st[(size_t)j * a.C + u];
+    }
+  }
+  for (int t = q0; t < q1; ++t) {
+    float own[CPT];
+    if constexpr (CPT == 2) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + (size_t)t * a.ldx + c));
+      own[0] = f.x;
+      own[1] = f.y;
+    } else {
+      own[0] = to_float(x[(size_t)t * a.ldx + c]);
+    }
+    float out[CPT];
+#pragma unroll
+    for (int u = 0; u < CPT; ++u) {
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < CONV_MAX_TAPS; ++j)
+        if (j <= K) acc = fmaf(w[u][j], j == K ? own[u] : win[u][j], acc);
+      out[u] = a.act ? silu_f(acc + bias[u]) : acc + bias[u];
+#pragma unroll
+      for (int j = 0; j < CONV_MAX_TAPS - 1; ++j)
+        if (j < K) win[u][j] = j + 1 == K ? own[u] : win[u][j + 1];
+    }
+    AT* o = (AT*)a.out + (size_t)t * a.ldo + c;
+    if constexpr (CPT == 2) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(out[0], out[1]);
+    else o[0] = from_float<AT>(out[0]);
+  }
+#pragma unroll
+  for (int u = 0; u < CPT; ++u)
+#pragma unroll
+    for (int j = 0; j < CONV_MAX_TAPS - 1; ++j)
+      if (j < K) st[(size_t)j * a.C + u] = win[u][j];
+}
+
 // any number of taps: one channel and one token a thread
 template <typename AT>
 __global__ void __launch_bounds__(128) conv_silu_long_kernel(ConvArgs a) {
@@ -1316,14 +1370,20 @@ int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const f
   if (C <= 0 || taps < 1) return FT_ERR_SHAPE;
   ConvArgs a{x, out, w, bias, state, token_seg, seg_slot, seg_q_start, ldx, ldo, slot_stride, C, taps, act};
   const int cb = (C + 127) / 128;
+  const bool pairs = dtype == FT_DTYPE_BF16 && !(C & 1) && !(ldx & 1) && !(ldo & 1) && !((uintptr_t)x & 3) &&
+                     !((uintptr_t)out & 3);
+  if (T == S && taps <= CONV_MAX_TAPS) {
+    if (pairs) launch_pdl(conv_step_kernel<__nv_bfloat16, 2>, dim3(S, (C / 2 + 127) / 128), dim3(128), 0, stream, a);
+    else FT_DISPATCH(dtype, AT, launch_pdl(conv_step_kernel<AT, 1>, dim3(S, cb), dim3(128), 0, stream, a));
+    FT_LAUNCH_CHECK();
+    return FT_OK;
+  }
   if (taps > CONV_MAX_TAPS) {
     FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_long_kernel<AT>, dim3(T, cb), dim3(128), 0, stream, a));
   } else {
     // many tokens: a thread walks 8 of them with its inputs in registers; few: a thread a token
     const bool many = T >= 1024;
     const dim3 rows(many ? (T + 7) / 8 : T);
-    const bool pairs = dtype == FT_DTYPE_BF16 && !(C & 1) && !(ldx & 1) && !(ldo & 1) && !((uintptr_t)x & 3) &&
-                       !((uintptr_t)out & 3);
     if (pairs) {
       const dim3 grid(rows.x, (C / 2 + 127) / 128);
       if (many) launch_pdl(conv_silu_kernel<__nv_bfloat16, 2, 8>, grid, dim3(128), 0, stream, a, T);

@@ -1,4 +1,4 @@
-"""The scans of the recurrent mixers: a launch of several tokens takes
+"""The scans of the recurrent mixers and the short convolution: a launch of several tokens takes
 other kernels than a launch of one token a segment, and gives the same bits."""
 
 import pytest
@@ -72,3 +72,40 @@ def test_scans_agree_bitwise(dtype, kind, H, P, D, lens, G):
         want[rows] = out
     _token_by_token(lens, launch)
     assert torch.equal(y, want) and torch.equal(whole, steps)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("C,taps,lens,act", [(6, 4, [5, 1, 9], True), (130, 2, [3], False), (7, 8, [12, 2], True),
+                                             (64, 1, [4], True), (33, 9, [3, 12], True)])
+def test_convolutions_agree_bitwise(dtype, C, taps, lens, act):
+    T, dt = sum(lens), DT[dtype]
+    slot, starts = _segments(lens)
+    seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(torch.int32).to(DEV)
+    x, w, b = rnd(T, C + 2, dtype=dt, seed=1)[:, :C], rnd(C, taps, seed=2), rnd(C, seed=3)
+    first = rnd(len(lens) + 2, max(1, (taps - 1) * C), seed=4)
+    whole, y = first.clone(), torch.empty(T, C, dtype=dt, device=DEV)
+    ops().conv_silu(x, y, w, b, whole, seg, slot, starts, activation=act)
+    steps, want = first.clone(), torch.empty(T, C, dtype=dt, device=DEV)
+
+    def launch(rows, s, q, t):
+        out = torch.empty(rows.numel(), C, dtype=dt, device=DEV)
+        ops().conv_silu(x[rows], out, w, b, steps, torch.arange(rows.numel(), dtype=torch.int32, device=DEV), s, q,
+                        activation=act)
+        want[rows] = out
+    _token_by_token(lens, launch)
+    assert torch.equal(y, want) and torch.equal(whole, steps)
+
+
+def test_convolution_of_as_many_tokens_as_segments_that_are_not_one_each():
+    """Two tokens in one segment and none in the other."""
+    x, w = rnd(2, 10, seed=1), rnd(10, 3, seed=2)
+    first = rnd(3, 20, seed=4)
+    out = []
+    for starts in ([0, 0, 2], [0, 2]):
+        state, y = first.clone(), torch.empty(2, 10, device=DEV)
+        S = len(starts) - 1
+        slot = torch.tensor([2, 1][-S:], dtype=torch.int32, device=DEV)
+        ops().conv_silu(x, y, w, None, state, torch.full((2,), S - 1, dtype=torch.int32, device=DEV), slot,
+                        torch.tensor(starts, dtype=torch.int32, device=DEV))
+        out.append((y, state))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
