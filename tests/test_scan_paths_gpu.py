@@ -1,4 +1,4 @@
-"""The scans of the recurrent mixers and the short convolution: a launch of several tokens takes
+"""The scans of the recurrent mixers, the short convolution and the latent store: a launch of several tokens takes
 other kernels than a launch of one token a segment, and gives the same bits."""
 
 import pytest
@@ -109,3 +109,25 @@ def test_convolution_of_as_many_tokens_as_segments_that_are_not_one_each():
                         torch.tensor(starts, dtype=torch.int32, device=DEV))
         out.append((y, state))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("heads,dq,rank,rot,interleaved", [(32, 16, 40, 64, False), (3, 8, 24, 6, True), (20, 8, 16, 32, True)])
+def test_latent_rows_of_few_and_many_tokens_agree_bitwise(dtype, heads, dq, rank, rot, interleaved):
+    T, dt, P = 70, DT[dtype], 16
+    down, q = rnd(T, rank + rot, dtype=dt, seed=1), rnd(T, heads * (dq + rot), dtype=dt, seed=2)
+    weight, turn = rnd(rank, seed=3), rnd(T, rot, seed=4)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    seg = torch.zeros(T, dtype=torch.int32, device=DEV)
+    table = torch.arange(1, 6, dtype=torch.int32, device=DEV).view(1, 5)
+    results = []
+    for rows in (T, 9):
+        pages = torch.zeros(6, 1, P, rank + rot, dtype=dt, device=DEV)
+        q_abs = torch.zeros(T, heads, rank + rot, dtype=dt, device=DEV)
+        turned = q.clone()
+        for a in range(0, T, rows):
+            b = min(T, a + rows)
+            ops().latent_store(down[a:b], turned[a:b], q_abs[a:b], pages, weight, turn, pos[a:b], seg[a:b], table,
+                               heads=heads, q_dim=dq, rank=rank, rot=rot, interleaved=interleaved, eps=1e-6, turn_q=True)
+        results.append((pages, q_abs, turned))
+    assert all(torch.equal(x, y) for x, y in zip(*results))
