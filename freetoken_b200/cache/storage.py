@@ -54,9 +54,15 @@ class CacheStorage:
         """Zero the state rows of newly admitted request slots."""
         if not slots or not self.state:
             return
-        index = torch.tensor(list(slots), dtype=torch.long, device=self.device)
-        for t in self.state:
-            t.index_fill_(1, index, 0)
+        # run by run of neighbouring slots: an index tensor would have to be copied to the device first, and
+        # that copy waits for the steps in flight
+        slots = sorted(slots)
+        first = 0
+        for i in range(1, len(slots) + 1):
+            if i == len(slots) or slots[i] != slots[i - 1] + 1:
+                for t in self.state:
+                    t[:, slots[first]:slots[i - 1] + 1].zero_()
+                first = i
 
     def poison(self, group: int, pages: Sequence[int]) -> None:
         """Overwrite pages (of every stop of a group, all they hold) with NaN: a

@@ -233,10 +233,17 @@ class Engine:
         segments: List[Segment] = []
         seen = set()
         q = 0
-        token_arrays: List[np.ndarray] = []
+        token_arrays: List[Sequence[int]] = []
+        counts: List[int] = []
         for e in entries:
-            arr = np.asarray(e.tokens, dtype=np.int64).reshape(-1)
-            n = arr.size
+            arr = e.tokens
+            if type(arr) is list and len(arr) == 1 and type(arr[0]) is int:
+                n, low, high = 1, arr[0], arr[0]        # a decoded token: no array work
+            else:
+                arr = np.asarray(arr, dtype=np.int64).reshape(-1)
+                n = arr.size
+                low, high = (int(arr.min()), int(arr.max())) if n else (0, 0)
+                arr = arr.astype(np.int32)
             if n == 0:
                 raise ValueError(f"request {e.request!r} brings no tokens to the step")
             if e.request in seen:
@@ -245,13 +252,14 @@ class Engine:
             for w in e.want:
                 if not 0 <= w < n:
                     raise ValueError(f"request {e.request!r}: wanted place {w} is outside its {n} tokens")
-            if arr.min() < 0 or arr.max() >= vocab:
+            if low < 0 or high >= vocab:
                 raise ValueError(f"request {e.request!r}: a token id is outside the vocabulary 0..{vocab - 1}")
             if e.device_token is not None:
                 if n != 1 or token_source is None or not 0 <= e.device_token < token_source.numel():
                     raise ValueError(f"request {e.request!r}: a token on the device stands for exactly one "
                                      f"token and needs a token_source that holds it")
-            token_arrays.append(arr.astype(np.int32))
+            token_arrays.append(arr)
+            counts.append(n)
         # New requests take a slot; every request takes the pages its tokens
         # need.  If that fails nothing of the step has run: requests that were
         # new give their slot and pages back, older ones keep pages they will
@@ -262,15 +270,15 @@ class Engine:
                 if not self.cache.has_request(e.request):
                     self.cache.admit(e.request)
                     fresh.append(e.request)
-            for e, arr in zip(entries, token_arrays):
-                self.cache.grow(e.request, self.cache.length(e.request) + arr.size)
+            for e, n in zip(entries, counts):
+                self.cache.grow(e.request, self.cache.length(e.request) + n)
         except Exception:
             for r in fresh:
                 self.cache.release(r)
             raise
-        for e, arr in zip(entries, token_arrays):
-            segments.append(Segment(self.cache.slot(e.request), self.cache.length(e.request), arr.size, q))
-            q += arr.size
+        for e, n in zip(entries, counts):
+            segments.append(Segment(self.cache.slot(e.request), self.cache.length(e.request), n, q))
+            q += n
         T, S = q, len(segments)
         N = sum(len(e.want) for e in entries)
         P = self.cache.page_size
@@ -311,21 +319,25 @@ class Engine:
             cur = _align4(cur + len(patches))
         host = self._staging(cur)
         h = host.numpy()
-        rows: List[int] = []
-        for i, (e, s) in enumerate(zip(entries, segments)):
-            a, b = s.q_start, s.q_start + s.n
-            h[off["token_ids"] + a: off["token_ids"] + b] = token_arrays[i]
-            h[off["token_pos"] + a: off["token_pos"] + b] = np.arange(s.pos0, s.pos0 + s.n, dtype=np.int32)
-            h[off["token_seg"] + a: off["token_seg"] + b] = i
-            h[off["seg_slot"] + i] = s.slot
-            h[off["seg_pos0"] + i] = s.pos0
-            h[off["seg_q_start"] + i] = s.q_start
-            h[off["seg_kv_len"] + i] = s.pos0 + s.n
-            rows.extend(s.q_start + w for w in e.want)
-            for g, group in enumerate(groups):
-                base = off[f"table{g}"] + i * width
-                h[base: base + width] = group.block_table[s.slot, :width]
-        h[off["seg_q_start"] + S] = T
+        rows: List[int] = [s.q_start + w for e, s in zip(entries, segments) for w in e.want]
+        h[off["seg_slot"]: off["seg_slot"] + S] = [s.slot for s in segments]
+        h[off["seg_pos0"]: off["seg_pos0"] + S] = [s.pos0 for s in segments]
+        h[off["seg_q_start"]: off["seg_q_start"] + S + 1] = [s.q_start for s in segments] + [T]
+        h[off["seg_kv_len"]: off["seg_kv_len"] + S] = [s.pos0 + s.n for s in segments]
+        if max_q == 1:
+            h[off["token_ids"]: off["token_ids"] + T] = [tokens[0] for tokens in token_arrays]
+            h[off["token_pos"]: off["token_pos"] + T] = h[off["seg_pos0"]: off["seg_pos0"] + S]
+            h[off["token_seg"]: off["token_seg"] + T] = np.arange(S, dtype=np.int32)
+        else:
+            for i, s in enumerate(segments):
+                a, b = s.q_start, s.q_start + s.n
+                h[off["token_ids"] + a: off["token_ids"] + b] = token_arrays[i]
+                h[off["token_pos"] + a: off["token_pos"] + b] = np.arange(s.pos0, s.pos0 + s.n, dtype=np.int32)
+                h[off["token_seg"] + a: off["token_seg"] + b] = i
+        slots = [s.slot for s in segments]
+        for g, group in enumerate(groups):
+            base = off[f"table{g}"]
+            h[base: base + S * width].reshape(S, width)[:] = group.block_table[slots, :width]
         if N:
             h[off["logit_rows"]: off["logit_rows"] + N] = np.asarray(rows, dtype=np.int32)
         for i, plan in enumerate(plans.values()):

@@ -65,16 +65,27 @@ class Workspace:
 
     ``get`` returns a view of a buffer at least as large as asked; a buffer is
     only ever replaced by a larger one, so steady-state steps allocate
-    nothing."""
+    nothing.  The views handed out are kept beside their buffer (the last
+    :data:`KEPT_VIEWS` shapes of it): a step asks for a few dozen of them, and
+    making one costs as much host time as a small launch."""
+
+    KEPT_VIEWS = 64
 
     def __init__(self, device):
         self.device = torch.device(device)
         self._buffers: Dict[str, torch.Tensor] = {}
+        self._views: Dict[str, Dict[Tuple, torch.Tensor]] = {}
         # bumped whenever a buffer is (re)allocated: captured CUDA graphs hold
         # raw addresses and must be dropped then
         self.generation = 0
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
+        key = (tuple(shape), dtype)
+        views = self._views.get(name)
+        if views is not None:
+            view = views.get(key)
+            if view is not None:
+                return view
         count = 1
         for s in shape:
             count *= int(s)
@@ -84,7 +95,11 @@ class Workspace:
             buf = torch.empty(grow, dtype=dtype, device=self.device)
             self._buffers[name] = buf
             self.generation += 1
-        return buf[:count].view(*shape)
+            views = None
+        if views is None or len(views) >= self.KEPT_VIEWS:
+            views = self._views[name] = {}
+        view = views[key] = buf[:count].view(*shape)
+        return view
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

@@ -4,7 +4,7 @@
   arithmetic with a fixed summation order (no tensor cores, no TF32), weights
   read as stored (float32 or bfloat16, upcast exactly in registers).
 * bfloat16 compute, bfloat16 result: a library product (cuBLAS through
-  ``torch.matmul``), as the reference does for its dense projections
+  ``torch.mm``), as the reference does for its dense projections
   (python/freetoken/layers/linear.py:31-32).  Few rows (decode) go through the
   weight-streaming kernel of ``skinny_gemm.cu`` instead.
 * bfloat16 compute, float32 result (logits of many rows, the router's logits
@@ -62,7 +62,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
             ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows))
             return out
         if out.dtype == torch.bfloat16:
-            torch.matmul(x, weight.t(), out=out)
+            torch.mm(x, weight.t(), out=out)
             return out
         if out.dtype == torch.float32 and library_f32_out(x, weight, out):
             return out
