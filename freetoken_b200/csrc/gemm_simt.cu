@@ -193,20 +193,6 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
     v[2 * i + 1] = f.y;
   }
 }
-__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
-  }
-}
 // Two fused multiply-adds in one instruction; each half rounds like fmaf.
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long x, unsigned long long y) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
@@ -333,19 +319,20 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
 }
 
 // Many rows: bound by the multiply-adds (72 TFLOP/s of them on this chip) and by what shared memory returns to
-// registers, 128 bytes a cycle whatever is broadcast (12 cycles a warp and k here, for 8 of arithmetic).  A block
-// takes 64 rows by 128 weight rows (GLU: 64 gate rows and the 64 up rows of the same features), a thread 4 rows by
-// 4 + 4 columns: three 16-byte shared loads feed 32 multiply-adds, issued two at a time.  The next 16 values of
-// k are fetched into registers while these are multiplied, and two shared buffers leave one barrier a step.
-// Measured: 342 x 3072 x 2048 in 126 us (64 x 64 tiles of 4 x 4 a thread, without the paired multiply-adds: 161),
-// gate_up + GLU of 684 rows over 8 experts, 2 x 2688 x 2048, in 571 us (the plain kernel: 1,124).  Tried and
-// slower at these sizes: 8 x 8 outputs a thread (545 and 158 us a launch, but 1,573 instead of 1,860 us for 2048 x
-// 4096 x 4096), 32 rows a block (158 us), two tiles of k ahead in registers (175 us).
+// registers, 128 bytes a cycle whatever is broadcast: 8 x 8 outputs a thread need 16 cycles of it for 16 of
+// arithmetic a warp and k, 4 x 8 need 12 for 8.  A block takes 64 rows by 128 weight rows (GLU: 64 gate rows and the
+// 64 up rows of the same features), a thread 8 rows by 4 + 4 columns, two multiply-adds an instruction.  A block is
+// often alone on its SM with one warp a scheduler (a chain over k can't be split), so nothing hides a latency but
+// the thread itself: the next k's operands are read from shared memory before this k's products, the tile after
+// next is on its way in registers.  Measured against 4 x 8 outputs with twice the threads: gate_up + GLU of 684 rows
+// over 8 experts, 2 x 2688 x 2048, 512 instead of 602 us (the plain kernel: 1,124), 1024 x 4096 x 2048 in 427 instead
+// of 454 us (40 TFLOP/s), 342 x 3072 x 2048 level at 124 (161 with the tiles of 64 x 64 before them).  Tried and
+// slower: 8 x 8 without the operands read ahead (158 us for the last), 32 rows a block (158), two tiles ahead (175).
 template <typename AT, typename WT, typename OT, bool GLU>
-__global__ void __launch_bounds__(256) gemm_tile_kernel(GemmArgs a) {
+__global__ void __launch_bounds__(128) gemm_tile_kernel(GemmArgs a) {
   constexpr int TBM = 64, TBN = 128, TBK = 16, HALF = 64;
-  __shared__ __align__(16) float As[2][TBK][TBM + 4];
-  __shared__ __align__(16) float Ws[2][TBK][TBN + 4];
+  __shared__ __align__(16) float As[2][TBK][TBM];
+  __shared__ __align__(16) float Ws[2][TBK][TBN];
   __shared__ int tile_info[3];
   pdl_wait();
   find_tile<TBM>(a, tile_info);
@@ -356,57 +343,77 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(GemmArgs a) {
   const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
   const WT* W = (const WT*)a.W + (size_t)group * a.w_group_stride + (size_t)blockIdx.z * a.w_batch_stride;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // this thread loads k ak .. ak + 3 of row ar and k wk .. wk + 7 of weight row wr; rows beyond the last repeat it
-  const int ar = threadIdx.x >> 2, ak = (threadIdx.x & 3) * 4, wr = threadIdx.x >> 1, wk = (threadIdx.x & 1) * 8;
+  // this thread loads eight k of row ar and sixteen of weight row threadIdx.x; rows beyond the last repeat it
+  const int ar = threadIdx.x & 63, ak = (threadIdx.x >> 6) * 8, wr = threadIdx.x;
   const int at = row0 + min(ar, rows - 1);
   const AT* ap = A + (size_t)(a.a_rows ? a.a_rows[at] : at) * a.lda + ak;
   const int col = GLU ? min(n0 + (wr & (HALF - 1)), a.N - 1) + (wr >= HALF ? a.N : 0) : min(n0 + wr, a.N - 1);
-  const WT* wp = W + (size_t)col * a.K + wk;
-  unsigned long long acc[4][4];
+  const WT* wp = W + (size_t)col * a.K;
+  unsigned long long acc[8][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-  float av[4], wv[8];
+  __align__(16) AT araw[8];
+  __align__(16) WT wraw[16];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 8 * (int)sizeof(AT) / 16; ++i)
+      reinterpret_cast<uint4*>(araw)[i] = reinterpret_cast<const uint4*>(ap + k0)[i];
+#pragma unroll
+    for (int i = 0; i < 16 * (int)sizeof(WT) / 16; ++i)
+      reinterpret_cast<uint4*>(wraw)[i] = reinterpret_cast<const uint4*>(wp + k0)[i];
+  };
   auto put = [&](int b) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) As[b][ak + i][ar] = av[i];
+    for (int i = 0; i < 8; ++i) As[b][ak + i][ar] = to_float(araw[i]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) Ws[b][wk + i][wr] = wv[i];
+    for (int i = 0; i < 16; ++i) Ws[b][i][wr] = to_float(wraw[i]);
   };
-  load4(ap, av);
-  load8(wp, wv);
+  struct Frag { float x[8]; ulonglong2 w0, w1; };
+  auto frag = [&](int b, int kk, Frag& f) {
+    load8(&As[b][kk][ty * 8], f.x);
+    f.w0 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][tx * 4]);
+    f.w1 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][HALF + tx * 4]);
+  };
+  auto mul = [&](const Frag& f) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const unsigned long long x2 = pack2(f.x[i], f.x[i]);
+      fma2(acc[i][0], x2, f.w0.x);
+      fma2(acc[i][1], x2, f.w0.y);
+      fma2(acc[i][2], x2, f.w1.x);
+      fma2(acc[i][3], x2, f.w1.y);
+    }
+  };
+  fetch(0);
   put(0);
+  if (TBK < a.K) fetch(TBK);
   __syncthreads();
+  Frag cur, nxt;
+  frag(0, 0, cur);
   int b = 0;
   for (int k0 = 0; k0 < a.K; k0 += TBK, b ^= 1) {
     const bool more = k0 + TBK < a.K;
-    if (more) {
-      load4(ap + k0 + TBK, av);
-      load8(wp + k0 + TBK, wv);
-    }
 #pragma unroll
     for (int kk = 0; kk < TBK; ++kk) {
-      const float4 x4 = *reinterpret_cast<const float4*>(&As[b][kk][ty * 4]);
-      const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][tx * 4]);
-      const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][HALF + tx * 4]);
-      const float xs[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const unsigned long long x2 = pack2(xs[i], xs[i]);
-        fma2(acc[i][0], x2, w0.x);
-        fma2(acc[i][1], x2, w0.y);
-        fma2(acc[i][2], x2, w1.x);
-        fma2(acc[i][3], x2, w1.y);
+      if (kk + 1 < TBK) frag(b, kk + 1, nxt);
+      if (kk == 4 && more) {
+        put(b ^ 1);
+        if (k0 + 2 * TBK < a.K) fetch(k0 + 2 * TBK);
       }
+      if (kk + 1 == TBK) {
+        __syncthreads();
+        if (more) frag(b ^ 1, 0, nxt);
+      }
+      mul(cur);
+      cur = nxt;
     }
-    if (more) put(b ^ 1);
-    __syncthreads();
   }
   OT* C = (OT*)a.C + (size_t)blockIdx.z * a.c_batch_stride;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty * 4 + i;
+  for (int i = 0; i < 8; ++i) {
+    const int r = ty * 8 + i;
     if (r >= rows) continue;
     const int crow = a.c_rows ? a.c_rows[row0 + r] : row0 + r;
     float v[8];
@@ -451,7 +458,7 @@ int launch_kind(const GemmArgs& a, cudaStream_t stream) {
     const int cols = (a.N + (GLU ? 63 : 127)) / (GLU ? 64 : 128);
     if (!(a.K & 15) && per_group >= 32 && (a.M + 63) / 64 * (long long)cols * a.batch >= 64) {
       const dim3 grid(a.group_offsets ? a.M / 64 + min(a.G, a.M) : (a.M + 63) / 64, cols, a.batch);
-      const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(256), 0, stream, a);
+      const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(128), 0, stream, a);
       return e == cudaSuccess ? FT_OK : (int)e;
     }
     // rows a block: about twice a group's mean, so that most busy groups are read once
