@@ -926,16 +926,13 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
                 c_rows: Optional[torch.Tensor] = None, row_scale: Optional[torch.Tensor] = None,
                 rows: Optional[int] = None, glu: bool = False, act: str = "silu",
                 act_alpha: float = 1.702, act_limit: float = 7.0, rows_per_pass: int = 8,
-                unary: Optional[str] = None, bias: Optional[torch.Tensor] = None, group_rows: int = 0,
-                early_weights: bool = False) -> None:
+                unary: Optional[str] = None, bias: Optional[torch.Tensor] = None, group_rows: int = 0) -> None:
     """c = a @ w^T for few rows, streaming bfloat16 weights once through
     mma.sync; same conventions as :func:`gemm_rows`.  ``unary`` (one of
     :data:`ACTIVATIONS`, without ``glu``): that function of the float32 accumulator is stored; ``bias``
     (float32 ``[N]``, without ``glu``) is added to the accumulator first.  ``group_rows``: ``w`` is ``[G, N, K]``
     and rows ``g * group_rows ..`` of ``a`` and ``c`` belong to matrix g.  With ``glu``, ``act`` may be
-    ``silu``, ``swigluoai`` or ``gelu_tanh``.  ``early_weights`` (a dense product or one of ``group_rows``): the caller
-    knows that the launch right before did not write ``w``, so its first pieces are fetched without waiting for that
-    launch to end."""
+    ``silu``, ``swigluoai`` or ``gelu_tanh``."""
     _need(a, "a", torch.bfloat16, contiguous=False)
     _need(w, "w", torch.bfloat16)
     _need(c, "c", contiguous=False)
@@ -967,12 +964,12 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
             raise KernelError("skinny_gemm: the active list needs G + 1 entries")
     if unary is not None and (glu or unary not in ACTIVATIONS):
         raise KernelError(f"skinny_gemm: cannot apply {unary!r} (with glu: {glu})")
-    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i")
+    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i")
     _check(f(_ptr(a), a.stride(0), _ptr(w), NW * K, _ptr(c), code(c.dtype), c.stride(0),
              _ptr(group_offsets), _ptr(active), _ptr(a_rows), _ptr(c_rows), _ptr(row_scale), M, N, K, G,
              int(glu), GLU_ACTS[act], float(act_alpha), float(act_limit),
-             rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], _ptr(bias), int(group_rows),
-             int(early_weights), _stream()), "skinny_gemm")
+             rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], _ptr(bias), int(group_rows), _stream()),
+           "skinny_gemm")
 
 
 # ------------------------------------------------ grouped GEMM on tcgen05

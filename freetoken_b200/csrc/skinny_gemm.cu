@@ -42,7 +42,6 @@ struct SkinnyArgs {
   int unary = 0;             // without GLU: 0 nothing, 1 relu(x)^2, 2 tanh-GELU, 3 SiLU, 5 tanh on the accumulator
   const float* bias = nullptr;   // [N], added to the accumulator (not with GLU)
   int group_rows = 0;            // > 0: every group has that many rows, group g the rows g * group_rows ..
-  int early = 0;                 // W was not written by the launch before: its first pieces need not wait for it
 };
 
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
@@ -93,46 +92,6 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
   constexpr int NG = GLU ? 2 : 1;
   __shared__ float red[KS][NT][NG][16][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 16;
-  const int K = a.K;
-  const int chunks = (K + 31) >> 5;
-  const int per = (chunks + KS - 1) / KS;
-  const int c_begin = warp * per, c_end = min(chunks, c_begin + per);
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  // weight row pointers of this lane (rows beyond N are clamped and masked)
-  const uint4* wrow[NG][2];
-  bool wvalid[2];
-  auto point = [&](int group) {
-    const __nv_bfloat16* W = a.W + (size_t)group * a.w_group_stride;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = n0 + g + 8 * h;
-      wvalid[h] = r < a.N;
-#pragma unroll
-      for (int q = 0; q < NG; ++q) {
-        const size_t rr = (size_t)(wvalid[h] ? r : 0) + (size_t)q * a.N;
-        wrow[q][h] = reinterpret_cast<const uint4*>(W + rr * K);
-      }
-    }
-  };
-  uint4 wv[U][NG][2];
-  auto load_weights = [&](int c) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k8 = ((c + u) << 2) + t;  // index in units of 8 elements
-      const bool kin = (c + u) < c_end && (k8 << 3) < K;
-#pragma unroll
-      for (int q = 0; q < NG; ++q)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          wv[u][q][h] = (kin && wvalid[h]) ? ld_stream(wrow[q][h] + k8) : zero;
-    }
-  };
-  bool have = a.early;                    // the first pieces are on their way
-  if (have) {
-    point(blockIdx.y);
-    load_weights(c_begin);
-  }
   pdl_wait();
 
   int group = blockIdx.y;
@@ -150,7 +109,26 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
     row_end = a.group_offsets[group + 1];
   }
   if (row_end <= row_begin) return;
-  if (!have) point(group);
+  const int n0 = blockIdx.x * 16;
+  const __nv_bfloat16* W = a.W + (size_t)group * a.w_group_stride;
+  const int K = a.K;
+  // weight row pointers of this lane (rows beyond N are clamped and masked)
+  const uint4* wrow[NG][2];
+  bool wvalid[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = n0 + g + 8 * h;
+    wvalid[h] = r < a.N;
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      const size_t rr = (size_t)(wvalid[h] ? r : 0) + (size_t)q * a.N;
+      wrow[q][h] = reinterpret_cast<const uint4*>(W + rr * K);
+    }
+  }
+  const int chunks = (K + 31) >> 5;
+  const int per = (chunks + KS - 1) / KS;
+  const int c_begin = warp * per, c_end = min(chunks, c_begin + per);
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 
   for (int pass = row_begin; pass < row_end; pass += 8 * NT) {
     const uint4* xrow[NT];
@@ -172,13 +150,17 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
         for (int i = 0; i < 4; ++i) acc[q][j][i] = 0.f;
 
     for (int c = c_begin; c < c_end; c += U) {
+      uint4 wv[U][NG][2];
       uint4 xv[U][NT];
-      if (!have) load_weights(c);
-      have = false;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int k8 = ((c + u) << 2) + t;
+        const int k8 = ((c + u) << 2) + t;  // index in units of 8 elements
         const bool kin = (c + u) < c_end && (k8 << 3) < K;
+#pragma unroll
+        for (int q = 0; q < NG; ++q)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            wv[u][q][h] = (kin && wvalid[h]) ? ld_stream(wrow[q][h] + k8) : zero;
 #pragma unroll
         for (int j = 0; j < NT; ++j)
           xv[u][j] = (kin && xrow[j]) ? __ldg(xrow[j] + k8) : zero;
@@ -266,7 +248,7 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
                               const int* group_offsets, const int* active, const int* a_rows,
                               const int* c_rows, const float* row_scale, int M, int N, int K, int G, int glu,
                               int act, float act_alpha, float act_limit, int rows_per_pass, int unary,
-                              const float* bias, int group_rows, int early, cudaStream_t stream) {
+                              const float* bias, int group_rows, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return FT_OK;
   if (K <= 0 || (K & 7) || (lda & 7) || G <= 0) return FT_ERR_SHAPE;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((w_group_stride * 2) & 15)) return FT_ERR_SHAPE;
@@ -278,7 +260,6 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
   a.unary = unary;
   a.bias = bias;
   a.group_rows = group_rows;
-  a.early = early && !group_offsets && !active;
   // with the list of busy groups, no more groups than rows can have any
   dim3 grid((N + 15) / 16, active ? min(G, M) : G);
   const int nt = rows_per_pass / 8;

@@ -38,7 +38,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
         rows = x.shape[0]
         if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and rows <= SKINNY_ROWS
                 and ops.skinny_gemm_takes(x, weight, out)):
-            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows), bias=bias, early_weights=True)
+            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows), bias=bias)
             return out
         if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
                 and out.is_contiguous()):
@@ -50,8 +50,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
     if activation is not None:
         if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[0] <= SKINNY_ROWS
                 and ops.skinny_gemm_takes(x, weight, out)):
-            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(x.shape[0]), unary=activation,
-                            early_weights=True)
+            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(x.shape[0]), unary=activation)
             return out
         linear(x, weight, out)
         ops.activation(out, activation)
@@ -60,7 +59,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
         rows = x.shape[0]
         takes = ops.skinny_gemm_takes(x, weight, out)
         if takes and rows <= SKINNY_ROWS:
-            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows), early_weights=True)
+            ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows))
             return out
         if out.dtype == torch.bfloat16:
             torch.mm(x, weight.t(), out=out)
@@ -88,7 +87,7 @@ def grouped(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> torch.T
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16:
         rows, flat = x.view(G * T, K), out.view(G * T, out.shape[2])
         if T <= SKINNY_ROWS and ops.skinny_gemm_takes(rows, weight, flat):
-            ops.skinny_gemm(rows, weight, flat, group_rows=T, rows_per_pass=ops.pass_rows(T), early_weights=True)
+            ops.skinny_gemm(rows, weight, flat, group_rows=T, rows_per_pass=ops.pass_rows(T))
             return out
         torch.bmm(x, weight.transpose(1, 2), out=out)
         return out
