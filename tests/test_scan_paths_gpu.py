@@ -131,3 +131,25 @@ def test_latent_rows_of_few_and_many_tokens_agree_bitwise(dtype, heads, dq, rank
                                heads=heads, q_dim=dq, rank=rank, rot=rot, interleaved=interleaved, eps=1e-6, turn_q=True)
         results.append((pages, q_abs, turned))
     assert all(torch.equal(x, y) for x, y in zip(*results))
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("C,taps,lens", [(258, 4, [1000, 1, 31]), (70, 3, [1024]), (33, 4, [500, 700]), (8, 8, [7] * 150)])
+def test_long_convolutions_agree_bitwise(dtype, C, taps, lens):
+    """1,024 tokens and more take runs of 32 a thread; here against the same segments a few at a time."""
+    dt = DT[dtype]
+    w, b = rnd(C, taps, seed=2), rnd(C, seed=3)
+    slot, starts = _segments(lens)
+    seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(torch.int32).to(DEV)
+    x = rnd(sum(lens), C, dtype=dt, seed=1)
+    first = rnd(len(lens) + 2, max(1, (taps - 1) * C), seed=4)
+    whole, y = first.clone(), torch.empty_like(x)
+    ops().conv_silu(x, y, w, b, whole, seg, slot, starts)
+    parts, want, at = first.clone(), torch.empty_like(x), 0
+    for i, n in enumerate(lens):
+        for a in range(0, n, 600):
+            m = min(600, n - a)
+            ops().conv_silu(x[at + a:at + a + m], want[at + a:at + a + m], w, b, parts, torch.zeros(m, dtype=torch.int32, device=DEV),
+                            slot[i:i + 1], torch.tensor([0, m], dtype=torch.int32, device=DEV))
+        at += n
+    assert torch.equal(y, want) and torch.equal(whole, parts)
