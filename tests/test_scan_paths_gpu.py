@@ -153,3 +153,37 @@ def test_long_convolutions_agree_bitwise(dtype, C, taps, lens):
                             slot[i:i + 1], torch.tensor([0, m], dtype=torch.int32, device=DEV))
         at += n
     assert torch.equal(y, want) and torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("S,H,k", [(4, 256, 1), (4, 2052, 2), (2, 4100, 5), (1, 1024, 8), (3, 64, 0)])
+def test_stream_norms_of_few_and_many_tokens_agree_bitwise(dtype, S, H, k):
+    T, dt, o = 70, DT[dtype], ops()
+    streams, branch = rnd(T, S, H, seed=1), rnd(T, max(k, 1), H, dtype=dt, seed=2)
+    mix, out, read = rnd(S, S, seed=3), rnd(S, seed=4), rnd(S, seed=5)
+    weight, bias = rnd(H, seed=6), rnd(H, seed=7)
+    results = []
+    for rows in (T, 9):
+        x, y = streams.clone(), torch.empty(T, H, dtype=dt, device=DEV)
+        for a in range(0, T, rows):
+            b = min(T, a + rows)
+            o.hyper_norm(x[a:b], branch[a:b] if k else None, mix if k else None, out if k else None, read, weight, bias, 1e-5,
+                         True, y[a:b])
+        results.append((x, y))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("H,k", [(512, 1), (2048, 3), (4096, 2), (6000, 1), (30, 2)])
+def test_branch_norms_of_few_and_many_tokens_agree_bitwise(dtype, H, k):
+    T, dt, o = 70, DT[dtype], ops()
+    residual, branch = rnd(T, H, seed=1), rnd(T, k, H, dtype=dt, seed=2)
+    w, w2 = rnd(H, seed=3), rnd(H, seed=4)
+    results = []
+    for rows in (T, 9):
+        x, y = residual.clone(), torch.empty(T, H, dtype=dt, device=DEV)
+        for a in range(0, T, rows):
+            b = min(T, a + rows)
+            o.norm_add(branch[a:b], x[a:b], w, 1e-5, True, 0.7, next_weight=w2, next_eps=1e-4, next_out=y[a:b])
+        results.append((x, y))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
