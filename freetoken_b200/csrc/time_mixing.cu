@@ -133,15 +133,18 @@ struct TimeMixArgs {
   int heads, P, D, vec;    // vec: state rows may be read in 16-byte pieces
 };
 
-constexpr int time_mix_buffer(int RPL, int LPC) { return TM_CHUNK * (3 * LPC * RPL + TM_THREADS / LPC + 1); }
+constexpr int time_mix_buffer(int RPL, int LPC, int CPL) { return TM_CHUNK * (3 * LPC * RPL + CPL * TM_THREADS / LPC + 1); }
 
-template <typename AT, int RPL, int LPC>
+// CPL: columns a lane owns (neighbouring ones, of the same rows).  With two, a row of r, k and w is read from shared
+// memory, and made on its way there, for twice as many columns: eight segments of 317
+// .. 958 tokens, 32 heads of 64 x 64, 326 instead of 496 us.
+template <typename AT, int RPL, int LPC, int CPL>
 __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) {
   constexpr int DP = LPC * RPL;                        // rows, filled up
   constexpr int NE = DP / 32;                          // channels a lane stages per token
-  constexpr int CPW = 32 / LPC, COLS = TM_WARPS * CPW; // columns of a warp, of a block
+  constexpr int CPW = 32 / LPC, COLS = TM_WARPS * CPW * CPL; // lanes' columns of a warp, columns of a block
   constexpr int LOG = LPC == 8 ? 3 : 4;
-  constexpr int PER = time_mix_buffer(RPL, LPC);
+  constexpr int PER = time_mix_buffer(RPL, LPC, CPL);
   static_assert((LPC == 8 || LPC == 16) && DP % 32 == 0 && TM_CHUNK * COLS <= TM_THREADS, "lanes, rows, columns");
   extern __shared__ __align__(16) float sm[];
   pdl_wait();
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
   const int D = a.D, P = a.P;
   const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1];
   if (q1 <= q0) return;
-  const int cb = warp * CPW + (lane >> LOG);           // this lane's column inside the block
+  const int cb = (warp * CPW + (lane >> LOG)) * CPL;   // this lane's first column inside the block
   const int col = blockIdx.x * COLS + cb;
   float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + ((size_t)head * P + col) * D;
   const AT* rp = (const AT*)a.r + (size_t)head * D;
@@ -158,22 +161,25 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
   const AT* vp = (const AT*)a.v + (size_t)head * P;
   const float* dp = a.decay + (size_t)head * D;
 
-  float S[RPL];
+  float S[CPL][RPL];
 #pragma unroll
-  for (int j = 0; j < RPL / 4; ++j) {
-    const int n = (LPC * j + l) * 4;
-    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (col < P && n < D) {
-      if (a.vec) f = *reinterpret_cast<const float4*>(st + n);
-      else {
-        f.x = st[n];
-        if (n + 1 < D) f.y = st[n + 1];
-        if (n + 2 < D) f.z = st[n + 2];
-        if (n + 3 < D) f.w = st[n + 3];
+  for (int c = 0; c < CPL; ++c)
+#pragma unroll
+    for (int j = 0; j < RPL / 4; ++j) {
+      const int n = (LPC * j + l) * 4;
+      const float* p = st + (size_t)c * D + n;
+      float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (col + c < P && n < D) {
+        if (a.vec) f = *reinterpret_cast<const float4*>(p);
+        else {
+          f.x = p[0];
+          if (n + 1 < D) f.y = p[1];
+          if (n + 2 < D) f.z = p[2];
+          if (n + 3 < D) f.w = p[3];
+        }
       }
+      S[c][4 * j] = f.x; S[c][4 * j + 1] = f.y; S[c][4 * j + 2] = f.z; S[c][4 * j + 3] = f.w;
     }
-    S[4 * j] = f.x; S[4 * j + 1] = f.y; S[4 * j + 2] = f.z; S[4 * j + 3] = f.w;
-  }
   float w0[NE], u[NE];
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
@@ -226,7 +232,7 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
 
   struct Row {
     float4 r[RPL / 4], k[RPL / 4], w[RPL / 4];
-    float v;
+    float v[CPL];
   };
   // one chunk: works through tokens t0 .. from buffer `turn`, puts the next chunk (`x`) into the other one and
   // fetches the chunk two further on in its place
@@ -237,9 +243,10 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
     const float* ws = ks + TM_CHUNK * DP;
     const float* vs = ws + TM_CHUNK * DP;
     const float* bs = vs + TM_CHUNK * COLS;
-    float part[TM_CHUNK];
+    float part[CPL][TM_CHUNK];
     auto load_row = [&](int tt, Row& row) {
-      row.v = vs[tt * COLS + cb];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) row.v[c] = vs[tt * COLS + cb + c];
 #pragma unroll
       for (int j = 0; j < RPL / 4; ++j) {
         const int n = tt * DP + (LPC * j + l) * 4;
@@ -248,20 +255,25 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
         row.w[j] = *reinterpret_cast<const float4*>(ws + n);
       }
     };
-    auto token = [&](const Row& row) {
-      float acc = 0.f;
+    auto token = [&](const Row& row, int tt) {
 #pragma unroll
-      for (int j = 0; j < RPL / 4; ++j) {
-        acc = fmaf(S[4 * j], row.r[j].x, acc);
-        acc = fmaf(S[4 * j + 1], row.r[j].y, acc);
-        acc = fmaf(S[4 * j + 2], row.r[j].z, acc);
-        acc = fmaf(S[4 * j + 3], row.r[j].w, acc);
-        S[4 * j] = fmaf(row.w[j].x, S[4 * j], row.k[j].x * row.v);
-        S[4 * j + 1] = fmaf(row.w[j].y, S[4 * j + 1], row.k[j].y * row.v);
-        S[4 * j + 2] = fmaf(row.w[j].z, S[4 * j + 2], row.k[j].z * row.v);
-        S[4 * j + 3] = fmaf(row.w[j].w, S[4 * j + 3], row.k[j].w * row.v);
+      for (int c = 0; c < CPL; ++c) {
+        float acc = 0.f;
+        float(&Sc)[RPL] = S[c];
+        const float v = row.v[c];
+#pragma unroll
+        for (int j = 0; j < RPL / 4; ++j) {
+          acc = fmaf(Sc[4 * j], row.r[j].x, acc);
+          acc = fmaf(Sc[4 * j + 1], row.r[j].y, acc);
+          acc = fmaf(Sc[4 * j + 2], row.r[j].z, acc);
+          acc = fmaf(Sc[4 * j + 3], row.r[j].w, acc);
+          Sc[4 * j] = fmaf(row.w[j].x, Sc[4 * j], row.k[j].x * v);
+          Sc[4 * j + 1] = fmaf(row.w[j].y, Sc[4 * j + 1], row.k[j].y * v);
+          Sc[4 * j + 2] = fmaf(row.w[j].z, Sc[4 * j + 2], row.k[j].z * v);
+          Sc[4 * j + 3] = fmaf(row.w[j].w, Sc[4 * j + 3], row.k[j].w * v);
+        }
+        part[c][tt] = acc;
       }
-      return acc;
     };
     if (nt == TM_CHUNK) {
       Row cur, ahead;                                  // the next token's row is on its way meanwhile
@@ -269,37 +281,41 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
 #pragma unroll
       for (int tt = 0; tt < TM_CHUNK; ++tt) {
         if (tt + 1 < TM_CHUNK) load_row(tt + 1, ahead);
-        part[tt] = token(cur);
+        token(cur, tt);
         cur = ahead;
       }
     } else {
 #pragma unroll
       for (int tt = 0; tt < TM_CHUNK; ++tt) {
-        part[tt] = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) part[c][tt] = 0.f;
         if (tt < nt) {
           Row cur;
           load_row(tt, cur);
-          part[tt] = token(cur);
+          token(cur, tt);
         }
       }
     }
     // lane l of a column's ends with the total of token l >> (LOG - 3)
-    int mask = LPC / 2;
-#pragma unroll
-    for (int w = TM_CHUNK / 2; w >= 1; w >>= 1) {
-      const bool upper = l & mask;
-#pragma unroll
-      for (int i = 0; i < w; ++i) {
-        const float send = upper ? part[i] : part[i + w];
-        const float keep = upper ? part[i + w] : part[i];
-        part[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
-      }
-      mask >>= 1;
-    }
-    if constexpr (LOG == 4) part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
     const int tok = l >> (LOG - 3);
-    if ((l & (LPC / 8 - 1)) == 0 && tok < nt && col < P)
-      a.o[(size_t)(t0 + tok) * a.heads * P + (size_t)head * P + col] = fmaf(bs[tok], vs[tok * COLS + cb], part[0]);
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      int mask = LPC / 2;
+#pragma unroll
+      for (int w = TM_CHUNK / 2; w >= 1; w >>= 1) {
+        const bool upper = l & mask;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const float send = upper ? part[c][i] : part[c][i + w];
+          const float keep = upper ? part[c][i + w] : part[c][i];
+          part[c][i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+        }
+        mask >>= 1;
+      }
+      if constexpr (LOG == 4) part[c][0] += __shfl_xor_sync(0xffffffffu, part[c][0], 1);
+      if ((l & (LPC / 8 - 1)) == 0 && tok < nt && col + c < P)
+        a.o[(size_t)(t0 + tok) * a.heads * P + (size_t)head * P + col + c] = fmaf(bs[tok], vs[tok * COLS + cb + c], part[c][0]);
+    }
     if (t0 + TM_CHUNK < q1) {
       put(sm + (turn ^ 1) * PER, x);
       fetch(t0 + 3 * TM_CHUNK, x);
@@ -317,17 +333,20 @@ __global__ void __launch_bounds__(TM_THREADS) time_mixing_kernel(TimeMixArgs a) 
     if (t0 + TM_CHUNK < q1) chunk(t0 + TM_CHUNK, 1, even);
   }
 #pragma unroll
-  for (int j = 0; j < RPL / 4; ++j) {
-    const int n = (LPC * j + l) * 4;
-    if (col < P && n < D) {
-      if (a.vec) *reinterpret_cast<float4*>(st + n) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
-      else {
+  for (int c = 0; c < CPL; ++c)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (n + i < D) st[n + i] = S[4 * j + i];
+    for (int j = 0; j < RPL / 4; ++j) {
+      const int n = (LPC * j + l) * 4;
+      float* p = st + (size_t)c * D + n;
+      if (col + c < P && n < D) {
+        if (a.vec) *reinterpret_cast<float4*>(p) = make_float4(S[c][4 * j], S[c][4 * j + 1], S[c][4 * j + 2], S[c][4 * j + 3]);
+        else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (n + i < D) p[i] = S[c][4 * j + i];
+        }
       }
     }
-  }
 }
 
 // Segments of one token each (a decode step): what it costs is reading and writing the states, so a lane holds
@@ -464,15 +483,24 @@ static int launch_time_mix_step(const TimeMixArgs& a, int S, cudaStream_t stream
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
+template <typename AT, int RPL, int LPC, int CPL>
+static int launch_time_mix(const TimeMixArgs& a, int S, cudaStream_t stream) {
+  const size_t smem = 2 * time_mix_buffer(RPL, LPC, CPL) * sizeof(float);
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(time_mixing_kernel<AT, RPL, LPC, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int cols = CPL * TM_THREADS / LPC;
+  const dim3 grid((a.P + cols - 1) / cols, a.heads, S);
+  const cudaError_t e = launch_pdl(time_mixing_kernel<AT, RPL, LPC, CPL>, grid, dim3(TM_THREADS), smem, stream, a);
+  return e == cudaSuccess ? FT_OK : (int)e;
+}
+// Two columns a lane where that leaves two blocks an SM; a few segments need all the blocks there are.
 template <typename AT, int RPL, int LPC>
 static int launch_time_mix(const TimeMixArgs& a, int S, cudaStream_t stream) {
-  const size_t smem = 2 * time_mix_buffer(RPL, LPC) * sizeof(float);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(time_mixing_kernel<AT, RPL, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int cols = TM_THREADS / LPC;
-  const dim3 grid((a.P + cols - 1) / cols, a.heads, S);
-  const cudaError_t e = launch_pdl(time_mixing_kernel<AT, RPL, LPC>, grid, dim3(TM_THREADS), smem, stream, a);
-  return e == cudaSuccess ? FT_OK : (int)e;
+  if constexpr (LPC == 16) {
+    const int cols = 2 * TM_THREADS / LPC;
+    if ((long long)((a.P + cols - 1) / cols) * a.heads * S >= 2 * 148) return launch_time_mix<AT, RPL, LPC, 2>(a, S, stream);
+  }
+  return launch_time_mix<AT, RPL, LPC, 1>(a, S, stream);
 }
 
 }  // namespace ft

@@ -134,6 +134,32 @@ def test_latent_rows_of_few_and_many_tokens_agree_bitwise(dtype, heads, dq, rank
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("H,P,D,lens", [(2, 36, 40, [3, 1, 17]), (1, 64, 64, [8, 9]), (3, 30, 20, [11]),
+                                        (40, 41, 41, [9] * 9), (20, 70, 100, [3, 8] * 5)])    # two columns a lane
+def test_time_mixing_agrees_bitwise(dtype, H, P, D, lens):
+    T, dt = sum(lens), DT[dtype]
+    slot, starts = _segments(lens)
+    r, k, v = rnd(T, H * D, dtype=dt, seed=1), rnd(T, H * D, dtype=dt, seed=2), rnd(T, H * P, dtype=dt, seed=3)
+    decay, w0, u = rnd(T, H * D, seed=4), rnd(H * D, seed=5), rnd(H, D, seed=6)
+    if P != D:                                   # one row stride
+        wide = max(P, D) * H
+        r, k, v = (torch.cat([x, torch.zeros(T, wide - x.shape[1], dtype=dt, device=DEV)], 1) for x in (r, k, v))
+    call = lambda state, y, rows, s, q: ops().time_mixing_scan(
+        r[rows][:, :H * D], k[rows][:, :H * D], v[rows][:, :H * P], decay[rows], w0, u, state, y, s, q, H, P, D)
+    first = rnd(len(lens) + 2, H * D * P, seed=7, scale=0.1)
+    whole, y = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+    call(whole, y, torch.arange(T, device=DEV), slot, starts)
+    steps, want = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+
+    def launch(rows, s, q, t):
+        out = torch.empty(rows.numel(), H * P, device=DEV)
+        call(steps, out, rows, s, q)
+        want[rows] = out
+    _token_by_token(lens, launch)
+    assert torch.equal(y, want) and torch.equal(whole, steps)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
 @pytest.mark.parametrize("C,taps,lens", [(258, 4, [1000, 1, 31]), (70, 3, [1024]), (33, 4, [500, 700]), (8, 8, [7] * 150)])
 def test_long_convolutions_agree_bitwise(dtype, C, taps, lens):
     """1,024 tokens and more take runs of 32 a thread; here against the same segments a few at a time."""
