@@ -591,6 +591,110 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
   }
 }
 
+// The same for many tokens, a block a token: a row's pieces stay in registers between the norm's sums and their
+// use, a thread NPT of them, one behind the other at a distance of the block, so that the row is read once, all its
+// loads (and the look-up of its page) in flight together; the other half of a turned pair is a shuffle away.  Heads
+// of 4, 8, 16 or 32 pieces, rotary halves of a power of two of them; the sums run in the order of the kernel above.
+// That one reads a row twice, looks up its page in between and walks work items with two divisions each.  8,192 rows,
+// before and now: 48 + 2 x 8 heads of 128, one norm a row, 130 -> 84 us (268 MB: 41 us); 32 + 2 x 8, a norm a head, 137
+// -> 66; 16 + 2 x 4, none, 60 -> 36.  2,048 rows of the first: 33 -> 23.  Up to a hundred tokens both take a launch's time.
+template <int NPT>
+__global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkRopeArgs a) {
+  __shared__ float scratch[66];
+  pdl_wait();
+  const int t = blockIdx.x, d = a.d, dc = d >> 3, shift = __ffs(dc) - 1;
+  const int qp = a.nq * dc, kp = a.nkv * dc, total = qp + 2 * kp;
+  const __nv_bfloat16* row = (const __nv_bfloat16*)a.qkv + (size_t)t * a.ld;
+  uint4 raw[NPT];
+#pragma unroll
+  for (int i = 0; i < NPT; ++i) {
+    const int p = threadIdx.x + 256 * i;
+    raw[i] = p < total ? *reinterpret_cast<const uint4*>(row + p * 8) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  const int pos = a.token_pos[t];
+  __nv_bfloat16* ko = nullptr;
+  __nv_bfloat16* vo = nullptr;
+  if (a.kv_pages) {
+    const int page = a.block_table[(size_t)a.token_seg[t] * a.table_width + pos / a.P];
+    ko = (__nv_bfloat16*)a.kv_pages + (size_t)page * a.page_stride + (size_t)(pos % a.P) * d;
+    vo = ko + a.kv_stride;
+  }
+  const size_t head_stride_cache = (size_t)a.P * d;
+  __nv_bfloat16* qo = (__nv_bfloat16*)a.q_out + (size_t)t * a.nq * d;
+  float inv_q = 1.f, inv_k = 1.f;
+  if (a.norm_mode == 1) {
+    float sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int i = 0; i < NPT; ++i) {
+      const int p = threadIdx.x + 256 * i;
+      if (p < qp) sq += sumsq8(unpack8(raw[i]));
+      else if (p < qp + kp) sk += sumsq8(unpack8(raw[i]));
+    }
+    block_sum2(sq, sk, scratch);
+    inv_q = rsqrtf(sq / (float)(a.nq * a.dn) + a.eps);
+    inv_k = rsqrtf(sk / (float)(a.nkv * a.dn) + a.eps);
+  }
+  const int half = a.R >> 1, hc = a.interleaved ? 0 : half >> 3;
+  const float* cs = (a.cos_sin && a.R > 0) ? a.cos_sin + (size_t)pos * a.R : nullptr;
+  const float one = a.plus_one ? 1.f : 0.f;
+#pragma unroll
+  for (int i = 0; i < NPT; ++i) {
+    const int p = threadIdx.x + 256 * i;
+    if (256 * i + (int)(threadIdx.x & ~31u) >= total) break;         // the whole warp is past the row
+    const bool is_q = p < qp, is_v = p >= qp + kp;
+    const int pp = is_q ? p : (is_v ? p - qp - kp : p - qp), h = pp >> shift, ci = pp & (dc - 1);
+    Chunk8 x = unpack8(raw[i]);
+    if (a.norm_mode) {
+      float inv = is_q ? inv_q : inv_k;
+      if (a.norm_mode == 2) {
+        float s = sumsq8(x);
+        for (int o = dc >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        inv = rsqrtf(s / (float)a.dn + a.eps);
+      }
+      if (!is_v) {
+        float w[8];
+        load8a((is_q ? a.q_weight : a.k_weight) + (a.norm_mode == 1 ? h * d : 0) + ci * 8, w);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x.v[j] = x.v[j] * inv * (w[j] + one);
+      }
+    }
+    if (cs && hc) {
+      Chunk8 o;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o.v[j] = __shfl_xor_sync(0xffffffffu, x.v[j], hc);
+      if (!is_v && ci < 2 * hc) {
+        const int i0 = (ci & (hc - 1)) * 8;
+        float c[8], sn[8];
+        load8a(cs + i0, c);
+        load8a(cs + half + i0, sn);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)                                    // rounded as the kernel above rounds
+          x.v[j] = ci < hc ? __fmaf_rn(x.v[j], c[j], -__fmul_rn(o.v[j], sn[j])) : __fmaf_rn(o.v[j], sn[j], __fmul_rn(x.v[j], c[j]));
+      }
+    } else if (cs && !is_v && ci * 8 < a.R) {
+      float c[4], sn[4];
+      load4p(cs + ci * 4, c);
+      load4p(cs + half + ci * 4, sn);
+      turn_pairs(x, c, sn);
+    }
+    if (p >= total) continue;
+    if (is_q) store8(qo + p * 8, x);
+    else if (!ko) continue;
+    else if (!is_v) store8(ko + (size_t)h * head_stride_cache + ci * 8, x);
+    else if (a.v_first) {
+      const float l = a.v_lambda[0];
+      Chunk8 f = {};
+      if (ci * 8 < a.d_first)
+        f = load8((const __nv_bfloat16*)a.v_first + (size_t)t * a.ld_first + (size_t)h * a.d_first + ci * 8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x.v[j] = (1.f - l) * x.v[j] + l * f.v[j];
+      store8(vo + (size_t)h * head_stride_cache + ci * 8, x);
+    } else {
+      *reinterpret_cast<uint4*>(vo + (size_t)h * head_stride_cache + ci * 8) = raw[i];
+    }
+  }
+}
+
 // --------------------------------------------------------------- top-k sum
 // out[t,:] = sum_j parts[t*k+j,:] in float32, j ascending.
 template <typename AT>
@@ -748,7 +852,20 @@ int ft_qk_rope_store(const void* qkv, void* q_out, void* kv_pages, const float* 
     if (parts < 1) parts = 1;
     const bool eager = T <= ROW_KERNEL_EAGER_TOKENS && !((uintptr_t)q_weight & 15) && !((uintptr_t)k_weight & 15) &&
                        !((uintptr_t)cos_sin & 15);
-    if (eager) launch_pdl(qk_rope_store_vec_kernel<true>, dim3(T, parts), dim3(256), smem, stream, a);
+    const int dc = d >> 3, hc = interleaved ? 0 : R >> 4, npt = ((nq + 2 * nkv) * dc + 255) / 256;
+    const bool in_rows = T > ROW_KERNEL_EAGER_TOKENS && dc >= 4 && dc <= 32 && !(dc & (dc - 1)) && !(hc & (hc - 1)) &&
+                         npt <= 8 && !((uintptr_t)q_weight & 15) && !((uintptr_t)k_weight & 15) &&
+                         !((uintptr_t)cos_sin & 15);
+    if (in_rows) {
+      switch (npt) {
+        case 1: launch_pdl(qk_rope_rows_kernel<1>, dim3(T), dim3(256), 0, stream, a); break;
+        case 2: launch_pdl(qk_rope_rows_kernel<2>, dim3(T), dim3(256), 0, stream, a); break;
+        case 3: launch_pdl(qk_rope_rows_kernel<3>, dim3(T), dim3(256), 0, stream, a); break;
+        case 4: launch_pdl(qk_rope_rows_kernel<4>, dim3(T), dim3(256), 0, stream, a); break;
+        case 5: case 6: launch_pdl(qk_rope_rows_kernel<6>, dim3(T), dim3(256), 0, stream, a); break;
+        default: launch_pdl(qk_rope_rows_kernel<8>, dim3(T), dim3(256), 0, stream, a); break;
+      }
+    } else if (eager) launch_pdl(qk_rope_store_vec_kernel<true>, dim3(T, parts), dim3(256), smem, stream, a);
     else launch_pdl(qk_rope_store_vec_kernel<false>, dim3(T, parts), dim3(256), smem, stream, a);
     FT_LAUNCH_CHECK();
     return FT_OK;
