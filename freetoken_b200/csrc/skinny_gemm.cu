@@ -44,11 +44,22 @@ struct SkinnyArgs {
   int group_rows = 0;            // > 0: every group has that many rows, group g the rows g * group_rows ..
 };
 
+// Plain loads with a memory clobber, and a warp barrier behind a round's loads (skinny_kernel): the compiler may not
+// sink such a load below the barrier, so a round's loads are all in flight before its first product.  As read-only
+// loads they were sunk between the products wherever that saved registers: eight chunks a round then took 54 registers
+// and longer than four.
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
+               : "l"(p) : "memory");
+  return v;
+}
+
+// the rows of A in the same way, through L1
+__device__ __forceinline__ uint4 ld_rows(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 
@@ -86,9 +97,8 @@ __device__ __forceinline__ float unary_act_s(float x, int kind) {
 // 8 or 16 for dense matrices with few rows (QKV, O), where 4 warps per
 // 16 weight rows would leave an SM with a handful of warps and too few loads in
 // flight to fill the memory pipe.  KS is chosen from the weight's shape alone.
-template <int NT, bool GLU, typename OT, int KS>
+template <int NT, bool GLU, typename OT, int KS, int U>      // U: 32-k chunks in flight per warp
 __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
-  constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);  // 32-k chunks in flight per warp
   constexpr int NG = GLU ? 2 : 1;
   __shared__ float red[KS][NT][NG][16][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -163,8 +173,9 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
             wv[u][q][h] = (kin && wvalid[h]) ? ld_stream(wrow[q][h] + k8) : zero;
 #pragma unroll
         for (int j = 0; j < NT; ++j)
-          xv[u][j] = (kin && xrow[j]) ? __ldg(xrow[j] + k8) : zero;
+          xv[u][j] = (kin && xrow[j]) ? (U == 8 ? ld_rows(xrow[j] + k8) : __ldg(xrow[j] + k8)) : zero;
       }
+      if constexpr (U == 8) __syncwarp();
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -209,12 +220,29 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
   }
 }
 
+// Eight chunks a round where a warp has more than four (a dense matrix, 8 tokens a pass): half the rounds, each of
+// which lasts a load's latency.  A four-layer decode of width 2,048, before and now: 16 tokens behind a prompt of 2,048
+// (Tonapel) 6.88 -> 6.63 ms, eight requests (Besuzen) 12.77 -> 12.5; Dizatar, width 4,096, 21.83 -> 21.58; one MiniMax-M3
+// request 11.54 -> 11.42.  Two warps a block (the head, an expert's down projection) gain nothing from it, nor does
+// the gated pair, whose four chunks are as many loads.
+template <int NT, bool GLU, typename OT, int KS>
+void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream) {
+  constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);
+  if constexpr (NT == 1 && !GLU && KS >= 4) {
+    const int per = ((a.K + 31) / 32 + KS - 1) / KS;
+    if (per > 4) {
+      launch_pdl(skinny_kernel<NT, GLU, OT, KS, 8>, grid, dim3(KS * 32), 0, stream, a);
+      return;
+    }
+  }
+  launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
+}
 template <bool GLU, typename OT, int KS>
 int launch_nt(const SkinnyArgs& a, int nt, dim3 grid, cudaStream_t stream) {
   switch (nt) {
-    case 1: launch_pdl(skinny_kernel<1, GLU, OT, KS>, grid, dim3(KS * 32), 0, stream, a); break;
-    case 2: launch_pdl(skinny_kernel<2, GLU, OT, KS>, grid, dim3(KS * 32), 0, stream, a); break;
-    case 4: launch_pdl(skinny_kernel<4, GLU, OT, KS>, grid, dim3(KS * 32), 0, stream, a); break;
+    case 1: launch_u<1, GLU, OT, KS>(a, grid, stream); break;
+    case 2: launch_u<2, GLU, OT, KS>(a, grid, stream); break;
+    case 4: launch_u<4, GLU, OT, KS>(a, grid, stream); break;
     default: return FT_ERR_SHAPE;
   }
   return FT_OK;
