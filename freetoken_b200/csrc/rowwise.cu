@@ -343,7 +343,7 @@ __device__ __forceinline__ float4 branch_at4(const BranchArgs& b, int t, int H, 
   float eg = 1.f;
   if (b.extra) {
     e = load4f((const AT*)b.extra + (size_t)t * H + 4 * gi);
-    if (b.extra_gate) eg = b.extra_gate[t];
+    if (b.extra && b.extra_gate) eg = b.extra_gate[t];
   }
   if (b.beside) {
     const AT* other = (const AT*)b.beside + (size_t)t * b.kb * H + 4 * gi;
@@ -379,6 +379,78 @@ __device__ __forceinline__ float4 branch_at4(const BranchArgs& b, int t, int H, 
   z.x = fmaf(back, h.x, z.x); z.y = fmaf(back, h.y, z.y); z.z = fmaf(back, h.z, z.z); z.w = fmaf(back, h.w, z.w);
   z.x += y.x; z.y += y.y; z.z += y.z; z.w += y.w;
   return z;
+}
+
+// The pieces gi = threadIdx.x + j * THREADS (j < KEEP) of token t's branch at once: a slot's pieces of all KEEP are in
+// flight together, and the first slots' beside the other sublayer's rows, for launches of few tokens, which last a row's
+// latency.  (Piece after piece, each waits for its own loads: norm_add of a token of 4,096 values 6.6 us, now 5.8.)
+// Every element's sum runs in the order above.
+template <typename AT, int KEEP, int THREADS>
+__device__ __forceinline__ void branch_all(const BranchArgs& b, int t, int H, unsigned slots, float back, float4 (&z)[KEEP]) {
+  constexpr int U = KEEP <= 2 ? 4 : 2;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int groups = H >> 2;
+  auto at = [&](const void* rows, size_t row, int j) {
+    const int gi = threadIdx.x + j * THREADS;
+    return gi < groups ? load4f((const AT*)rows + row * H + 4 * gi) : zero;
+  };
+  float4 v[U][KEEP], e[KEEP], h[KEEP], y[KEEP];
+  float s[U], eg = 1.f;
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = j0 + u < b.k && (slots >> (j0 + u) & 1u);
+      s[u] = (b.part_scale && j0 + u < b.k) ? b.part_scale[j0 + u] : 1.f;
+#pragma unroll
+      for (int j = 0; j < KEEP; ++j) v[u][j] = in ? at(b.rows, (size_t)t * b.k + j0 + u, j) : zero;
+    }
+  };
+  fetch(0);
+  if (b.extra && b.extra_gate) eg = b.extra_gate[t];
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    e[j] = b.extra ? at(b.extra, t, j) : zero;
+    h[j] = back != 0.f ? at(b.source, t, j) : zero;
+    y[j] = z[j] = zero;
+  }
+  if (b.beside) {
+    for (int j0 = 0; j0 < b.kb; j0 += 2) {
+      float4 o[2][KEEP];
+      float os[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const bool in = j0 + u < b.kb;
+        os[u] = in && b.beside_scale ? b.beside_scale[j0 + u] : 1.f;
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) o[u][j] = in ? at(b.beside, (size_t)t * b.kb + j0 + u, j) : zero;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+          y[j].x = fmaf(os[u], o[u][j].x, y[j].x); y[j].y = fmaf(os[u], o[u][j].y, y[j].y);
+          y[j].z = fmaf(os[u], o[u][j].z, y[j].z); y[j].w = fmaf(os[u], o[u][j].w, y[j].w);
+        }
+    }
+  }
+  for (int j0 = 0; j0 < b.k; j0 += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < KEEP; ++j) {
+        z[j].x = fmaf(s[u], v[u][j].x, z[j].x); z[j].y = fmaf(s[u], v[u][j].y, z[j].y);
+        z[j].z = fmaf(s[u], v[u][j].z, z[j].z); z[j].w = fmaf(s[u], v[u][j].w, z[j].w);
+      }
+    if (j0 + U < b.k) fetch(j0 + U);
+  }
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    z[j].x = fmaf(eg, e[j].x, z[j].x); z[j].y = fmaf(eg, e[j].y, z[j].y);
+    z[j].z = fmaf(eg, e[j].z, z[j].z); z[j].w = fmaf(eg, e[j].w, z[j].w);
+    z[j].x = fmaf(back, h[j].x, z[j].x); z[j].y = fmaf(back, h[j].y, z[j].y);
+    z[j].z = fmaf(back, h[j].z, z[j].z); z[j].w = fmaf(back, h[j].w, z[j].w);
+    z[j].x += y[j].x; z[j].y += y[j].y; z[j].z += y[j].z; z[j].w += y[j].w;
+  }
 }
 
 // out[t, :] = z of token t, for a consumer that wants one plain row
@@ -479,10 +551,12 @@ __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
         w[j] = load4f(a.weight + 4 * gi);
         if constexpr (EAGER) {
           if (a.next_weight) w_next[j] = load4f(a.next_weight + 4 * gi);
+        } else {
+          keep[j] = branch_at4<AT>(a.b, t, H, gi, slots, back);
         }
-        keep[j] = branch_at4<AT>(a.b, t, H, gi, slots, back);
       }
     }
+    if constexpr (EAGER) branch_all<AT, KEEP, 256>(a.b, t, H, slots, back, keep);
 #pragma unroll
     for (int j = 0; j < KEEP; ++j) {
       const int gi = threadIdx.x + j * 256;
@@ -588,14 +662,26 @@ __global__ void __launch_bounds__(THREADS) join_layer_norm_kernel(JoinNormArgs a
       }
     }
     const unsigned slots = a.b.rows ? branch_slots(a.b, t, back) : 0u;
+    constexpr bool ALL = EAGER && KEEP <= 2;       // more do not fit the registers of 512 threads
+    float4 zs[ALL ? KEEP : 1];
+    if constexpr (ALL) {
+#pragma unroll
+      for (int j = 0; j < KEEP; ++j) {
+        const int gi = threadIdx.x + j * THREADS;
+        x[j] = gi < groups ? load4f(r + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      if (a.b.rows) branch_all<AT, KEEP, THREADS>(a.b, t, H, slots, back, zs);
+    }
 #pragma unroll
     for (int j = 0; j < KEEP; ++j) {
       const int gi = threadIdx.x + j * THREADS;
-      x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (!ALL) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (gi < groups) {
-        x[j] = load4f(r + 4 * gi);
+        if constexpr (!ALL) x[j] = load4f(r + 4 * gi);
         if (a.b.rows) {
-          const float4 z = branch_at4<AT, EAGER>(a.b, t, H, gi, slots, back);
+          float4 z;
+          if constexpr (ALL) z = zs[j];
+          else z = branch_at4<AT, EAGER>(a.b, t, H, gi, slots, back);
           x[j].x += z.x; x[j].y += z.y; x[j].z += z.z; x[j].w += z.w;
           store4f(r + 4 * gi, x[j]);
         }
@@ -808,9 +894,10 @@ hyper_norm_kernel(float* __restrict__ streams, const AT* __restrict__ branch, in
 // a thread owns up to KEEP groups of 4 consecutive values; it first fetches all its pieces of every
 // stream and of the branch (all loads in flight together), then joins, reads and keeps u in registers
 // between the passes.  The sums run in the order of the generic kernel.
-// EAGER (up to 64 tokens, where a launch is one row's latency): the branch's partial rows are fetched four at a
-// time and weight and bias - cold in L2, the step's weights have been through it - before the sums instead of
-// behind them: four rows of 4 x 4,096 values 7.1 -> 5.7 us, one to eight of 4 x 2,048 4.4 -> 3.7.  With every SM full of rows those registers would cost occupancy.
+// EAGER (up to 64 tokens, where a launch is one row's latency): the branch's partial rows are fetched two or four at a
+// time, for all of a thread's pieces together, and weight and bias - cold in L2, the step's weights have been through
+// it - before the sums instead of behind them: four rows of 4 x 4,096 values 7.1 -> 4.9 us, one to eight of 4 x 2,048
+// 4.4 -> 3.7.  With every SM full of rows those registers would cost occupancy.
 template <typename AT, int S, int KEEP, bool EAGER>
 __global__ void __launch_bounds__(256)
 hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch, int k, const float* __restrict__ mix,
@@ -844,22 +931,30 @@ hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch
           b_early[j] = bias ? load4f(bias + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
-      if (branch && EAGER) {
-        for (int q0 = 0; q0 < k; q0 += 4) {
-          float4 more[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            more[u] = q0 + u < k ? load4f(y_rows + (size_t)(q0 + u) * H + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (q0 + u < k) { y[j].x += more[u].x; y[j].y += more[u].y; y[j].z += more[u].z; y[j].w += more[u].w; }
-        }
-      } else if (branch) {
+      if (branch && !EAGER) {
         for (int q = 0; q < k; ++q) {
           const float4 v = load4f(y_rows + (size_t)q * H + 4 * gi);
           y[j].x += v.x; y[j].y += v.y; y[j].z += v.z; y[j].w += v.w;
         }
       }
+    }
+  }
+  if constexpr (EAGER) {
+    constexpr int U = KEEP <= 2 ? 4 : KEEP <= 4 ? 2 : 1;
+    for (int q0 = 0; branch && q0 < k; q0 += U) {
+      float4 more[U][KEEP];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+          const int gi = threadIdx.x + j * 256;
+          more[u][j] = q0 + u < k && gi < groups ? load4f(y_rows + (size_t)(q0 + u) * H + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j)
+          if (q0 + u < k) { y[j].x += more[u][j].x; y[j].y += more[u][j].y; y[j].z += more[u][j].z; y[j].w += more[u][j].w; }
     }
   }
   float sum = 0.f;

@@ -213,3 +213,27 @@ def test_branch_norms_of_few_and_many_tokens_agree_bitwise(dtype, H, k):
             o.norm_add(branch[a:b], x[a:b], w, 1e-5, True, 0.7, next_weight=w2, next_eps=1e-4, next_out=y[a:b])
         results.append((x, y))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+# a thread keeps one, two and four pieces of the row, the last with and without a remainder; fewer and more slots than
+# are fetched at a time
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("H,k,m", [(1000, 1, 1), (2048, 5, 2), (2040, 2, 3), (4096, 3, 1), (3000, 9, 2), (8192, 2, 2)])
+def test_routed_branches_of_few_and_many_tokens_agree_bitwise(dtype, H, k, m):
+    T, dt, o = 70, DT[dtype], ops()
+    residual, extra, source = rnd(T, H, seed=1), rnd(T, H, dtype=dt, seed=2), rnd(T, H, dtype=dt, seed=3)
+    rows, beside = rnd(T, k, H, dtype=dt, seed=4), rnd(T, m, H, dtype=dt, seed=5)
+    ids = (torch.arange(T * k, device=DEV, dtype=torch.int32) * 5 % 7).view(T, k)      # ids of 4 and more hand back
+    rows[ids >= 4] = float("nan")                                                       # and are not read
+    weights, gate, scale = rnd(T, k, seed=6), rnd(T, seed=7), rnd(m, seed=8)
+    w, w2 = rnd(H, seed=9), rnd(H, seed=10)
+    results = []
+    for step in (T, 9):
+        x, y, u = residual.clone(), torch.empty(T, H, dtype=dt, device=DEV), torch.empty(T, H, dtype=dt, device=DEV)
+        for a in range(0, T, step):
+            c = slice(a, min(T, a + step))
+            branch = o.RoutedRows(rows[c], ids[c], weights[c], 4, source[c], extra[c], None, gate[c], beside[c], scale)
+            o.norm_add(branch, x[c], w, 1e-5, True, 0.7, next_weight=w2, next_eps=1e-4, next_out=y[c])
+            o.join_layer_norm(branch, x[c], w, 1e-5, u[c])
+        results.append((x, y, u))
+    assert all(torch.isfinite(r).all() and torch.equal(r, other) for r, other in zip(*results))
