@@ -335,8 +335,16 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const Chunk8& c) {
 __device__ __forceinline__ float sumsq8(const Chunk8& c) {
   float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) s += c.v[i] * c.v[i];
+  for (int i = 0; i < 8; ++i) s = __fmaf_rn(c.v[i], c.v[i], s);
   return s;
+}
+// A turned pair of two halves (neighbours: turn_pairs) and a blended value.  Which product is rounded before the sum is
+// written out, once for the kernels of few and of many tokens: left to the compiler it may come out one way in one kernel
+// and the other way in another, and a token's stored key would then depend on how many tokens its launch holds.
+__device__ __forceinline__ float turn_first(float x0, float x1, float c, float s) { return __fmaf_rn(x0, c, -__fmul_rn(x1, s)); }
+__device__ __forceinline__ float turn_second(float x0, float x1, float c, float s) { return __fmaf_rn(x1, c, __fmul_rn(x0, s)); }
+__device__ __forceinline__ float blend_values(float own, float first, float l) {
+  return __fmaf_rn(1.f - l, own, __fmul_rn(l, first));
 }
 
 // Sum of two values over the block in one round; every thread gets both.
@@ -388,8 +396,8 @@ __device__ __forceinline__ void turn_pairs(Chunk8& x, const float (&c)[4], const
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float u = x.v[2 * i], v = x.v[2 * i + 1];
-    x.v[2 * i] = u * c[i] - v * s[i];
-    x.v[2 * i + 1] = v * c[i] + u * s[i];
+    x.v[2 * i] = turn_first(u, v, c[i], s[i]);
+    x.v[2 * i + 1] = __fmaf_rn(u, s[i], __fmul_rn(v, c[i]));
   }
 }
 
@@ -498,8 +506,8 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
         if (cs) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            y0.v[i] = x0.v[i] * c[i] - x1.v[i] * sn[i];
-            y1.v[i] = x1.v[i] * c[i] + x0.v[i] * sn[i];
+            y0.v[i] = turn_first(x0.v[i], x1.v[i], c[i], sn[i]);
+            y1.v[i] = turn_second(x0.v[i], x1.v[i], c[i], sn[i]);
           }
         }
         store8(dst + i0, y0);
@@ -544,8 +552,8 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
         load8w(cs + half + i0, sn);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          y0.v[i] = x0.v[i] * c[i] - x1.v[i] * sn[i];
-          y1.v[i] = x1.v[i] * c[i] + x0.v[i] * sn[i];
+          y0.v[i] = turn_first(x0.v[i], x1.v[i], c[i], sn[i]);
+          y1.v[i] = turn_second(x0.v[i], x1.v[i], c[i], sn[i]);
         }
       }
       store8(dst + i0, y0);
@@ -582,7 +590,7 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
         if (i < a.d_first)
           f = load8((const __nv_bfloat16*)a.v_first + (size_t)t * a.ld_first + (size_t)h * a.d_first + i);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x.v[j] = (1.f - l) * x.v[j] + l * f.v[j];
+        for (int j = 0; j < 8; ++j) x.v[j] = blend_values(x.v[j], f.v[j], l);
         store8(vo + (size_t)h * head_stride_cache + i, x);
       } else {
         *reinterpret_cast<uint4*>(vo + (size_t)h * head_stride_cache + i) = piece;
@@ -594,13 +602,14 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
 // The same for many tokens, a block a token: a row's pieces stay in registers between the norm's sums and their
 // use, a thread NPT of them, one behind the other at a distance of the block, so that the row is read once, all its
 // loads (and the look-up of its page) in flight together; the other half of a turned pair is a shuffle away.  Heads
-// of 4, 8, 16 or 32 pieces, rotary halves of a power of two of them; the sums run in the order of the kernel above.
+// of 4, 8, 16 or 32 pieces, rotary halves of a power of two of them.  Sums and roundings are those of the kernel above,
+// bit for bit: a token's result does not depend on how many tokens the launch holds.
 // That one reads a row twice, looks up its page in between and walks work items with two divisions each.  8,192 rows,
 // before and now: 48 + 2 x 8 heads of 128, one norm a row, 130 -> 84 us (268 MB: 41 us); 32 + 2 x 8, a norm a head, 137
 // -> 66; 16 + 2 x 4, none, 60 -> 36.  2,048 rows of the first: 33 -> 23.  Up to a hundred tokens both take a launch's time.
 template <int NPT>
 __global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkRopeArgs a) {
-  __shared__ float scratch[66];
+  __shared__ float scratch[66], k_sums[256 * NPT];
   pdl_wait();
   const int t = blockIdx.x, d = a.d, dc = d >> 3, shift = __ffs(dc) - 1;
   const int qp = a.nq * dc, kp = a.nkv * dc, total = qp + 2 * kp;
@@ -623,12 +632,23 @@ __global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkR
   __nv_bfloat16* qo = (__nv_bfloat16*)a.q_out + (size_t)t * a.nq * d;
   float inv_q = 1.f, inv_k = 1.f;
   if (a.norm_mode == 1) {
+    // The kernel above deals the key's pieces to the threads from thread 0 on.  Here they begin wherever the
+    // query's end: where that is not thread 0 their sums change hands, so that the total has the same bits.
     float sq = 0.f, sk = 0.f;
+    const bool moved = qp & 255;
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
       const int p = threadIdx.x + 256 * i;
       if (p < qp) sq += sumsq8(unpack8(raw[i]));
-      else if (p < qp + kp) sk += sumsq8(unpack8(raw[i]));
+      else if (p < qp + kp) {
+        const float s = sumsq8(unpack8(raw[i]));
+        if (moved) k_sums[p - qp] = s;
+        else sk += s;
+      }
+    }
+    if (moved) {
+      __syncthreads();
+      for (int c = threadIdx.x; c < kp; c += 256) sk += k_sums[c];
     }
     block_sum2(sq, sk, scratch);
     inv_q = rsqrtf(sq / (float)(a.nq * a.dn) + a.eps);
@@ -668,8 +688,8 @@ __global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkR
         load8a(cs + i0, c);
         load8a(cs + half + i0, sn);
 #pragma unroll
-        for (int j = 0; j < 8; ++j)                                    // rounded as the kernel above rounds
-          x.v[j] = ci < hc ? __fmaf_rn(x.v[j], c[j], -__fmul_rn(o.v[j], sn[j])) : __fmaf_rn(o.v[j], sn[j], __fmul_rn(x.v[j], c[j]));
+        for (int j = 0; j < 8; ++j)
+          x.v[j] = ci < hc ? turn_first(x.v[j], o.v[j], c[j], sn[j]) : turn_second(o.v[j], x.v[j], c[j], sn[j]);
       }
     } else if (cs && !is_v && ci * 8 < a.R) {
       float c[4], sn[4];
@@ -687,7 +707,7 @@ __global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkR
       if (ci * 8 < a.d_first)
         f = load8((const __nv_bfloat16*)a.v_first + (size_t)t * a.ld_first + (size_t)h * a.d_first + ci * 8);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) x.v[j] = (1.f - l) * x.v[j] + l * f.v[j];
+      for (int j = 0; j < 8; ++j) x.v[j] = blend_values(x.v[j], f.v[j], l);
       store8(vo + (size_t)h * head_stride_cache + ci * 8, x);
     } else {
       *reinterpret_cast<uint4*>(vo + (size_t)h * head_stride_cache + ci * 8) = raw[i];
