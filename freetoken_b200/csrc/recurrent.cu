@@ -845,6 +845,9 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
   constexpr int PER = seq_buffer(NPL, CPL, MODE == 1 ? 3 : 2);
   constexpr int VR = (SEQ_CHUNK * COLS + 32 * SEQ_WARPS - 1) / (32 * SEQ_WARPS);
   extern __shared__ __align__(16) float sm[];
+  // what a token writes, for its read-out: words of their own, since lanes behind the one that stores may still have to
+  // read the token's value (retention writes the value itself)
+  __shared__ float us[MODE == 2 ? 1 : SEQ_CHUNK * COLS];
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % SEQ_WARPS, l = lane & 15;
   const bool stages = threadIdx.x >= 32 * SEQ_WARPS;
@@ -1025,7 +1028,7 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
     const float* qs = sm + turn * PER;
     const float* ks = qs + SEQ_CHUNK * DP;
     const float* gs = ks + SEQ_CHUNK * DP;
-    float* vs = sm + turn * PER + (MODE == 1 ? 3 : 2) * SEQ_CHUNK * DP;
+    const float* vs = sm + turn * PER + (MODE == 1 ? 3 : 2) * SEQ_CHUNK * DP;
     const float4* gates = reinterpret_cast<const float4*>(vs + SEQ_CHUNK * COLS);
     float part[CPL][SEQ_CHUNK];
     auto token = [&](int tt) {
@@ -1075,7 +1078,7 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           u[c] = gate.x * (v[c] - gate.y * u[c]);
-          if (l == 0) vs[tt * COLS + cb + c] = u[c];             // for the read-out, by lanes of this column only
+          if (l == 0) us[tt * COLS + cb + c] = u[c];             // for the read-out, by lanes of this column only
         }
       }
 #pragma unroll
@@ -1096,7 +1099,7 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
         }
       }
     }
-    __syncwarp();
+    if constexpr (MODE != 2) __syncwarp();
     const int tok = l >> 1;
 #pragma unroll
     for (int c = 0; c < CPL; ++c) {
@@ -1104,8 +1107,9 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
       if (!(l & 1) && tok < nt && col + c < P) {
         // the read-out already contains the token's own write: decay * (S^T q) + (k . q) u
         const float4 gate = gates[tok];
+        const float u = MODE == 2 ? vs[tok * COLS + cb + c] : us[tok * COLS + cb + c];
         a.o[(size_t)(t0 + tok) * width + (size_t)head * P + col + c] =
-            fmaf(gate.z, vs[tok * COLS + cb + c], MODE == 1 ? part[c][0] : gate.y * part[c][0]);
+            fmaf(gate.z, u, MODE == 1 ? part[c][0] : gate.y * part[c][0]);
       }
     }
     __syncthreads();

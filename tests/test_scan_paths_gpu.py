@@ -237,3 +237,24 @@ def test_routed_branches_of_few_and_many_tokens_agree_bitwise(dtype, H, k, m):
             o.join_layer_norm(branch, x[c], w, 1e-5, u[c])
         results.append((x, y, u))
     assert all(torch.isfinite(r).all() and torch.equal(r, other) for r, other in zip(*results))
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("H,P,D,lens", [(40, 130, 128, [29, 16, 8]), (4, 30, 64, [61]), (6, 70, 200, [13, 24])])
+def test_delta_rule_repeats_itself(dtype, per_channel, H, P, D, lens):
+    """A token's write is read out later in its chunk by other lanes than computed it: the same bits in every launch."""
+    T, dt, o = sum(lens), DT[dtype], ops()
+    slot, starts = _segments(lens)
+    a_log, bias = rnd(H, seed=3, scale=0.5) - 1, rnd(H, seed=4, scale=0.5) - 1
+    gates, first = rnd(T, 2 * H, dtype=dt, seed=2), rnd(len(lens) + 2, H * D * P, seed=5, scale=0.1)
+    x, decay, channel_bias = rnd(T, 2 * H * D + H * P, dtype=dt, seed=1), rnd(T, H * D, seed=8), rnd(H * D, seed=9, scale=0.5) - 1
+    results = []
+    for _ in range(12):
+        state, y = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+        if per_channel:
+            o.channel_delta_scan(x, gates[:, :H], decay, channel_bias, a_log, state, y, slot, starts, H, H, D, P, 1e-6, D ** -0.5)
+        else:
+            o.delta_scan(x, gates[:, :H], gates[:, H:], bias, a_log, state, y, slot, starts, H, H, D, P, 1e-6, D ** -0.5)
+        results.append((state, y))
+    assert all(torch.equal(a, b) for r in results[1:] for a, b in zip(results[0], r))
