@@ -346,58 +346,83 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
 // out row = sum_s o_s 2^(m_s - m) / sum_s l_s 2^(m_s - m), splits ascending; a block per row
 // The splits' maxima and sums are fetched once, together, and the partial rows MERGE_AHEAD at a time (one after
 // the other, each behind its own factor's load, a token of 32 heads on 3,000 keys took 10.3 us, now 5.8).  The sums run over
-// ascending splits.
-constexpr int MERGE_AHEAD = 8;
-__global__ void __launch_bounds__(128) latent_merge_kernel(LatentAttnArgs a, int rt) {
+// ascending splits.  Shared memory holds the factors of MERGE_SPLITS splits (a launch has 64 at most unless its caller
+// asks for more); further ones follow in rounds of as many.
+constexpr int MERGE_AHEAD = 8, MERGE_SPLITS = 1024, MERGE_THREADS = 128;
+__global__ void __launch_bounds__(MERGE_THREADS) latent_merge_kernel(LatentAttnArgs a, int rt) {
   pdl_wait();
   const int tile = blockIdx.x, r = blockIdx.y;
   const int seg = a.tile_seg[tile], row0 = a.tile_row[tile];
   const int seg_begin = a.seg_q_start[seg];
   if (r >= (a.seg_q_start[seg + 1] - seg_begin) * a.nq - row0) return;
   const size_t base = ((size_t)tile * rt + r) * a.splits;
-  extern __shared__ float split_ml[];                  // [splits] sums, [splits] maxima, then factors
+  extern __shared__ float split_ml[];                  // of a round: sums, then maxima, then factors
   __shared__ float warp_m[4], total;
+  const int round = min(a.splits, MERGE_SPLITS);
   float* ls = split_ml;
-  float* fs = split_ml + a.splits;
+  float* fs = split_ml + round;
   float m = -INFINITY;
-  for (int s = threadIdx.x; s < a.splits; s += blockDim.x) {
-    const float2 ml = *reinterpret_cast<const float2*>(a.part_ml + (base + s) * 2);
-    fs[s] = ml.x;
-    ls[s] = ml.y;
-    m = fmaxf(m, ml.x);
+  for (int s = threadIdx.x; s < a.splits; s += MERGE_THREADS) {
+    const float ms = a.part_ml[(base + s) * 2];
+    if (s < round) {
+      fs[s] = ms;
+      ls[s] = a.part_ml[(base + s) * 2 + 1];
+    }
+    m = fmaxf(m, ms);
   }
   m = warp_max(m);
   if ((threadIdx.x & 31) == 0) warp_m[threadIdx.x >> 5] = m;
   __syncthreads();
   m = fmaxf(fmaxf(warp_m[0], warp_m[1]), fmaxf(warp_m[2], warp_m[3]));
-  for (int s = threadIdx.x; s < a.splits; s += blockDim.x) fs[s] = fs[s] == -INFINITY ? 0.f : fast_exp2(fs[s] - m);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float l = 0.f;
+  float l = 0.f;                                       // thread 0's
+  float4 acc[2];                                       // rank <= 1024: two pieces a thread
+#pragma unroll
+  for (int u = 0; u < 2; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int first = 0; first < a.splits; first += round) {
+    const int n = min(round, a.splits - first);
+    if (first > 0) {
+      __syncthreads();                                 // the round before is used up
+      for (int s = threadIdx.x; s < n; s += MERGE_THREADS) {
+        fs[s] = a.part_ml[(base + first + s) * 2];
+        ls[s] = a.part_ml[(base + first + s) * 2 + 1];
+      }
+    }
+    for (int s = threadIdx.x; s < n; s += MERGE_THREADS) fs[s] = fs[s] == -INFINITY ? 0.f : fast_exp2(fs[s] - m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
 #pragma unroll 8
-    for (int s = 0; s < a.splits; ++s) l += fs[s] == 0.f ? 0.f : ls[s] * fs[s];
-    total = l;
+      for (int s = 0; s < n; ++s) l += fs[s] == 0.f ? 0.f : ls[s] * fs[s];
+      total = l;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int c = (threadIdx.x + u * MERGE_THREADS) * 4;
+      if (c >= a.rank) break;
+      for (int s0 = 0; s0 < n; s0 += MERGE_AHEAD) {
+        float4 v[MERGE_AHEAD];
+        float f[MERGE_AHEAD];
+#pragma unroll
+        for (int i = 0; i < MERGE_AHEAD; ++i) {
+          f[i] = s0 + i < n ? fs[s0 + i] : 0.f;        // a split that saw no key left nothing to read
+          if (f[i] != 0.f) v[i] = *reinterpret_cast<const float4*>(a.part_o + (base + first + s0 + i) * a.rank + c);
+        }
+#pragma unroll
+        for (int i = 0; i < MERGE_AHEAD; ++i)
+          if (f[i] != 0.f) {
+            acc[u].x += v[i].x * f[i]; acc[u].y += v[i].y * f[i]; acc[u].z += v[i].z * f[i]; acc[u].w += v[i].w * f[i];
+          }
+      }
+    }
   }
   __syncthreads();
   const float inv = total > 0.f ? 1.f / total : 0.f;
   __nv_bfloat16* out = a.out + ((long long)seg_begin * a.nq + row0 + r) * a.ldo;
-  for (int c = threadIdx.x * 4; c < a.rank; c += blockDim.x * 4) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < a.splits; s0 += MERGE_AHEAD) {
-      float4 v[MERGE_AHEAD];
-      float f[MERGE_AHEAD];
 #pragma unroll
-      for (int i = 0; i < MERGE_AHEAD; ++i) {
-        f[i] = s0 + i < a.splits ? fs[s0 + i] : 0.f;   // a split that saw no key left nothing to read
-        if (f[i] != 0.f) v[i] = *reinterpret_cast<const float4*>(a.part_o + (base + s0 + i) * a.rank + c);
-      }
-#pragma unroll
-      for (int i = 0; i < MERGE_AHEAD; ++i)
-        if (f[i] != 0.f) {
-          acc.x += v[i].x * f[i]; acc.y += v[i].y * f[i]; acc.z += v[i].z * f[i]; acc.w += v[i].w * f[i];
-        }
-    }
-    *reinterpret_cast<uint2*>(out + c) = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+  for (int u = 0; u < 2; ++u) {
+    const int c = (threadIdx.x + u * MERGE_THREADS) * 4;
+    if (c < a.rank)
+      *reinterpret_cast<uint2*>(out + c) =
+          make_uint2(pack_bf16(acc[u].x * inv, acc[u].y * inv), pack_bf16(acc[u].z * inv, acc[u].w * inv));
   }
 }
 
@@ -464,7 +489,6 @@ int ft_attn_latent(const void* q, void* out, long long ldo, float* part_o, float
                    const int* block_table, int* status, long long page_stride, int nq, int d, int rank, int P,
                    int table_width, int window, int tiles, int mt, int splits, int split_keys, float scale, cudaStream_t stream) {
   if (tiles <= 0) return FT_OK;
-  if (splits > 6144) return FT_ERR_SHAPE;              // what the merge keeps of the splits in shared memory
   if ((d & 7) || (rank & 7) || rank <= 0 || rank > d || d > 1024 || (mt != 1 && mt != 2) || splits < 1 ||
       split_keys < LT_KEYS || split_keys % LT_KEYS || (ldo & 7) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
       ((uintptr_t)pages & 15) || (page_stride & 7) || P <= 0 || (splits > 1 && (!part_o || !part_ml)))
@@ -477,7 +501,8 @@ int ft_attn_latent(const void* q, void* out, long long ldo, float* part_o, float
   const int rc = mt == 1 ? launch_latent_by_size<1>(a, tiles, stream) : launch_latent_by_size<2>(a, tiles, stream);
   if (rc != FT_OK) return rc;
   if (splits > 1)
-    launch_pdl(latent_merge_kernel, dim3(tiles, 16 * mt), dim3(128), 2 * splits * sizeof(float), stream, a, 16 * mt);
+    launch_pdl(latent_merge_kernel, dim3(tiles, 16 * mt), dim3(MERGE_THREADS),
+               2 * (splits < MERGE_SPLITS ? splits : MERGE_SPLITS) * sizeof(float), stream, a, 16 * mt);
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
