@@ -17,6 +17,7 @@ from typing import List, Sequence
 
 import torch
 
+from ..csrc import ops
 from .manager import CacheManager
 
 _STATE_DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
@@ -54,15 +55,13 @@ class CacheStorage:
         """Zero the state rows of newly admitted request slots."""
         if not slots or not self.state:
             return
-        # run by run of neighbouring slots: an index tensor would have to be copied to the device first, and
-        # that copy waits for the steps in flight
-        slots = sorted(slots)
-        first = 0
-        for i in range(1, len(slots) + 1):
-            if i == len(slots) or slots[i] != slots[i - 1] + 1:
-                for t in self.state:
-                    t[:, slots[first]:slots[i - 1] + 1].zero_()
-                first = i
+        # the slots travel with the launch: an index tensor would have to be copied to the device first, and that
+        # copy waits for the steps in flight
+        for t in self.state:
+            if t.is_cuda:
+                ops.zero_slots(t, slots)
+            else:
+                t.index_fill_(1, torch.tensor(list(slots), dtype=torch.long), 0)
 
     def poison(self, group: int, pages: Sequence[int]) -> None:
         """Overwrite pages (of every stop of a group, all they hold) with NaN: a

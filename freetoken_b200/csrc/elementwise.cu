@@ -750,6 +750,26 @@ __global__ void gather_rows_kernel(const AT* __restrict__ src, const int* __rest
   for (int i = threadIdx.x; i < H; i += blockDim.x) d[i] = s[i];
 }
 
+// -------------------------------------------------------------- zero slots
+// State rows of newly admitted slots set to zero: t[stop][slot] for every stop, `row_bytes` each.  The slots travel in
+// the launch itself, so any set of them is one launch without a copy to the device.
+constexpr int ZERO_SLOTS = 128;
+struct ZeroSlotsArgs {
+  unsigned char* base;
+  long long stop_bytes, row_bytes;
+  int slots[ZERO_SLOTS];
+};
+__global__ void __launch_bounds__(256) zero_slots_kernel(const __grid_constant__ ZeroSlotsArgs a) {
+  pdl_wait();
+  unsigned char* row = a.base + (long long)blockIdx.z * a.stop_bytes + (long long)a.slots[blockIdx.y] * a.row_bytes;
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  if (!(((uintptr_t)a.base | a.stop_bytes | a.row_bytes) & 15)) {
+    for (long long i = first; i < a.row_bytes >> 4; i += stride) reinterpret_cast<uint4*>(row)[i] = make_uint4(0u, 0u, 0u, 0u);
+  } else {
+    for (long long i = first; i < a.row_bytes; i += stride) row[i] = 0;
+  }
+}
+
 // ------------------------------------------------------------ read stream
 // Sums a buffer of 16-byte words: nothing but loads, eight in flight per thread.
 // What a read-only stream reaches on this GPU - the ceiling of a decode step, which
@@ -898,6 +918,19 @@ int ft_qk_rope_store(const void* qkv, void* q_out, void* kv_pages, const float* 
 int ft_combine(const void* parts, void* out, int dtype, int T, int k, int H, cudaStream_t stream) {
   if (T <= 0) return FT_OK;
   FT_DISPATCH(dtype, AT, launch_pdl(combine_kernel<AT>, dim3(T), dim3(256), 0, stream, (const AT*)parts, (AT*)out, k, H));
+  FT_LAUNCH_CHECK();
+  return FT_OK;
+}
+
+// Zeroes rows `slots` (`n` of them, on the host) of every stop: stops of `stop_bytes`, rows of `row_bytes`.
+int ft_zero_slots(void* base, long long stop_bytes, long long row_bytes, const int* slots, int n, int stops,
+                  cudaStream_t stream) {
+  if (n <= 0 || stops <= 0 || row_bytes <= 0) return FT_OK;
+  if (n > ZERO_SLOTS || stops > 65535) return FT_ERR_SHAPE;
+  ZeroSlotsArgs a{(unsigned char*)base, stop_bytes, row_bytes, {}};
+  for (int i = 0; i < n; ++i) a.slots[i] = slots[i];
+  const long long blocks = (row_bytes + 256 * 64 - 1) / (256 * 64);      // four 16-byte pieces a thread, more of long rows
+  launch_pdl(zero_slots_kernel, dim3(blocks < 64 ? (unsigned)blocks : 64u, n, stops), dim3(256), 0, stream, a);
   FT_LAUNCH_CHECK();
   return FT_OK;
 }

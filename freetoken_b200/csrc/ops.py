@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Dict, Optional
+from typing import Dict, Optional, Sequence
 
 import torch
 
@@ -98,6 +98,25 @@ def _need_pages(kv_pages: torch.Tensor, dtype) -> None:
     if kv_pages.dim() != 5 or kv_pages.shape[0] != 2 or not kv_pages[0].is_contiguous() \
             or kv_pages.stride(0) not in (0, kv_pages[0].numel()):
         raise KernelError("kv_pages must be [2, pages, kv_heads, page, head_dim], planes dense")
+
+
+# ----------------------------------------------------------------- state
+ZERO_SLOTS = 128        # slots a launch of the clearing kernel carries
+
+
+def zero_slots(state: torch.Tensor, slots: Sequence[int]) -> None:
+    """Zero ``state[:, slots]`` of a dense ``[stops, slots, ...]`` tensor; a negative slot counts from the end."""
+    _need(state, "state")
+    stops, rows = state.shape[:2]
+    slots = [int(s) for s in slots]
+    if any(not -rows <= s < rows for s in slots):
+        raise IndexError(f"zero_slots: slots {slots} of {rows}")
+    row_bytes = state[0, 0].numel() * state.element_size() if state.numel() else 0
+    f = _fn("elementwise", "ft_zero_slots", "p q q p i i")
+    for i in range(0, len(slots), ZERO_SLOTS):
+        part = [s % rows for s in slots[i:i + ZERO_SLOTS]]
+        _check(f(_ptr(state), rows * row_bytes, row_bytes, (ctypes.c_int * len(part))(*part), len(part), stops, _stream()),
+               "zero_slots")
 
 
 # ------------------------------------------------------------------ rows
