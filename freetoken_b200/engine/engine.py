@@ -394,7 +394,7 @@ class Engine:
         self._poison_freed()        # pages a window has passed
         self.steps += 1
         self.tokens_run += ctx.num_tokens
-        return logits
+        return logits.view(logits.shape)        # the caller's own: the workspace keeps the view it handed out
 
     def _replay_graph(self, ctx: StepContext, logit_rows, logits, N: int, in_order: bool, probe) -> bool:
         """Decode-only steps with every row's logits wanted run as a captured
