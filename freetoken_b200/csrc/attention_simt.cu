@@ -41,6 +41,7 @@ struct AttnArgs {
   int sink_mode;          // 0 none, 1 the score sink_value, 2 sink[h]
   float sink_value;
   const float* sink;      // [nq]
+  const int* seg_q_start; // [S + 1] first token of every request, or nullptr
 };
 
 // MAXD: output dims per lane (head sizes up to 32 * MAXD)
@@ -121,11 +122,13 @@ __global__ void __launch_bounds__(128) attn_paged_kernel(AttnArgs a) {
   }
 }
 
-// A block's eight warps are (token, query head) rows of one KV head: `tokens` tokens by `heads` heads.  The
-// rows of one request walk the chunks together: every chunk is fetched once by all threads (cp.async, 16-byte
+// A block's eight warps are (token, query head) rows of one KV head and one request: `tokens` tokens by `heads`
+// heads.  They walk the chunks together: every chunk is fetched once by all threads (cp.async, 16-byte
 // pieces, the next chunk on its way while this one is used), and a warp leaves out the chunks that its own
 // token does not see, so its arithmetic is attn_paged_kernel's, operation by operation.  That kernel is bound
 // by latency: a lane reads its key's row from global memory value by value.
+// Blocks of several tokens begin every `tokens` tokens (`packs` of them) and end at their request's last token; the
+// first tokens of a request that begins inside one have a block of their own (blockIdx.x >= packs).
 // Measured (16 heads of 128 on 4 KV heads, float32): two prompts of 214 and 128 tokens in 70 us, a token behind
 // each in 25; four launches of the one and sixteen of the other took 4,552 us and take 686.
 constexpr int SHARED_WARPS = 8;
@@ -146,19 +149,28 @@ __device__ __forceinline__ void piece_of(const __nv_bfloat16* p, float (&v)[8]) 
 }
 
 template <typename AT, bool EXACT>
-__global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs a, int T, int tokens, int heads) {
+__global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs a, int T, int tokens, int heads, int packs) {
   constexpr int MAXD = 8, PIECE = 16 / sizeof(AT), CHUNK = 32;
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ int row_seg[SHARED_WARPS], row_lo[SHARED_WARPS], row_pos[SHARED_WARPS];
+  __shared__ int row_lo[SHARED_WARPS], row_pos[SHARED_WARPS];
   pdl_wait();
+  int r_begin = blockIdx.x * tokens, r_end = min(T, r_begin + tokens);
+  if ((int)blockIdx.x >= packs) {              // request blockIdx.x - packs + 1, up to where the next pack begins
+    const int s = blockIdx.x - packs + 1;
+    r_begin = a.seg_q_start[s];
+    r_end = min(min((r_begin / tokens + 1) * tokens, a.seg_q_start[s + 1]), T);
+    if (r_begin % tokens == 0 || r_end <= r_begin) return;
+  } else if (a.seg_q_start) {
+    r_end = min(r_end, a.seg_q_start[a.token_seg[r_begin] + 1]);
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d = a.d, group = a.nq / a.nkv, slices = (group + heads - 1) / heads;
   const int krow = d * sizeof(AT) + 16, vrow = d * sizeof(AT);       // padded key rows: no bank conflicts
   const int stage_bytes = CHUNK * (krow + vrow);
   float* qv = reinterpret_cast<float*>(sm + 2 * stage_bytes) + warp * d;
   const int kvh = blockIdx.y / slices, in_group = (blockIdx.y % slices) * heads + warp % heads;
-  const int r = blockIdx.x * tokens + warp / heads;
-  const bool live = r < T && warp / heads < tokens && in_group < group;
+  const int r = r_begin + warp / heads;
+  const bool live = r < r_end && in_group < group;
   const int h = kvh * group + in_group;
   int t = 0, pos = -1, lo = 0;
   if (live) {
@@ -170,8 +182,7 @@ __global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs
     for (int i = lane; i < d; i += 32) qv[i] = to_float(q[i]);
   }
   if (lane == 0) {
-    row_seg[warp] = live ? a.token_seg[t] : -1;
-    row_lo[warp] = lo;
+    row_lo[warp] = live ? lo : INT_MAX;
     row_pos[warp] = pos;
   }
   __syncthreads();
@@ -183,22 +194,18 @@ __global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs
   const AT* kbase = (const AT*)a.kv_pages + (size_t)kvh * a.P * d;
   const AT* vbase = kbase + a.kv_stride;
 
-  unsigned todo = 0;
-  for (int w = 0; w < SHARED_WARPS; ++w) todo |= row_seg[w] >= 0 ? 1u << w : 0u;
-  while (todo) {                               // one request after the other (mostly there is one)
-    const int seg = row_seg[__ffs(todo) - 1];
-    int first = INT_MAX, last = -1;
-    for (int w = 0; w < SHARED_WARPS; ++w) {
-      if (row_seg[w] != seg) continue;
-      todo &= ~(1u << w);
-      first = min(first, row_lo[w]);
-      last = max(last, row_pos[w]);
-    }
-    const int* table = a.block_table + (size_t)seg * a.table_width;
+  int first = INT_MAX, last = -1;
+  for (int w = 0; w < SHARED_WARPS; ++w) {
+    first = min(first, row_lo[w]);
+    last = max(last, row_pos[w]);
+  }
+  if (first <= last) {
+    const int* table = a.block_table + (size_t)a.token_seg[a.rows ? a.rows[r_begin] : r_begin] * a.table_width;
     auto fetch = [&](int stage, int c0) {      // keys outside first .. last are never read: those repeat one of them
       unsigned char* ks = sm + stage * stage_bytes;
       unsigned char* vs = ks + CHUNK * krow;
       const int pieces = d / PIECE;
+#pragma unroll 4
       for (int i = threadIdx.x; i < CHUNK * pieces; i += 32 * SHARED_WARPS) {
         const int jj = i / pieces, piece = i % pieces;
         const int j = min(max(c0 + jj, first), last);
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs
       cp_async_commit();
       cp_async_wait<1>();
       __syncthreads();
-      if (row_seg[warp] == seg && c0 <= pos && c0 + CHUNK > lo) {
+      if (c0 <= pos && c0 + CHUNK > lo) {
         const unsigned char* ks = sm + stage * stage_bytes;
         const AT* kr = reinterpret_cast<const AT*>(ks + lane * krow);
         const AT* vs = reinterpret_cast<const AT*>(ks + CHUNK * krow);
@@ -275,17 +282,29 @@ __global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs
   }
 }
 
+// How many tokens share a block of attn_shared_kernel (at most `fit`); T rows of S requests, `rest` blocks a token.
+// One while that leaves SMs without a block, or where every request has one token: rows of different requests share no
+// key, and packed into one block they were walked one request after the other (64 requests of 200 keys, 8 heads of 64,
+// float32: 147 us, apart 27; row by row from global memory 89).  One as well for rows picked out of several requests:
+// where each begins is not known then.  Otherwise neighbours share the chunks: a prompt of 512, 16 heads of 128, 221 us
+// (651 with a token a block).
+static int attn_tokens_per_block(int T, int S, int rest, int fit, bool starts_known) {
+  if ((long long)T * rest <= 2 * 148 || T == S || (S > 1 && !starts_known)) return 1;
+  return fit;
+}
+
 template <typename AT, bool EXACT>
-static int launch_shared(const AttnArgs& a, int T, cudaStream_t stream) {
+static int launch_shared(AttnArgs a, int T, int S, cudaStream_t stream) {
   const size_t smem = 2 * (size_t)32 * (2 * a.d * sizeof(AT) + 16) + (size_t)SHARED_WARPS * a.d * sizeof(float);
   const auto kernel = attn_shared_kernel<AT, EXACT>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int group = a.nq / a.nkv, heads = min(group, SHARED_WARPS), slices = (group + heads - 1) / heads;
-  // a token a block while that leaves SMs without one; otherwise neighbouring tokens share the chunks
-  const int tokens = (long long)T * a.nkv * slices <= 2 * 148 ? 1 : SHARED_WARPS / heads;
-  const cudaError_t le = launch_pdl(kernel, dim3((T + tokens - 1) / tokens, a.nkv * slices), dim3(32 * SHARED_WARPS),
-                                    smem, stream, a, T, tokens, heads);
+  const int tokens = attn_tokens_per_block(T, S, a.nkv * slices, SHARED_WARPS / heads, a.seg_q_start != nullptr);
+  if (tokens == 1 || S == 1) a.seg_q_start = nullptr;
+  const int packs = (T + tokens - 1) / tokens;
+  const cudaError_t le = launch_pdl(kernel, dim3(packs + (a.seg_q_start ? S - 1 : 0), a.nkv * slices), dim3(32 * SHARED_WARPS),
+                                    smem, stream, a, T, tokens, heads, packs);
   return le == cudaSuccess ? FT_OK : (int)le;
 }
 
@@ -293,17 +312,23 @@ static int launch_shared(const AttnArgs& a, int T, cudaStream_t stream) {
 
 using namespace ft;
 
+extern "C" int ft_attn_tokens_per_block(int T, int S, int rest, int fit, int starts_known) {
+  return attn_tokens_per_block(T, S, rest, fit, starts_known != 0);
+}
+
+// S: rows of the block table, or of seg_q_start where it is given (tokens lie request by request then).
 extern "C" int ft_attn_paged_simt(const void* q, void* out, const void* kv_pages,
                                   const int* token_pos, const int* token_seg,
                                   const int* block_table, const int* rows,
                                   long long page_stride, long long kv_stride, int nq, int nkv, int d, int P,
                                   int table_width, int window, float scale, int dtype, int T,
                                   int chunk, float softcap, int sink_mode, float sink_value,
-                                  const float* sink, cudaStream_t stream) {
+                                  const float* sink, const int* seg_q_start, int S, cudaStream_t stream) {
   if (T <= 0) return FT_OK;
   if (d > 1024 || d <= 0 || nkv <= 0 || nq % nkv) return FT_ERR_SHAPE;
   AttnArgs a{q, out, kv_pages, token_pos, token_seg, block_table, rows, page_stride, kv_stride,
-             nq, nkv, d, P, table_width, window, scale, chunk, softcap, sink_mode, sink_value, sink};
+             nq, nkv, d, P, table_width, window, scale, chunk, softcap, sink_mode, sink_value, sink,
+             rows ? nullptr : seg_q_start};
   if (sink_mode == 2 && !sink) return FT_ERR_SHAPE;
   dim3 grid(T, (nq + 3) / 4);
   const size_t smem = 4 * (size_t)d * sizeof(float);
@@ -311,8 +336,8 @@ extern "C" int ft_attn_paged_simt(const void* q, void* out, const void* kv_pages
   const int in_piece = dtype == FT_DTYPE_F32 ? 3 : 7;              // 16-byte pieces along a row, from its start
   if (d <= 256 && !(d & in_piece) && !(page_stride & in_piece) && !(kv_stride & in_piece) && !((uintptr_t)kv_pages & 15) &&
       (long long)nkv * nq <= 65535) {
-    const int rc = dtype == FT_DTYPE_F32 ? launch_shared<float, true>(a, T, stream)
-                                         : launch_shared<__nv_bfloat16, false>(a, T, stream);
+    const int rc = dtype == FT_DTYPE_F32 ? launch_shared<float, true>(a, T, S, stream)
+                                         : launch_shared<__nv_bfloat16, false>(a, T, S, stream);
     if (rc != FT_OK) return rc;
   } else if (d <= 256) {
     if (dtype == FT_DTYPE_F32) attn_paged_kernel<float, true, 8><<<grid, 128, smem, stream>>>(a);

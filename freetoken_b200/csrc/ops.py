@@ -1199,8 +1199,10 @@ def attn_paged_simt(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
                     token_pos: torch.Tensor, token_seg: torch.Tensor, block_table: torch.Tensor,
                     num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
                     window: Optional[int], rows: Optional[torch.Tensor] = None,
-                    options: Optional[ScoreOptions] = None) -> None:
-    """Generic paged attention; ``rows`` limits it to those token rows."""
+                    options: Optional[ScoreOptions] = None, seg_q_start: Optional[torch.Tensor] = None) -> None:
+    """Generic paged attention; ``rows`` limits it to those token rows.  ``seg_q_start`` (``[S + 1]``: the first token of
+    every request, whose tokens lie one behind the other) lets a block take several tokens of a request where there are
+    several requests."""
     _need(q, "q")
     _need(out, "out", q.dtype)
     _need_pages(kv_pages, q.dtype)
@@ -1211,11 +1213,16 @@ def attn_paged_simt(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
         _need(rows, "rows", torch.int32)
     if q.shape[1] != num_heads * head_dim or out.shape != q.shape:
         raise KernelError("attn_paged_simt: q/out must be [T, heads*head_dim]")
-    f = _fn("attention_simt", "ft_attn_paged_simt", "p p p p p p p q q i i i i i i f i i i f i f p")
+    S = block_table.shape[0]
+    if seg_q_start is not None:
+        _need(seg_q_start, "seg_q_start", torch.int32)
+        S = seg_q_start.numel() - 1
+    f = _fn("attention_simt", "ft_attn_paged_simt", "p p p p p p p q q i i i i i i f i i i f i f p p i")
     _check(f(_ptr(q), _ptr(out), _ptr(kv_pages), _ptr(token_pos), _ptr(token_seg),
              _ptr(block_table), _ptr(rows), kv_pages.stride(1), kv_pages.stride(0), num_heads, num_kv_heads,
              head_dim, kv_pages.shape[3], block_table.shape[1], int(window or 0), float(scale),
-             code(q.dtype), T, *(options or NO_SCORE_OPTIONS).args(num_heads), _stream()), "attn_paged_simt")
+             code(q.dtype), T, *(options or NO_SCORE_OPTIONS).args(num_heads), _ptr(seg_q_start), S, _stream()),
+           "attn_paged_simt")
 
 
 DECODE_HEAD_DIMS = (32, 64, 128)

@@ -123,7 +123,8 @@ class PagedSoftmaxCore:
                                  table, self.nq, self.nkv, self.d, self.scale, self.window, options=self.options)
             return
         ops.attn_paged_simt(q, o, kv_pages, ctx.token_pos, ctx.token_seg, table,
-                            self.nq, self.nkv, self.d, self.scale, self.window, options=self.options)
+                            self.nq, self.nkv, self.d, self.scale, self.window, options=self.options,
+                            seg_q_start=ctx.seg_q_start)
 
 
 @register_mixer("paged_attention")
