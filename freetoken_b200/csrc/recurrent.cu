@@ -70,14 +70,15 @@ struct ConvArgs {
 constexpr int CONV_MAX_TAPS = 8;     // longer convolutions take the plain loop
 
 // A thread owns one channel (two neighbouring ones where rows allow 4-byte pieces of bfloat16)
-// and `groups` runs of RUN consecutive tokens: while they belong to one segment it keeps the last taps inputs
+// and GROUPS runs of RUN consecutive tokens: while they belong to one segment it keeps the last taps inputs
 // in registers and fetches one new input a token, a run ahead; at a segment's first token (and always when
 // run is 1) it fetches the whole reach, from earlier rows or from the slot.  The sum runs over
 // ascending taps either way.  TAPS: the number of taps where the launch knows it (0: any up to CONV_MAX_TAPS); a
-// window of known length is shifted by renaming registers, and four runs share one fetch of
-// the weights: 3,951 rows of 12,288 channels in 132 instead of 243 us, 2,048 of 6,144 and 2,304 in 26 instead of 44.
-template <typename AT, int CPT, int RUN, int TAPS>
-__global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T, int groups) {
+// window of known length is shifted by renaming registers, and several runs share one fetch of the weights
+// (conv_groups says when).  bfloat16, four taps, before both and now: 1,024 rows of 512 channels 8.1 -> 6.1 us, 2,048 of
+// 2,304 27 -> 16, 4,096 of 6,144 127 -> 73.
+template <typename AT, int CPT, int RUN, int TAPS, int GROUPS>
+__global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T) {
   constexpr int W = TAPS ? TAPS : CONV_MAX_TAPS;
   pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * CPT;
@@ -101,28 +102,24 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T, int g
     }
   };
   int prev_seg = -1;
-  const int t_first = blockIdx.x * RUN * groups, t_end = min(T, t_first + RUN * groups);
+  const int t_first = blockIdx.x * RUN * GROUPS, t_end = min(T, t_first + RUN * GROUPS);
   // every token's own input and segment of a run first, all loads in flight together, the next run's meanwhile
-  float own[RUN][CPT], next[RUN][CPT];
-  int segs[RUN], next_segs[RUN];
-  auto fetch_run = [&](int t0) {
+  float own[RUN][CPT];
+  int segs[RUN];
+  auto fetch_run = [&](int t0, float (&v)[RUN][CPT], int (&seg)[RUN]) {
 #pragma unroll
     for (int i = 0; i < RUN; ++i) {
       if (t0 + i < t_end) {
-        fetch(t0 + i, next[i]);
-        next_segs[i] = a.token_seg[t0 + i];
+        fetch(t0 + i, v[i]);
+        seg[i] = a.token_seg[t0 + i];
       }
     }
   };
-  fetch_run(t_first);
+  fetch_run(t_first, own, segs);
   for (int t0 = t_first; t0 < t_end; t0 += RUN) {
-#pragma unroll
-    for (int i = 0; i < RUN; ++i) {
-      segs[i] = next_segs[i];
-#pragma unroll
-      for (int u = 0; u < CPT; ++u) own[i][u] = next[i][u];
-    }
-    fetch_run(t0 + RUN);
+    float next[RUN][CPT];
+    int next_segs[RUN];
+    if constexpr (GROUPS > 1) fetch_run(t0 + RUN, next, next_segs);
 #pragma unroll
     for (int i = 0; i < RUN; ++i) {
       const int t = t0 + i;
@@ -172,6 +169,13 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T, int g
       AT* o = (AT*)a.out + (size_t)t * a.ldo + c;
       if constexpr (CPT == 2) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(out[0], out[1]);
       else o[0] = from_float<AT>(out[0]);
+    }
+    if constexpr (GROUPS == 1) break;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      segs[i] = next_segs[i];
+#pragma unroll
+      for (int u = 0; u < CPT; ++u) own[i][u] = next[i][u];
     }
   }
 }
@@ -1374,11 +1378,25 @@ static int dispatch_delta(DeltaArgs a, int S, int T, int dtype, cudaStream_t str
   return FT_OK;
 }
 
+// Runs of eight tokens a thread of conv_silu_kernel walks; 0: a thread a token, below 1,024 tokens.  More than one run
+// saves fetches of the weights and of the reach, where it leaves blocks enough (1,000 of 128 threads; measured, us with one run and with
+// four: 1,024 rows of 512 channels 6.1 and 11.7; two, 4,096 rows of 6,144: 80 and 73) and segments are long (63 single
+// tokens beside 961 of 2,304 channels: a window is fetched anew at each, 14 and 26).  Single channels (float32) walk
+// four; two channels of other than four taps never gained (4,096 rows of 6,144, three taps: 117 and 129).
+static int conv_groups(int C, int T, int S, int taps, bool pairs) {
+  if (T < 1024) return 0;
+  if (T < 64LL * S) return 1;
+  if (pairs) return taps == 4 && (long long)(T / 16) * ((C / 2 + 127) / 128) >= 1000 ? 2 : 1;
+  return (long long)(T / 32) * ((C + 127) / 128) >= 1100 ? 4 : 1;
+}
+
 }  // namespace ft
 
 using namespace ft;
 
 extern "C" {
+
+int ft_conv_groups(int C, int T, int S, int taps, int pairs) { return conv_groups(C, T, S, taps, pairs != 0); }
 
 // Both kernels of the short convolution: outputs first, then the slots' new contents.
 int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const float* w, const float* bias,
@@ -1399,19 +1417,22 @@ int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const f
   if (taps > CONV_MAX_TAPS) {
     FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_long_kernel<AT>, dim3(T, cb), dim3(128), 0, stream, a));
   } else {
-    // many tokens: a thread walks 32 of them with its inputs in registers; few: a thread a token
-    const bool many = T >= 1024;
-    constexpr int GROUPS = 4;
-    const unsigned rows = many ? (T + 8 * GROUPS - 1) / (8 * GROUPS) : T;
+    // many tokens: a thread walks eight of them and more with its inputs in registers; few: a thread a token
+    const int groups = conv_groups(C, T, S, taps, pairs);
+    const int walked = groups == 0 ? 1 : 8 * groups;
+    const dim3 grid((T + walked - 1) / walked, pairs ? (C / 2 + 127) / 128 : cb), block(128);
+    using B = __nv_bfloat16;
     if (pairs) {
-      const dim3 grid(rows, (C / 2 + 127) / 128);
-      if (many && taps == 4) launch_pdl(conv_silu_kernel<__nv_bfloat16, 2, 8, 4>, grid, dim3(128), 0, stream, a, T, GROUPS);
-      else if (many) launch_pdl(conv_silu_kernel<__nv_bfloat16, 2, 8, 0>, grid, dim3(128), 0, stream, a, T, GROUPS);
-      else launch_pdl(conv_silu_kernel<__nv_bfloat16, 2, 1, 0>, grid, dim3(128), 0, stream, a, T, 1);
-    } else if (many) {
-      FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_kernel<AT, 1, 8, 0>, dim3(rows, cb), dim3(128), 0, stream, a, T, GROUPS));
+      if (groups == 0) launch_pdl(conv_silu_kernel<B, 2, 1, 0, 1>, grid, block, 0, stream, a, T);
+      else if (taps != 4) launch_pdl(conv_silu_kernel<B, 2, 8, 0, 1>, grid, block, 0, stream, a, T);
+      else if (groups == 1) launch_pdl(conv_silu_kernel<B, 2, 8, 4, 1>, grid, block, 0, stream, a, T);
+      else launch_pdl(conv_silu_kernel<B, 2, 8, 4, 2>, grid, block, 0, stream, a, T);
+    } else if (groups == 0) {
+      FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_kernel<AT, 1, 1, 0, 1>, grid, block, 0, stream, a, T));
+    } else if (groups == 1) {
+      FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_kernel<AT, 1, 8, 0, 1>, grid, block, 0, stream, a, T));
     } else {
-      FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_kernel<AT, 1, 1, 0>, dim3(rows, cb), dim3(128), 0, stream, a, T, 1));
+      FT_DISPATCH(dtype, AT, launch_pdl(conv_silu_kernel<AT, 1, 8, 0, 4>, grid, block, 0, stream, a, T));
     }
   }
   FT_LAUNCH_CHECK();

@@ -258,3 +258,11 @@ def test_delta_rule_repeats_itself(dtype, per_channel, H, P, D, lens):
             o.delta_scan(x, gates[:, :H], gates[:, H:], bias, a_log, state, y, slot, starts, H, H, D, P, 1e-6, D ** -0.5)
         results.append((state, y))
     assert all(torch.equal(a, b) for r in results[1:] for a, b in zip(results[0], r))
+
+
+# two runs a thread (bfloat16 pairs, four taps), four (single channels), and one beside: a request's edges inside runs
+@pytest.mark.parametrize("dtype,C,taps,lens", [("bfloat16", 2006, 4, [1500, 20, 541]), ("bfloat16", 2311, 4, [2050]),
+                                               ("float32", 2310, 3, [1201, 850]), ("bfloat16", 2006, 3, [1500, 20, 541]),
+                                               ("bfloat16", 512, 4, [7, 1022])])
+def test_long_convolutions_of_several_runs(dtype, C, taps, lens):
+    test_long_convolutions_agree_bitwise(dtype, C, taps, lens)
