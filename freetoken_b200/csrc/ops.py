@@ -693,10 +693,11 @@ def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Op
 
 def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
              d_skip: torch.Tensor, state: torch.Tensor, y: torch.Tensor, seg_slot: torch.Tensor,
-             seg_q_start: torch.Tensor, heads: int, head_dim: int, state_dim: int, groups: int) -> None:
+             seg_q_start: torch.Tensor, heads: int, head_dim: int, state_dim: int, groups: int, longest: int = 0) -> None:
     """Per head: ``S <- exp(-exp(a_log) * step) * S + step * B x^T``, ``y = S^T C + d_skip * x`` with
     ``step = softplus(dt + dt_bias)``; ``xbc`` rows are ``x | B | C``; ``state`` ``[slots, >= heads *
-    state_dim * head_dim]`` float32; ``y`` ``[T, heads * head_dim]`` float32."""
+    state_dim * head_dim]`` float32; ``y`` ``[T, heads * head_dim]`` float32.  ``longest`` (tokens of the longest segment, 0:
+    not known) helps to choose between kernels of equal results."""
     _need(xbc, "xbc", contiguous=False)
     _need(dt, "dt", xbc.dtype, contiguous=False)
     _need(state, "state", torch.float32, contiguous=False)
@@ -711,20 +712,21 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         raise KernelError("ssd_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * state_dim * head_dim:
         raise KernelError("ssd_scan: a state row must hold heads * state_dim * head_dim values")
-    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i")
+    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i i")
     _check(f(_ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
              _ptr(state), state.stride(0), _ptr(y), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim,
-             state_dim, groups, seg_slot.numel(), T, code(xbc.dtype), _stream()), "ssd_scan")
+             state_dim, groups, seg_slot.numel(), T, longest, code(xbc.dtype), _stream()), "ssd_scan")
 
 
 def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
                a_log: torch.Tensor, state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor,
                seg_q_start: torch.Tensor, heads: int, key_heads: int, key_dim: int, value_dim: int,
-               unit_eps: float, q_scale: float) -> None:
+               unit_eps: float, q_scale: float, longest: int = 0) -> None:
     """The gated delta rule per head: q and k made unit vectors (q times ``q_scale``), ``g =
     exp(-exp(a_log) * softplus(decay + dt_bias))``, ``b = sigmoid(beta)``; ``S <- g S``; ``u = b (v -
     S^T k)``; ``S <- S + k u^T``; ``o = S^T q``.  ``qkv`` rows are ``q | k | v``; ``beta`` and ``decay``
-    ``[T, heads]`` with the same row stride; ``state`` ``[slots, >= heads * key_dim * value_dim]``."""
+    ``[T, heads]`` with the same row stride; ``state`` ``[slots, >= heads * key_dim * value_dim]``.  ``longest`` (tokens of the longest segment, 0:
+    not known) helps to choose between kernels of equal results."""
     _need(qkv, "qkv", contiguous=False)
     _need(beta, "beta", qkv.dtype, contiguous=False)
     _need(decay, "decay", qkv.dtype, contiguous=False)
@@ -741,20 +743,21 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bi
         raise KernelError("delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i")
+    f = _fn("recurrent", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), _ptr(decay), beta.stride(0), _ptr(dt_bias), _ptr(a_log),
              _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, code(qkv.dtype),
+             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
              _stream()), "delta_scan")
 
 
 def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
                        a_log: torch.Tensor, state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor,
                        seg_q_start: torch.Tensor, heads: int, key_heads: int, key_dim: int, value_dim: int,
-                       unit_eps: float, q_scale: float) -> None:
+                       unit_eps: float, q_scale: float, longest: int = 0) -> None:
     """The gated delta rule with a decay per key channel: as :func:`delta_scan`, but row ``n`` of head
     ``h``'s state is multiplied by ``exp(-exp(a_log[h]) * softplus(decay[t, h * key_dim + n] + dt_bias[h *
-    key_dim + n]))`` before the token reads and writes.  ``decay`` is float32 ``[T, heads * key_dim]``."""
+    key_dim + n]))`` before the token reads and writes.  ``decay`` is float32 ``[T, heads * key_dim]``.  ``longest`` (tokens of the longest segment, 0:
+    not known) helps to choose between kernels of equal results."""
     _need(qkv, "qkv", contiguous=False)
     _need(beta, "beta", qkv.dtype, contiguous=False)
     _need(decay, "decay", torch.float32, contiguous=False)
@@ -771,20 +774,21 @@ def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tenso
         raise KernelError("channel_delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("channel_delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i")
+    f = _fn("recurrent", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(decay), decay.stride(0), _ptr(dt_bias),
              _ptr(a_log), _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, code(qkv.dtype), _stream()),
+             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype), _stream()),
            "channel_delta_scan")
 
 
 def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[torch.Tensor], seg_pos0: torch.Tensor,
                    state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor, seg_q_start: torch.Tensor,
-                   heads: int, key_dim: int, value_dim: int, k_scale: float) -> None:
+                   heads: int, key_dim: int, value_dim: int, k_scale: float, longest: int = 0) -> None:
     """Retention per head: ``S <- decay[h] S + k v^T``, ``o = S^T q``.  ``qkv`` rows are ``q | k | v``
     (``heads * key_dim`` twice, then ``heads * value_dim``); the first ``cos_sin.shape[1]`` dimensions of
     every q and k head are turned by the token's position (dimension i with i + half) in float32 and k is
-    multiplied by ``k_scale`` afterwards; ``state`` ``[slots, >= heads * key_dim * value_dim]`` float32."""
+    multiplied by ``k_scale`` afterwards; ``state`` ``[slots, >= heads * key_dim * value_dim]`` float32.  ``longest`` (tokens of the longest segment, 0:
+    not known) helps to choose between kernels of equal results."""
     _need(qkv, "qkv", contiguous=False)
     _need(decay, "decay", torch.float32)
     _need(state, "state", torch.float32, contiguous=False)
@@ -800,10 +804,10 @@ def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[tor
         raise KernelError("retention_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("retention_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i")
+    f = _fn("recurrent", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(decay), _ptr(cos_sin), rot, _ptr(seg_pos0), _ptr(state), state.stride(0),
              _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim, key_dim, float(k_scale),
-             seg_slot.numel(), T, code(qkv.dtype), _stream()), "retention_scan")
+             seg_slot.numel(), T, longest, code(qkv.dtype), _stream()), "retention_scan")
 
 
 def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: torch.Tensor, token_seg: torch.Tensor,

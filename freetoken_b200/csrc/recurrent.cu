@@ -20,9 +20,9 @@
 // products are one warp reduction; a block's four warps share the tokens of a
 // chunk, which all threads stage into shared memory together.  Which WC a launch
 // takes depends on the step's shape, never on a token's place in it, and the
-// operations on a column are the same for every WC.  Launches in which some segment
-// has several tokens take kernels with 16 lanes a column that perform the same
-// operations (see there).
+// operations on a column are the same for every WC.  Launches whose segments have several
+// tokens may take kernels with 16 lanes a column that perform the same operations (see
+// there, and seq_scan for which).
 #include "common.cuh"
 
 namespace ft {
@@ -1272,8 +1272,8 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) ssd_seq_kernel(S
   seq_store_state<NPL, CPL>(st, N, P, col, l, a.vec, S);
 }
 
-// A few segments of a long prompt leave most SMs without a block when a warp owns 8 columns:
-// then a warp owns 2 and four times as many blocks share the work.
+// Few columns in all (single tokens of a few requests, short portions) leave most SMs without a block when a warp owns
+// 8 of them: then a warp owns 2 and four times as many blocks share the work.
 #ifndef NARROW_WC
 #define NARROW_WC 2
 #endif
@@ -1351,14 +1351,41 @@ static int launch_ssd_seq(const SsdArgs& a, int S, cudaStream_t stream) {
   return FT_ERR_DTYPE;
 }
 
-// T tokens in S segments: one token each (decode) is bound by the states' traffic, which the kernels with 32
-// lanes a column read and write in wider pieces; any segment of more takes the others.
+// Which kernels take T tokens in S segments: those with 16 lanes a column (true) or those with 32.  The former take a third
+// of the time a token of a chain and read and write states in narrower pieces, so that they pay with the tokens a state
+// stays in registers for, and with a long chain's share of the launch; `longest`: tokens of the longest segment (0: not
+// known, the mean).  All lines from both kernels' times over S = 1 .. 64 segments of 2 .. 256 tokens, even ones and a
+// long one beside single tokens, heads of 64, 128 and 256 (bfloat16, 16 heads of 128, delta rule, us with 32 and 16
+// lanes: 32 segments of 2 tokens 29 and 39, of 16 91 and 73; 31 single tokens beside 16 tokens 36 and 42, beside 128 105
+// and 71).  Up to 8,192 columns every block finds a place at once: from the first tokens on.  More: where the long
+// segment's chain outlasts the other segments' states, or all segments have several tokens.  Float32 launches take
+// two columns a lane and pay later, states of more than 128 rows one: there only long segments that nothing else
+// outweighs.
+enum ScanKind { SCAN_DELTA, SCAN_CHANNEL, SCAN_RETENTION, SCAN_SSD };
+static bool seq_scan(int kind, bool f32, int heads, int P, int D, int S, int T, int longest) {
+  if (T <= S) return false;
+  const long long head_columns = (long long)heads * P, columns = head_columns * S;
+  const long long L = longest > 0 ? longest : (T + S - 1) / S;
+  const bool light = kind == SCAN_DELTA || kind == SCAN_SSD;       // a scalar decay a head, nothing turned
+  if (D > 128) {
+    const bool alone = T <= 2 * L;
+    if (columns > 8192) return alone && L * (kind == SCAN_DELTA ? 300 : kind == SCAN_SSD ? 128 : 64) >= columns;
+    return light && L >= (kind == SCAN_SSD && columns > 4096 ? 128 : 32);
+  }
+  if (columns <= 8192) return L >= 4 || (columns > 4096 && (light || !f32));
+  constexpr int chain[2][4] = {{1600, 1600, 1600, 1600}, {1024, 700, 800, 512}};       // columns a chain's token stands for
+  constexpr int tokens[2][4] = {{8, 8, 8, 12}, {28, 42, 16, 90}};                       // mean tokens more than one
+  // float32 work gains little a token: there the others' tokens count against the chain
+  const long long beside = f32 ? head_columns * (S + T - L) / 2 : columns;
+  return L * chain[f32][kind] >= beside || T - S >= (long long)tokens[f32][kind] * S;
+}
+
 template <int MODE>
-static int dispatch_delta(DeltaArgs a, int S, int T, int dtype, cudaStream_t stream) {
+static int dispatch_delta(DeltaArgs a, int S, int T, int longest, int dtype, cudaStream_t stream) {
   int rc = FT_OK;
   const int D = a.D;
   const bool narrow = narrow_warps(a.P, a.heads, S);
-  if (T > S) {
+  if (seq_scan(MODE, dtype == FT_DTYPE_F32, a.heads, a.P, D, S, T, longest)) {         // the modes are the first three kinds
     FT_DISPATCH(dtype, AT, {
       if (D <= 32) rc = launch_delta_seq<AT, 1, MODE>(a, S, stream);
       else if (D <= 64) rc = launch_delta_seq<AT, 2, MODE>(a, S, stream);
@@ -1396,6 +1423,9 @@ using namespace ft;
 
 extern "C" {
 
+int ft_scan_several(int kind, int f32, int heads, int P, int D, int S, int T, int longest) {
+  return seq_scan(kind, f32 != 0, heads, P, D, S, T, longest);
+}
 int ft_conv_groups(int C, int T, int S, int taps, int pairs) { return conv_groups(C, T, S, taps, pairs != 0); }
 
 // Both kernels of the short convolution: outputs first, then the slots' new contents.
@@ -1446,13 +1476,13 @@ int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const f
 int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, const float* dt_bias,
                 const float* A_log, const float* D, float* state, long long slot_stride, float* y,
                 const int* seg_slot, const int* seg_q_start, int heads, int P, int N, int G, int S,
-                int T, int dtype, cudaStream_t stream) {
+                int T, int longest, int dtype, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || N <= 0 || N > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   SsdArgs a{xbc, dt, dt_bias, A_log, D, state, y, seg_slot, seg_q_start, ld, ld_dt, slot_stride, heads, P, N, G, 0};
   int rc = FT_OK;
   const bool narrow = narrow_warps(P, heads, S);
-  if (T > S) {                                          // see dispatch_delta
+  if (seq_scan(SCAN_SSD, dtype == FT_DTYPE_F32, heads, P, N, S, T, longest)) {
     FT_DISPATCH(dtype, AT, {
       if (N <= 32) rc = launch_ssd_seq<AT, 1>(a, S, stream);
       else if (N <= 64) rc = launch_ssd_seq<AT, 2>(a, S, stream);
@@ -1475,12 +1505,12 @@ int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, 
 int ft_delta_scan(const void* qkv, long long ld, const void* beta, const void* decay, long long ld_gate,
                   const float* dt_bias, const float* A_log, float* state, long long slot_stride, float* o,
                   const int* seg_slot, const int* seg_q_start, int heads, int P, int D, int G, float unit_eps,
-                  float q_scale, int S, int T, int dtype, cudaStream_t stream) {
+                  float q_scale, int S, int T, int longest, int dtype, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   DeltaArgs a{qkv, beta, decay, dt_bias, A_log, state, o, seg_slot, seg_q_start, ld, ld_gate, slot_stride,
               heads, P, D, G, unit_eps, q_scale, 0, nullptr, 0, nullptr, nullptr, 0};
-  return dispatch_delta<0>(a, S, T, dtype, stream);
+  return dispatch_delta<0>(a, S, T, longest, dtype, stream);
 }
 
 // The delta rule with a decay per key channel: `decay` is float32 [T, ld_decay] (channel n of head
@@ -1488,27 +1518,27 @@ int ft_delta_scan(const void* qkv, long long ld, const void* beta, const void* d
 int ft_channel_delta_scan(const void* qkv, long long ld, const void* beta, long long ld_gate, const float* decay,
                           long long ld_decay, const float* dt_bias, const float* A_log, float* state,
                           long long slot_stride, float* o, const int* seg_slot, const int* seg_q_start, int heads,
-                          int P, int D, int G, float unit_eps, float q_scale, int S, int T, int dtype,
+                          int P, int D, int G, float unit_eps, float q_scale, int S, int T, int longest, int dtype,
                           cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
   DeltaArgs a{qkv, beta, nullptr, dt_bias, A_log, state, o, seg_slot, seg_q_start, ld, ld_gate, slot_stride,
               heads, P, D, G, unit_eps, q_scale, 0, decay, ld_decay, nullptr, nullptr, 0};
-  return dispatch_delta<1>(a, S, T, dtype, stream);
+  return dispatch_delta<1>(a, S, T, longest, dtype, stream);
 }
 
 // Retention: rows of `qkv` are q (heads * D) | k (heads * D) | v (heads * P); `decay` [heads] float32 holds
 // each head's constant factor; cos_sin [positions, rot_dims] (rot_dims 0: nothing turns).
 int ft_retention_scan(const void* qkv, long long ld, const float* decay, const float* cos_sin, int rot_dims,
                       const int* seg_pos0, float* state, long long slot_stride, float* o, const int* seg_slot,
-                      const int* seg_q_start, int heads, int P, int D, float k_scale, int S, int T, int dtype,
+                      const int* seg_q_start, int heads, int P, int D, float k_scale, int S, int T, int longest, int dtype,
                       cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || rot_dims < 0 || (rot_dims & 1) || rot_dims > D)
     return FT_ERR_SHAPE;
   DeltaArgs a{qkv, nullptr, nullptr, decay, nullptr, state, o, seg_slot, seg_q_start, ld, 0, slot_stride,
               heads, P, D, heads, 0.f, k_scale, 0, nullptr, 0, cos_sin, seg_pos0, cos_sin ? rot_dims : 0};
-  return dispatch_delta<2>(a, S, T, dtype, stream);
+  return dispatch_delta<2>(a, S, T, longest, dtype, stream);
 }
 
 }  // extern "C"

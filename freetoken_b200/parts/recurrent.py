@@ -122,7 +122,7 @@ class SelectiveStateSpace(_Recurrent):
                       ctx.seg_slot, ctx.seg_q_start)
         y = ws.get("ssd.y", (T, inner), torch.float32)
         ops.ssd_scan(xbc, proj[:, inner + C:], w["dt_bias"], w["a_log"], w["d"], state, y, ctx.seg_slot,
-                     ctx.seg_q_start, self.heads, self.P, self.N, self.G)
+                     ctx.seg_q_start, self.heads, self.P, self.N, self.G, ctx.max_q_len)
         gated = ws.get("ssd.gated", (T, inner), ctx.dtype)
         ops.gated_norm(y, proj[:, :inner], w["norm"], gated, self.norm_groups, self.eps, gate_first=True)
         if out is None:
@@ -191,7 +191,7 @@ class GatedDelta(_Recurrent):
         gates = C + inner
         ops.delta_scan(qkv, proj[:, gates:gates + heads], proj[:, gates + heads:], w["dt_bias"], w["a_log"],
                        state, o, ctx.seg_slot, ctx.seg_q_start, heads, self.G, self.D, self.P, self.unit_eps,
-                       self.D ** -0.5)
+                       self.D ** -0.5, ctx.max_q_len)
         gated = ws.get("delta.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, proj[:, C:C + inner], w["norm"], gated, heads, self.eps, gate_first=False)
         if out is None:
@@ -270,7 +270,8 @@ class ChannelDelta(_Recurrent):
         gate = linear.linear(proj[:, C + low:C + both], w["gate_up"], ws.get("cdelta.gate", (T, inner), ctx.dtype))
         o = ws.get("cdelta.o", (T, inner), torch.float32)
         ops.channel_delta_scan(qkv, proj[:, C + both:], decay, w["dt_bias"], w["a_log"], state, o, ctx.seg_slot,
-                               ctx.seg_q_start, heads, self.G, self.D, self.P, self.unit_eps, self.D ** -0.5)
+                               ctx.seg_q_start, heads, self.G, self.D, self.P, self.unit_eps, self.D ** -0.5,
+                               ctx.max_q_len)
         gated = ws.get("cdelta.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, gate, w["norm"], gated, heads, self.eps, gate_first=False, gate_kind="sigmoid")
         if out is None:
@@ -338,7 +339,7 @@ class Retention(_Recurrent):
         o = ws.get("retention.o", (T, inner), torch.float32)
         ops.retention_scan(proj[:, :2 * kd + inner], self.decay, self.position.table(ctx.device, ctx.max_positions),
                            ctx.seg_pos0, state, o, ctx.seg_slot, ctx.seg_q_start, self.heads, self.D, self.P,
-                           self.D ** -0.5)
+                           self.D ** -0.5, ctx.max_q_len)
         gated = ws.get("retention.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, proj[:, 2 * kd + inner:], self.ones, gated, self.heads, self.eps, gate_first=False)
         if out is None:

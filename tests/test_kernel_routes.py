@@ -23,3 +23,21 @@ def test_tokens_that_share_an_attention_block(T, S, rest, fit, known, tokens):
     (6144, 4096, 1, 3, 1, 1), (1024, 4096, 1, 4, 0, 1), (2304, 2048, 1, 3, 0, 4), (2304, 2048, 64, 3, 0, 1)])
 def test_runs_of_a_long_convolution(C, T, S, taps, pairs, groups):
     assert build.load("recurrent").ft_conv_groups(C, T, S, taps, pairs) == groups
+
+
+DELTA, CHANNEL, RETENTION, SSD = range(4)
+
+
+# kind, float32, heads, value size, key size, segments, tokens, longest (0: not known): sixteen lanes a column or not
+@pytest.mark.parametrize("kind,f32,H,P,D,S,T,longest,several", [
+    (DELTA, 0, 16, 128, 128, 32, 32, 1, 0), (DELTA, 0, 16, 128, 128, 32, 33, 2, 0),    # single tokens, one of two
+    (DELTA, 0, 16, 128, 128, 1, 2048, 2048, 1), (DELTA, 0, 16, 128, 128, 4, 12, 3, 1), (CHANNEL, 0, 4, 64, 64, 1, 2, 2, 0),
+    (DELTA, 0, 16, 128, 128, 32, 64, 2, 0), (DELTA, 0, 16, 128, 128, 32, 512, 16, 1),  # a full chip, even segments
+    (DELTA, 0, 16, 128, 128, 64, 263, 200, 1), (DELTA, 0, 16, 128, 128, 64, 263, 0, 0),       # a long one beside single tokens
+    (DELTA, 1, 16, 128, 128, 32, 512, 16, 0), (DELTA, 1, 16, 128, 128, 32, 1024, 32, 1),      # two columns a lane
+    (SSD, 1, 32, 64, 128, 32, 1024, 32, 0), (RETENTION, 1, 16, 128, 128, 32, 1024, 32, 1),
+    (DELTA, 0, 8, 256, 256, 1, 16, 16, 0), (DELTA, 0, 8, 256, 256, 1, 512, 512, 1),    # one column a lane
+    (DELTA, 0, 8, 256, 256, 32, 512, 16, 0), (CHANNEL, 0, 8, 256, 256, 4, 4096, 1335, 0), (RETENTION, 0, 8, 256, 256, 8, 307, 300, 1),
+    (SSD, 0, 8, 256, 256, 8, 135, 128, 1), (SSD, 0, 8, 256, 256, 32, 159, 128, 0)])
+def test_lanes_of_a_scan(kind, f32, H, P, D, S, T, longest, several):
+    assert build.load("recurrent").ft_scan_several(kind, f32, H, P, D, S, T, longest) == several

@@ -266,3 +266,37 @@ def test_delta_rule_repeats_itself(dtype, per_channel, H, P, D, lens):
                                                ("bfloat16", 512, 4, [7, 1022])])
 def test_long_convolutions_of_several_runs(dtype, C, taps, lens):
     test_long_convolutions_agree_bitwise(dtype, C, taps, lens)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("kind", ["delta", "channel_delta", "retention", "ssd"])
+@pytest.mark.parametrize("H,P,D,lens", [(2, 130, 200, [12, 5]), (1, 7, 129, [8]), (2, 8, 256, [10]), (16, 66, 256, [9, 3] * 5),
+                                        (40, 64, 64, [3, 1] * 8)])
+def test_scans_agree_whichever_lanes_they_take(dtype, kind, H, P, D, lens):
+    """The same launch told that its longest segment has one token, and so many that it is worth a chain."""
+    T, dt, o = sum(lens), DT[dtype], ops()
+    slot, starts = _segments(lens)
+    a_log, bias = rnd(H, seed=3, scale=0.5) - 1, rnd(H, seed=4, scale=0.5) - 1
+    gates, first = rnd(T, 2 * H, dtype=dt, seed=2), rnd(len(lens) + 2, H * D * P, seed=5, scale=0.1)
+    results, kinds = [], ["delta", "channel_delta", "retention", "ssd"]
+    for longest in (1, 1 << 20):
+        state, y = first.clone(), torch.full((T, H * P), float("nan"), device=DEV)
+        if kind == "ssd":
+            o.ssd_scan(rnd(T, H * P + 2 * D, dtype=dt, seed=1), gates[:, :H], bias, a_log, rnd(H, seed=6), state, y, slot, starts, H, P,
+                       D, 1, longest)
+        elif kind == "retention":
+            o.retention_scan(rnd(T, 2 * H * D + H * P, dtype=dt, seed=1), torch.linspace(0.9, 0.999, H, device=DEV), rnd(64, 2 * (D // 4),
+                             seed=7), torch.arange(len(lens), dtype=torch.int32, device=DEV), state, y, slot, starts, H, D, P, D ** -0.5,
+                             longest)
+        elif kind == "delta":
+            o.delta_scan(rnd(T, 2 * H * D + H * P, dtype=dt, seed=1), gates[:, :H], gates[:, H:], bias, a_log, state, y, slot, starts, H,
+                         H, D, P, 1e-6, D ** -0.5, longest)
+        else:
+            o.channel_delta_scan(rnd(T, 2 * H * D + H * P, dtype=dt, seed=1), gates[:, :H], rnd(T, H * D, seed=8), rnd(H * D, seed=9) - 1,
+                                 a_log, state, y, slot, starts, H, H, D, P, 1e-6, D ** -0.5, longest)
+        results.append((state, y))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    from freetoken_b200.csrc import build
+    worth = D <= 128 or H * P * len(lens) > 8192 or kind in ("delta", "ssd")       # others of more than 128 rows stay
+    for longest, took in ((1, False), (1 << 20, worth)):
+        assert took == build.load("recurrent").ft_scan_several(kinds.index(kind), dtype == "float32", H, P, D, len(lens), T, longest)
