@@ -6,9 +6,9 @@
 // row's result does not depend on how many rows the launch holds, on the tile
 // shape chosen, or on which expert group the row fell into.
 //
-// Three kernels share that arithmetic: gemm_stream_kernel (few rows: the weights are
-// streamed once), gemm_tile_kernel (many rows: register tiles) and gemm_rows_kernel (any
-// size and alignment).  launch() says which takes what.
+// Four kernels share that arithmetic: gemm_stream_kernel (few rows: the weights are
+// streamed once), gemm_tile_kernel (many rows: register tiles), gemm_dense_kernel (between
+// the two) and gemm_rows_kernel (any size and alignment).  gemm_route() says which takes what.
 //
 // Grouped use (routed experts; reference python/freetoken/moe/fused.py:267-337,
 // python/freetoken/kernel/triton/fused_moe.py:156-302): rows are sorted by
@@ -249,11 +249,14 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
   const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
   const WT* W = (const WT*)a.W + (size_t)group * a.w_group_stride + (size_t)blockIdx.z * a.w_batch_stride;
 
-  auto fetch = [&](int stage, int k0) {        // rows and columns beyond the last repeat it; k stops at K
+  // Rows beyond the last repeat it; columns beyond the last repeat the first ones, spread out (hundreds of blocks that
+  // all fetched one row of eight 25 times stood in each other's way: 4,096 rows of 8 columns, K = 512, 34 us); k stops at K.
+  const int here = min(a.N - n0, STREAM_COLS), spread = (1 << (31 - __clz(here))) - 1;
+  auto fetch = [&](int stage, int k0) {
     unsigned char* to = stream_sm + stage * STAGE;
     for (int i = threadIdx.x; i < WROWS * WPIECES; i += THREADS) {
-      const int n = i / WPIECES, piece = i % WPIECES, k = k0 + piece * (16 / (int)sizeof(WT));
-      const int col = min(n0 + n % STREAM_COLS, a.N - 1) + (n / STREAM_COLS) * a.N;
+      const int n = i / WPIECES, piece = i % WPIECES, k = k0 + piece * (16 / (int)sizeof(WT)), c = n % STREAM_COLS;
+      const int col = n0 + (c < here ? c : c & spread) + (n / STREAM_COLS) * a.N;
       if (k < a.K) cp_async16(to + n * WROW + piece * 16, W + (size_t)col * a.K + k);
     }
     to += WROWS * WROW;
@@ -431,6 +434,68 @@ __global__ void __launch_bounds__(128) gemm_tile_kernel(GemmArgs a) {
   }
 }
 
+// Dense products whose tiles of 64 x 64 find an SM each: twice as many blocks as above, twice as many threads; 16-byte
+// global loads, k-major shared tiles, 128-bit shared loads, the next tile on its way meanwhile.  K % 32 == 0.
+template <typename AT, typename WT, typename OT>
+__global__ void __launch_bounds__(256) gemm_dense_kernel(GemmArgs a) {
+  constexpr int TBM = 64, TBN = 64, TBK = 32;
+  __shared__ __align__(16) float As[TBK][TBM + 4];
+  __shared__ __align__(16) float Ws[TBK][TBN + 4];
+  pdl_wait();
+  const int row0 = blockIdx.x * TBM, n0 = blockIdx.y * TBN;
+  const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
+  const WT* W = (const WT*)a.W + (size_t)blockIdx.z * a.w_batch_stride;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 8;      // this thread loads row lr, k lk..lk+7
+  const bool a_ok = row0 + lr < a.M, w_ok = n0 + lr < a.N;
+  const AT* ap = A + (size_t)(a_ok ? row0 + lr : 0) * a.lda + lk;
+  const WT* wp = W + (size_t)(w_ok ? n0 + lr : 0) * a.K + lk;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  float av[8], wv[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) av[i] = wv[i] = 0.f;
+  if (a_ok) load8(ap, av);
+  if (w_ok) load8(wp, wv);
+  for (int k0 = 0; k0 < a.K; k0 += TBK) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      As[lk + i][lr] = av[i];
+      Ws[lk + i][lr] = wv[i];
+    }
+    __syncthreads();
+    if (k0 + TBK < a.K) {            // next tile's loads fly while this one is multiplied
+      if (a_ok) load8(ap + k0 + TBK, av);
+      if (w_ok) load8(wp + k0 + TBK, wv);
+    }
+#pragma unroll
+    for (int kk = 0; kk < TBK; ++kk) {
+      const float4 a4 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
+      const float4 w4 = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
+      const float ar[4] = {a4.x, a4.y, a4.z, a4.w}, wr[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+  OT* C = (OT*)a.C + (size_t)blockIdx.z * a.c_batch_stride;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = row0 + ty * 4 + i;
+    if (r >= a.M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + tx * 4 + j;
+      if (n < a.N) C[(size_t)r * a.ldc + n] = from_float<OT>(acc[i][j]);
+    }
+  }
+}
+
 template <typename AT, typename WT, typename OT, int MR, bool GLU>
 int launch_stream(const GemmArgs& a, cudaStream_t stream) {
   constexpr size_t smem = stream_smem<AT, WT, MR, GLU>();
@@ -445,6 +510,42 @@ int launch_stream(const GemmArgs& a, cudaStream_t stream) {
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
+// Which kernel takes a product of M rows (`grouped`: M over G groups), N columns and K, `batch` of them.  Dense ones go
+// to the least estimate of time: rounds of blocks on 148 SMs times what a round took per k (0.1 ns; measured over M = 64 ..
+// 4,096, N = 8 .. 3,072, K = 64 .. 2,048: the choice is 0.6 % behind the best of the four on average).  gemm_stream_kernel
+// reads the weights again for every 16 rows and wins while few blocks share an SM (64 rows, K = N = 2,048: 36 us, tiles of
+// 64 x 64 93); gemm_dense_kernel's tiles give twice as many blocks as gemm_tile_kernel's and win where those fit one round
+// (2,048 x 256, K = 512: 26 us, 34 and 32), gemm_tile_kernel beyond (1,024 x 4,096, K = 2,048: 427 us); gemm_rows_kernel takes
+// many tiles of a K that is no multiple of 16 (2,048 x 4,096, K = 1,000: 694 us, streamed 846).
+enum GemmRoute { GEMM_STREAM, GEMM_TILE, GEMM_DENSE, GEMM_ROWS };
+static int gemm_route(int M, int N, int K, int G, int batch, bool grouped, bool glu, bool plain, bool bf16_rows,
+                      bool f32_weights) {
+  const int half = glu ? 64 : 128;
+  const long long wide = (N + half - 1) / half;
+  if (M / G < 32) return GEMM_STREAM;
+  // Groups take register tiles from 32 rows each on, where those give half of the SMs a block.
+  if (grouped && !(K & 15)) return (M + 63) / 64 * wide >= 64 ? GEMM_TILE : GEMM_STREAM;
+  const auto rounds = [](long long blocks) { return (blocks + 147) / 148; };
+  const int part = grouped ? G : 0;
+  const long long m64 = ((M + 63) / 64 + part) * (long long)batch, narrow = rounds(m64 * ((N + 63) / 64));
+  long long best = (f32_weights ? 108 : bf16_rows ? 100 : 85) * (glu ? 2 : 1) *
+                   rounds(((M + 15) / 16 + part) * (long long)batch * ((N + STREAM_COLS - 1) / STREAM_COLS)) * (K + 128);
+  int route = GEMM_STREAM;
+  const auto offer = [&](int r, long long cost) {
+    if (cost < best) {
+      best = cost;
+      route = r;
+    }
+  };
+  if (K & 15) {
+    offer(GEMM_ROWS, (780 + 475 * (narrow - 1)) * (glu ? 2 : 1) * (K + 32));
+  } else {
+    offer(GEMM_TILE, (580 + 500 * (rounds(m64 * wide) - 1)) * (K + 64));
+    if (plain && M >= 64 && !(K & 31)) offer(GEMM_DENSE, (453 + 333 * (narrow - 1)) * (K + 56));
+  }
+  return route;
+}
+
 template <typename AT, typename WT, typename OT, bool GLU>
 int launch_kind(const GemmArgs& a, cudaStream_t stream) {
   const int per_group = a.group_offsets ? a.M / max(a.G, 1) : a.M;
@@ -452,15 +553,24 @@ int launch_kind(const GemmArgs& a, cudaStream_t stream) {
   const bool pieces = !(a.K & 7) && !(a.lda & a_align) && !(a.a_batch_stride & a_align) &&
                       !(a.w_batch_stride & w_align) && !(a.w_group_stride & w_align) && !((uintptr_t)a.A & 15) &&
                       !((uintptr_t)a.W & 15);
-  if (pieces) {
-    // Register tiles from 32 rows a group on, where they give half of the SMs a block; below that, and for few
-    // columns (a router's), the weights are streamed by many small blocks (342 rows of 8 columns: 24 instead of 99 us).
+  const bool plain = !GLU && !a.group_offsets && !a.a_rows && !a.c_rows && !a.row_scale;
+  const int route = pieces ? gemm_route(a.M, a.N, a.K, a.G, a.batch, a.group_offsets != nullptr, GLU, plain, sizeof(AT) == 2,
+                                        sizeof(WT) == 4)
+                           : GEMM_ROWS;
+  if (route == GEMM_TILE) {
     const int cols = (a.N + (GLU ? 63 : 127)) / (GLU ? 64 : 128);
-    if (!(a.K & 15) && per_group >= 32 && (a.M + 63) / 64 * (long long)cols * a.batch >= 64) {
-      const dim3 grid(a.group_offsets ? a.M / 64 + min(a.G, a.M) : (a.M + 63) / 64, cols, a.batch);
-      const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(128), 0, stream, a);
+    const dim3 grid(a.group_offsets ? a.M / 64 + min(a.G, a.M) : (a.M + 63) / 64, cols, a.batch);
+    const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(128), 0, stream, a);
+    return e == cudaSuccess ? FT_OK : (int)e;
+  }
+  if constexpr (!GLU) {
+    if (route == GEMM_DENSE) {
+      const cudaError_t e = launch_pdl(gemm_dense_kernel<AT, WT, OT>, dim3((a.M + 63) / 64, (a.N + 63) / 64, a.batch), dim3(256),
+                                       0, stream, a);
       return e == cudaSuccess ? FT_OK : (int)e;
     }
+  }
+  if (route == GEMM_STREAM) {
     // rows a block: about twice a group's mean, so that most busy groups are read once
     const int want = a.group_offsets ? 2 * ((a.M + a.G - 1) / a.G) : a.M;
     if (want <= 1) return launch_stream<AT, WT, OT, 1, GLU>(a, stream);
@@ -492,6 +602,10 @@ using namespace ft;
 extern "C" int ft_gemm_heads(const void* A, int a_dtype, long long lda, long long a_batch_stride, const void* W,
                              int w_dtype, long long w_batch_stride, void* C, int c_dtype, long long ldc,
                              long long c_batch_stride, int M, int N, int K, int batch, cudaStream_t stream);
+
+extern "C" int ft_gemm_route(int M, int N, int K, int G, int batch, int grouped, int glu, int plain, int bf16_rows, int f32_weights) {
+  return gemm_route(M, N, K, G, batch, grouped != 0, glu != 0, plain != 0, bf16_rows != 0, f32_weights != 0);
+}
 
 // A, W, C element types are given by code; supported triples:
 //   (f32,f32,f32) (f32,bf16,f32) (bf16,bf16,bf16) (bf16,bf16,f32) (bf16,f32,f32)

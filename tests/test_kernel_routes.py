@@ -41,3 +41,21 @@ DELTA, CHANNEL, RETENTION, SSD = range(4)
     (SSD, 0, 8, 256, 256, 8, 135, 128, 1), (SSD, 0, 8, 256, 256, 32, 159, 128, 0)])
 def test_lanes_of_a_scan(kind, f32, H, P, D, S, T, longest, several):
     assert build.load("recurrent").ft_scan_several(kind, f32, H, P, D, S, T, longest) == several
+
+
+STREAM, TILE, DENSE, ROWS = range(4)
+
+
+# rows, columns, K, groups, batch, grouped, gated, plain, bfloat16 rows, float32 weights
+@pytest.mark.parametrize("M,N,K,G,batch,grouped,glu,plain,b16,w32,route", [
+    (1, 4096, 2048, 1, 1, 0, 0, 1, 0, 0, STREAM), (64, 2048, 2048, 1, 1, 0, 0, 1, 0, 0, STREAM),
+    (4096, 32, 512, 1, 1, 0, 0, 1, 0, 0, STREAM), (342, 8, 2048, 1, 1, 0, 0, 1, 0, 0, STREAM),
+    (1024, 4096, 2048, 1, 1, 0, 0, 1, 0, 0, TILE), (342, 3072, 2048, 1, 1, 0, 0, 1, 0, 0, TILE),
+    (2048, 256, 512, 1, 1, 0, 0, 1, 0, 0, DENSE), (64, 512, 128, 1, 16, 0, 0, 1, 0, 0, DENSE),
+    (700, 512, 1024, 1, 1, 0, 0, 1, 0, 1, DENSE), (2048, 256, 512, 1, 1, 0, 0, 0, 0, 0, TILE),
+    (2048, 4096, 1000, 1, 1, 0, 0, 1, 0, 0, ROWS), (512, 2048, 2056, 1, 1, 0, 0, 1, 0, 1, ROWS),
+    (64, 1024, 1000, 1, 1, 0, 0, 1, 0, 0, STREAM),
+    (2000, 1024, 2048, 8, 1, 1, 1, 0, 0, 0, TILE), (2000, 1024, 1000, 8, 1, 1, 1, 0, 0, 1, ROWS),
+    (8, 512, 1024, 64, 1, 1, 1, 0, 0, 0, STREAM)])
+def test_kernel_of_a_float32_product(M, N, K, G, batch, grouped, glu, plain, b16, w32, route):
+    assert build.load("gemm_simt").ft_gemm_route(M, N, K, G, batch, grouped, glu, plain, b16, w32) == route

@@ -61,3 +61,23 @@ def test_attention_rows_do_not_depend_on_their_block(dtype, nq, nkv, d, window):
         one = torch.zeros_like(q)
         ops().attn_paged_simt(q, one, *args, rows=torch.tensor([t], dtype=torch.int32, device=DEV))
         assert torch.equal(one[t], out[t]), t
+
+
+STREAM, TILE, DENSE, ROWS = range(4)
+
+
+# each kernel at its edges: tiles of 64 x 64 that end inside rows and columns, one and several of K's tiles; fewer
+# columns than a block's, of every number of them that repeats differently; K in pieces of 8 with many tiles
+@pytest.mark.parametrize("at,wt,ct", GEMM_TYPES)
+@pytest.mark.parametrize("M,N,K,route", [
+    (64, 3000, 32, DENSE), (65, 3009, 64, DENSE), (2000, 200, 96, DENSE), (2048, 256, 512, DENSE),
+    (40, 1, 64, STREAM), (33, 3, 136, STREAM), (50, 20, 64, STREAM), (9, 31, 264, STREAM), (70, 33, 64, STREAM),
+    (1000, 2000, 104, ROWS), (515, 4100, 1000, ROWS), (2048, 1024, 48, TILE)])
+def test_dense_products_by_kernel_agree_bitwise(at, wt, ct, M, N, K, route):
+    from freetoken_b200.csrc import build
+    assert build.load("gemm_simt").ft_gemm_route(M, N, K, 1, 1, 0, 0, 1, int(at == "bfloat16"), int(wt == "float32")) == route
+    a, w = rnd(M, K, dtype=DT[at], seed=1), rnd(N, K, dtype=DT[wt], seed=2, scale=0.1)
+    got, want = (torch.full((M, N), float("nan"), dtype=DT[ct], device=DEV) for _ in range(2))
+    ops().gemm_rows(a, w, got)
+    ops().gemm_rows(_misaligned(a), w, want)
+    assert torch.equal(got, want)
