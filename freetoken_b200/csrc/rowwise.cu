@@ -343,7 +343,7 @@ __device__ __forceinline__ float4 branch_at4(const BranchArgs& b, int t, int H, 
   float eg = 1.f;
   if (b.extra) {
     e = load4f((const AT*)b.extra + (size_t)t * H + 4 * gi);
-    if (b.extra && b.extra_gate) eg = b.extra_gate[t];
+    if (b.extra_gate) eg = b.extra_gate[t];
   }
   if (b.beside) {
     const AT* other = (const AT*)b.beside + (size_t)t * b.kb * H + 4 * gi;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(THREADS) join_layer_norm_kernel(JoinNormArgs a
       }
     }
     const unsigned slots = a.b.rows ? branch_slots(a.b, t, back) : 0u;
-    constexpr bool ALL = EAGER && KEEP <= 2;       // more do not fit the registers of 512 threads
+    constexpr bool ALL = EAGER && KEEP == 2;       // one piece a thread gains nothing, four do not fit the registers
     float4 zs[ALL ? KEEP : 1];
     if constexpr (ALL) {
 #pragma unroll
@@ -1022,11 +1022,20 @@ hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch
   }
 }
 
+// Whether rows of few tokens take the form that fetches early: with up to four partial rows always; with more, whose
+// rounds of two or four wait for each other, where it still won (eight partial rows, us without and with: float32, 4 x 2,048
+// values 4.7 and 3.8; bfloat16 4.7 and 4.3, 2 x 3,000 4.4 and 5.5, 2 x 6,144 6.9 and 5.9; float32, 4 x 6,144 7.6 and 8.1).
+static bool hyper_fetches_early(bool f32, int S, int H, int k) {
+  if (k <= 4) return true;
+  return f32 ? S < 4 || H <= 4096 : (H > 1024 && H <= 2048) || H > 4096;
+}
+
 template <typename AT, int S, int KEEP>
 static cudaError_t launch_hyper_keep(cudaStream_t stream, int T, int H, float* streams, const AT* branch, int k,
                                      const float* mix, const float* out_w, const float* read, const float* weight,
                                      const float* bias, float eps, int center, AT* normed) {
-  return T <= 64 ? launch_pdl(hyper_norm_vec_kernel<AT, S, KEEP, true>, dim3(T), dim3(256), 0, stream, streams, branch, k,
+  const bool eager = T <= 64 && hyper_fetches_early(sizeof(AT) == 4, S, H, k);
+  return eager   ? launch_pdl(hyper_norm_vec_kernel<AT, S, KEEP, true>, dim3(T), dim3(256), 0, stream, streams, branch, k,
                               mix, out_w, read, weight, bias, eps, center, normed, H)
                  : launch_pdl(hyper_norm_vec_kernel<AT, S, KEEP, false>, dim3(T), dim3(256), 0, stream, streams, branch, k,
                               mix, out_w, read, weight, bias, eps, center, normed, H);
@@ -1346,6 +1355,14 @@ static bool branch_aligned(const BranchArgs& b) {
   return !((uintptr_t)b.rows & 15) && !((uintptr_t)b.source & 15) && !((uintptr_t)b.extra & 15) && !((uintptr_t)b.beside & 15);
 }
 
+// Whether rows of few tokens take the form that fetches all of a thread's pieces at once (branch_all).  In bfloat16 only
+// where one round takes all the partial rows: behind it the rounds wait for each other, which branch_at4's, a piece
+// each, do not (4,096 values, us: one partial row 4.6 -> 3.8, three 4.6 -> 5.1, eight 5.9 -> 7.4; float32, eight: 5.7 -> 4.6).
+static bool norm_add_fetches_early(bool f32, int H, int k) { return f32 || k <= (H <= 2048 ? 4 : 2); }
+
+int ft_hyper_fetches_early(int f32, int S, int H, int k) { return hyper_fetches_early(f32 != 0, S, H, k); }
+int ft_norm_add_fetches_early(int f32, int H, int k) { return norm_add_fetches_early(f32 != 0, H, k); }
+
 int ft_norm_add(const BranchArgs* branch, const float* weight, int plus_one, float eps, float mult, float* residual, const float* next_weight, int next_plus_one, float next_eps,
                 void* next_out, void* copy_out, long long copy_ld, int T, int H, int dtype, cudaStream_t stream) {
   if (T <= 0) return FT_OK;
@@ -1362,7 +1379,7 @@ int ft_norm_add(const BranchArgs* branch, const float* weight, int plus_one, flo
                    !((uintptr_t)copy_out & 15) && !(copy_ld & 3);
   if (vec && a.b.k <= 32) {
     const dim3 g(T), th(256);
-    const bool few = T <= 64;
+    const bool few = T <= 64 && norm_add_fetches_early(dtype == FT_DTYPE_F32, H, a.b.k);
     if (few && H <= 1024) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 1, true>, g, th, 0, stream, a))); }
     else if (few && H <= 2048) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 2, true>, g, th, 0, stream, a))); }
     else if (few && H <= 4096) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 4, true>, g, th, 0, stream, a))); }

@@ -59,3 +59,16 @@ STREAM, TILE, DENSE, ROWS = range(4)
     (8, 512, 1024, 64, 1, 1, 1, 0, 0, 0, STREAM)])
 def test_kernel_of_a_float32_product(M, N, K, G, batch, grouped, glu, plain, b16, w32, route):
     assert build.load("gemm_simt").ft_gemm_route(M, N, K, G, batch, grouped, glu, plain, b16, w32) == route
+
+
+# float32, width, partial rows
+@pytest.mark.parametrize("f32,H,k,early", [(0, 2048, 4, 1), (0, 2048, 5, 0), (0, 4096, 1, 1), (0, 4096, 2, 1), (0, 4096, 3, 0),
+                                           (1, 4096, 8, 1), (0, 512, 8, 0)])
+def test_early_fetches_of_an_output_norm(f32, H, k, early):
+    assert build.load("rowwise").ft_norm_add_fetches_early(f32, H, k) == early
+
+
+@pytest.mark.parametrize("f32,S,H,k,early", [(0, 4, 4096, 4, 1), (0, 2, 3000, 8, 0), (0, 4, 512, 8, 0), (0, 4, 2048, 8, 1),
+                                             (0, 2, 8192, 8, 1), (1, 4, 6144, 8, 0), (1, 4, 4096, 8, 1), (1, 2, 8192, 8, 1)])
+def test_early_fetches_of_a_stream_norm(f32, S, H, k, early):
+    assert build.load("rowwise").ft_hyper_fetches_early(f32, S, H, k) == early
