@@ -220,17 +220,23 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
   }
 }
 
-// Eight chunks a round where a warp has more than four (a dense matrix, 8 tokens a pass): half the rounds, each of
-// which lasts a load's latency.  A four-layer decode of width 2,048, before and now: 16 tokens behind a prompt of 2,048
-// (Tonapel) 6.88 -> 6.63 ms, eight requests (Besuzen) 12.77 -> 12.5; Dizatar, width 4,096, 21.83 -> 21.58; one MiniMax-M3
-// request 11.54 -> 11.42.  Two warps a block (the head, an expert's down projection) gain nothing from it, nor does
-// the gated pair, whose four chunks are as many loads.
+// Eight chunks a round (8 tokens a pass, not gated) or four.  Eight are half the rounds, each of which lasts a load's
+// latency, but take 128 registers instead of 72.  Where all blocks then still find a place at once (16 / ks an SM) they won
+// at every size (dense 6,144 x 4,096 0.84 of the time, one expert of 2,048 x 2,688 0.72); where they only do with four
+// chunks (28 / ks, three at ks = 8) they lost (12,288 x 4,096 1.15, five experts of 2,048 x 2,304 1.20); beyond that they
+// won again (20,480 x 3,072 0.86).  Of experts the launch knows only the most that can be busy: there from rows on that
+// are long enough for the rounds to win by themselves (sixteen of 2,048 x 2,304 1.11, of 4,096 x 4,736 0.95).
+static bool eight_chunks(long long blocks, int ks, int K, bool experts) {
+  const int per = ((K + 31) / 32 + ks - 1) / ks;
+  if (per <= 4) return false;
+  if (blocks <= 148 * (16 / ks)) return true;
+  return experts ? per >= 21 && blocks > 1300 : blocks > 148 * (ks == 8 ? 3 : 28 / ks);
+}
 template <int NT, bool GLU, typename OT, int KS>
 void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream) {
   constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);
   if constexpr (NT == 1 && !GLU && KS >= 4) {
-    const int per = ((a.K + 31) / 32 + KS - 1) / KS;
-    if (per > 4) {
+    if (eight_chunks((long long)grid.x * grid.y, KS, a.K, a.group_offsets != nullptr)) {
       launch_pdl(skinny_kernel<NT, GLU, OT, KS, 8>, grid, dim3(KS * 32), 0, stream, a);
       return;
     }
@@ -267,6 +273,10 @@ static int dense_k_split(int N, int K) {
 }  // namespace ft
 
 using namespace ft;
+
+extern "C" int ft_skinny_eight_chunks(long long blocks, int ks, int K, int experts) {
+  return eight_chunks(blocks, ks, K, experts != 0);
+}
 
 // A, W bfloat16; C bfloat16 or float32.  `rows_per_pass` in {8,16,32} picks
 // how many tokens share one pass over the weights.  Needs K % 8 == 0,

@@ -72,3 +72,12 @@ def test_early_fetches_of_an_output_norm(f32, H, k, early):
                                              (0, 2, 8192, 8, 1), (1, 4, 6144, 8, 0), (1, 4, 4096, 8, 1), (1, 2, 8192, 8, 1)])
 def test_early_fetches_of_a_stream_norm(f32, S, H, k, early):
     assert build.load("rowwise").ft_hyper_fetches_early(f32, S, H, k) == early
+
+
+# blocks, warps a block, K, experts
+@pytest.mark.parametrize("blocks,ks,K,experts,eight", [
+    (384, 4, 4096, 0, 1), (592, 4, 4096, 0, 1), (593, 4, 4096, 0, 0), (1036, 4, 4096, 0, 0), (1037, 4, 4096, 0, 1),
+    (296, 8, 4096, 0, 1), (297, 8, 4096, 0, 0), (445, 8, 4096, 0, 1), (128, 4, 512, 0, 0),
+    (512, 4, 2304, 1, 1), (640, 4, 2304, 1, 0), (4096, 4, 2304, 1, 0), (4096, 4, 2688, 1, 1), (1024, 4, 4736, 1, 0)])
+def test_chunks_a_round_of_a_weight_streaming_product(blocks, ks, K, experts, eight):
+    assert build.load("skinny_gemm").ft_skinny_eight_chunks(blocks, ks, K, experts) == eight

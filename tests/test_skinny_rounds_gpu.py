@@ -22,3 +22,19 @@ def test_eight_chunks_a_round(ct, M, N, K):
     assert torch.equal(c, two)                   # the same products in the same order
     want = a.float() @ w.float().t()
     assert torch.allclose(c.float(), want, atol=TOL[ct]["atol"] * 3, rtol=TOL[ct]["rtol"])
+
+
+# experts of rows longer than 2,048 values: groups without a row, of one, of more than a pass
+@pytest.mark.parametrize("ct", ["bfloat16", "float32"])
+@pytest.mark.parametrize("rows,N,K", [([1, 0, 2], 40, 2056), ([9, 1, 0, 3], 33, 2688), ([0, 8], 100, 4736), ([3] * 6, 1600, 2312)])
+def test_eight_chunks_a_round_of_experts(ct, rows, N, K):
+    o, E, M = ops(), len(rows), sum(rows)
+    a = rnd(M, K, dtype=torch.bfloat16, seed=1)
+    w = rnd(E, N, K, dtype=torch.bfloat16, seed=2, scale=0.1)
+    offsets = torch.tensor([sum(rows[:i]) for i in range(E + 1)], dtype=torch.int32, device=DEV)
+    c, two = (torch.empty(M, N, dtype=DT[ct], device=DEV) for _ in range(2))
+    o.skinny_gemm(a, w, c, group_offsets=offsets, rows_per_pass=8)
+    o.skinny_gemm(a, w, two, group_offsets=offsets, rows_per_pass=16)
+    assert torch.equal(c, two)
+    want = torch.cat([a[offsets[e]:offsets[e + 1]].float() @ w[e].float().t() for e in range(E)])
+    assert torch.allclose(c.float(), want, atol=TOL[ct]["atol"] * 3, rtol=TOL[ct]["rtol"])
