@@ -170,12 +170,13 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T) {
       if constexpr (CPT == 2) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(out[0], out[1]);
       else o[0] = from_float<AT>(out[0]);
     }
-    if constexpr (GROUPS == 1) break;
+    if constexpr (GROUPS > 1) {
 #pragma unroll
-    for (int i = 0; i < RUN; ++i) {
-      segs[i] = next_segs[i];
+      for (int i = 0; i < RUN; ++i) {
+        segs[i] = next_segs[i];
 #pragma unroll
-      for (int u = 0; u < CPT; ++u) own[i][u] = next[i][u];
+        for (int u = 0; u < CPT; ++u) own[i][u] = next[i][u];
+      }
     }
   }
 }
