@@ -62,7 +62,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
             ops.skinny_gemm(x, weight, out, rows_per_pass=ops.pass_rows(rows))
             return out
         if out.dtype == torch.bfloat16:
-            torch.mm(x, weight.t(), out=out)
+            if x.dim() == 2:
+                torch.mm(x, weight.t(), out=out)        # what matmul would call, without its look at the shapes
+            else:
+                torch.matmul(x, weight.t(), out=out)
             return out
         if out.dtype == torch.float32 and library_f32_out(x, weight, out):
             return out
