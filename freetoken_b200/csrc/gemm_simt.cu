@@ -516,21 +516,27 @@ int launch_stream(const GemmArgs& a, cudaStream_t stream) {
 // reads the weights again for every 16 rows and wins while few blocks share an SM (64 rows, K = N = 2,048: 36 us, tiles of
 // 64 x 64 93); gemm_dense_kernel's tiles give twice as many blocks as gemm_tile_kernel's and win where those fit one round
 // (2,048 x 256, K = 512: 26 us, 34 and 32), gemm_tile_kernel beyond (1,024 x 4,096, K = 2,048: 427 us); gemm_rows_kernel takes
-// many tiles of a K that is no multiple of 16 (2,048 x 4,096, K = 1,000: 694 us, streamed 846).
+// many tiles of a K that is no multiple of 16 (2,048 x 4,096, K = 1,000: 694 us, streamed 846).  More columns than a grid's
+// second dimension holds blocks of 32 for are not streamed.
 enum GemmRoute { GEMM_STREAM, GEMM_TILE, GEMM_DENSE, GEMM_ROWS };
 static int gemm_route(int M, int N, int K, int G, int batch, bool grouped, bool glu, bool plain, bool bf16_rows,
                       bool f32_weights) {
   const int half = glu ? 64 : 128;
   const long long wide = (N + half - 1) / half;
-  if (M / G < 32) return GEMM_STREAM;
+  const bool streams = (N + STREAM_COLS - 1) / STREAM_COLS <= 65535;
+  if (M / G < 32) return streams ? GEMM_STREAM : GEMM_ROWS;
   // Groups take register tiles from 32 rows each on, where those give half of the SMs a block.
-  if (grouped && !(K & 15)) return (M + 63) / 64 * wide >= 64 ? GEMM_TILE : GEMM_STREAM;
+  if (grouped && !(K & 15)) return (M + 63) / 64 * wide >= 64 ? GEMM_TILE : GEMM_STREAM;      // many columns: tiles
   const auto rounds = [](long long blocks) { return (blocks + 147) / 148; };
   const int part = grouped ? G : 0;
   const long long m64 = ((M + 63) / 64 + part) * (long long)batch, narrow = rounds(m64 * ((N + 63) / 64));
   long long best = (f32_weights ? 108 : bf16_rows ? 100 : 85) * (glu ? 2 : 1) *
                    rounds(((M + 15) / 16 + part) * (long long)batch * ((N + STREAM_COLS - 1) / STREAM_COLS)) * (K + 128);
   int route = GEMM_STREAM;
+  if (!streams) {
+    best = LLONG_MAX;
+    route = GEMM_ROWS;
+  }
   const auto offer = [&](int r, long long cost) {
     if (cost < best) {
       best = cost;

@@ -56,7 +56,9 @@ STREAM, TILE, DENSE, ROWS = range(4)
     (2048, 4096, 1000, 1, 1, 0, 0, 1, 0, 0, ROWS), (512, 2048, 2056, 1, 1, 0, 0, 1, 0, 1, ROWS),
     (64, 1024, 1000, 1, 1, 0, 0, 1, 0, 0, STREAM),
     (2000, 1024, 2048, 8, 1, 1, 1, 0, 0, 0, TILE), (2000, 1024, 1000, 8, 1, 1, 1, 0, 0, 1, ROWS),
-    (8, 512, 1024, 64, 1, 1, 1, 0, 0, 0, STREAM)])
+    (8, 512, 1024, 64, 1, 1, 1, 0, 0, 0, STREAM),
+    (1, 65535 * 32, 8, 1, 1, 0, 0, 1, 0, 0, STREAM), (1, 65535 * 32 + 1, 8, 1, 1, 0, 0, 1, 0, 0, ROWS),     # a grid's most blocks
+    (64, 65535 * 32 + 1, 8, 1, 1, 0, 0, 1, 0, 0, ROWS), (8, 65535 * 32 + 1, 16, 8, 1, 1, 1, 0, 0, 0, ROWS)])
 def test_kernel_of_a_float32_product(M, N, K, G, batch, grouped, glu, plain, b16, w32, route):
     assert build.load("gemm_simt").ft_gemm_route(M, N, K, G, batch, grouped, glu, plain, b16, w32) == route
 

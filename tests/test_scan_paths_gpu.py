@@ -182,7 +182,7 @@ def test_long_convolutions_agree_bitwise(dtype, C, taps, lens):
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
-@pytest.mark.parametrize("S,H,k", [(4, 256, 1), (4, 2052, 2), (2, 4100, 5), (1, 1024, 8), (3, 64, 0)])
+@pytest.mark.parametrize("S,H,k", [(4, 256, 1), (4, 2052, 2), (2, 4100, 5), (1, 1024, 8), (3, 64, 0), (4, 6144, 2), (4, 8192, 5)])
 def test_stream_norms_of_few_and_many_tokens_agree_bitwise(dtype, S, H, k):
     T, dt, o = 70, DT[dtype], ops()
     streams, branch = rnd(T, S, H, seed=1), rnd(T, max(k, 1), H, dtype=dt, seed=2)

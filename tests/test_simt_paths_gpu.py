@@ -20,7 +20,8 @@ def _misaligned(x):
 @pytest.mark.parametrize("M,N,K", [
     (1, 31, 8), (2, 33, 136), (3, 32, 128), (5, 100, 512), (9, 70, 392), (17, 40, 1040),   # streamed, 1 .. 16 rows a block
     (64, 8192, 16), (65, 8200, 48), (130, 4100, 144),                                      # register tiles and their edges
-    (400, 8, 264)])                                                                        # many rows, few columns: streamed
+    (400, 8, 264),                                                                         # many rows, few columns: streamed
+    (1, 65535 * 32, 8), (2, 65535 * 32 + 33, 8)])                                          # as many blocks as a grid holds; more
 def test_dense_products_agree_bitwise(at, wt, ct, M, N, K):
     a, w = rnd(M, K, dtype=DT[at], seed=1), rnd(N, K, dtype=DT[wt], seed=2, scale=0.1)
     got, want = (torch.full((M, N), float("nan"), dtype=DT[ct], device=DEV) for _ in range(2))
