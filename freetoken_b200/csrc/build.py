@@ -50,10 +50,16 @@ LIBRARIES: Dict[str, str] = {
     "attention_prefill_mha": "attention_prefill_mha.cu",
     "moe_gemm_tc": "moe_gemm_tc.cu",
     "recurrent": "recurrent.cu",
+    "delta_scan": "delta_scan.cu",
+    "channel_delta": "channel_delta.cu",
+    "retention": "retention.cu",
     "gated_norm": "gated_norm.cu",
     "time_mixing": "time_mixing.cu",
 }
 HEADERS: List[str] = ["common.cuh", "mma_utils.cuh", "tcgen05.cuh", "status_codes.h", "sampling_static.h"]
+# headers of some libraries only
+OWN_HEADERS: Dict[str, List[str]] = {"recurrent": ["scans.cuh"]}
+OWN_HEADERS.update({name: ["scans.cuh", "delta_scan.cuh"] for name in ("delta_scan", "channel_delta", "retention")})
 EXTRA_LINK: Dict[str, List[str]] = {}
 
 
@@ -102,7 +108,7 @@ def build_dir() -> str:
 
 def _digest(name: str) -> str:
     h = hashlib.sha256()
-    for rel in [LIBRARIES[name]] + HEADERS:
+    for rel in [LIBRARIES[name]] + HEADERS + OWN_HEADERS.get(name, []):
         with open(os.path.join(HERE, rel), "rb") as f:
             h.update(f.read())
     h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS + EXTRA_LINK.get(name, [])).encode())

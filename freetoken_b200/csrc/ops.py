@@ -743,7 +743,7 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bi
         raise KernelError("delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i")
+    f = _fn("delta_scan", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), _ptr(decay), beta.stride(0), _ptr(dt_bias), _ptr(a_log),
              _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
              key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
@@ -774,7 +774,7 @@ def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tenso
         raise KernelError("channel_delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("channel_delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i")
+    f = _fn("channel_delta", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(decay), decay.stride(0), _ptr(dt_bias),
              _ptr(a_log), _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
              key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype), _stream()),
@@ -804,7 +804,7 @@ def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[tor
         raise KernelError("retention_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("retention_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("recurrent", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i")
+    f = _fn("retention", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(decay), _ptr(cos_sin), rot, _ptr(seg_pos0), _ptr(state), state.stride(0),
              _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim, key_dim, float(k_scale),
              seg_slot.numel(), T, longest, code(qkv.dtype), _stream()), "retention_scan")

@@ -35,7 +35,7 @@ state in per-request slots too (python/freetoken/kvcache/linear_state_pool.py:32
 
 from __future__ import annotations
 
-from typing import Dict, List
+from typing import Dict, List, Tuple
 
 import torch
 
@@ -53,6 +53,7 @@ class _Recurrent(Mixer):
     conv_channels: int
     taps: int
     state_values: int
+    kernels: Tuple[str, ...]     # libraries of the convolution and the scan
 
     def cache_need(self):
         return StateNeed(((self.taps - 1) * self.conv_channels + self.state_values,), "float32")
@@ -65,7 +66,7 @@ class _Recurrent(Mixer):
         return cache.state[:, :cut], cache.state[:, cut:]
 
     def libraries(self, dtype) -> List[str]:
-        return ["recurrent", "gated_norm"] + linear.libraries(dtype)
+        return list(self.kernels) + ["gated_norm"] + linear.libraries(dtype)
 
 
 @register_mixer("ssd")
@@ -73,6 +74,8 @@ class SelectiveStateSpace(_Recurrent):
     """params: ``hidden_size, heads, head_dim, state_dim, groups, conv_taps, norm_groups,
     norm_eps``, ``scope`` and ``names`` (in, conv, conv_bias, dt_bias, a_log, d, norm, o below
     the scope).  The input projection's rows are ``z | x | B | C | dt``."""
+
+    kernels = ("recurrent",)
 
     def __init__(self, spec, prefix):
         super().__init__(spec, prefix)
@@ -137,6 +140,8 @@ class GatedDelta(_Recurrent):
     beta, decay: the projections; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv:
     the merged projection and convolution the model keeps).  Query / key head ``h // (heads /
     key_heads)`` serves head ``h``; q is multiplied by ``key_dim ** -0.5`` after its unit norm."""
+
+    kernels = ("recurrent", "delta_scan")
 
     def __init__(self, spec, prefix):
         super().__init__(spec, prefix)
@@ -208,6 +213,8 @@ class ChannelDelta(_Recurrent):
     of the decay's and the gate's; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv: the
     merged projection and convolution the model keeps).  ``dt_bias`` has one entry per head and key
     channel, ``norm`` one per value of a head (shared by the heads)."""
+
+    kernels = ("recurrent", "channel_delta")
 
     def __init__(self, spec, prefix):
         super().__init__(spec, prefix)
@@ -287,6 +294,7 @@ class Retention(_Recurrent):
     ** -0.5`` after the rotation; the read-out of a head is divided by its root mean square (no
     weight), the row gated by ``silu(W_g h)``."""
 
+    kernels = ("retention",)
     taps = 1
     conv_channels = 0
 

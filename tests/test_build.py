@@ -1,6 +1,7 @@
 """The library builder's housekeeping (no compiler needed)."""
 
 import os
+import re
 
 from freetoken_b200.csrc import build
 
@@ -23,3 +24,16 @@ def test_every_library_has_its_source_and_a_digest():
         assert len(build._digest(name)) == 16
     for header in build.HEADERS:
         assert os.path.exists(os.path.join(build.HERE, header)), header
+
+
+def test_a_digest_covers_every_header_that_is_included():
+    def included(path, seen):
+        with open(os.path.join(build.HERE, path)) as f:
+            for header in re.findall(r'^#include "(.+)"', f.read(), re.M):
+                if header not in seen:
+                    seen.add(header)
+                    included(header, seen)
+        return seen
+
+    for name, src in build.LIBRARIES.items():
+        assert included(src, set()) <= set(build.HEADERS + build.OWN_HEADERS.get(name, [])), name
