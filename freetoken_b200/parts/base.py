@@ -65,9 +65,9 @@ class Workspace:
 
     ``get`` returns a view of a buffer at least as large as asked; a buffer is
     only ever replaced by a larger one, so steady-state steps allocate
-    nothing.  The views handed out are kept beside their buffer (the last
-    :data:`KEPT_VIEWS` shapes of it): a step asks for a few dozen of them, and
-    making one costs as much host time as a small launch."""
+    nothing.  The views handed out are kept beside their buffer (up to
+    :data:`KEPT_VIEWS` shapes of it, all dropped when one more comes): a step asks for a few
+    dozen of them, and making one costs as much host time as a small launch."""
 
     KEPT_VIEWS = 64
 
