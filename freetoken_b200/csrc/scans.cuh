@@ -16,8 +16,8 @@
 // chunk, which all threads stage into shared memory together.  Which WC a launch
 // takes depends on the step's shape, never on a token's place in it, and the
 // operations on a column are the same for every WC.  Launches whose segments have several
-// tokens may take kernels with 16 lanes a column that perform the same operations (see
-// there, and seq_scan for which).
+// tokens may take kernels with 16 lanes a column that perform the same operations (seq_scan
+// says which).
 #pragma once
 #include "common.cuh"
 
@@ -98,11 +98,12 @@ __device__ __forceinline__ void store_cols(float* p, const float (&v)[WC], int v
 }
 
 // ------------------------------------------------- segments of several tokens
-// A prompt portion's tokens are a chain, and the kernels above spend a microsecond and more on four of them: 32
-// lanes a column, five shuffle stages for the unit vectors, five for the column sums, a broadcast.  Here a column
+// A prompt portion's tokens are a chain, and ssd_scan_kernel and delta_scan_kernel spend a microsecond and more on four
+// of them: 32 lanes a column, five shuffle stages for the unit vectors, five for the column sums, a broadcast.  In
+// ssd_seq_kernel and delta_seq_kernel a column
 // belongs to 16 lanes; lane l keeps rows l + 32 e and l + 16 + 32 e of CPL columns, sums them in two chains (what
-// lanes l and l + 16 sum above) and adds the two, so that four shuffle stages remain and every sum has the bits of
-// the kernels above: which of the two a launch takes does not show in the results.  What does not wait for the
+// lanes l and l + 16 sum there) and adds the two, so that four shuffle stages remain and every sum has the bits of
+// the former: which of the two a launch takes does not show in the results.  What does not wait for the
 // state (unit vectors, gates, rotations, k . q) is done while a chunk is staged, a warp a token; what nothing waits
 // for (the read-outs) is added over the lanes once a chunk, for its eight tokens together.  q and k rows lie in
 // shared memory in the lanes' order, so that a lane reads its rows in 16-byte pieces.  Four warps work and four stage (the staging's chain of
