@@ -193,8 +193,10 @@ static bool narrow_warps(int P, int heads, int S) {
 }
 
 // Columns a lane of the kernels for several tokens a segment.  Four need fewer shared loads and less staging a
-// column, two leave twice as many blocks: measured, two win while the columns of a launch (heads, segments) fill
-// the chip once (4,096: delta 499 against 594 us for 2,048 tokens), four from there on (16,384: 911 against 750).
+// column, two leave twice as many blocks.  Time with four over time with two, by the columns of a launch (heads, segments),
+// states of 128 x 128, one and four segments of 64 and 512 tokens: delta rule 1.3 .. 1.5 at 2,048, 1.08 .. 1.20 at 4,096,
+// 0.90 .. 0.95 at 5,120, 0.80 .. 0.95 from 6,144 to 16,384 (level at 10,240, where two fill a round exactly); a decay
+// per channel 1.09 .. 1.16 at 4,096, 0.81 at 5,120; retention and the state space 1.1 .. 1.2 at 2,048, 0.88 .. 0.92 at 4,096.
 static int seq_columns(int P, int heads, int S) { return (long long)P * heads * S <= 5000 ? 2 : 4; }
 
 // Which kernels take T tokens in S segments: those with 16 lanes a column (true) or those with 32.  The former take a third
