@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
   __nv_bfloat16* sV = sK + STAGES * TILE * LD;                            // [STAGES][TILE][LD]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
-  pdl_wait();
+  pdl_wait_only();
 
   const int G = a.nq / a.nkv;
   const int gtiles = (G + 15) / 16;
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
 __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                   __nv_bfloat16* __restrict__ out, const int* __restrict__ rows,
                                   int nq, int d, int splits) {
-  pdl_wait();
+  pdl_wait_only();
 
   const int row = blockIdx.x, head = blockIdx.y;
   const int tok = rows ? rows[row] : row;

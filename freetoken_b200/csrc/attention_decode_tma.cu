@@ -79,8 +79,6 @@ __global__ void __launch_bounds__(160) attn_decode_tma_kernel(const __grid_const
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  pdl_wait();
-
   const int G = a.nq / a.nkv;
   const int gtiles = (G + 15) / 16;
   const int kvh = blockIdx.y / gtiles, gt = blockIdx.y % gtiles;
@@ -96,6 +94,11 @@ __global__ void __launch_bounds__(160) attn_decode_tma_kernel(const __grid_const
   const int k_end = min(pos + 1, (split + 1) * a.split_keys);
   const int first_valid = max(lo, split * a.split_keys);
   const int ntiles = k_end > k_begin ? (k_end - k_begin + TILE - 1) / TILE : 0;
+  // What stands above is the step's metadata.  A launch that fills the chip lets the next one in only as it leaves: a
+  // product that becomes resident beside these blocks works in the little L1 that their stages leave an SM, to its end
+  // (a projection of 192 blocks behind 256 of these: 10 -> 21 us).
+  pdl_wait_only();
+  if (gridDim.x * gridDim.y * gridDim.z <= 74) pdl_release();
 
   // Q tile -> shared (rows >= heads are zero), by the consumers
   if (warp < 4) {

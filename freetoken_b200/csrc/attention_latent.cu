@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
     for (int c = chunks + lane; c < dp / 8; c += 32)
       *reinterpret_cast<uint4*>((r < RT ? sQ + r * ld : sK + (size_t)(r - RT) * ld) + c * 8) = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  pdl_wait();
 
   const int seg = a.tile_seg[blockIdx.x], row0 = a.tile_row[blockIdx.x];
   const int split = blockIdx.y;
@@ -110,6 +109,7 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
   const int k_end = min(pos_last + 1, (split + 1) * a.split_keys);
   const int k_begin = k_lo / LT_KEYS * LT_KEYS;
   const int ntiles = k_end > k_lo ? (k_end - k_begin + LT_KEYS - 1) / LT_KEYS : 0;
+  pdl_wait();          // what stands above is the step's metadata
 
   if (warp >= 8) {
     // 16 rows a warp, four at a time: eight lanes a row, 128 bytes of it per copy instruction.  Rows outside
@@ -350,10 +350,10 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
 // asks for more); further ones follow in rounds of as many.
 constexpr int MERGE_AHEAD = 8, MERGE_SPLITS = 1024, MERGE_THREADS = 128;
 __global__ void __launch_bounds__(MERGE_THREADS) latent_merge_kernel(LatentAttnArgs a, int rt) {
-  pdl_wait();
   const int tile = blockIdx.x, r = blockIdx.y;
   const int seg = a.tile_seg[tile], row0 = a.tile_row[tile];
   const int seg_begin = a.seg_q_start[seg];
+  pdl_wait();
   if (r >= (a.seg_q_start[seg + 1] - seg_begin) * a.nq - row0) return;
   const size_t base = ((size_t)tile * rt + r) * a.splits;
   extern __shared__ float split_ml[];                  // of a round: sums, then maxima, then factors

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * SHARED_WARPS) attn_shared_kernel(AttnArgs
   constexpr int MAXD = 8, PIECE = 16 / sizeof(AT), CHUNK = 32;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ int row_lo[SHARED_WARPS], row_pos[SHARED_WARPS];
-  pdl_wait();
+  pdl_wait_only();
   int r_begin = blockIdx.x * tokens, r_end = min(T, r_begin + tokens);
   if ((int)blockIdx.x >= packs) {              // request blockIdx.x - packs + 1, up to where the next pack begins
     const int s = blockIdx.x - packs + 1;

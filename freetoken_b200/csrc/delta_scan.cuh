@@ -30,6 +30,7 @@ struct DeltaArgs {
   const float* cos_sin;      // [positions, rot_dims]: cos | sin (nullptr or rot_dims 0: no rotation)
   const int* seg_pos0;       // [S]: position of a segment's first token
   int rot_dims;
+  int state_ahead;           // the launch right in front does not write the state: it is fetched ahead of the wait
 };
 
 // MODE 0: the gated delta rule with one decay per head.
@@ -45,7 +46,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   constexpr int NB = (NPL * 32 + SCAN_THREADS - 1) / SCAN_THREADS;
   constexpr int XR = (SCAN_CHUNK * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
   extern __shared__ float sm[];
-  pdl_wait();
+  if (!a.state_ahead) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int head = blockIdx.y, seg = blockIdx.z;
   const int D = a.D, P = a.P;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
       for (int c = 0; c < WC; ++c) S[e][c] = 0.f;
     }
   }
+  if (a.state_ahead) pdl_wait();
 
   AT pq[SCAN_CHUNK][NB], pk[SCAN_CHUNK][NB], pv[XR], pbeta, pdecay;
   float pg[MODE == 1 ? SCAN_CHUNK : 1][NB];                   // MODE 1: the channels' decay projections

@@ -71,13 +71,9 @@ __device__ __forceinline__ void store4f(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
-// EAGER (a step of few tokens, where a launch is a chain of waits for L2 rather than a
-// stream): the k partial rows of a piece are fetched four at a time before they are added,
-// in the same order.  With every SM full of such blocks the extra loads in flight cost more
-// than they save (25 -> 29 us at 2,048 tokens), so many tokens keep the one-by-one loop.
 constexpr int ROW_KERNEL_EAGER_TOKENS = 64;   // up to this many tokens the row kernels fetch eagerly
 
-template <typename AT, bool VEC, bool EAGER = false>
+template <typename AT, bool VEC>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_kernel(const AT* __restrict__ delta, float* __restrict__ residual,
                const float* __restrict__ weight, AT* __restrict__ out, int H, float eps,
@@ -100,21 +96,9 @@ rmsnorm_kernel(const AT* __restrict__ delta, float* __restrict__ residual,
         float4 z = load4f(r + 4 * gi);
         if (d) {
           float4 add = load4f(d + 4 * gi);
-          if (EAGER) {
-            for (int q0 = 1; q0 < k; q0 += 4) {
-              float4 more[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u)
-                more[u] = q0 + u < k ? load4f(d + (size_t)(q0 + u) * H + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int u = 0; u < 4; ++u)
-                if (q0 + u < k) { add.x += more[u].x; add.y += more[u].y; add.z += more[u].z; add.w += more[u].w; }
-            }
-          } else {
-            for (int q = 1; q < k; ++q) {
-              const float4 more = load4f(d + (size_t)q * H + 4 * gi);
-              add.x += more.x; add.y += more.y; add.z += more.z; add.w += more.w;
-            }
+          for (int q = 1; q < k; ++q) {
+            const float4 more = load4f(d + (size_t)q * H + 4 * gi);
+            add.x += more.x; add.y += more.y; add.z += more.z; add.w += more.w;
           }
           z.x += add.x; z.y += add.y; z.z += add.z; z.w += add.w;
           store4f(r + 4 * gi, z);
@@ -154,6 +138,95 @@ rmsnorm_kernel(const AT* __restrict__ delta, float* __restrict__ residual,
   const float inv = rsqrtf(ss / (float)H + eps);
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
     o[i] = from_float<AT>(r[i] * inv * (weight[i] + one));
+  }
+}
+
+// four elements as they lie in memory, and as float32
+template <typename AT> struct Raw4;
+template <> struct Raw4<float> { float4 v; };
+template <> struct Raw4<__nv_bfloat16> { uint2 v; };
+__device__ __forceinline__ float4 widen4(const Raw4<float>& r) { return r.v; }
+__device__ __forceinline__ float4 widen4(const Raw4<__nv_bfloat16>& r) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.v.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// For a step of few tokens, where a launch is a chain of waits for L2 rather than a
+// stream: the k partial rows are fetched four at a time, of two pieces together, before they are
+// added, in the same order, and the weight - cold in L2 after a step's worth of others - is asked
+// for ahead of the wait.  With every SM full of such blocks the extra loads in flight cost more
+// than they save (25 -> 29 us at 2,048 tokens), so many tokens keep the one-by-one loop.  Of 64 registers
+// a thread, so that a block finds a place beside those of the launch in front: with 128 it waited for an
+// SM to fall empty, 7.0 instead of 5.1 us behind eight partial rows of 3,072 values.
+template <typename AT>
+__global__ void __launch_bounds__(NORM_THREADS, 2)
+rmsnorm_few_kernel(const AT* __restrict__ delta, float* __restrict__ residual, const float* __restrict__ weight,
+                   AT* __restrict__ out, int H, float eps, int plus_one, int k) {
+  __shared__ float scratch[33];
+  for (int i = threadIdx.x * 32; i < H; i += NORM_THREADS * 32) warm(weight + i);
+  pdl_wait();
+  const int t = blockIdx.x, groups = H >> 2;
+  float* r = residual + (size_t)t * H;
+  const AT* d = delta ? delta + (size_t)t * k * H : nullptr;
+  AT* o = out + (size_t)t * H;
+  const float one = plus_one ? 1.f : 0.f;
+  float ss = 0.f;
+  float4 keep[NORM_KEEP];
+#pragma unroll
+  for (int j0 = 0; j0 < NORM_KEEP; j0 += 2) {
+    if (j0 * NORM_THREADS >= groups) break;
+    float4 z[2], add[2];
+    bool in[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int gi = threadIdx.x + (j0 + p) * NORM_THREADS;
+      in[p] = gi < groups;
+      z[p] = in[p] ? load4f(r + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+      add[p] = in[p] && d ? load4f(d + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int q0 = 1; d && q0 < k; q0 += 4) {
+      Raw4<AT> more[2][4];
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (in[p] && q0 + u < k)
+            more[p][u] = *reinterpret_cast<const Raw4<AT>*>(d + (size_t)(q0 + u) * H + 4 * (threadIdx.x + (j0 + p) * NORM_THREADS));
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (in[p] && q0 + u < k) {
+            const float4 m = widen4(more[p][u]);
+            add[p].x += m.x; add[p].y += m.y; add[p].z += m.z; add[p].w += m.w;
+          }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      if (!in[p]) continue;
+      if (d) {
+        z[p].x += add[p].x; z[p].y += add[p].y; z[p].z += add[p].z; z[p].w += add[p].w;
+        store4f(r + 4 * (threadIdx.x + (j0 + p) * NORM_THREADS), z[p]);
+      }
+      keep[j0 + p] = z[p];
+      ss += z[p].x * z[p].x;
+      ss += z[p].y * z[p].y;
+      ss += z[p].z * z[p].z;
+      ss += z[p].w * z[p].w;
+    }
+  }
+  ss = block_sum(ss, scratch);
+  const float inv = rsqrtf(ss / (float)H + eps);
+#pragma unroll
+  for (int j = 0; j < NORM_KEEP; ++j) {
+    const int gi = threadIdx.x + j * NORM_THREADS;
+    if (gi < groups) {
+      const float4 w = load4f(weight + 4 * gi);
+      const float4 z = keep[j];
+      store4f(o + 4 * gi, make_float4(z.x * inv * (w.x + one), z.y * inv * (w.y + one),
+                                      z.z * inv * (w.z + one), z.w * inv * (w.w + one)));
+    }
   }
 }
 
@@ -411,8 +484,24 @@ template <bool EAGER>
 __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
   extern __shared__ float head_inv[];
   __shared__ float scratch[66];
-  pdl_wait();
   const int t = blockIdx.x;
+  const int pos = a.token_pos[t];
+  size_t page_base = 0;
+  if (EAGER && a.kv_pages) {
+    const int page = a.block_table[(size_t)a.token_seg[t] * a.table_width + pos / a.P];
+    page_base = (size_t)page * a.page_stride + (size_t)(pos % a.P) * a.d;
+  }
+  if (EAGER && gridDim.x * gridDim.y <= 296) {
+    // what no launch of the step writes, four lookups deep, is near before the wait (of blocks that are there by then)
+    if (a.cos_sin)
+      for (int i = threadIdx.x * 32; i < a.R; i += blockDim.x * 32) warm(a.cos_sin + (size_t)pos * a.R + i);
+    if (a.norm_mode) {
+      const int per = a.norm_mode == 1 ? a.d : 0;
+      for (int i = threadIdx.x * 32; i < (per ? per * a.nq : a.d); i += blockDim.x * 32) warm(a.q_weight + i);
+      for (int i = threadIdx.x * 32; i < (per ? per * a.nkv : a.d); i += blockDim.x * 32) warm(a.k_weight + i);
+    }
+  }
+  pdl_wait();
   const __nv_bfloat16* row = (const __nv_bfloat16*)a.qkv + (size_t)t * a.ld;
   const int d = a.d, dc = d >> 3;                 // pieces per head
   const int qn = a.nq * d, kn = a.nkv * d;
@@ -448,7 +537,6 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
     }
     __syncthreads();
   }
-  const int pos = a.token_pos[t];
   const int half = a.R >> 1;
   const int hc = a.interleaved ? 0 : half >> 3;   // rotary half, in pieces (halves; pairs stay inside a piece)
   const float* cs = (a.cos_sin && a.R > 0) ? a.cos_sin + (size_t)pos * a.R : nullptr;
@@ -457,9 +545,11 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
   __nv_bfloat16* ko = nullptr;
   __nv_bfloat16* vo = nullptr;
   if (a.kv_pages) {
-    const int seg = a.token_seg[t];
-    const int page = a.block_table[(size_t)seg * a.table_width + pos / a.P];
-    const size_t base = (size_t)page * a.page_stride + (size_t)(pos % a.P) * d;
+    size_t base = page_base;
+    if (!EAGER) {
+      const int page = a.block_table[(size_t)a.token_seg[t] * a.table_width + pos / a.P];
+      base = (size_t)page * a.page_stride + (size_t)(pos % a.P) * d;
+    }
     ko = (__nv_bfloat16*)a.kv_pages + base;
     vo = (__nv_bfloat16*)a.kv_pages + a.kv_stride + base;
   }
@@ -468,7 +558,7 @@ __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
   const int total_q = a.nq * per_head, total = total_q + a.nkv * per_head;
   // this block's share of the work items and of the V pieces
   const int parts = gridDim.y, part = blockIdx.y;
-  const int w_begin = (int)((long long)total * part / parts), w_end = (int)((long long)total * (part + 1) / parts);
+  const int w_begin = total * part / parts, w_end = total * (part + 1) / parts;      // a few thousand pieces, 8 parts
   for (int w = w_begin + threadIdx.x; w < w_end; w += blockDim.x) {
     const bool is_q = w < total_q;
     const int ww = is_q ? w : w - total_q;
@@ -849,7 +939,7 @@ int ft_rmsnorm(const void* delta, float* residual, const float* weight, void* ou
                    !((uintptr_t)residual & 15) && !((uintptr_t)weight & 15) && !((uintptr_t)out & 15);
   if (vec && T <= ROW_KERNEL_EAGER_TOKENS) {
     FT_DISPATCH(dtype, AT,
-                (launch_pdl(rmsnorm_kernel<AT, true, true>, dim3(T), dim3(NORM_THREADS), 0, stream,
+                (launch_pdl(rmsnorm_few_kernel<AT>, dim3(T), dim3(NORM_THREADS), 0, stream,
                             (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
   } else if (vec) {
     FT_DISPATCH(dtype, AT,

@@ -69,13 +69,15 @@ __global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* __rest
                                                              int weight_len, AT* __restrict__ out, int T, int width,
                                                              int groups, float eps, int gate_first, int gate_kind) {
   __shared__ float scratch[33];
-  pdl_wait();
   const int sub = threadIdx.x % TPI;
-  const long long item = (long long)blockIdx.x * (128 / TPI) + threadIdx.x / TPI;
-  const bool live = item < (long long)T * groups;
-  if (TPI >= 32 && !live) return;                     // a warp (TPI 32) or the whole block (TPI 128) leaves
-  const int t = live ? (int)(item / groups) : 0, grp = live ? (int)(item % groups) : 0;
+  // 32 bits (the host sees to it): a division of 64 took as long as the load behind it
+  const unsigned item = blockIdx.x * (128 / TPI) + threadIdx.x / TPI;
+  const bool live = item < (unsigned)T * (unsigned)groups;
+  const int t = live ? (int)(item / (unsigned)groups) : 0, grp = live ? (int)(item - (unsigned)t * (unsigned)groups) : 0;
   const int size = width / groups, base = grp * size, pieces = live ? size >> 2 : 0;
+  for (int i = sub * 32; i < (live ? size : 0); i += TPI * 32) warm(weight + (base + i) % weight_len);
+  pdl_wait();
+  if (TPI >= 32 && !live) return;                     // a warp (TPI 32) or the whole block (TPI 128) leaves
   const float* row = y + (size_t)t * width + base;
   const AT* gate = z + (size_t)t * ldz + base;
   float4 keep[KEEP], gk[KEEP];
@@ -127,7 +129,7 @@ int ft_gated_norm(const float* y, const void* z, long long ldz, const float* wei
   if (width <= 0 || groups <= 0 || width % groups || weight_len <= 0) return FT_ERR_SHAPE;
   const long long items = (long long)T * groups;
   const int size = width / groups;
-  const bool vec = !(size & 3) && !(weight_len & 3) && !(ldz & 3) && !((uintptr_t)y & 15) && !((uintptr_t)z & 15) &&
+  const bool vec = items < (1ll << 31) - 128 && !(size & 3) && !(weight_len & 3) && !(ldz & 3) && !((uintptr_t)y & 15) && !((uintptr_t)z & 15) &&
                    !((uintptr_t)weight & 15) && !((uintptr_t)out & 15);
   if (vec && size <= 16 * 8) {
     FT_DISPATCH(dtype, AT, launch_pdl(gated_norm_vec_kernel<AT, 8, 4>, dim3((unsigned)((items + 15) / 16)), dim3(128), 0, stream,

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(GemmArgs a) {
   __shared__ float Ws[BN][BK + 1];
   __shared__ float Us[GLU ? BN : 1][BK + 1];
   __shared__ int tile_info[3];  // group, first row, rows
-  pdl_wait();
+  pdl_wait_only();
   find_tile<BM>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
   constexpr int STAGE = WROWS * WROW + MR * AROW;
   extern __shared__ __align__(16) unsigned char stream_sm[];
   __shared__ int tile_info[3];
-  pdl_wait();
+  pdl_wait_only();
   find_tile<MR>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(128) gemm_tile_kernel(GemmArgs a) {
   __shared__ __align__(16) float As[2][TBK][TBM];
   __shared__ __align__(16) float Ws[2][TBK][TBN];
   __shared__ int tile_info[3];
-  pdl_wait();
+  pdl_wait_only();
   find_tile<TBM>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256) gemm_dense_kernel(GemmArgs a) {
   constexpr int TBM = 64, TBN = 64, TBK = 32;
   __shared__ __align__(16) float As[TBK][TBM + 4];
   __shared__ __align__(16) float Ws[TBK][TBN + 4];
-  pdl_wait();
+  pdl_wait_only();
   const int row0 = blockIdx.x * TBM, n0 = blockIdx.y * TBN;
   const AT* A = (const AT*)a.A + (size_t)blockIdx.z * a.a_batch_stride;
   const WT* W = (const WT*)a.W + (size_t)blockIdx.z * a.w_batch_stride;
@@ -506,7 +506,9 @@ int launch_stream(const GemmArgs& a, cudaStream_t stream) {
   }
   const int tiles = a.group_offsets ? a.M / MR + min(a.G, a.M) : (a.M + MR - 1) / MR;
   const dim3 grid(tiles, (a.N + STREAM_COLS - 1) / STREAM_COLS, a.batch);
-  const cudaError_t e = launch_pdl(kernel, grid, dim3(32 * (MR < 8 ? MR : 8)), smem, stream, a);
+  const dim3 block(32 * (MR < 8 ? MR : 8));
+  const cudaError_t e = a.group_offsets ? launch_behind(kernel, grid, block, smem, stream, a)
+                                        : launch_pdl(kernel, grid, block, smem, stream, a);
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
@@ -566,12 +568,12 @@ int launch_kind(const GemmArgs& a, cudaStream_t stream) {
   if (route == GEMM_TILE) {
     const int cols = (a.N + (GLU ? 63 : 127)) / (GLU ? 64 : 128);
     const dim3 grid(a.group_offsets ? a.M / 64 + min(a.G, a.M) : (a.M + 63) / 64, cols, a.batch);
-    const cudaError_t e = launch_pdl(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(128), 0, stream, a);
+    const cudaError_t e = launch_behind(gemm_tile_kernel<AT, WT, OT, GLU>, grid, dim3(128), 0, stream, a);
     return e == cudaSuccess ? FT_OK : (int)e;
   }
   if constexpr (!GLU) {
     if (route == GEMM_DENSE) {
-      const cudaError_t e = launch_pdl(gemm_dense_kernel<AT, WT, OT>, dim3((a.M + 63) / 64, (a.N + 63) / 64, a.batch), dim3(256),
+      const cudaError_t e = launch_behind(gemm_dense_kernel<AT, WT, OT>, dim3((a.M + 63) / 64, (a.N + 63) / 64, a.batch), dim3(256),
                                        0, stream, a);
       return e == cudaSuccess ? FT_OK : (int)e;
     }
@@ -589,8 +591,8 @@ int launch_kind(const GemmArgs& a, cudaStream_t stream) {
   const int bm = big ? 64 : 16;
   const int tiles = (a.M + bm - 1) / bm + (a.group_offsets ? a.G : 0);
   const dim3 grid(tiles, (a.N + BN - 1) / BN, a.batch);
-  const cudaError_t e = big ? launch_pdl(gemm_rows_kernel<AT, WT, OT, 64, GLU>, grid, dim3(256), 0, stream, a)
-                            : launch_pdl(gemm_rows_kernel<AT, WT, OT, 16, GLU>, grid, dim3(256), 0, stream, a);
+  const cudaError_t e = big ? launch_behind(gemm_rows_kernel<AT, WT, OT, 64, GLU>, grid, dim3(256), 0, stream, a)
+                            : launch_behind(gemm_rows_kernel<AT, WT, OT, 16, GLU>, grid, dim3(256), 0, stream, a);
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 

@@ -661,14 +661,19 @@ def latent_store(down: torch.Tensor, q: torch.Tensor, q_abs: Optional[torch.Tens
 
 
 # ------------------------------------------------------- mixers with a carried state
+# STATE_AHEAD.  A scan's or convolution's ``state_ahead`` promises that the launch right in front of this one does not write
+# ``state``: a step of one token a request then fetches it while that launch still runs.  So it is where a mixer's own
+# projection comes in between; two scans of one state back to back leave it out.
 def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
               state: torch.Tensor, token_seg: torch.Tensor, seg_slot: torch.Tensor,
-              seg_q_start: torch.Tensor, activation: bool = True) -> None:
+              seg_q_start: torch.Tensor, activation: bool = True,
+              state_ahead: bool = False) -> None:
     """A causal convolution over time per channel, then SiLU: ``out[t, c] = silu(bias[c] +
     sum_j weight[c, j] * u[t - (taps - 1) + j, c])`` where ``u`` is the request's inputs so far
     (``activation=False``: the sum itself, no SiLU).
     ``x`` ``[T, C]`` (a column range of a wider matrix is fine), ``state`` ``[slots, >= (taps - 1) *
-    C]`` float32: a request's last ``taps - 1`` inputs, read first and then brought up to date."""
+    C]`` float32: a request's last ``taps - 1`` inputs, read first and then brought up to date.
+    ``state_ahead``: see STATE_AHEAD."""
     _need(x, "x", contiguous=False)
     _need(out, "out", x.dtype, contiguous=False)
     _need(weight, "weight", torch.float32)
@@ -685,19 +690,21 @@ def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Op
         _need(t, name, torch.int32)
     global LAUNCHES
     LAUNCHES += 1 if taps > 1 and (T != seg_slot.numel() or taps > 8) else 0      # a kernel for the slots' new contents
-    f = _fn("recurrent", "ft_conv_silu", "p q p q p p p q p p p i i i i i i")
+    f = _fn("recurrent", "ft_conv_silu", "p q p q p p p q p p p i i i i i i i")
     _check(f(_ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(weight), _ptr(bias), _ptr(state),
              state.stride(0), _ptr(token_seg), _ptr(seg_slot), _ptr(seg_q_start), C, taps, T,
-             seg_slot.numel(), code(x.dtype), int(activation), _stream()), "conv_silu")
+             seg_slot.numel(), code(x.dtype), int(activation), int(state_ahead), _stream()), "conv_silu")
 
 
 def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
              d_skip: torch.Tensor, state: torch.Tensor, y: torch.Tensor, seg_slot: torch.Tensor,
-             seg_q_start: torch.Tensor, heads: int, head_dim: int, state_dim: int, groups: int, longest: int = 0) -> None:
+             seg_q_start: torch.Tensor, heads: int, head_dim: int, state_dim: int, groups: int, longest: int = 0,
+             state_ahead: bool = False) -> None:
     """Per head: ``S <- exp(-exp(a_log) * step) * S + step * B x^T``, ``y = S^T C + d_skip * x`` with
     ``step = softplus(dt + dt_bias)``; ``xbc`` rows are ``x | B | C``; ``state`` ``[slots, >= heads *
     state_dim * head_dim]`` float32; ``y`` ``[T, heads * head_dim]`` float32.  ``longest`` (tokens of the longest segment, 0:
-    not known) helps to choose between kernels of equal results."""
+    not known) helps to choose between kernels of equal results.
+    ``state_ahead``: see STATE_AHEAD."""
     _need(xbc, "xbc", contiguous=False)
     _need(dt, "dt", xbc.dtype, contiguous=False)
     _need(state, "state", torch.float32, contiguous=False)
@@ -712,21 +719,23 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         raise KernelError("ssd_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * state_dim * head_dim:
         raise KernelError("ssd_scan: a state row must hold heads * state_dim * head_dim values")
-    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i i")
+    f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i i i")
     _check(f(_ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
              _ptr(state), state.stride(0), _ptr(y), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim,
-             state_dim, groups, seg_slot.numel(), T, longest, code(xbc.dtype), _stream()), "ssd_scan")
+             state_dim, groups, seg_slot.numel(), T, longest, code(xbc.dtype), int(state_ahead), _stream()), "ssd_scan")
 
 
 def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
                a_log: torch.Tensor, state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor,
                seg_q_start: torch.Tensor, heads: int, key_heads: int, key_dim: int, value_dim: int,
-               unit_eps: float, q_scale: float, longest: int = 0) -> None:
+               unit_eps: float, q_scale: float, longest: int = 0,
+               state_ahead: bool = False) -> None:
     """The gated delta rule per head: q and k made unit vectors (q times ``q_scale``), ``g =
     exp(-exp(a_log) * softplus(decay + dt_bias))``, ``b = sigmoid(beta)``; ``S <- g S``; ``u = b (v -
     S^T k)``; ``S <- S + k u^T``; ``o = S^T q``.  ``qkv`` rows are ``q | k | v``; ``beta`` and ``decay``
     ``[T, heads]`` with the same row stride; ``state`` ``[slots, >= heads * key_dim * value_dim]``.  ``longest`` (tokens of the longest segment, 0:
-    not known) helps to choose between kernels of equal results."""
+    not known) helps to choose between kernels of equal results.
+    ``state_ahead``: see STATE_AHEAD."""
     _need(qkv, "qkv", contiguous=False)
     _need(beta, "beta", qkv.dtype, contiguous=False)
     _need(decay, "decay", qkv.dtype, contiguous=False)
@@ -743,21 +752,23 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bi
         raise KernelError("delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("delta_scan", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i")
+    f = _fn("delta_scan", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), _ptr(decay), beta.stride(0), _ptr(dt_bias), _ptr(a_log),
              _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
              key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
-             _stream()), "delta_scan")
+             int(state_ahead), _stream()), "delta_scan")
 
 
 def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
                        a_log: torch.Tensor, state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor,
                        seg_q_start: torch.Tensor, heads: int, key_heads: int, key_dim: int, value_dim: int,
-                       unit_eps: float, q_scale: float, longest: int = 0) -> None:
+                       unit_eps: float, q_scale: float, longest: int = 0,
+                       state_ahead: bool = False) -> None:
     """The gated delta rule with a decay per key channel: as :func:`delta_scan`, but row ``n`` of head
     ``h``'s state is multiplied by ``exp(-exp(a_log[h]) * softplus(decay[t, h * key_dim + n] + dt_bias[h *
     key_dim + n]))`` before the token reads and writes.  ``decay`` is float32 ``[T, heads * key_dim]``.  ``longest`` (tokens of the longest segment, 0:
-    not known) helps to choose between kernels of equal results."""
+    not known) helps to choose between kernels of equal results.
+    ``state_ahead``: see STATE_AHEAD."""
     _need(qkv, "qkv", contiguous=False)
     _need(beta, "beta", qkv.dtype, contiguous=False)
     _need(decay, "decay", torch.float32, contiguous=False)
@@ -774,21 +785,23 @@ def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tenso
         raise KernelError("channel_delta_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("channel_delta_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("channel_delta", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i")
+    f = _fn("channel_delta", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(decay), decay.stride(0), _ptr(dt_bias),
              _ptr(a_log), _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype), _stream()),
-           "channel_delta_scan")
+             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
+             int(state_ahead), _stream()), "channel_delta_scan")
 
 
 def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[torch.Tensor], seg_pos0: torch.Tensor,
                    state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor, seg_q_start: torch.Tensor,
-                   heads: int, key_dim: int, value_dim: int, k_scale: float, longest: int = 0) -> None:
+                   heads: int, key_dim: int, value_dim: int, k_scale: float, longest: int = 0,
+                   state_ahead: bool = False) -> None:
     """Retention per head: ``S <- decay[h] S + k v^T``, ``o = S^T q``.  ``qkv`` rows are ``q | k | v``
     (``heads * key_dim`` twice, then ``heads * value_dim``); the first ``cos_sin.shape[1]`` dimensions of
     every q and k head are turned by the token's position (dimension i with i + half) in float32 and k is
     multiplied by ``k_scale`` afterwards; ``state`` ``[slots, >= heads * key_dim * value_dim]`` float32.  ``longest`` (tokens of the longest segment, 0:
-    not known) helps to choose between kernels of equal results."""
+    not known) helps to choose between kernels of equal results.
+    ``state_ahead``: see STATE_AHEAD."""
     _need(qkv, "qkv", contiguous=False)
     _need(decay, "decay", torch.float32)
     _need(state, "state", torch.float32, contiguous=False)
@@ -804,10 +817,10 @@ def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[tor
         raise KernelError("retention_scan: shapes do not match")
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("retention_scan: a state row must hold heads * key_dim * value_dim values")
-    f = _fn("retention", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i")
+    f = _fn("retention", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i i")
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(decay), _ptr(cos_sin), rot, _ptr(seg_pos0), _ptr(state), state.stride(0),
              _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim, key_dim, float(k_scale),
-             seg_slot.numel(), T, longest, code(qkv.dtype), _stream()), "retention_scan")
+             seg_slot.numel(), T, longest, code(qkv.dtype), int(state_ahead), _stream()), "retention_scan")
 
 
 def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: torch.Tensor, token_seg: torch.Tensor,
@@ -832,11 +845,13 @@ def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: tor
 
 def time_mixing_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, w0: torch.Tensor,
                      u: torch.Tensor, state: torch.Tensor, o: torch.Tensor, seg_slot: torch.Tensor,
-                     seg_q_start: torch.Tensor, heads: int, head_dim: int, key_dim: int) -> None:
+                     seg_q_start: torch.Tensor, heads: int, head_dim: int, key_dim: int,
+                     state_ahead: bool = False) -> None:
     """Per head, with ``w = exp(-exp(decay + w0))`` per key channel: ``o_t = (S + diag(u) k_t v_t^T)^T r_t``, then ``S
     <- diag(w_t) S + k_t v_t^T``.  ``r`` and ``k`` are ``[T, heads * key_dim]``, ``v`` ``[T, heads * head_dim]`` (one
     row stride), ``decay`` float32; the state of head h lies at ``h * head_dim * key_dim`` of its slot's row, ``[head_dim,
-    key_dim]``.  Every segment brings at least one token; as many tokens as segments: one each, a kernel of its own."""
+    key_dim]``.  Every segment brings at least one token; as many tokens as segments: one each, a kernel of its own.
+    ``state_ahead``: see STATE_AHEAD."""
     for name, t in (("r", r), ("k", k), ("v", v)):
         _need(t, name, r.dtype, contiguous=False)
     for name, t in (("decay", decay), ("state", state)):
@@ -852,10 +867,10 @@ def time_mixing_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
         raise KernelError("time_mixing_scan: shapes do not match")
     if len({t.stride(0) for t in (r, k, v)}) != 1 or any(t.stride(1) != 1 for t in (r, k, v, decay)):
         raise KernelError("time_mixing_scan: r, k and v need one row stride and unit column strides")
-    f = _fn("time_mixing", "ft_time_mixing_scan", "p p p q p q p p p q p p p i i i i i i")
+    f = _fn("time_mixing", "ft_time_mixing_scan", "p p p q p q p p p q p p p i i i i i i i")
     _check(f(_ptr(r), _ptr(k), _ptr(v), r.stride(0), _ptr(decay), decay.stride(0), _ptr(w0), _ptr(u), _ptr(state),
              state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim, key_dim,
-             seg_slot.numel(), T, code(r.dtype), _stream()), "time_mixing_scan")
+             seg_slot.numel(), T, code(r.dtype), int(state_ahead), _stream()), "time_mixing_scan")
 
 
 GATES = {"silu": 0, "sigmoid": 1}
@@ -949,13 +964,16 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
                 c_rows: Optional[torch.Tensor] = None, row_scale: Optional[torch.Tensor] = None,
                 rows: Optional[int] = None, glu: bool = False, act: str = "silu",
                 act_alpha: float = 1.702, act_limit: float = 7.0, rows_per_pass: int = 8,
-                unary: Optional[str] = None, bias: Optional[torch.Tensor] = None, group_rows: int = 0) -> None:
+                unary: Optional[str] = None, bias: Optional[torch.Tensor] = None, group_rows: int = 0,
+                lists_ahead: bool = False) -> None:
     """c = a @ w^T for few rows, streaming bfloat16 weights once through
     mma.sync; same conventions as :func:`gemm_rows`.  ``unary`` (one of
     :data:`ACTIVATIONS`, without ``glu``): that function of the float32 accumulator is stored; ``bias``
     (float32 ``[N]``, without ``glu``) is added to the accumulator first.  ``group_rows``: ``w`` is ``[G, N, K]``
     and rows ``g * group_rows ..`` of ``a`` and ``c`` belong to matrix g.  With ``glu``, ``act`` may be
-    ``silu``, ``swigluoai`` or ``gelu_tanh``."""
+    ``silu``, ``swigluoai`` or ``gelu_tanh``.  The kernel fetches its first weights while the launch in front of it
+    still runs: ``w`` is never what that launch writes.  ``lists_ahead`` promises the same of ``group_offsets``, ``active``,
+    ``a_rows`` and ``c_rows``, and lets a grouped product do so too."""
     _need(a, "a", torch.bfloat16, contiguous=False)
     _need(w, "w", torch.bfloat16)
     _need(c, "c", contiguous=False)
@@ -987,11 +1005,12 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
             raise KernelError("skinny_gemm: the active list needs G + 1 entries")
     if unary is not None and (glu or unary not in ACTIVATIONS):
         raise KernelError(f"skinny_gemm: cannot apply {unary!r} (with glu: {glu})")
-    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i")
+    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i")
     _check(f(_ptr(a), a.stride(0), _ptr(w), NW * K, _ptr(c), code(c.dtype), c.stride(0),
              _ptr(group_offsets), _ptr(active), _ptr(a_rows), _ptr(c_rows), _ptr(row_scale), M, N, K, G,
              int(glu), GLU_ACTS[act], float(act_alpha), float(act_limit),
-             rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], _ptr(bias), int(group_rows), _stream()),
+             rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], _ptr(bias), int(group_rows),
+             int(lists_ahead), _stream()),
            "skinny_gemm")
 
 

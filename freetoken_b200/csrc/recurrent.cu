@@ -28,6 +28,7 @@ struct ConvArgs {
   long long ldx, ldo, slot_stride;
   int C, taps;
   int act;              // 1: SiLU behind the sum; 0: the sum itself
+  int state_ahead;      // the launch right in front does not write the state: it is fetched ahead of the wait
 };
 
 constexpr int CONV_MAX_TAPS = 8;     // longer convolutions take the plain loop
@@ -149,11 +150,13 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(ConvArgs a, int T) {
 // value read twice.  (One row of 6,144 channels: 2.6 us instead of 2.8 + 2.4.)  It walks whatever tokens the segment has.
 template <typename AT, int CPT>
 __global__ void __launch_bounds__(128) conv_step_kernel(ConvArgs a) {
-  pdl_wait();
+  if (!a.state_ahead) pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * CPT, seg = blockIdx.x;
-  if (c >= a.C) return;
   const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1], K = a.taps - 1;
-  if (q1 <= q0) return;
+  if (c >= a.C || q1 <= q0) {
+    if (a.state_ahead) pdl_wait();
+    return;
+  }
   const AT* x = (const AT*)a.x;
   float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + c;
   float w[CPT][CONV_MAX_TAPS], win[CPT][CONV_MAX_TAPS], bias[CPT];
@@ -166,6 +169,7 @@ __global__ void __launch_bounds__(128) conv_step_kernel(ConvArgs a) {
       if (j < K) win[u][j] = st[(size_t)j * a.C + u];
     }
   }
+  if (a.state_ahead) pdl_wait();
   for (int t = q0; t < q1; ++t) {
     float own[CPT];
     if constexpr (CPT == 2) {
@@ -251,6 +255,7 @@ struct SsdArgs {
   long long ld, ld_dt, slot_stride;
   int heads, P, N, G;
   int vec;              // state rows may be read in 16-byte (WC % 4 == 0) or 8-byte pieces
+  int state_ahead;      // the launch right in front does not write the state: it is fetched ahead of the wait
 };
 
 // NPL: state rows a lane holds (N <= 32 * NPL); WC: state columns a warp owns
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
   constexpr int NB = (NPL * 32 + SCAN_THREADS - 1) / SCAN_THREADS;       // B (or C) values a thread stages per token
   constexpr int XR = (SCAN_CHUNK * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
   extern __shared__ float sm[];
-  pdl_wait();
+  if (!a.state_ahead) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int head = blockIdx.y, seg = blockIdx.z;
   const int N = a.N, P = a.P;
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
       for (int c = 0; c < WC; ++c) S[e][c] = 0.f;
     }
   }
+  if (a.state_ahead) pdl_wait();
 
   AT pb[SCAN_CHUNK][NB], pc[SCAN_CHUNK][NB], px[XR], pdt;
   auto fetch = [&](int t0, int nt) {
@@ -597,10 +603,11 @@ int ft_conv_groups(int C, int T, int S, int taps, int pairs) { return conv_group
 // Both kernels of the short convolution: outputs first, then the slots' new contents.
 int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const float* w, const float* bias,
                  float* state, long long slot_stride, const int* token_seg, const int* seg_slot,
-                 const int* seg_q_start, int C, int taps, int T, int S, int dtype, int act, cudaStream_t stream) {
+                 const int* seg_q_start, int C, int taps, int T, int S, int dtype, int act, int state_ahead,
+                 cudaStream_t stream) {
   if (T <= 0 || S <= 0) return FT_OK;
   if (C <= 0 || taps < 1) return FT_ERR_SHAPE;
-  ConvArgs a{x, out, w, bias, state, token_seg, seg_slot, seg_q_start, ldx, ldo, slot_stride, C, taps, act};
+  ConvArgs a{x, out, w, bias, state, token_seg, seg_slot, seg_q_start, ldx, ldo, slot_stride, C, taps, act, state_ahead};
   const int cb = (C + 127) / 128;
   const bool pairs = dtype == FT_DTYPE_BF16 && !(C & 1) && !(ldx & 1) && !(ldo & 1) && !((uintptr_t)x & 3) &&
                      !((uintptr_t)out & 3);
@@ -642,10 +649,10 @@ int ft_conv_silu(const void* x, long long ldx, void* out, long long ldo, const f
 int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, const float* dt_bias,
                 const float* A_log, const float* D, float* state, long long slot_stride, float* y,
                 const int* seg_slot, const int* seg_q_start, int heads, int P, int N, int G, int S,
-                int T, int longest, int dtype, cudaStream_t stream) {
+                int T, int longest, int dtype, int state_ahead, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || N <= 0 || N > 256 || G <= 0 || heads % G) return FT_ERR_SHAPE;
-  SsdArgs a{xbc, dt, dt_bias, A_log, D, state, y, seg_slot, seg_q_start, ld, ld_dt, slot_stride, heads, P, N, G, 0};
+  SsdArgs a{xbc, dt, dt_bias, A_log, D, state, y, seg_slot, seg_q_start, ld, ld_dt, slot_stride, heads, P, N, G, 0, state_ahead};
   int rc = FT_OK;
   const bool narrow = narrow_warps(P, heads, S);
   if (seq_scan(SCAN_SSD, dtype == FT_DTYPE_F32, heads, P, N, S, T, longest)) {

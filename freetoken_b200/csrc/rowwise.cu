@@ -523,14 +523,25 @@ struct NormAddArgs {
 // aligned: each row is read once, in 16-byte pieces, and stays in registers between the passes; the branch
 // rows, the residual and both weights are fetched before the first sum, all loads in flight together.
 // KEEP = 0: any row, element by element through shared memory.
-// EAGER (up to 64 tokens): the next norm's weight - cold in L2, the step's weights have been through it - is fetched
-// with the rest instead of under the second sum: a row of 2,048 values 4.5 -> 3.8 us.
+// EAGER (up to 64 tokens): both weights - cold in L2, the step's weights have been through it - are fetched ahead of the
+// wait for the launch in front (with the rest instead of under the second sum: a row of 2,048 values 4.5 -> 3.8 us).
 template <typename AT, int KEEP, bool EAGER = false>
 __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
-  pdl_wait();
   const int t = blockIdx.x, H = a.H;
+  float4 w[KEEP > 0 ? KEEP : 1], w_next[EAGER ? KEEP : 1];
+  if constexpr (EAGER) {
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int gi = threadIdx.x + j * 256;
+      if (gi < (H >> 2)) {
+        w[j] = ld_ahead4(a.weight + 4 * gi);
+        if (a.next_weight) w_next[j] = ld_ahead4(a.next_weight + 4 * gi);
+      }
+    }
+  }
+  pdl_wait();
   float* r = a.residual + (size_t)t * H;
   const float one = a.plus_one ? 1.f : 0.f;
   const float one2 = a.next_plus_one ? 1.f : 0.f;
@@ -539,7 +550,7 @@ __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
   AT* o = (AT*)a.next_out + (size_t)t * H;
   float ss = 0.f, ss2 = 0.f;
   if constexpr (KEEP > 0) {
-    float4 keep[KEEP], x0[KEEP], w[KEEP], w_next[EAGER ? KEEP : 1];
+    float4 keep[KEEP], x0[KEEP];
     const int groups = H >> 2;
     float back;
     const unsigned slots = branch_slots(a.b, t, back);
@@ -548,10 +559,8 @@ __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
       const int gi = threadIdx.x + j * 256;
       if (gi < groups) {
         x0[j] = load4f(r + 4 * gi);
-        w[j] = load4f(a.weight + 4 * gi);
-        if constexpr (EAGER) {
-          if (a.next_weight) w_next[j] = load4f(a.next_weight + 4 * gi);
-        } else {
+        if constexpr (!EAGER) {
+          w[j] = load4f(a.weight + 4 * gi);
           keep[j] = branch_at4<AT>(a.b, t, H, gi, slots, back);
         }
       }
@@ -634,33 +643,36 @@ struct JoinNormArgs {
   float eps1, eps2;
 };
 
-// EAGER (few tokens): the weights are fetched with the rows, before the sums.
+// EAGER (few tokens): the weights are fetched ahead of the wait for the launch in front.
 template <typename AT, int KEEP, int THREADS, bool EAGER = false>
 __global__ void __launch_bounds__(THREADS) join_layer_norm_kernel(JoinNormArgs a) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
-  pdl_wait();
   const int t = blockIdx.x, H = a.H;
+  float4 e1[EAGER ? KEEP : 1], e2[EAGER ? KEEP : 1];
+  if constexpr (EAGER) {
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int gi = threadIdx.x + j * THREADS;
+      e1[j] = e2[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (gi < (H >> 2)) {
+        e1[j] = ld_ahead4(a.w1 + 4 * gi);
+        if (a.w2) e2[j] = ld_ahead4(a.w2 + 4 * gi);
+        if (a.b1) warm(a.b1 + 4 * gi);
+        if (a.b2) warm(a.b2 + 4 * gi);
+      }
+    }
+  }
+  pdl_wait();
   float* r = a.residual + (size_t)t * H;
   AT* o1 = (AT*)a.out1 + (size_t)t * H;
   AT* o2 = (AT*)a.out2 + (size_t)t * H;
   const bool two = a.w2 != nullptr;
   float sum = 0.f, sq = 0.f;
   if constexpr (KEEP > 0) {
-    float4 x[KEEP], e1[EAGER ? KEEP : 1], e2[EAGER ? KEEP : 1];
+    float4 x[KEEP];
     const int groups = H >> 2;
     float back = 0.f;
-    if constexpr (EAGER) {
-#pragma unroll
-      for (int j = 0; j < KEEP; ++j) {
-        const int gi = threadIdx.x + j * THREADS;
-        e1[j] = e2[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gi < groups) {
-          e1[j] = load4f(a.w1 + 4 * gi);
-          if (two) e2[j] = load4f(a.w2 + 4 * gi);
-        }
-      }
-    }
     const unsigned slots = a.b.rows ? branch_slots(a.b, t, back) : 0u;
     constexpr bool ALL = EAGER && KEEP == 2;       // one piece a thread gains nothing, four do not fit the registers
     float4 zs[ALL ? KEEP : 1];
@@ -896,8 +908,8 @@ hyper_norm_kernel(float* __restrict__ streams, const AT* __restrict__ branch, in
 // between the passes.  The sums run in the order of the generic kernel.
 // EAGER (up to 64 tokens, where a launch is one row's latency): the branch's partial rows are fetched two or four at a
 // time, for all of a thread's pieces together, and weight and bias - cold in L2, the step's weights have been through
-// it - before the sums instead of behind them: four rows of 4 x 4,096 values 7.1 -> 4.9 us, one to eight of 4 x 2,048
-// 4.4 -> 3.7.  With every SM full of rows those registers would cost occupancy.
+// it - ahead of the wait for the launch in front (before the sums instead of behind them: four rows of 4 x 4,096 values 7.1 -> 4.9 us, one to eight of 4 x 2,048
+// 4.4 -> 3.7).  With every SM full of rows those registers would cost occupancy.
 template <typename AT, int S, int KEEP, bool EAGER>
 __global__ void __launch_bounds__(256)
 hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch, int k, const float* __restrict__ mix,
@@ -905,19 +917,30 @@ hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch
                       const float* __restrict__ weight, const float* __restrict__ bias, float eps, int center,
                       AT* __restrict__ normed, int H) {
   __shared__ float scratch[33];
-  pdl_wait();
   const int t = blockIdx.x, groups = H >> 2;
   float m[S * S], ow[S], rd[S];
+  float4 w_early[EAGER ? KEEP : 1], b_early[EAGER ? KEEP : 1];
 #pragma unroll
-  for (int i = 0; i < S * S; ++i) m[i] = branch ? mix[i] : 0.f;
+  for (int i = 0; i < S * S; ++i) m[i] = branch ? ld_ahead(mix + i) : 0.f;
 #pragma unroll
   for (int i = 0; i < S; ++i) {
-    ow[i] = branch ? out_w[i] : 0.f;
-    rd[i] = read ? read[i] : 1.f;
+    ow[i] = branch ? ld_ahead(out_w + i) : 0.f;
+    rd[i] = read ? ld_ahead(read + i) : 1.f;
   }
+  if constexpr (EAGER) {
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int gi = threadIdx.x + j * 256;
+      if (gi < groups && normed) {
+        w_early[j] = ld_ahead4(weight + 4 * gi);
+        b_early[j] = bias ? ld_ahead4(bias + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
+  pdl_wait();
   float* x = streams + (size_t)t * S * H;
   const AT* y_rows = branch ? branch + (size_t)t * k * H : nullptr;
-  float4 xs[KEEP][S], y[KEEP], w_early[EAGER ? KEEP : 1], b_early[EAGER ? KEEP : 1];
+  float4 xs[KEEP][S], y[KEEP];
 #pragma unroll
   for (int j = 0; j < KEEP; ++j) {
     const int gi = threadIdx.x + j * 256;
@@ -925,12 +948,6 @@ hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch
     if (gi < groups) {
 #pragma unroll
       for (int s_ = 0; s_ < S; ++s_) xs[j][s_] = load4f(x + (size_t)s_ * H + 4 * gi);
-      if constexpr (EAGER) {
-        if (normed) {
-          w_early[j] = load4f(weight + 4 * gi);
-          b_early[j] = bias ? load4f(bias + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
       if (branch && !EAGER) {
         for (int q = 0; q < k; ++q) {
           const float4 v = load4f(y_rows + (size_t)q * H + 4 * gi);
@@ -1058,6 +1075,7 @@ __global__ void __launch_bounds__(128)
 rms_rows_kernel(const AT* __restrict__ x, long long ldx, const float* __restrict__ w, AT* __restrict__ out,
                 long long ldo, int n, float eps) {
   __shared__ float scratch[33];
+  for (int c = threadIdx.x * 32; c < n; c += blockDim.x * 32) warm(w + c);
   pdl_wait();
   const AT* row = x + (size_t)blockIdx.x * ldx;
   float sq = 0.f;
@@ -1098,11 +1116,16 @@ struct LatentStoreArgs {
 template <typename AT>
 __global__ void __launch_bounds__(128) latent_store_kernel(LatentStoreArgs a) {
   __shared__ float scratch[33];
-  pdl_wait();
   const int t = blockIdx.x;
   const int pos = a.token_pos[t];
   const int half = a.rot >> 1;
   const float* cs = a.cos_sin + (size_t)pos * a.rot;
+  const bool stores = a.pages && blockIdx.y == 0;
+  const int page = stores ? a.block_table[(size_t)a.token_seg[t] * a.table_width + pos / a.P] : 0;
+  for (int i = threadIdx.x * 32; i < a.rot; i += blockDim.x * 32) warm(cs + i);
+  if (stores)
+    for (int i = threadIdx.x * 32; i < a.rank; i += blockDim.x * 32) warm(a.weight + i);
+  pdl_wait();
   auto turn = [&](const AT* src, AT* dst, AT* self, int i) {       // pair i of a rotated part
     const int ia = a.interleaved ? 2 * i : i, ib = a.interleaved ? 2 * i + 1 : i + half;
     const float u = to_float(src[ia]), v = to_float(src[ib]);
@@ -1123,9 +1146,8 @@ __global__ void __launch_bounds__(128) latent_store_kernel(LatentStoreArgs a) {
       turn(tail, qa ? qa + (size_t)h * width + a.rank : nullptr, a.turn_q ? tail : nullptr, p);
     }
   }
-  if (!a.pages || blockIdx.y > 0) return;
+  if (!stores) return;
   const AT* down = (const AT*)a.down + (size_t)t * a.ld_down;
-  const int page = a.block_table[(size_t)a.token_seg[t] * a.table_width + pos / a.P];
   AT* dst = (AT*)a.pages + (size_t)page * a.page_stride + (size_t)(pos % a.P) * width;
   float sq = 0.f;
   for (int c = threadIdx.x; c < a.rank; c += blockDim.x) {

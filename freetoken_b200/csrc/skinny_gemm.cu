@@ -42,6 +42,8 @@ struct SkinnyArgs {
   int unary = 0;             // without GLU: 0 nothing, 1 relu(x)^2, 2 tanh-GELU, 3 SiLU, 5 tanh on the accumulator
   const float* bias = nullptr;   // [N], added to the accumulator (not with GLU)
   int group_rows = 0;            // > 0: every group has that many rows, group g the rows g * group_rows ..
+  int lists_ahead = 0;           // the lists were written before the launch right in front of this one began
+  int first_round = 0;           // blocks that find a place on the chip at once
 };
 
 // Plain loads with a memory clobber, and a warp barrier behind a round's loads (skinny_kernel): the compiler may not
@@ -102,11 +104,19 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
   constexpr int NG = GLU ? 2 : 1;
   __shared__ float red[KS][NT][NG][16][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  pdl_wait();
+  // Weights are nobody's output: the first round of them is under way before the wait for the launch in front,
+  // whose end this block would otherwise only idle through.  Later blocks find that launch at its end, and a wait
+  // between their loads would only hold the second half up (the head, 12,504 blocks: 176 -> 194 us).
+  const bool ahead = (int)(blockIdx.y * gridDim.x + blockIdx.x) < a.first_round &&
+                     (a.lists_ahead || (!a.active && !a.group_offsets));
+  if (!ahead) pdl_wait();
 
   int group = blockIdx.y;
   if (a.active) {
-    if ((int)blockIdx.y >= a.active[a.G]) return;
+    if ((int)blockIdx.y >= a.active[a.G]) {
+      if (ahead) pdl_wait();
+      return;
+    }
     group = a.active[blockIdx.y];
   }
   int row_begin = 0, row_end = a.M;
@@ -118,7 +128,10 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
     row_begin = a.group_offsets[group];
     row_end = a.group_offsets[group + 1];
   }
-  if (row_end <= row_begin) return;
+  if (row_end <= row_begin) {
+    if (ahead) pdl_wait();
+    return;
+  }
   const int n0 = blockIdx.x * 16;
   const __nv_bfloat16* W = a.W + (size_t)group * a.w_group_stride;
   const int K = a.K;
@@ -139,6 +152,24 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
   const int per = (chunks + KS - 1) / KS;
   const int c_begin = warp * per, c_end = min(chunks, c_begin + per);
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 wv[U][NG][2];
+  auto fetch_weights = [&](int c) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k8 = ((c + u) << 2) + t;  // index in units of 8 elements
+      const bool kin = (c + u) < c_end && (k8 << 3) < K;
+#pragma unroll
+      for (int q = 0; q < NG; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          wv[u][q][h] = (kin && wvalid[h]) ? ld_stream(wrow[q][h] + k8) : zero;
+    }
+  };
+  bool fetched = ahead;
+  if (ahead) {
+    fetch_weights(c_begin);
+    pdl_wait();
+  }
 
   for (int pass = row_begin; pass < row_end; pass += 8 * NT) {
     const uint4* xrow[NT];
@@ -160,22 +191,18 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
         for (int i = 0; i < 4; ++i) acc[q][j][i] = 0.f;
 
     for (int c = c_begin; c < c_end; c += U) {
-      uint4 wv[U][NG][2];
       uint4 xv[U][NT];
+      if (!fetched) fetch_weights(c);
+      fetched = false;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int k8 = ((c + u) << 2) + t;  // index in units of 8 elements
+        const int k8 = ((c + u) << 2) + t;
         const bool kin = (c + u) < c_end && (k8 << 3) < K;
 #pragma unroll
-        for (int q = 0; q < NG; ++q)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            wv[u][q][h] = (kin && wvalid[h]) ? ld_stream(wrow[q][h] + k8) : zero;
-#pragma unroll
         for (int j = 0; j < NT; ++j)
-          xv[u][j] = (kin && xrow[j]) ? (U == 8 ? ld_rows(xrow[j] + k8) : __ldg(xrow[j] + k8)) : zero;
+          xv[u][j] = (kin && xrow[j]) ? (U >= 4 ? ld_rows(xrow[j] + k8) : __ldg(xrow[j] + k8)) : zero;
       }
-      if constexpr (U == 8) __syncwarp();
+      if constexpr (U >= 4) __syncwarp();
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -232,16 +259,26 @@ static bool eight_chunks(long long blocks, int ks, int K, bool experts) {
   if (blocks <= 148 * (16 / ks)) return true;
   return experts ? per >= 21 && blocks > 1300 : blocks > 148 * (ks == 8 ? 3 : 28 / ks);
 }
+template <int NT, bool GLU, typename OT, int KS, int U>
+void launch_one(SkinnyArgs a, dim3 grid, cudaStream_t stream) {
+  static const int resident = [] {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, skinny_kernel<NT, GLU, OT, KS, U>, KS * 32, 0) == cudaSuccess
+               ? 148 * n : 0;
+  }();
+  a.first_round = resident;
+  launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
+}
 template <int NT, bool GLU, typename OT, int KS>
 void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream) {
   constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);
   if constexpr (NT == 1 && !GLU && KS >= 4) {
     if (eight_chunks((long long)grid.x * grid.y, KS, a.K, a.group_offsets != nullptr)) {
-      launch_pdl(skinny_kernel<NT, GLU, OT, KS, 8>, grid, dim3(KS * 32), 0, stream, a);
+      launch_one<NT, GLU, OT, KS, 8>(a, grid, stream);
       return;
     }
   }
-  launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
+  launch_one<NT, GLU, OT, KS, U>(a, grid, stream);
 }
 template <bool GLU, typename OT, int KS>
 int launch_nt(const SkinnyArgs& a, int nt, dim3 grid, cudaStream_t stream) {
@@ -286,7 +323,7 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
                               const int* group_offsets, const int* active, const int* a_rows,
                               const int* c_rows, const float* row_scale, int M, int N, int K, int G, int glu,
                               int act, float act_alpha, float act_limit, int rows_per_pass, int unary,
-                              const float* bias, int group_rows, cudaStream_t stream) {
+                              const float* bias, int group_rows, int lists_ahead, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return FT_OK;
   if (K <= 0 || (K & 7) || (lda & 7) || G <= 0) return FT_ERR_SHAPE;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((w_group_stride * 2) & 15)) return FT_ERR_SHAPE;
@@ -298,6 +335,7 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
   a.unary = unary;
   a.bias = bias;
   a.group_rows = group_rows;
+  a.lists_ahead = lists_ahead;
   // with the list of busy groups, no more groups than rows can have any
   dim3 grid((N + 15) / 16, active ? min(G, M) : G);
   const int nt = rows_per_pass / 8;

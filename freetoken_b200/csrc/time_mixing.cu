@@ -131,6 +131,7 @@ struct TimeMixArgs {
   const int* seg_q_start;
   long long ld, ld_decay, slot_stride;
   int heads, P, D, vec;    // vec: state rows may be read in 16-byte pieces
+  int state_ahead;         // the launch right in front does not write the state: it is fetched ahead of the wait
 };
 
 constexpr int time_mix_buffer(int RPL, int LPC, int CPL) { return TM_CHUNK * (3 * LPC * RPL + CPL * TM_THREADS / LPC + 1); }
@@ -359,12 +360,15 @@ __global__ void __launch_bounds__(128) time_mixing_step_kernel(TimeMixArgs a) {
   constexpr int CPW = 32 / LPC;
   constexpr int LOG = LPC == 8 ? 3 : 4;
   static_assert(CPL <= LPC, "a lane per column when they are added up");
-  pdl_wait();
+  if (!a.state_ahead) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = lane & (LPC - 1);
   const int head = blockIdx.y, seg = blockIdx.z;
   const int D = a.D, P = a.P;
   const int col0 = (blockIdx.x * 4 + warp) * CPL * CPW + (lane >> LOG);       // columns col0 + c * CPW
-  if ((blockIdx.x * 4 + warp) * CPL * CPW >= P) return;                        // the whole warp leaves
+  if ((blockIdx.x * 4 + warp) * CPL * CPW >= P) {                              // the whole warp leaves
+    if (a.state_ahead) pdl_wait();
+    return;
+  }
   const size_t t = a.seg_q_start[seg];
   float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * P * D;
   const AT* rp = (const AT*)a.r + t * a.ld + (size_t)head * D;
@@ -392,6 +396,7 @@ __global__ void __launch_bounds__(128) time_mixing_step_kernel(TimeMixArgs a) {
         }
       }
     }
+  if (a.state_ahead) pdl_wait();
   float v[CPL];
 #pragma unroll
   for (int c = 0; c < CPL; ++c) v[c] = col0 + c * CPW < P ? to_float(vp[col0 + c * CPW]) : 0.f;
@@ -540,10 +545,10 @@ int ft_token_shift(const void* x, long long ldx, const float* mu, void* out, flo
 int ft_time_mixing_scan(const void* r, const void* k, const void* v, long long ld, const float* decay,
                         long long ld_decay, const float* w0, const float* u, float* state, long long slot_stride,
                         float* o, const int* seg_slot, const int* seg_q_start, int heads, int P, int D, int S, int T,
-                        int dtype, cudaStream_t stream) {
+                        int dtype, int state_ahead, cudaStream_t stream) {
   if (S <= 0) return FT_OK;
   if (heads <= 0 || P <= 0 || D <= 0 || D > 256 || heads > 65535 || S > 65535) return FT_ERR_SHAPE;
-  TimeMixArgs a{r, k, v, decay, w0, u, state, o, seg_slot, seg_q_start, ld, ld_decay, slot_stride, heads, P, D, 0};
+  TimeMixArgs a{r, k, v, decay, w0, u, state, o, seg_slot, seg_q_start, ld, ld_decay, slot_stride, heads, P, D, 0, state_ahead};
   a.vec = !(D & 3) && !(slot_stride & 3) && !((uintptr_t)state & 15);
   int rc = FT_OK;
   if (T == S) {                                        // one token a segment

@@ -355,7 +355,7 @@ class PagedAttention(PagedSoftmaxCore, Mixer):
             if not cache.writes:
                 raise ValueError("a mixer with a convolution's state cannot read another stop's cache")
             ops.conv_silu(qkv, mixed, self.w_conv, None, conv.state, ctx.token_seg, ctx.seg_slot, ctx.seg_q_start,
-                          activation=False)
+                          activation=False, state_ahead=True)
             qkv = mixed
         elif self.taps == 1:
             # one tap: a factor per channel, nothing carried from step to step

@@ -256,7 +256,7 @@ class RoutedExperts(FeedForward):
                             act_limit=self.act_limit, rows_per_pass=per_pass)
             ops.skinny_gemm(mid, self.w_down, parts, group_offsets=offsets, active=active,
                             c_rows=sorted_route,
-                            row_scale=route_weight, rows=R, rows_per_pass=per_pass)
+                            row_scale=route_weight, rows=R, rows_per_pass=per_pass, lists_ahead=True)
             return
         ops.gemm_rows(x, self.w_gate_up, mid, group_offsets=offsets, a_rows=sorted_token, rows=R,
                       glu=True, act=self.act, act_alpha=self.act_alpha, act_limit=self.act_limit)

@@ -122,10 +122,10 @@ class SelectiveStateSpace(_Recurrent):
         proj = linear.linear(x, w["in"], ws.get("ssd.in", (T, inner + C + self.heads), ctx.dtype))
         xbc = ws.get("ssd.xbc", (T, C), ctx.dtype)
         ops.conv_silu(proj[:, inner:inner + C], xbc, w["conv"], w["conv_bias"], conv_state, ctx.token_seg,
-                      ctx.seg_slot, ctx.seg_q_start)
+                      ctx.seg_slot, ctx.seg_q_start, state_ahead=True)
         y = ws.get("ssd.y", (T, inner), torch.float32)
         ops.ssd_scan(xbc, proj[:, inner + C:], w["dt_bias"], w["a_log"], w["d"], state, y, ctx.seg_slot,
-                     ctx.seg_q_start, self.heads, self.P, self.N, self.G, ctx.max_q_len)
+                     ctx.seg_q_start, self.heads, self.P, self.N, self.G, ctx.max_q_len, state_ahead=True)
         gated = ws.get("ssd.gated", (T, inner), ctx.dtype)
         ops.gated_norm(y, proj[:, :inner], w["norm"], gated, self.norm_groups, self.eps, gate_first=True)
         if out is None:
@@ -191,12 +191,12 @@ class GatedDelta(_Recurrent):
         proj = linear.linear(x, w["in"], ws.get("delta.in", (T, C + inner + 2 * heads), ctx.dtype))
         qkv = ws.get("delta.qkv", (T, C), ctx.dtype)
         ops.conv_silu(proj[:, :C], qkv, w["conv"], None, conv_state, ctx.token_seg, ctx.seg_slot,
-                      ctx.seg_q_start)
+                      ctx.seg_q_start, state_ahead=True)
         o = ws.get("delta.o", (T, inner), torch.float32)
         gates = C + inner
         ops.delta_scan(qkv, proj[:, gates:gates + heads], proj[:, gates + heads:], w["dt_bias"], w["a_log"],
                        state, o, ctx.seg_slot, ctx.seg_q_start, heads, self.G, self.D, self.P, self.unit_eps,
-                       self.D ** -0.5, ctx.max_q_len)
+                       self.D ** -0.5, ctx.max_q_len, state_ahead=True)
         gated = ws.get("delta.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, proj[:, C:C + inner], w["norm"], gated, heads, self.eps, gate_first=False)
         if out is None:
@@ -270,7 +270,7 @@ class ChannelDelta(_Recurrent):
         proj = linear.linear(x, w["in"], ws.get("cdelta.in", (T, C + both + heads), ctx.dtype))
         qkv = ws.get("cdelta.qkv", (T, C), ctx.dtype)
         ops.conv_silu(proj[:, :C], qkv, w["conv"], None, conv_state, ctx.token_seg, ctx.seg_slot,
-                      ctx.seg_q_start)
+                      ctx.seg_q_start, state_ahead=True)
         # the decay's second step leaves its float32 accumulator: softplus and exp follow in float32
         decay = linear.linear(proj[:, C:C + low], w["decay_up"], ws.get("cdelta.decay", (T, heads * self.D),
                                                                         torch.float32))
@@ -278,7 +278,7 @@ class ChannelDelta(_Recurrent):
         o = ws.get("cdelta.o", (T, inner), torch.float32)
         ops.channel_delta_scan(qkv, proj[:, C + both:], decay, w["dt_bias"], w["a_log"], state, o, ctx.seg_slot,
                                ctx.seg_q_start, heads, self.G, self.D, self.P, self.unit_eps, self.D ** -0.5,
-                               ctx.max_q_len)
+                               ctx.max_q_len, state_ahead=True)
         gated = ws.get("cdelta.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, gate, w["norm"], gated, heads, self.eps, gate_first=False, gate_kind="sigmoid")
         if out is None:
@@ -347,7 +347,7 @@ class Retention(_Recurrent):
         o = ws.get("retention.o", (T, inner), torch.float32)
         ops.retention_scan(proj[:, :2 * kd + inner], self.decay, self.position.table(ctx.device, ctx.max_positions),
                            ctx.seg_pos0, state, o, ctx.seg_slot, ctx.seg_q_start, self.heads, self.D, self.P,
-                           self.D ** -0.5, ctx.max_q_len)
+                           self.D ** -0.5, ctx.max_q_len, state_ahead=True)
         gated = ws.get("retention.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, proj[:, 2 * kd + inner:], self.ones, gated, self.heads, self.eps, gate_first=False)
         if out is None:
@@ -426,7 +426,7 @@ class TimeMixing(Mixer):
         decay = linear.linear(low, w["decay_up"], ws.get("tmix.decay", (T, inner), torch.float32))
         o = ws.get("tmix.o", (T, inner), torch.float32)
         ops.time_mixing_scan(rkvg[0], rkvg[1], rkvg[2], decay, w["w0"], w["u"], state, o, ctx.seg_slot, ctx.seg_q_start,
-                             self.heads, self.P, self.D)
+                             self.heads, self.P, self.D, state_ahead=True)
         gated = ws.get("tmix.gated", (T, inner), ctx.dtype)
         ops.gated_norm(o, rkvg[3], w["norm"], gated, self.heads, self.eps, gate_first=False)
         if out is None:
