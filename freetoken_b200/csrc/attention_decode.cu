@@ -362,3 +362,6 @@ extern "C" int ft_attn_merge(const float* part_o, const float* part_ml, void* ou
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_attn_merge)
+FT_PACKED(ft_attn_decode)

@@ -436,3 +436,5 @@ extern "C" int ft_attn_decode_tma(const void* map_kv, const void* q, void* out, 
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_attn_decode_tma)

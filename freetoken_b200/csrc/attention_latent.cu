@@ -508,3 +508,5 @@ int ft_attn_latent(const void* q, void* out, long long ldo, float* part_o, float
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_attn_latent)

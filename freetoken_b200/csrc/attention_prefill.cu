@@ -265,3 +265,5 @@ extern "C" int ft_attn_prefill(const void* q, void* out, const void* kv, const i
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_attn_prefill)

@@ -472,3 +472,6 @@ int ft_attn_prefill_mha(const void* map_q, const void* map_k, const void* map_r,
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_latent_gather)
+FT_PACKED(ft_attn_prefill_mha)

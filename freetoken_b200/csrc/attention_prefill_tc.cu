@@ -562,3 +562,5 @@ int ft_attn_prefill_tc(const void* map_q, const void* map_q2, const void* map_kv
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_attn_prefill_tc)

@@ -352,3 +352,5 @@ extern "C" int ft_attn_paged_simt(const void* q, void* out, const void* kv_pages
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_attn_paged_simt)

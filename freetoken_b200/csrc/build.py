@@ -16,11 +16,14 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -171,6 +174,54 @@ def drop_stale(folder: str, name: str, keep: str) -> List[str]:
     return removed
 
 
+HOST_SOURCE = "host_call.c"
+HOST_FLAGS = ["-O2", "-fPIC", "-shared"]
+
+
+def host_path(folder: Optional[str] = None) -> str:
+    h = hashlib.sha256()
+    with open(os.path.join(HERE, HOST_SOURCE), "rb") as f:
+        h.update(f.read())
+    h.update(" ".join(HOST_FLAGS + [sys.implementation.cache_tag]).encode())
+    return os.path.join(folder or build_dir(), f"libft_host_{h.hexdigest()[:16]}.so")
+
+
+def _compile_host(out: str) -> None:
+    """The host module is plain C against the interpreter's headers; nvcc's own host compiler takes it."""
+    cc = shutil.which(os.environ.get("CC", "gcc")) or shutil.which("cc")
+    if cc is None:
+        raise BuildError("the host side of a launch is not built and no C compiler was found (looked for $CC, gcc and cc)")
+    tmp = f"{out}.{os.getpid()}.{threading.get_ident()}.tmp"
+    cmd = [cc] + HOST_FLAGS + ["-I", sysconfig.get_paths()["include"], "-o", tmp, os.path.join(HERE, HOST_SOURCE)]
+    done = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if done.returncode != 0:
+        raise BuildError(f"{cc} failed for {HOST_SOURCE}:\n{done.stdout}")
+    os.replace(tmp, out)
+    drop_stale(os.path.dirname(out), "host", out)
+
+
+_host_lock = threading.Lock()
+_host_module = None
+
+
+def load_host():
+    """The compiled module between the ops' Python faces and their launchers, built first if need be."""
+    global _host_module
+    with _host_lock:
+        if _host_module is None:
+            path = host_path()
+            if not os.path.exists(path):
+                _compile_host(path)
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("ft_host", path)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("ft_host", loader))
+                loader.exec_module(module)
+            except ImportError as exc:
+                raise BuildError(f"cannot load {path}: {exc}") from exc
+            _host_module = module
+    return _host_module
+
+
 _loaded: Dict[str, ctypes.CDLL] = {}
 _locks: Dict[str, threading.Lock] = {}
 _global_lock = threading.Lock()
@@ -181,6 +232,7 @@ def ensure_built(names: Optional[Iterable[str]] = None, verbose_ptxas: bool = Fa
     parallel.  Returns the library paths."""
     names = list(names) if names is not None else list(LIBRARIES)
     folder = build_dir()
+    load_host()
     todo = [n for n in names if verbose_ptxas or not os.path.exists(library_path(n, folder))]
     if todo:
         with ThreadPoolExecutor(max_workers=min(len(todo), os.cpu_count() or 4)) as pool:

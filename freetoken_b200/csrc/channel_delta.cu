@@ -15,3 +15,5 @@ extern "C" int ft_channel_delta_scan(const void* qkv, long long ld, const void* 
               heads, P, D, G, unit_eps, q_scale, 0, decay, ld_decay, nullptr, nullptr, 0, state_ahead};
   return dispatch_delta<1>(a, S, T, longest, dtype, stream);
 }
+
+FT_PACKED(ft_channel_delta_scan)

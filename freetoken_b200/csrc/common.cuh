@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <utility>
 
 #define FT_DTYPE_F32 0
 #define FT_DTYPE_BF16 1
@@ -133,6 +134,27 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// The packed form of an extern "C" launcher: the arguments in an array of 8-byte words, taken apart by the types of the
+// launcher's own parameters.  FT_PACKED(name), behind the launcher, defines `name_packed`, which the host side calls.
+union PackedArg {
+  void* p;
+  long long i;
+  double f;
+};
+template <typename T> struct Unpack { static T get(const PackedArg& a) { return (T)a.i; } };
+template <typename T> struct Unpack<T*> { static T* get(const PackedArg& a) { return (T*)a.p; } };
+template <> struct Unpack<float> { static float get(const PackedArg& a) { return (float)a.f; } };
+template <typename... P, size_t... I>
+inline int call_packed(int (*f)(P...), const PackedArg* a, std::index_sequence<I...>) {
+  return f(Unpack<P>::get(a[I])...);
+}
+template <typename... P>
+inline int call_packed(int (*f)(P...), const PackedArg* a) {
+  return call_packed(f, a, std::index_sequence_for<P...>());
+}
+#define FT_PACKED(NAME) \
+  extern "C" int NAME##_packed(const ft::PackedArg* a) { return ft::call_packed(NAME, a); }
 
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }

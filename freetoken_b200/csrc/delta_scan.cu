@@ -14,3 +14,5 @@ extern "C" int ft_delta_scan(const void* qkv, long long ld, const void* beta, co
               heads, P, D, G, unit_eps, q_scale, 0, nullptr, 0, nullptr, nullptr, 0, state_ahead};
   return dispatch_delta<0>(a, S, T, longest, dtype, stream);
 }
+
+FT_PACKED(ft_delta_scan)

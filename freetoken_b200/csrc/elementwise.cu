@@ -1044,3 +1044,12 @@ int ft_gather_rows(const void* src, const int* rows, void* dst, int dtype, int n
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_zero_slots)
+FT_PACKED(ft_embed_gather)
+FT_PACKED(ft_patch_tokens)
+FT_PACKED(ft_rmsnorm)
+FT_PACKED(ft_qk_rope_store)
+FT_PACKED(ft_combine)
+FT_PACKED(ft_read_sum)
+FT_PACKED(ft_gather_rows)

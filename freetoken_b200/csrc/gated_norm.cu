@@ -167,3 +167,5 @@ int ft_gated_norm(const float* y, const void* z, long long ldz, const float* wei
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_gated_norm)

@@ -665,3 +665,6 @@ extern "C" int ft_gemm_heads(const void* A, int a_dtype, long long lda, long lon
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_gemm_heads)
+FT_PACKED(ft_gemm_rows)

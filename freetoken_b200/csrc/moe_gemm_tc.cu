@@ -555,3 +555,7 @@ int ft_moe_gemm_tc(const void* map_w, const void* maps_x, void* C, long long ldc
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_wait_selftest)
+FT_PACKED(ft_moe_tile_map)
+FT_PACKED(ft_moe_gemm_tc)

@@ -662,3 +662,8 @@ int ft_moe_sort(const int* ids, int* counts, int* offsets, int* sorted_route, in
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_router_select)
+FT_PACKED(ft_route_small)
+FT_PACKED(ft_router_logits)
+FT_PACKED(ft_moe_sort)

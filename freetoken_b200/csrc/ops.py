@@ -1,7 +1,8 @@
 """Python faces of the CUDA launchers.
 
 Each function checks what the kernel assumes (device, dtype, contiguity,
-sizes), then calls the ``extern "C"`` launcher on the current CUDA stream.  A
+sizes), then calls the ``extern "C"`` launcher on the current CUDA stream, through
+a small compiled module (host_call.c).  A
 non-zero return code raises :class:`KernelError`; nothing here computes on the
 CPU or through a library in a kernel's place.
 """
@@ -18,8 +19,6 @@ from . import build
 
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
-
-_C = {"p": ctypes.c_void_p, "i": ctypes.c_int, "q": ctypes.c_longlong, "f": ctypes.c_float}
 
 
 class KernelError(RuntimeError):
@@ -38,65 +37,65 @@ def code(dtype: torch.dtype) -> int:
 
 
 _bound = {}
+_host = None            # the compiled host side of a launch (host_call.c), loaded with the first of them
 
 # How many of this package's kernels were launched since the counter was last
-# reset; a launcher that starts two kernels counts as two.
+# reset; a launcher that starts two kernels counts as two.  Launches are counted by the
+# host module; here is what is added to its count.
 LAUNCHES = 0
 _KERNELS_PER_CALL = {"ft_moe_sort": 2, "ft_attn_decode": 2}
 
 
 def reset_launch_count() -> None:
     global LAUNCHES
-    LAUNCHES = 0
+    LAUNCHES = -_host.count() if _host is not None else 0
 
 
 def launch_count() -> int:
-    return LAUNCHES
+    return LAUNCHES + (_host.count() if _host is not None else 0)
+
+
+def _host_module():
+    global _host, _need
+    if _host is None:
+        module = build.load_host()
+        module.setup(torch.Tensor, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, KernelError, _ERRORS)
+        _need = module.need
+        _host = module
+    return _host
 
 
 def _fn(lib: str, name: str, sig: str):
+    """The launcher ``name``: called with its arguments as ``sig`` lists them (p: a tensor, None, a buffer or an address; i,
+    q: whole numbers of 32 and 64 bits; f: a float32), without the stream, which is the current one.  Raises
+    :class:`KernelError` on any code but 0."""
     key = (lib, name)
     f = _bound.get(key)
     if f is None:
-        f = getattr(build.load(lib), name)
-        f.argtypes = [_C[c] for c in sig.split()] + [ctypes.c_void_p]
-        f.restype = ctypes.c_int
-        _bound[key] = f
+        address = ctypes.cast(getattr(build.load(lib), name + "_packed"), ctypes.c_void_p).value
+        f = _bound[key] = _host_module().Launcher(address, sig, name, _KERNELS_PER_CALL.get(name, 1))
     return f
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else t.data_ptr()
-
-
-def _stream() -> int:
-    # torch.cuda.current_stream() builds a Stream object and looks its device up anew: 4 us of a launch's 15
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
-
-
-def _check(rc: int, name: str) -> None:
-    global LAUNCHES
-    LAUNCHES += _KERNELS_PER_CALL.get("ft_" + name, 1)
-    if rc != 0:
-        what = _ERRORS.get(rc, f"CUDA error {rc}")
-        raise KernelError(f"{name}: {what}")
-
-
 def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
-    if not t.is_cuda:
-        raise KernelError(f"{name} must be a CUDA tensor")
-    if dtype is not None and t.dtype != dtype:
-        raise KernelError(f"{name} must be {dtype}, is {t.dtype}")
-    if contiguous and not t.is_contiguous():
-        raise KernelError(f"{name} must be contiguous")
+    """``t`` must be a CUDA tensor, of type ``dtype`` if that is given.  (Replaced by the host module's own with the first
+    call.)"""
+    _host_module().need(t, name, dtype, contiguous)
 
 
 def _need_pages(kv_pages: torch.Tensor, dtype) -> None:
     """Pages are ``[2 (K, V), pages, kv_heads, page, head_dim]`` with every plane dense.  A
     cache whose values ARE its keys is one plane seen twice (a stride of 0 between the two)."""
     _need(kv_pages, "kv_pages", dtype, contiguous=False)
-    if kv_pages.dim() != 5 or kv_pages.shape[0] != 2 or not kv_pages[0].is_contiguous() \
-            or kv_pages.stride(0) not in (0, kv_pages[0].numel()):
+    shape, stride = kv_pages.shape, kv_pages.stride()
+    dense = len(shape) == 5 and shape[0] == 2
+    if dense:
+        step = 1                                # the planes' own strides (of a size of 1: any)
+        for n, at in zip(shape[:0:-1], stride[:0:-1]):
+            dense = dense and (n == 1 or at == step or 0 in shape)
+            step *= n
+        dense = dense and stride[0] in (0, step)
+    if not dense:
         raise KernelError("kv_pages must be [2, pages, kv_heads, page, head_dim], planes dense")
 
 
@@ -115,8 +114,7 @@ def zero_slots(state: torch.Tensor, slots: Sequence[int]) -> None:
     f = _fn("elementwise", "ft_zero_slots", "p q q p i i")
     for i in range(0, len(slots), ZERO_SLOTS):
         part = [s % rows for s in slots[i:i + ZERO_SLOTS]]
-        _check(f(_ptr(state), rows * row_bytes, row_bytes, (ctypes.c_int * len(part))(*part), len(part), stops, _stream()),
-               "zero_slots")
+        f(state, rows * row_bytes, row_bytes, (ctypes.c_int * len(part))(*part), len(part), stops)
 
 
 # ------------------------------------------------------------------ rows
@@ -130,8 +128,7 @@ def embed_gather(ids: torch.Tensor, table: torch.Tensor, residual: torch.Tensor)
     if table.shape[1] != H or ids.numel() != T or residual.dim() not in (2, 3):
         raise KernelError("embed_gather: shapes do not match")
     f = _fn("elementwise", "ft_embed_gather", "p p i p i i i i")
-    _check(f(_ptr(ids), _ptr(table), code(table.dtype), _ptr(residual), T, H, table.shape[0], copies,
-             _stream()), "embed_gather")
+    f(ids, table, code(table.dtype), residual, T, H, table.shape[0], copies)
 
 
 def patch_tokens(ids: torch.Tensor, rows: torch.Tensor, src: torch.Tensor, src_index: torch.Tensor,
@@ -142,8 +139,7 @@ def patch_tokens(ids: torch.Tensor, rows: torch.Tensor, src: torch.Tensor, src_i
     if rows.numel() != src_index.numel():
         raise KernelError("patch_tokens: rows and src_index differ in length")
     f = _fn("elementwise", "ft_patch_tokens", "p p p p i i")
-    _check(f(_ptr(ids), _ptr(rows), _ptr(src), _ptr(src_index), rows.numel(), vocab, _stream()),
-           "patch_tokens")
+    f(ids, rows, src, src_index, rows.numel(), vocab)
 
 
 def rmsnorm(delta: Optional[torch.Tensor], residual: torch.Tensor, weight: torch.Tensor,
@@ -165,8 +161,8 @@ def rmsnorm(delta: Optional[torch.Tensor], residual: torch.Tensor, weight: torch
     if out.shape != residual.shape or weight.numel() != H:
         raise KernelError("rmsnorm: shapes do not match")
     f = _fn("elementwise", "ft_rmsnorm", "p p p p i i i f i i")
-    _check(f(_ptr(delta), _ptr(residual), _ptr(weight), _ptr(out), code(out.dtype), T, H,
-             float(eps), int(plus_one), k, _stream()), "rmsnorm")
+    f(delta, residual, weight, out, code(out.dtype), T, H,
+      float(eps), int(plus_one), k)
 
 
 def qk_rope_store(qkv: torch.Tensor, q_out: torch.Tensor, kv_pages: Optional[torch.Tensor],
@@ -220,12 +216,12 @@ def qk_rope_store(qkv: torch.Tensor, q_out: torch.Tensor, kv_pages: Optional[tor
             raise KernelError("qk_rope_store: value_first must be [T, kv_heads * size] with one lambda")
     f = _fn("elementwise", "ft_qk_rope_store",
             "p p p p p p p p p q q q i i i i i i i i i f i i i p p q i")
-    _check(f(_ptr(qkv), _ptr(q_out), _ptr(kv_pages), _ptr(q_weight), _ptr(k_weight),
-             _ptr(cos_sin) if rotary_dim else None, _ptr(token_pos), _ptr(token_seg),
-             _ptr(block_table), qkv.stride(0), page_stride, kv_stride, num_heads, num_kv_heads,
-             head_dim, rotary_dim, P, block_table.shape[1], norm_mode, int(plus_one),
-             int(interleaved), float(eps), code(qkv.dtype), T, int(norm_dim), _ptr(value_first), _ptr(value_lambda),
-             value_first.stride(0) if value_first is not None else 0, d_first, _stream()), "qk_rope_store")
+    f(qkv, q_out, kv_pages, q_weight, k_weight,
+      cos_sin if rotary_dim else None, token_pos, token_seg,
+      block_table, qkv.stride(0), page_stride, kv_stride, num_heads, num_kv_heads,
+      head_dim, rotary_dim, P, block_table.shape[1], norm_mode, int(plus_one),
+      int(interleaved), float(eps), code(qkv.dtype), T, int(norm_dim), value_first, value_lambda,
+      value_first.stride(0) if value_first is not None else 0, d_first)
 
 
 def combine(parts: torch.Tensor, out: torch.Tensor, k: int) -> None:
@@ -236,7 +232,7 @@ def combine(parts: torch.Tensor, out: torch.Tensor, k: int) -> None:
     if parts.shape[0] != T * k or parts.shape[1] != H:
         raise KernelError("combine: shapes do not match")
     f = _fn("elementwise", "ft_combine", "p p i i i i")
-    _check(f(_ptr(parts), _ptr(out), code(out.dtype), T, k, H, _stream()), "combine")
+    f(parts, out, code(out.dtype), T, k, H)
 
 
 def read_sum(src: torch.Tensor, partial: torch.Tensor) -> None:
@@ -246,7 +242,7 @@ def read_sum(src: torch.Tensor, partial: torch.Tensor) -> None:
     _need(partial, "partial", torch.int32)
     nbytes = src.numel() * src.element_size()
     f = _fn("elementwise", "ft_read_sum", "p q p i")
-    _check(f(_ptr(src), nbytes, _ptr(partial), partial.numel(), _stream()), "read_sum")
+    f(src, nbytes, partial, partial.numel())
 
 
 def gather_rows(src: torch.Tensor, rows: torch.Tensor, dst: torch.Tensor) -> None:
@@ -257,7 +253,7 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, dst: torch.Tensor) -> Non
     if src.shape[1] != H or rows.numel() != n:
         raise KernelError("gather_rows: shapes do not match")
     f = _fn("elementwise", "ft_gather_rows", "p p p i i i")
-    _check(f(_ptr(src), _ptr(rows), _ptr(dst), code(src.dtype), n, H, _stream()), "gather_rows")
+    f(src, rows, dst, code(src.dtype), n, H)
 
 
 # -------------------------------------------- rows of one-tensor caches, gates, caps
@@ -272,8 +268,8 @@ def embed_norm(ids: torch.Tensor, table: torch.Tensor, weight: torch.Tensor, res
     if table.shape[1] != H or ids.numel() != T or weight.numel() != H:
         raise KernelError("embed_norm: shapes do not match")
     f = _fn("rowwise", "ft_embed_norm", "p p i p p i i i f")
-    _check(f(_ptr(ids), _ptr(table), code(table.dtype), _ptr(weight), _ptr(residual), T, H, table.shape[0],
-             float(eps), _stream()), "embed_norm")
+    f(ids, table, code(table.dtype), weight, residual, T, H, table.shape[0],
+      float(eps))
 
 
 def embed_pair(ids: torch.Tensor, token_pos: torch.Tensor, token_seg: torch.Tensor, seg_slot: torch.Tensor,
@@ -303,9 +299,9 @@ def embed_pair(ids: torch.Tensor, token_pos: torch.Tensor, token_seg: torch.Tens
                         ("seg_q_start", seg_q_start)):
             _need(t, name, torch.int32)
     f = _fn("rowwise", "ft_embed_pair", "p p p p p p p p p q q q i i i i f i i")
-    _check(f(_ptr(ids), _ptr(token_pos), _ptr(token_seg), _ptr(seg_slot), _ptr(seg_q_start), _ptr(table),
-             _ptr(pair_table), _ptr(last_token), _ptr(residual), stride, int(mul_prev), int(mul_cur), int(buckets),
-             H, table.shape[0], copies, float(scale), code(table.dtype), T, _stream()), "embed_pair")
+    f(ids, token_pos, token_seg, seg_slot, seg_q_start, table,
+      pair_table, last_token, residual, stride, int(mul_prev), int(mul_cur), int(buckets),
+      H, table.shape[0], copies, float(scale), code(table.dtype), T)
 
 
 def key_store(src: torch.Tensor, q_out: Optional[torch.Tensor], pages: Optional[torch.Tensor],
@@ -343,10 +339,10 @@ def key_store(src: torch.Tensor, q_out: Optional[torch.Tensor], pages: Optional[
         if k_weight.numel() != k_dim:
             raise KernelError("key_store: the norm weight has the wrong length")
     f = _fn("rowwise", "ft_key_store", "p p p p p p p q q i i i i i i i i i f f i i")
-    _check(f(_ptr(src), _ptr(q_out), _ptr(pages), _ptr(k_weight), _ptr(token_pos), _ptr(token_seg),
-             _ptr(block_table), src.stride(0), page_stride, q_off, k_off, num_heads, q_dim, num_kv_heads,
-             k_dim, P, block_table.shape[1], int(temp_every), float(temp_coef), float(eps),
-             code(src.dtype), T, _stream()), "key_store")
+    f(src, q_out, pages, k_weight, token_pos, token_seg,
+      block_table, src.stride(0), page_stride, q_off, k_off, num_heads, q_dim, num_kv_heads,
+      k_dim, P, block_table.shape[1], int(temp_every), float(temp_coef), float(eps),
+      code(src.dtype), T)
 
 
 def gate_heads(o: torch.Tensor, z: torch.Tensor, heads: int, head_dim: int) -> None:
@@ -357,7 +353,7 @@ def gate_heads(o: torch.Tensor, z: torch.Tensor, heads: int, head_dim: int) -> N
     if o.shape[1] != heads * head_dim or z.shape != (T, heads) or z.stride(1) != 1:
         raise KernelError("gate_heads: shapes do not match")
     f = _fn("rowwise", "ft_gate_heads", "p p q i i i i")
-    _check(f(_ptr(o), _ptr(z), z.stride(0), heads, head_dim, code(o.dtype), T, _stream()), "gate_heads")
+    f(o, z, z.stride(0), heads, head_dim, code(o.dtype), T)
 
 
 ACTIVATIONS = {"relu2": 0, "gelu_tanh": 1, "silu": 2, "tanh": 4}
@@ -369,14 +365,14 @@ def activation(x: torch.Tensor, kind: str) -> None:
     if kind not in ACTIVATIONS:
         raise KernelError(f"activation: unknown kind {kind!r}")
     f = _fn("rowwise", "ft_activation", "p q i i")
-    _check(f(_ptr(x), x.numel(), ACTIVATIONS[kind], code(x.dtype), _stream()), "activation")
+    f(x, x.numel(), ACTIVATIONS[kind], code(x.dtype))
 
 
 def softcap(x: torch.Tensor, cap: float) -> None:
     """In place: x = cap * tanh(x / cap) (float32)."""
     _need(x, "x", torch.float32)
     f = _fn("rowwise", "ft_softcap", "p q f")
-    _check(f(_ptr(x), x.numel(), float(cap), _stream()), "softcap")
+    f(x, x.numel(), float(cap))
 
 
 
@@ -480,9 +476,9 @@ def norm_add(branch, residual: torch.Tensor, weight: torch.Tensor, eps: float,
         if copy_out.shape != residual.shape or copy_out.stride(1) != 1:
             raise KernelError("norm_add: copy_out must be [T, H] with unit stride")
     f = _fn("rowwise", "ft_norm_add", "p p i f f p p i f p p q i i i")
-    _check(f(address, _ptr(weight), int(plus_one), float(eps), float(mult), _ptr(residual), _ptr(next_weight),
-             int(next_plus_one), float(next_eps), _ptr(next_out), _ptr(copy_out),
-             copy_out.stride(0) if copy_out is not None else 0, T, H, code(dtype), _stream()), "norm_add")
+    f(address, weight, int(plus_one), float(eps), float(mult), residual, next_weight,
+      int(next_plus_one), float(next_eps), next_out, copy_out,
+      copy_out.stride(0) if copy_out is not None else 0, T, H, code(dtype))
 
 
 def join_layer_norm(branch, residual: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor,
@@ -504,8 +500,8 @@ def join_layer_norm(branch, residual: torch.Tensor, weight: torch.Tensor, eps: f
         if t.numel() != H or o.shape != residual.shape or (b is not None and b.numel() != H):
             raise KernelError("join_layer_norm: shapes do not match")
     f = _fn("rowwise", "ft_join_layer_norm", "p p p p f p p p f p i i i")
-    _check(f(address, _ptr(residual), _ptr(weight), _ptr(bias), float(eps), _ptr(out), _ptr(weight2), _ptr(bias2),
-             float(eps2), _ptr(out2), T, H, code(dtype), _stream()), "join_layer_norm")
+    f(address, residual, weight, bias, float(eps), out, weight2, bias2,
+      float(eps2), out2, T, H, code(dtype))
 
 
 def branch_sum(branch, out: torch.Tensor) -> None:
@@ -514,7 +510,7 @@ def branch_sum(branch, out: torch.Tensor) -> None:
     address, dtype, _alive = _branch_args(branch, T, H, "branch_sum")
     _need(out, "out", dtype)
     f = _fn("rowwise", "ft_branch_sum", "p p i i i")
-    _check(f(address, _ptr(out), T, H, code(dtype), _stream()), "branch_sum")
+    f(address, out, T, H, code(dtype))
 
 
 def cast_rows(x: torch.Tensor, dst: torch.Tensor, branch=None) -> None:
@@ -531,7 +527,7 @@ def cast_rows(x: torch.Tensor, dst: torch.Tensor, branch=None) -> None:
         if dtype != dst.dtype:
             raise KernelError("cast_rows: the branch and dst must have one element type")
     f = _fn("rowwise", "ft_cast_rows", "p p p q i i i")
-    _check(f(_ptr(x), address, _ptr(dst), dst.stride(0), T, H, code(dst.dtype), _stream()), "cast_rows")
+    f(x, address, dst, dst.stride(0), T, H, code(dst.dtype))
 
 
 def scaled_sum(parts: torch.Tensor, scale: torch.Tensor, out: torch.Tensor) -> None:
@@ -543,7 +539,7 @@ def scaled_sum(parts: torch.Tensor, scale: torch.Tensor, out: torch.Tensor) -> N
     if out.shape != (T, H) or scale.numel() != k:
         raise KernelError("scaled_sum: shapes do not match")
     f = _fn("rowwise", "ft_scaled_sum", "p p p i i i i")
-    _check(f(_ptr(parts), _ptr(scale), _ptr(out), k, T, H, code(out.dtype), _stream()), "scaled_sum")
+    f(parts, scale, out, k, T, H, code(out.dtype))
 
 
 def bias_add(x: torch.Tensor, bias: torch.Tensor) -> None:
@@ -553,7 +549,7 @@ def bias_add(x: torch.Tensor, bias: torch.Tensor) -> None:
     if x.dim() != 2 or x.stride(1) != 1 or bias.numel() != x.shape[1]:
         raise KernelError("bias_add: x must be [T, width] with unit stride and one bias per column")
     f = _fn("rowwise", "ft_bias_add", "p q p i i i")
-    _check(f(_ptr(x), x.stride(0), _ptr(bias), x.shape[0], x.shape[1], code(x.dtype), _stream()), "bias_add")
+    f(x, x.stride(0), bias, x.shape[0], x.shape[1], code(x.dtype))
 
 
 GLU_KINDS = {"relu2": 0, "gelu_tanh": 1, "silu": 2, "swigluoai": 3}
@@ -569,8 +565,7 @@ def glu_rows(gate_up: torch.Tensor, mid: torch.Tensor, kind: str, alpha: float =
     if gate_up.shape != (T, 2 * I) or kind not in GLU_KINDS:
         raise KernelError("glu_rows: gate_up must be [T, 2 * I] and the activation a known one")
     f = _fn("rowwise", "ft_glu_rows", "p p i i i f f i")
-    _check(f(_ptr(gate_up), _ptr(mid), T, I, GLU_KINDS[kind], float(alpha), float(limit), code(mid.dtype),
-             _stream()), "glu_rows")
+    f(gate_up, mid, T, I, GLU_KINDS[kind], float(alpha), float(limit), code(mid.dtype))
 
 
 def hyper_norm(streams: torch.Tensor, branch: Optional[torch.Tensor], mix: Optional[torch.Tensor],
@@ -604,8 +599,8 @@ def hyper_norm(streams: torch.Tensor, branch: Optional[torch.Tensor], mix: Optio
         if normed.shape != (T, H):
             raise KernelError("hyper_norm: normed must be [T, H]")
     f = _fn("rowwise", "ft_hyper_norm", "p p i p p p p p f i p i i i i")
-    _check(f(_ptr(streams), _ptr(branch), k, _ptr(mix), _ptr(out_weights), _ptr(read), _ptr(weight), _ptr(bias),
-             float(eps), int(center), _ptr(normed), T, S, H, code(dtype), _stream()), "hyper_norm")
+    f(streams, branch, k, mix, out_weights, read, weight, bias,
+      float(eps), int(center), normed, T, S, H, code(dtype))
 
 
 def rms_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float) -> None:
@@ -618,8 +613,7 @@ def rms_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: floa
     if out.shape != x.shape or weight.numel() != n or x.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("rms_rows: shapes do not match")
     f = _fn("rowwise", "ft_rms_rows", "p q p p q i i f i")
-    _check(f(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), out.stride(0), T, n, float(eps), code(x.dtype),
-             _stream()), "rms_rows")
+    f(x, x.stride(0), weight, out, out.stride(0), T, n, float(eps), code(x.dtype))
 
 
 def latent_store(down: torch.Tensor, q: torch.Tensor, q_abs: Optional[torch.Tensor], pages: Optional[torch.Tensor],
@@ -655,9 +649,9 @@ def latent_store(down: torch.Tensor, q: torch.Tensor, q_abs: Optional[torch.Tens
             raise KernelError("latent_store: pages must be [pages, 1, page, rank + rot]")
         P, page_stride = pages.shape[2], pages.stride(0)
     f = _fn("rowwise", "ft_latent_store", "p q p q p p q p p p p p i i i i i i i i f i i")
-    _check(f(_ptr(down), down.stride(0), _ptr(q), q.stride(0), _ptr(q_abs), _ptr(pages), page_stride, _ptr(weight),
-             _ptr(cos_sin), _ptr(token_pos), _ptr(token_seg), _ptr(block_table), heads, q_dim, rank, rot, P,
-             block_table.shape[1], int(interleaved), int(turn_q), float(eps), code(down.dtype), T, _stream()), "latent_store")
+    f(down, down.stride(0), q, q.stride(0), q_abs, pages, page_stride, weight,
+      cos_sin, token_pos, token_seg, block_table, heads, q_dim, rank, rot, P,
+      block_table.shape[1], int(interleaved), int(turn_q), float(eps), code(down.dtype), T)
 
 
 # ------------------------------------------------------- mixers with a carried state
@@ -691,9 +685,9 @@ def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Op
     global LAUNCHES
     LAUNCHES += 1 if taps > 1 and (T != seg_slot.numel() or taps > 8) else 0      # a kernel for the slots' new contents
     f = _fn("recurrent", "ft_conv_silu", "p q p q p p p q p p p i i i i i i i")
-    _check(f(_ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(weight), _ptr(bias), _ptr(state),
-             state.stride(0), _ptr(token_seg), _ptr(seg_slot), _ptr(seg_q_start), C, taps, T,
-             seg_slot.numel(), code(x.dtype), int(activation), int(state_ahead), _stream()), "conv_silu")
+    f(x, x.stride(0), out, out.stride(0), weight, bias, state,
+      state.stride(0), token_seg, seg_slot, seg_q_start, C, taps, T,
+      seg_slot.numel(), code(x.dtype), int(activation), int(state_ahead))
 
 
 def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
@@ -720,9 +714,9 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     if state.stride(1) != 1 or state.shape[1] < heads * state_dim * head_dim:
         raise KernelError("ssd_scan: a state row must hold heads * state_dim * head_dim values")
     f = _fn("recurrent", "ft_ssd_scan", "p q p q p p p p q p p p i i i i i i i i i")
-    _check(f(_ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-             _ptr(state), state.stride(0), _ptr(y), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim,
-             state_dim, groups, seg_slot.numel(), T, longest, code(xbc.dtype), int(state_ahead), _stream()), "ssd_scan")
+    f(xbc, xbc.stride(0), dt, dt.stride(0), dt_bias, a_log, d_skip,
+      state, state.stride(0), y, seg_slot, seg_q_start, heads, head_dim,
+      state_dim, groups, seg_slot.numel(), T, longest, code(xbc.dtype), int(state_ahead))
 
 
 def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
@@ -753,10 +747,10 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bi
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("delta_scan: a state row must hold heads * key_dim * value_dim values")
     f = _fn("delta_scan", "ft_delta_scan", "p q p p q p p p q p p p i i i i f f i i i i i")
-    _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), _ptr(decay), beta.stride(0), _ptr(dt_bias), _ptr(a_log),
-             _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
-             int(state_ahead), _stream()), "delta_scan")
+    f(qkv, qkv.stride(0), beta, decay, beta.stride(0), dt_bias, a_log,
+      state, state.stride(0), o, seg_slot, seg_q_start, heads, value_dim,
+      key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
+      int(state_ahead))
 
 
 def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
@@ -786,10 +780,10 @@ def channel_delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tenso
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("channel_delta_scan: a state row must hold heads * key_dim * value_dim values")
     f = _fn("channel_delta", "ft_channel_delta_scan", "p q p q p q p p p q p p p i i i i f f i i i i i")
-    _check(f(_ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(decay), decay.stride(0), _ptr(dt_bias),
-             _ptr(a_log), _ptr(state), state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim,
-             key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
-             int(state_ahead), _stream()), "channel_delta_scan")
+    f(qkv, qkv.stride(0), beta, beta.stride(0), decay, decay.stride(0), dt_bias,
+      a_log, state, state.stride(0), o, seg_slot, seg_q_start, heads, value_dim,
+      key_dim, key_heads, float(unit_eps), float(q_scale), seg_slot.numel(), T, longest, code(qkv.dtype),
+      int(state_ahead))
 
 
 def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[torch.Tensor], seg_pos0: torch.Tensor,
@@ -818,9 +812,9 @@ def retention_scan(qkv: torch.Tensor, decay: torch.Tensor, cos_sin: Optional[tor
     if state.stride(1) != 1 or state.shape[1] < heads * key_dim * value_dim:
         raise KernelError("retention_scan: a state row must hold heads * key_dim * value_dim values")
     f = _fn("retention", "ft_retention_scan", "p q p p i p p q p p p i i i f i i i i i")
-    _check(f(_ptr(qkv), qkv.stride(0), _ptr(decay), _ptr(cos_sin), rot, _ptr(seg_pos0), _ptr(state), state.stride(0),
-             _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, value_dim, key_dim, float(k_scale),
-             seg_slot.numel(), T, longest, code(qkv.dtype), int(state_ahead), _stream()), "retention_scan")
+    f(qkv, qkv.stride(0), decay, cos_sin, rot, seg_pos0, state, state.stride(0),
+      o, seg_slot, seg_q_start, heads, value_dim, key_dim, float(k_scale),
+      seg_slot.numel(), T, longest, code(qkv.dtype), int(state_ahead))
 
 
 def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: torch.Tensor, token_seg: torch.Tensor,
@@ -839,8 +833,8 @@ def token_shift(x: torch.Tensor, mu: torch.Tensor, out: torch.Tensor, state: tor
     if mu.shape != (M, W) or out.shape != (M, T, W) or x.stride(1) != 1 or state.shape[1] < W or state.stride(1) != 1:
         raise KernelError("token_shift: shapes do not match")
     f = _fn("time_mixing", "ft_token_shift", "p q p p p q p p p i i i i")
-    _check(f(_ptr(x), x.stride(0), _ptr(mu), _ptr(out), _ptr(state), state.stride(0), _ptr(token_seg), _ptr(seg_slot),
-             _ptr(seg_q_start), T, W, M, code(x.dtype), _stream()), "token_shift")
+    f(x, x.stride(0), mu, out, state, state.stride(0), token_seg, seg_slot,
+      seg_q_start, T, W, M, code(x.dtype))
 
 
 def time_mixing_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, w0: torch.Tensor,
@@ -868,9 +862,9 @@ def time_mixing_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     if len({t.stride(0) for t in (r, k, v)}) != 1 or any(t.stride(1) != 1 for t in (r, k, v, decay)):
         raise KernelError("time_mixing_scan: r, k and v need one row stride and unit column strides")
     f = _fn("time_mixing", "ft_time_mixing_scan", "p p p q p q p p p q p p p i i i i i i i")
-    _check(f(_ptr(r), _ptr(k), _ptr(v), r.stride(0), _ptr(decay), decay.stride(0), _ptr(w0), _ptr(u), _ptr(state),
-             state.stride(0), _ptr(o), _ptr(seg_slot), _ptr(seg_q_start), heads, head_dim, key_dim,
-             seg_slot.numel(), T, code(r.dtype), int(state_ahead), _stream()), "time_mixing_scan")
+    f(r, k, v, r.stride(0), decay, decay.stride(0), w0, u, state,
+      state.stride(0), o, seg_slot, seg_q_start, heads, head_dim, key_dim,
+      seg_slot.numel(), T, code(r.dtype), int(state_ahead))
 
 
 GATES = {"silu": 0, "sigmoid": 1}
@@ -890,8 +884,8 @@ def gated_norm(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: t
             or width % weight.numel() or gate_kind not in GATES:
         raise KernelError("gated_norm: shapes do not match")
     f = _fn("gated_norm", "ft_gated_norm", "p p q p i p i i i f i i i")
-    _check(f(_ptr(y), _ptr(gate), gate.stride(0), _ptr(weight), weight.numel(), _ptr(out), T, width, groups,
-             float(eps), int(gate_first), GATES[gate_kind], code(out.dtype), _stream()), "gated_norm")
+    f(y, gate, gate.stride(0), weight, weight.numel(), out, T, width, groups,
+      float(eps), int(gate_first), GATES[gate_kind], code(out.dtype))
 
 # ------------------------------------------------------------------ gemm
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
@@ -906,8 +900,8 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
     if w.shape != (heads, N, K) or c.shape != (T, heads, N) or a.stride(2) != 1 or c.stride(2) != 1:
         raise KernelError("gemm_heads: shapes do not match")
     f = _fn("gemm_simt", "ft_gemm_heads", "p i q q p i q p i q q i i i i")
-    _check(f(_ptr(a), code(a.dtype), a.stride(0), a.stride(1), _ptr(w), code(w.dtype), N * K, _ptr(c),
-             code(c.dtype), c.stride(0), c.stride(1), T, N, K, heads, _stream()), "gemm_heads")
+    f(a, code(a.dtype), a.stride(0), a.stride(1), w, code(w.dtype), N * K, c,
+      code(c.dtype), c.stride(0), c.stride(1), T, N, K, heads)
 
 
 def gemm_rows(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
@@ -939,10 +933,10 @@ def gemm_rows(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
     if row_scale is not None:
         _need(row_scale, "row_scale", torch.float32)
     f = _fn("gemm_simt", "ft_gemm_rows", "p i q p i q p i q p p p p i i i i i i f f")
-    _check(f(_ptr(a), code(a.dtype), a.stride(0), _ptr(w), code(w.dtype), NW * K, _ptr(c),
-             code(c.dtype), c.stride(0), _ptr(group_offsets), _ptr(a_rows), _ptr(c_rows),
-             _ptr(row_scale), M, N, K, G, int(glu), 0 if act == "silu" else 1, float(act_alpha),
-             float(act_limit), _stream()), "gemm_rows")
+    f(a, code(a.dtype), a.stride(0), w, code(w.dtype), NW * K, c,
+      code(c.dtype), c.stride(0), group_offsets, a_rows, c_rows,
+      row_scale, M, N, K, G, int(glu), 0 if act == "silu" else 1, float(act_alpha),
+      float(act_limit))
 
 
 # gated pairs the weight-streaming kernel applies to its accumulators
@@ -1006,12 +1000,11 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
     if unary is not None and (glu or unary not in ACTIVATIONS):
         raise KernelError(f"skinny_gemm: cannot apply {unary!r} (with glu: {glu})")
     f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i")
-    _check(f(_ptr(a), a.stride(0), _ptr(w), NW * K, _ptr(c), code(c.dtype), c.stride(0),
-             _ptr(group_offsets), _ptr(active), _ptr(a_rows), _ptr(c_rows), _ptr(row_scale), M, N, K, G,
-             int(glu), GLU_ACTS[act], float(act_alpha), float(act_limit),
-             rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], _ptr(bias), int(group_rows),
-             int(lists_ahead), _stream()),
-           "skinny_gemm")
+    f(a, a.stride(0), w, NW * K, c, code(c.dtype), c.stride(0),
+      group_offsets, active, a_rows, c_rows, row_scale, M, N, K, G,
+      int(glu), GLU_ACTS[act], float(act_alpha), float(act_limit),
+      rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], bias, int(group_rows),
+      int(lists_ahead))
 
 
 # ------------------------------------------------ grouped GEMM on tcgen05
@@ -1069,7 +1062,7 @@ def wait_selftest(device, limit_ns: int, arrive: bool) -> None:
     by its own limit and the kernel returns)."""
     f = _fn("moe_gemm_tc", "ft_wait_selftest", "p q i")
     with torch.cuda.device(torch.device(device)):
-        _check(f(_ptr(tc_status(device)), int(limit_ns), int(bool(arrive)), _stream()), "wait_selftest")
+        f(tc_status(device), int(limit_ns), int(bool(arrive)))
 
 
 def _tc_map(t: torch.Tensor, rows: int, K: int, row_stride: int, groups: int, box_rows: int):
@@ -1117,8 +1110,7 @@ def moe_tile_map(group_offsets: torch.Tensor, active: torch.Tensor, rows: int, g
     bound = -(-rows // TC_TOKENS_PER_TILE) + min(groups, rows)
     tile_info = workspace.get("moe.tile_info", (bound, 4), torch.int32)
     f = _fn("moe_gemm_tc", "ft_moe_tile_map", "p p p i i i")
-    _check(f(_ptr(group_offsets), _ptr(active), _ptr(tile_info), rows, groups, TC_TOKENS_PER_TILE, _stream()),
-           "moe_tile_map")
+    f(group_offsets, active, tile_info, rows, groups, TC_TOKENS_PER_TILE)
     return tile_info
 
 
@@ -1152,10 +1144,9 @@ def moe_gemm_tc(x: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *, tile_map: 
         maps_x = _TC_MAPS[key] = ctypes.create_string_buffer(joined, 256)
     status = tc_status(x.device)
     f = _fn("moe_gemm_tc", "ft_moe_gemm_tc", "p p p q p p p p i i i i i i i f f")
-    _check(f(ctypes.cast(map_w, ctypes.c_void_p), ctypes.cast(maps_x, ctypes.c_void_p), _ptr(c),
-             c.stride(0), _ptr(tile_map), _ptr(c_rows), _ptr(row_scale), _ptr(status), rows, N, K, G,
-             TC_TOKENS_PER_TILE, form, 0 if act == "silu" else 1, float(act_alpha), float(act_limit),
-             _stream()), "moe_gemm_tc")
+    f(map_w, maps_x, c,
+      c.stride(0), tile_map, c_rows, row_scale, status, rows, N, K, G,
+      TC_TOKENS_PER_TILE, form, 0 if act == "silu" else 1, float(act_alpha), float(act_limit))
 
 
 def moe_experts_tc(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, mid: torch.Tensor,
@@ -1212,7 +1203,7 @@ class ScoreOptions:
             _need(self.sink, "sink", torch.float32)
             if self.sink.numel() != num_heads:
                 raise KernelError("the sink has one score per query head")
-        return (self.chunk, self.softcap, self.sink_mode, float(self.sink_value or 0.0), _ptr(self.sink))
+        return (self.chunk, self.softcap, self.sink_mode, float(self.sink_value or 0.0), self.sink)
 
 
 NO_SCORE_OPTIONS = ScoreOptions()
@@ -1241,11 +1232,10 @@ def attn_paged_simt(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
         _need(seg_q_start, "seg_q_start", torch.int32)
         S = seg_q_start.numel() - 1
     f = _fn("attention_simt", "ft_attn_paged_simt", "p p p p p p p q q i i i i i i f i i i f i f p p i")
-    _check(f(_ptr(q), _ptr(out), _ptr(kv_pages), _ptr(token_pos), _ptr(token_seg),
-             _ptr(block_table), _ptr(rows), kv_pages.stride(1), kv_pages.stride(0), num_heads, num_kv_heads,
-             head_dim, kv_pages.shape[3], block_table.shape[1], int(window or 0), float(scale),
-             code(q.dtype), T, *(options or NO_SCORE_OPTIONS).args(num_heads), _ptr(seg_q_start), S, _stream()),
-           "attn_paged_simt")
+    f(q, out, kv_pages, token_pos, token_seg,
+      block_table, rows, kv_pages.stride(1), kv_pages.stride(0), num_heads, num_kv_heads,
+      head_dim, kv_pages.shape[3], block_table.shape[1], int(window or 0), float(scale),
+      code(q.dtype), T, *(options or NO_SCORE_OPTIONS).args(num_heads), seg_q_start, S)
 
 
 DECODE_HEAD_DIMS = (32, 64, 128)
@@ -1342,22 +1332,22 @@ def attn_decode(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
         map_kv = _attn_tc_map("kv", (kv_pages.data_ptr(),) + tuple(kv_pages.shape) + tuple(kv_pages.stride()),
                               make_kv)
         f = _fn("attention_decode_tma", "ft_attn_decode_tma", "p p p p p p p p p p i i i i i i i i i f i i f i f p")
-        _check(f(ctypes.cast(map_kv, ctypes.c_void_p), _ptr(q), _ptr(out), _ptr(part_o), _ptr(part_ml),
-                 _ptr(rows), _ptr(token_pos), _ptr(token_seg), _ptr(block_table), _ptr(tc_status(q.device)),
-                 num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
-                 int(window or 0), n_rows, splits, split_keys, float(scale),
-                 1 if kv_pages.stride(0) else 0, *extra, _stream()), "attn_decode_tma")
+        f(map_kv, q, out, part_o, part_ml,
+          rows, token_pos, token_seg, block_table, tc_status(q.device),
+          num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
+          int(window or 0), n_rows, splits, split_keys, float(scale),
+          1 if kv_pages.stride(0) else 0, *extra)
         if part_o is not None:
             fm = _fn("attention_decode", "ft_attn_merge", "p p p p i i i i")
-            _check(fm(_ptr(part_o), _ptr(part_ml), _ptr(out), _ptr(rows), n_rows, num_heads, head_dim,
-                      splits, _stream()), "attn_merge")
+            fm(part_o, part_ml, out, rows, n_rows, num_heads, head_dim,
+               splits)
         return
     f = _fn("attention_decode", "ft_attn_decode", "p p p p p p p p p q q i i i i i i i i i f i f i f p")
-    _check(f(_ptr(q), _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(kv_pages), _ptr(rows),
-             _ptr(token_pos), _ptr(token_seg), _ptr(block_table), kv_pages.stride(1),
-             kv_pages.stride(0), num_heads, num_kv_heads, head_dim, kv_pages.shape[3],
-             block_table.shape[1], int(window or 0), n_rows, splits, split_keys, float(scale),
-             *extra, _stream()), "attn_decode")
+    f(q, out, part_o, part_ml, kv_pages, rows,
+      token_pos, token_seg, block_table, kv_pages.stride(1),
+      kv_pages.stride(0), num_heads, num_kv_heads, head_dim, kv_pages.shape[3],
+      block_table.shape[1], int(window or 0), n_rows, splits, split_keys, float(scale),
+      *extra)
 
 
 def attn_prefill(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
@@ -1376,10 +1366,10 @@ def attn_prefill(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
                     ("seg_pos0", seg_pos0), ("block_table", block_table)):
         _need(t, name, torch.int32)
     f = _fn("attention_prefill", "ft_attn_prefill", "p p p p p p p p q q i i i i i i i f i f i f p")
-    _check(f(_ptr(q), _ptr(out), _ptr(kv_pages), _ptr(tile_seg), _ptr(tile_q0), _ptr(seg_q_start),
-             _ptr(seg_pos0), _ptr(block_table), kv_pages.stride(1), kv_pages.stride(0), num_heads,
-             num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1], int(window or 0),
-             tile_seg.numel(), float(scale), *(options or NO_SCORE_OPTIONS).args(num_heads), _stream()), "attn_prefill")
+    f(q, out, kv_pages, tile_seg, tile_q0, seg_q_start,
+      seg_pos0, block_table, kv_pages.stride(1), kv_pages.stride(0), num_heads,
+      num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1], int(window or 0),
+      tile_seg.numel(), float(scale), *(options or NO_SCORE_OPTIONS).args(num_heads))
 
 
 # A step whose prompt portions score at least this many query-key pairs uses the
@@ -1451,12 +1441,12 @@ def attn_prefill_tc(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
                           make_kv)
     status = tc_status(q.device)
     f = _fn("attention_prefill_tc", "ft_attn_prefill_tc", "p p p p p p p p p p i i i i i i f i i i f i f p")
-    _check(f(ctypes.cast(map_q, ctypes.c_void_p), ctypes.cast(map_q2, ctypes.c_void_p),
-             ctypes.cast(map_kv, ctypes.c_void_p), _ptr(out),
-             _ptr(tile_seg), _ptr(tile_q0), _ptr(seg_q_start), _ptr(seg_pos0), _ptr(block_table),
-             _ptr(status), num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
-             tile_seg.numel(), float(scale), 1 if kv_pages.stride(0) else 0, int(window or 0),
-             *(options or NO_SCORE_OPTIONS).args(num_heads), _stream()), "attn_prefill_tc")
+    f(map_q, map_q2,
+      map_kv, out,
+      tile_seg, tile_q0, seg_q_start, seg_pos0, block_table,
+      status, num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
+      tile_seg.numel(), float(scale), 1 if kv_pages.stride(0) else 0, int(window or 0),
+      *(options or NO_SCORE_OPTIONS).args(num_heads))
 
 
 # ------------------------------------------- attention over latent rows, absorbed and expanded
@@ -1521,11 +1511,10 @@ def attn_latent(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, tile_se
         part_o = workspace.get("attn.part_o", (tiles * 16 * mt, splits, rank), torch.float32)
         part_ml = workspace.get("attn.part_ml", (tiles * 16 * mt, splits, 2), torch.float32)
     f = _fn("attention_latent", "ft_attn_latent", "p p q p p p p p p p p p q i i i i i i i i i i f")
-    _check(f(_ptr(q), _ptr(out), out.stride(1), _ptr(part_o), _ptr(part_ml), _ptr(pages), _ptr(tile_seg),
-             _ptr(tile_row), _ptr(seg_q_start), _ptr(seg_pos0), _ptr(block_table), _ptr(tc_status(q.device)),
-             pages.stride(0), H, d, rank,
-             pages.shape[2], block_table.shape[1], int(window or 0), tiles, mt, splits, split_keys, float(scale),
-             _stream()), "attn_latent")
+    f(q, out, out.stride(1), part_o, part_ml, pages, tile_seg,
+      tile_row, seg_q_start, seg_pos0, block_table, tc_status(q.device),
+      pages.stride(0), H, d, rank,
+      pages.shape[2], block_table.shape[1], int(window or 0), tiles, mt, splits, split_keys, float(scale))
     if splits > 1:
         global LAUNCHES
         LAUNCHES += 1
@@ -1545,10 +1534,9 @@ def latent_gather(pages: torch.Tensor, dst: torch.Tensor, seg: torch.Tensor, key
     if pages.dim() != 4 or pages.shape[1] != 1 or dst.shape[1] != pages.shape[3] or dst.shape[0] < 64 * seg.numel():
         raise KernelError("latent_gather: shapes do not match")
     f = _fn("attention_prefill_mha", "ft_latent_gather", "p p p p p p p p q i i i i i")
-    _check(f(_ptr(pages), _ptr(dst), _ptr(seg), _ptr(key0), _ptr(row0), _ptr(seg_kv_len), _ptr(seg_pos0),
-             _ptr(block_table), pages.stride(0), pages.shape[3], pages.shape[2], block_table.shape[1],
-             int(window or 0), seg.numel(), _stream()),
-           "latent_gather")
+    f(pages, dst, seg, key0, row0, seg_kv_len, seg_pos0,
+      block_table, pages.stride(0), pages.shape[3], pages.shape[2], block_table.shape[1],
+      int(window or 0), seg.numel())
 
 
 MHA_QUERY_TILE = 128
@@ -1590,17 +1578,16 @@ def attn_prefill_mha(q: torch.Tensor, keys: torch.Tensor, shared_keys: Optional[
             f.argtypes = [ctypes.c_void_p, ctypes.c_void_p] + [ctypes.c_longlong] * 5 + [ctypes.c_int]
             f.restype = ctypes.c_int
             return f(dst, t.data_ptr(), n_rows, cols, heads, row_stride, head_stride, box)
-        return ctypes.cast(_attn_tc_map(kind, (t.data_ptr(), n_rows, cols, heads, row_stride, head_stride, box), make),
-                           ctypes.c_void_p)
+        return _attn_tc_map(kind, (t.data_ptr(), n_rows, cols, heads, row_stride, head_stride, box), make)
 
     map_q = mapped("mha_q", q, T, q.shape[1], 0, q.stride(0), 0, MHA_QUERY_TILE)
     map_k = mapped("mha_kv", keys, rows, dk, H, keys.stride(0), keys.stride(1), 64)
     map_v = mapped("mha_kv", values, rows, dv, H, values.stride(0), values.stride(1), 64)
     map_r = mapped("mha_r", shared_keys, rows, rot, 0, shared_keys.stride(0), 0, 64) if rot else None
     f = _fn("attention_prefill_mha", "ft_attn_prefill_mha", "p p p p p p p p p p p i i i i i i f")
-    _check(f(map_q, map_k, map_r, map_v, _ptr(out), _ptr(tile_seg), _ptr(tile_q0), _ptr(tile_row0),
-             _ptr(seg_q_start), _ptr(seg_pos0), _ptr(tc_status(q.device)), H, dk, rot, dv, int(window or 0),
-             tile_seg.numel(), float(scale), _stream()), "attn_prefill_mha")
+    f(map_q, map_k, map_r, map_v, out, tile_seg, tile_q0, tile_row0,
+      seg_q_start, seg_pos0, tc_status(q.device), H, dk, rot, dv, int(window or 0),
+      tile_seg.numel(), float(scale))
 
 
 # ---------------------------------------------------------------- router
@@ -1625,9 +1612,8 @@ def router_select(logits: torch.Tensor, bias: Optional[torch.Tensor], ids: torch
     if logits.shape[1] % terms or E < 1 or not logits.is_contiguous() or (tail is not None and tail.numel() < T):
         raise KernelError(f"router_select: logits {tuple(logits.shape)} do not hold {terms} terms per expert")
     f = _fn("moe_route", "ft_router_select", "p p p p i i i i i f i i i i p")
-    _check(f(_ptr(logits), _ptr(bias), _ptr(ids), _ptr(weights), T, E, k, int(softmax_scoring),
-             int(renormalize), float(scale), int(terms), int(groups), int(keep), int(group_top), _ptr(tail), _stream()),
-           "router_select")
+    f(logits, bias, ids, weights, T, E, k, int(softmax_scoring),
+      int(renormalize), float(scale), int(terms), int(groups), int(keep), int(group_top), tail)
 
 
 ROUTE_SMALL_MAX_T = 8
@@ -1663,10 +1649,10 @@ def route_small(logits: torch.Tensor, bias: Optional[torch.Tensor], ids: torch.T
             or sorted_token.numel() < R or active.numel() < busy_of + 1 or ids.numel() < R or weights.numel() < R:
         raise KernelError("route_small: output buffers are too small")
     f = _fn("moe_route", "ft_route_small", "p p p p p p p p p i i i i i i f i i i i p")
-    _check(f(_ptr(logits), _ptr(bias), _ptr(ids), _ptr(weights), _ptr(counts), _ptr(offsets),
-             _ptr(sorted_route), _ptr(sorted_token), _ptr(active), T, E, busy_of, k, int(softmax_scoring),
-             int(renormalize), float(scale), int(terms), int(groups), int(keep), int(group_top),
-             _ptr(tail), _stream()), "route_small")
+    f(logits, bias, ids, weights, counts, offsets,
+      sorted_route, sorted_token, active, T, E, busy_of, k, int(softmax_scoring),
+      int(renormalize), float(scale), int(terms), int(groups), int(keep), int(group_top),
+      tail)
 
 
 def router_logits_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -1684,8 +1670,7 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor) -> Non
     if w.shape[1] != H or logits.shape != (T, E) or x.stride(1) != 1:
         raise KernelError("router_logits: shapes do not match")
     f = _fn("moe_route", "ft_router_logits", "p i q p p i i i")
-    _check(f(_ptr(x), code(x.dtype), x.stride(0), _ptr(w), _ptr(logits), T, E, H, _stream()),
-           "router_logits")
+    f(x, code(x.dtype), x.stride(0), w, logits, T, E, H)
 
 
 def moe_sort(ids: torch.Tensor, counts: torch.Tensor, offsets: torch.Tensor,
@@ -1712,8 +1697,8 @@ def moe_sort(ids: torch.Tensor, counts: torch.Tensor, offsets: torch.Tensor,
         if scratch.numel() < moe_sort_scratch(R, num_experts):
             raise KernelError("moe_sort: the scratch buffer is too small")
     f = _fn("moe_route", "ft_moe_sort", "p p p p p p p i i i i")
-    _check(f(_ptr(ids), _ptr(counts), _ptr(offsets), _ptr(sorted_route), _ptr(sorted_token),
-             _ptr(active), _ptr(scratch), R, num_experts, busy_of, k, _stream()), "moe_sort")
+    f(ids, counts, offsets, sorted_route, sorted_token,
+      active, scratch, R, num_experts, busy_of, k)
     if scratch is not None:
         global LAUNCHES
         LAUNCHES += 1      # three kernels instead of two
@@ -1747,5 +1732,5 @@ def sample(logits: torch.Tensor, temperature: Optional[torch.Tensor], top_k: Opt
     if top_p is not None:
         _need(top_p, "top_p", torch.float32)
     f = _fn("sampling", "ft_sample", "p p p p p p p i i")
-    _check(f(_ptr(logits), _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(uniform), _ptr(out),
-             _ptr(probs), rows, V, _stream()), "sample")
+    f(logits, temperature, top_k, top_p, uniform, out,
+      probs, rows, V)

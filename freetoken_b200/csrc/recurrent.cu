@@ -676,3 +676,6 @@ int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, 
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_conv_silu)
+FT_PACKED(ft_ssd_scan)

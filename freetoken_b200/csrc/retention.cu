@@ -15,3 +15,5 @@ extern "C" int ft_retention_scan(const void* qkv, long long ld, const float* dec
               heads, P, D, heads, 0.f, k_scale, 0, nullptr, 0, cos_sin, seg_pos0, cos_sin ? rot_dims : 0, state_ahead};
   return dispatch_delta<2>(a, S, T, longest, dtype, stream);
 }
+
+FT_PACKED(ft_retention_scan)

@@ -1585,3 +1585,20 @@ int ft_latent_store(const void* down, long long ld_down, void* q, long long ld_q
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_embed_norm)
+FT_PACKED(ft_embed_pair)
+FT_PACKED(ft_key_store)
+FT_PACKED(ft_gate_heads)
+FT_PACKED(ft_activation)
+FT_PACKED(ft_softcap)
+FT_PACKED(ft_norm_add)
+FT_PACKED(ft_join_layer_norm)
+FT_PACKED(ft_branch_sum)
+FT_PACKED(ft_cast_rows)
+FT_PACKED(ft_scaled_sum)
+FT_PACKED(ft_bias_add)
+FT_PACKED(ft_glu_rows)
+FT_PACKED(ft_hyper_norm)
+FT_PACKED(ft_rms_rows)
+FT_PACKED(ft_latent_store)

@@ -214,3 +214,5 @@ extern "C" int ft_sample_static(const float* logits, const float* temperature, c
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_sample)

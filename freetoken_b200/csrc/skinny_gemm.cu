@@ -366,3 +366,5 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
+
+FT_PACKED(ft_skinny_gemm)

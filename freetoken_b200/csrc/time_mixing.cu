@@ -574,3 +574,6 @@ int ft_time_mixing_scan(const void* r, const void* k, const void* v, long long l
 }
 
 }  // extern "C"
+
+FT_PACKED(ft_token_shift)
+FT_PACKED(ft_time_mixing_scan)
