@@ -40,11 +40,13 @@ struct DeltaArgs {
 //         strength and no unit norms; q and k have the first rot_dims dimensions of each head turned
 //         by the token's position (dimension i with i + rot_dims / 2) in shared memory, in float32;
 //         k is multiplied by q_scale after the rotation.
-template <typename AT, int NPL, int WC, int MODE>
+// CH: tokens of a chunk.  Segments of one token each take a chunk of one: the rows staged for a chunk of eight took
+// registers that left four requests of 32 heads of 128 x 128 two rounds of blocks.
+template <typename AT, int NPL, int WC, int MODE, int CH>
 __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   constexpr int COLS = SCAN_WARPS * WC;
   constexpr int NB = (NPL * 32 + SCAN_THREADS - 1) / SCAN_THREADS;
-  constexpr int XR = (SCAN_CHUNK * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
+  constexpr int XR = (CH * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
   extern __shared__ float sm[];
   if (!a.state_ahead) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -54,7 +56,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   const int col0 = blockIdx.x * COLS;
   const int j0 = col0 + warp * WC;
   const int width = a.heads * P;
-  const int per = SCAN_CHUNK * ((MODE == 1 ? 3 : 2) * D + COLS + 2);
+  const int per = CH * ((MODE == 1 ? 3 : 2) * D + COLS + 2);
   const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1];
   float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * D * P;
   const float rate = MODE == 2 ? 0.f : -expf(a.A_log[head]);
@@ -83,12 +85,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   }
   if (a.state_ahead) pdl_wait();
 
-  AT pq[SCAN_CHUNK][NB], pk[SCAN_CHUNK][NB], pv[XR], pbeta, pdecay;
-  float pg[MODE == 1 ? SCAN_CHUNK : 1][NB];                   // MODE 1: the channels' decay projections
+  AT pq[CH][NB], pk[CH][NB], pv[XR], pbeta, pdecay;
+  float pg[MODE == 1 ? CH : 1][NB];                   // MODE 1: the channels' decay projections
   float pcos[MODE == 2 ? NPL : 1], psin[MODE == 2 ? NPL : 1]; // MODE 2: pair (tt, i) = threadIdx.x + 128 r
   auto fetch = [&](int t0, int nt) {
 #pragma unroll
-    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+    for (int tt = 0; tt < CH; ++tt) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const int n = threadIdx.x + SCAN_THREADS * b;
@@ -127,11 +129,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   };
   auto put = [&](float* buf, int nt) {
     float* qs = buf;
-    float* ks = qs + SCAN_CHUNK * D;
-    float* vs = ks + SCAN_CHUNK * D;
-    float* gates = vs + SCAN_CHUNK * COLS;
+    float* ks = qs + CH * D;
+    float* vs = ks + CH * D;
+    float* gates = vs + CH * COLS;
 #pragma unroll
-    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+    for (int tt = 0; tt < CH; ++tt) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const int n = threadIdx.x + SCAN_THREADS * b;
@@ -139,22 +141,22 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
           qs[tt * D + n] = to_float(pq[tt][b]);
           ks[tt * D + n] = to_float(pk[tt][b]);
           if constexpr (MODE == 1)
-            gates[2 * SCAN_CHUNK + tt * D + n] = expf(rate * softplus_f(pg[tt][b] + ch_bias[b]));
+            gates[2 * CH + tt * D + n] = expf(rate * softplus_f(pg[tt][b] + ch_bias[b]));
         }
       }
     }
 #pragma unroll
     for (int r = 0; r < XR; ++r) {
       const int i = threadIdx.x + SCAN_THREADS * r;
-      if (i < SCAN_CHUNK * COLS) vs[i] = to_float(pv[r]);
+      if (i < CH * COLS) vs[i] = to_float(pv[r]);
     }
     if ((int)threadIdx.x < nt) {
       if constexpr (MODE == 2) {
         gates[threadIdx.x] = 1.f;
-        gates[SCAN_CHUNK + threadIdx.x] = bias;
+        gates[CH + threadIdx.x] = bias;
       } else {
         gates[threadIdx.x] = 1.f / (1.f + expf(-to_float(pbeta)));
-        gates[SCAN_CHUNK + threadIdx.x] = MODE == 1 ? 1.f : expf(rate * softplus_f(to_float(pdecay) + bias));
+        gates[CH + threadIdx.x] = MODE == 1 ? 1.f : expf(rate * softplus_f(to_float(pdecay) + bias));
       }
     }
   };
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
   auto turn_rows = [&](float* buf, int nt) {
     if constexpr (MODE == 2) {
       float* qs = buf;
-      float* ks = qs + SCAN_CHUNK * D;
+      float* ks = qs + CH * D;
 #pragma unroll
       for (int r = 0; r < NPL; ++r) {
         const int idx = threadIdx.x + SCAN_THREADS * r;
@@ -181,24 +183,24 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
     }
   };
 
-  fetch(q0, min(SCAN_CHUNK, q1 - q0));
-  put(sm, min(SCAN_CHUNK, q1 - q0));
+  fetch(q0, min(CH, q1 - q0));
+  put(sm, min(CH, q1 - q0));
   if constexpr (MODE == 2) {
     __syncthreads();
-    turn_rows(sm, min(SCAN_CHUNK, q1 - q0));
+    turn_rows(sm, min(CH, q1 - q0));
   }
   __syncthreads();
   int turn = 0;
-  for (int t0 = q0; t0 < q1; t0 += SCAN_CHUNK, turn ^= 1) {
-    const int nt = min(SCAN_CHUNK, q1 - t0);
-    const int next = min(SCAN_CHUNK, q1 - t0 - SCAN_CHUNK);
-    if (next > 0) fetch(t0 + SCAN_CHUNK, next);
+  for (int t0 = q0; t0 < q1; t0 += CH, turn ^= 1) {
+    const int nt = min(CH, q1 - t0);
+    const int next = min(CH, q1 - t0 - CH);
+    if (next > 0) fetch(t0 + CH, next);
     const float* qs = sm + turn * per;
-    const float* ks = qs + SCAN_CHUNK * D;
-    const float* vs = ks + SCAN_CHUNK * D;
-    const float* gates = vs + SCAN_CHUNK * COLS;
+    const float* ks = qs + CH * D;
+    const float* vs = ks + CH * D;
+    const float* gates = vs + CH * COLS;
     auto token = [&](int tt) {
-      const float beta = gates[tt], decay = gates[SCAN_CHUNK + tt];
+      const float beta = gates[tt], decay = gates[CH + tt];
       float qv[NPL], kv[NPL];
       // sums of squares of the raw q and k rows and their product: unit vectors without a pass of
       // their own (every warp of the block forms them for itself; they do not wait for the state)
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
 #pragma unroll
         for (int e = 0; e < NPL; ++e) {
           const int n = lane + 32 * e;
-          const float gn = n < D ? gates[2 * SCAN_CHUNK + tt * D + n] : 1.f;
+          const float gn = n < D ? gates[2 * CH + tt * D + n] : 1.f;
 #pragma unroll
           for (int c = 0; c < WC; ++c) S[e][c] *= gn;
         }
@@ -268,9 +270,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a) {
         for (int e = 0; e < NPL; ++e) S[e][c] = fmaf(kv[e], u, decay * S[e][c]);
       }
     };
-    if (nt == SCAN_CHUNK) {
+    if (nt == CH) {
 #pragma unroll
-      for (int tt = 0; tt < SCAN_CHUNK; ++tt) token(tt);
+      for (int tt = 0; tt < CH; ++tt) token(tt);
     } else {
       for (int tt = 0; tt < nt; ++tt) token(tt);
     }
@@ -573,15 +575,20 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) delta_seq_kernel
 }
 
 template <typename AT, int NPL, int WC, int MODE = 0>
-static int launch_delta(DeltaArgs a, int S, cudaStream_t stream) {
+static int launch_delta(DeltaArgs a, int S, int T, cudaStream_t stream) {
   constexpr int COLS = SCAN_WARPS * WC;
+  a.vec = !(a.P % (WC % 4 == 0 ? 4 : 2)) && !(a.slot_stride % 4) && !((uintptr_t)a.state & 15);
+  const dim3 grid((a.P + COLS - 1) / COLS, a.heads, S);
+  if (T == S) {
+    const size_t one = (size_t)2 * ((MODE == 1 ? 3 : 2) * a.D + COLS + 2) * sizeof(float);
+    const cudaError_t e = launch_pdl(delta_scan_kernel<AT, NPL, WC, MODE, 1>, grid, dim3(SCAN_THREADS), one, stream, a);
+    return e == cudaSuccess ? FT_OK : (int)e;
+  }
   const size_t smem = (size_t)2 * SCAN_CHUNK * ((MODE == 1 ? 3 : 2) * a.D + COLS + 2) * sizeof(float);
   if (smem > 96 * 1024) return FT_ERR_SHAPE;
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(delta_scan_kernel<AT, NPL, WC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  a.vec = !(a.P % (WC % 4 == 0 ? 4 : 2)) && !(a.slot_stride % 4) && !((uintptr_t)a.state & 15);
-  const dim3 grid((a.P + COLS - 1) / COLS, a.heads, S);
-  cudaError_t e = launch_pdl(delta_scan_kernel<AT, NPL, WC, MODE>, grid, dim3(SCAN_THREADS), smem, stream, a);
+    cudaFuncSetAttribute(delta_scan_kernel<AT, NPL, WC, MODE, SCAN_CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = launch_pdl(delta_scan_kernel<AT, NPL, WC, MODE, SCAN_CHUNK>, grid, dim3(SCAN_THREADS), smem, stream, a);
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
@@ -621,10 +628,10 @@ static int dispatch_delta(DeltaArgs a, int S, int T, int longest, int dtype, cud
     });
   } else {
     FT_DISPATCH(dtype, AT, {
-      if (D <= 32) rc = narrow ? launch_delta<AT, 1, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 1, 8, MODE>(a, S, stream);
-      else if (D <= 64) rc = narrow ? launch_delta<AT, 2, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 2, 8, MODE>(a, S, stream);
-      else if (D <= 128) rc = narrow ? launch_delta<AT, 4, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 4, 8, MODE>(a, S, stream);
-      else rc = narrow ? launch_delta<AT, 8, NARROW_WC, MODE>(a, S, stream) : launch_delta<AT, 8, 8, MODE>(a, S, stream);
+      if (D <= 32) rc = narrow ? launch_delta<AT, 1, NARROW_WC, MODE>(a, S, T, stream) : launch_delta<AT, 1, 8, MODE>(a, S, T, stream);
+      else if (D <= 64) rc = narrow ? launch_delta<AT, 2, NARROW_WC, MODE>(a, S, T, stream) : launch_delta<AT, 2, 8, MODE>(a, S, T, stream);
+      else if (D <= 128) rc = narrow ? launch_delta<AT, 4, NARROW_WC, MODE>(a, S, T, stream) : launch_delta<AT, 4, 8, MODE>(a, S, T, stream);
+      else rc = narrow ? launch_delta<AT, 8, NARROW_WC, MODE>(a, S, T, stream) : launch_delta<AT, 8, 8, MODE>(a, S, T, stream);
     });
   }
   if (rc != FT_OK) return rc;

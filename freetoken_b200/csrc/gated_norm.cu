@@ -82,12 +82,19 @@ __global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* __rest
   const AT* gate = z + (size_t)t * ldz + base;
   float4 keep[KEEP], gk[KEEP];
   float ss = 0.f;
+  // every piece is on its way before the first is used: behind one another's branches the loads waited in turn
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    const int gi = min(sub + j * TPI, max(pieces - 1, 0));
+    keep[j] = ld4(row + 4 * gi);
+    gk[j] = ld4(gate + 4 * gi);
+  }
 #pragma unroll
   for (int j = 0; j < KEEP; ++j) {
     const int gi = sub + j * TPI;
     if (gi < pieces) {
-      float4 v = ld4(row + 4 * gi);
-      const float4 gr = ld4(gate + 4 * gi);
+      float4 v = keep[j];
+      const float4 gr = gk[j];
       const float4 gv = make_float4(gate_f(gr.x, gate_kind), gate_f(gr.y, gate_kind), gate_f(gr.z, gate_kind), gate_f(gr.w, gate_kind));
       if (gate_first) { v.x *= gv.x; v.y *= gv.y; v.z *= gv.z; v.w *= gv.w; }
       keep[j] = v;

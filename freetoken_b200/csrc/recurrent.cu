@@ -259,11 +259,12 @@ struct SsdArgs {
 };
 
 // NPL: state rows a lane holds (N <= 32 * NPL); WC: state columns a warp owns
-template <typename AT, int NPL, int WC>
+// CH: tokens of a chunk; segments of one token each take a chunk of one, whose rows need few registers.
+template <typename AT, int NPL, int WC, int CH>
 __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
   constexpr int COLS = SCAN_WARPS * WC;
   constexpr int NB = (NPL * 32 + SCAN_THREADS - 1) / SCAN_THREADS;       // B (or C) values a thread stages per token
-  constexpr int XR = (SCAN_CHUNK * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
+  constexpr int XR = (CH * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
   extern __shared__ float sm[];
   if (!a.state_ahead) pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
   const int inner = a.heads * P;
   const int col0 = blockIdx.x * COLS;
   const int j0 = col0 + warp * WC;
-  const int per = SCAN_CHUNK * (2 * N + COLS + 2);                         // floats of one buffer
+  const int per = CH * (2 * N + COLS + 2);                         // floats of one buffer
   const int q0 = a.seg_q_start[seg], q1 = a.seg_q_start[seg + 1];
   float* st = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * N * P;
   const float rate = -expf(a.A_log[head]), bias = a.dt_bias[head], skip = a.D[head];
@@ -292,10 +293,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
   }
   if (a.state_ahead) pdl_wait();
 
-  AT pb[SCAN_CHUNK][NB], pc[SCAN_CHUNK][NB], px[XR], pdt;
+  AT pb[CH][NB], pc[CH][NB], px[XR], pdt;
   auto fetch = [&](int t0, int nt) {
 #pragma unroll
-    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+    for (int tt = 0; tt < CH; ++tt) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const int n = threadIdx.x + SCAN_THREADS * b;
@@ -315,11 +316,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
   };
   auto put = [&](float* buf, int nt) {
     float* Bs = buf;
-    float* Cs = Bs + SCAN_CHUNK * N;
-    float* xs = Cs + SCAN_CHUNK * N;
-    float* dts = xs + SCAN_CHUNK * COLS;
+    float* Cs = Bs + CH * N;
+    float* xs = Cs + CH * N;
+    float* dts = xs + CH * COLS;
 #pragma unroll
-    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+    for (int tt = 0; tt < CH; ++tt) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const int n = threadIdx.x + SCAN_THREADS * b;
@@ -332,29 +333,29 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
 #pragma unroll
     for (int r = 0; r < XR; ++r) {
       const int i = threadIdx.x + SCAN_THREADS * r;
-      if (i < SCAN_CHUNK * COLS) xs[i] = to_float(px[r]);
+      if (i < CH * COLS) xs[i] = to_float(px[r]);
     }
     if ((int)threadIdx.x < nt) {
       const float step = softplus_f(to_float(pdt) + bias);
       dts[threadIdx.x] = step;
-      dts[SCAN_CHUNK + threadIdx.x] = expf(rate * step);
+      dts[CH + threadIdx.x] = expf(rate * step);
     }
   };
 
-  fetch(q0, min(SCAN_CHUNK, q1 - q0));
-  put(sm, min(SCAN_CHUNK, q1 - q0));
+  fetch(q0, min(CH, q1 - q0));
+  put(sm, min(CH, q1 - q0));
   __syncthreads();
   int turn = 0;
-  for (int t0 = q0; t0 < q1; t0 += SCAN_CHUNK, turn ^= 1) {
-    const int nt = min(SCAN_CHUNK, q1 - t0);
-    const int next = min(SCAN_CHUNK, q1 - t0 - SCAN_CHUNK);
-    if (next > 0) fetch(t0 + SCAN_CHUNK, next);
+  for (int t0 = q0; t0 < q1; t0 += CH, turn ^= 1) {
+    const int nt = min(CH, q1 - t0);
+    const int next = min(CH, q1 - t0 - CH);
+    if (next > 0) fetch(t0 + CH, next);
     const float* Bs = sm + turn * per;
-    const float* Cs = Bs + SCAN_CHUNK * N;
-    const float* xs = Cs + SCAN_CHUNK * N;
-    const float* dts = xs + SCAN_CHUNK * COLS;
+    const float* Cs = Bs + CH * N;
+    const float* xs = Cs + CH * N;
+    const float* dts = xs + CH * COLS;
     auto token = [&](int tt) {
-      const float step = dts[tt], decay = dts[SCAN_CHUNK + tt];
+      const float step = dts[tt], decay = dts[CH + tt];
       float Bv[NPL], Cv[NPL];
 #pragma unroll
       for (int e = 0; e < NPL; ++e) {
@@ -384,9 +385,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(SsdArgs a) {
         a.y[(size_t)(t0 + tt) * inner + (size_t)head * P + j0 + c] = part[0] + skip * mine;
       }
     };
-    if (nt == SCAN_CHUNK) {
+    if (nt == CH) {
 #pragma unroll
-      for (int tt = 0; tt < SCAN_CHUNK; ++tt) token(tt);
+      for (int tt = 0; tt < CH; ++tt) token(tt);
     } else {
       for (int tt = 0; tt < nt; ++tt) token(tt);
     }
@@ -549,13 +550,15 @@ __global__ void __launch_bounds__(SEQ_THREADS, NPL < 8 ? 2 : 1) ssd_seq_kernel(S
 }
 
 template <typename AT, int NPL, int WC>
-static int launch_ssd(SsdArgs a, int S, cudaStream_t stream) {
+static int launch_ssd(SsdArgs a, int S, int T, cudaStream_t stream) {
   constexpr int COLS = SCAN_WARPS * WC;
   const size_t smem = (size_t)2 * SCAN_CHUNK * (2 * a.N + COLS + 2) * sizeof(float);
   if (smem > 48 * 1024) return FT_ERR_SHAPE;
   a.vec = !(a.P % (WC % 4 == 0 ? 4 : 2)) && !(a.slot_stride % 4) && !((uintptr_t)a.state & 15);
   const dim3 grid((a.P + COLS - 1) / COLS, a.heads, S);
-  cudaError_t e = launch_pdl(ssd_scan_kernel<AT, NPL, WC>, grid, dim3(SCAN_THREADS), smem, stream, a);
+  const cudaError_t e =
+      T == S ? launch_pdl(ssd_scan_kernel<AT, NPL, WC, 1>, grid, dim3(SCAN_THREADS), smem / SCAN_CHUNK, stream, a)
+             : launch_pdl(ssd_scan_kernel<AT, NPL, WC, SCAN_CHUNK>, grid, dim3(SCAN_THREADS), smem, stream, a);
   return e == cudaSuccess ? FT_OK : (int)e;
 }
 
@@ -664,10 +667,10 @@ int ft_ssd_scan(const void* xbc, long long ld, const void* dt, long long ld_dt, 
     });
   } else {
     FT_DISPATCH(dtype, AT, {
-      if (N <= 32) rc = narrow ? launch_ssd<AT, 1, NARROW_WC>(a, S, stream) : launch_ssd<AT, 1, 8>(a, S, stream);
-      else if (N <= 64) rc = narrow ? launch_ssd<AT, 2, NARROW_WC>(a, S, stream) : launch_ssd<AT, 2, 8>(a, S, stream);
-      else if (N <= 128) rc = narrow ? launch_ssd<AT, 4, NARROW_WC>(a, S, stream) : launch_ssd<AT, 4, 8>(a, S, stream);
-      else rc = narrow ? launch_ssd<AT, 8, NARROW_WC>(a, S, stream) : launch_ssd<AT, 8, 8>(a, S, stream);
+      if (N <= 32) rc = narrow ? launch_ssd<AT, 1, NARROW_WC>(a, S, T, stream) : launch_ssd<AT, 1, 8>(a, S, T, stream);
+      else if (N <= 64) rc = narrow ? launch_ssd<AT, 2, NARROW_WC>(a, S, T, stream) : launch_ssd<AT, 2, 8>(a, S, T, stream);
+      else if (N <= 128) rc = narrow ? launch_ssd<AT, 4, NARROW_WC>(a, S, T, stream) : launch_ssd<AT, 4, 8>(a, S, T, stream);
+      else rc = narrow ? launch_ssd<AT, 8, NARROW_WC>(a, S, T, stream) : launch_ssd<AT, 8, 8>(a, S, T, stream);
     });
   }
   if (rc != FT_OK) return rc;
