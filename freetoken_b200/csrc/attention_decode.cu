@@ -63,9 +63,10 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
   const int pos = a.token_pos[tok];
   const int* table = a.block_table + (size_t)a.token_seg[tok] * a.table_width;
   const int lo = first_visible(pos, a.window, a.opt.chunk);
-  const int k_begin = max(lo, split * a.split_keys) / TILE * TILE;
-  const int k_end = min(pos + 1, (split + 1) * a.split_keys);
-  const int first_valid = max(lo, split * a.split_keys);
+  // the splits divide what the row sees, from the tile of its first key on
+  const int k_begin = lo / TILE * TILE + split * a.split_keys;
+  const int k_end = min(pos + 1, k_begin + a.split_keys);
+  const int first_valid = max(lo, k_begin);
 
   // Q tile -> shared (rows >= heads are zero)
   for (int idx = tid; idx < 16 * CH; idx += 128) {

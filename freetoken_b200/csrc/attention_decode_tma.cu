@@ -51,6 +51,7 @@ struct DecodeTmaArgs {
   float scale;
   ScoreOpts opt;             // chunks, cap, sink (the sink joins the partial of split 0)
   int v_plane = 1;           // which plane of the cache holds the values (0: the keys are the values)
+  int lets_in = 0;           // the next launch becomes resident beside this one
 };
 
 constexpr int DT_TILE = 64;
@@ -90,15 +91,17 @@ __global__ void __launch_bounds__(160) attn_decode_tma_kernel(const __grid_const
   const int pos = a.token_pos[tok];
   const int* table = a.block_table + (size_t)a.token_seg[tok] * a.table_width;
   const int lo = first_visible(pos, a.window, a.opt.chunk);
-  const int k_begin = max(lo, split * a.split_keys) / TILE * TILE;
-  const int k_end = min(pos + 1, (split + 1) * a.split_keys);
-  const int first_valid = max(lo, split * a.split_keys);
+  // the splits divide what the row sees, from the tile of its first key on
+  const int base = lo / TILE * TILE;
+  const int k_begin = base + split * a.split_keys;
+  const int k_end = min(pos + 1, k_begin + a.split_keys);
+  const int first_valid = max(lo, k_begin);
   const int ntiles = k_end > k_begin ? (k_end - k_begin + TILE - 1) / TILE : 0;
   // What stands above is the step's metadata.  A launch that fills the chip lets the next one in only as it leaves: a
   // product that becomes resident beside these blocks works in the little L1 that their stages leave an SM, to its end
   // (a projection of 192 blocks behind 256 of these: 10 -> 21 us).
   pdl_wait_only();
-  if (gridDim.x * gridDim.y * gridDim.z <= 74) pdl_release();
+  if (a.lets_in) pdl_release();
 
   // Q tile -> shared (rows >= heads are zero), by the consumers
   if (warp < 4) {
@@ -365,18 +368,44 @@ __global__ void __launch_bounds__(160) attn_decode_tma_kernel(const __grid_const
 constexpr int DT_MAX_CLUSTER = 8;      // portable cluster size
 
 template <int D>
-int launch_decode_tma(const CUtensorMap& mkv, const DecodeTmaArgs& a, cudaStream_t stream) {
-  const int G = a.nq / a.nkv;
-  const size_t smem = (size_t)DT_STAGES * 2 * (D / 64) * DT_TILE * 128 + 16 * (D + 8) * sizeof(__nv_bfloat16) + 1024;
+constexpr size_t decode_tma_smem() {
+  return (size_t)DT_STAGES * 2 * (D / 64) * DT_TILE * 128 + 16 * (D + 8) * sizeof(__nv_bfloat16) + 1024;
+}
+template <int D>
+cudaError_t configure_decode_tma() {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    constexpr int smem = (int)decode_tma_smem<D>();
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
     configured = true;
   }
+  return cudaSuccess;
+}
+template <int D>
+int clusters_at_once(int size) {
+  if (configure_decode_tma<D>() != cudaSuccess) return -1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, (unsigned)size);
+  cfg.blockDim = dim3(160);
+  cfg.dynamicSmemBytes = decode_tma_smem<D>();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = (unsigned)size;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<D, true>, &cfg) == cudaSuccess ? n : -1;
+}
+template <int D>
+int launch_decode_tma(const CUtensorMap& mkv, const DecodeTmaArgs& a, cudaStream_t stream) {
+  const int G = a.nq / a.nkv;
+  constexpr size_t smem = decode_tma_smem<D>();
+  const cudaError_t ready = configure_decode_tma<D>();
+  if (ready != cudaSuccess) return (int)ready;
   dim3 grid(a.n_rows, a.nkv * ((G + 15) / 16), a.splits);
   if (a.splits > 1 && a.splits <= DT_MAX_CLUSTER && !a.part_o) {
     // the splits of a (row, head tile) as one cluster along z
@@ -405,6 +434,12 @@ int launch_decode_tma(const CUtensorMap& mkv, const DecodeTmaArgs& a, cudaStream
 
 using namespace ft;
 
+// How many clusters of `size` (2 .. 8) CTAs find a place at once; negative: not known.
+extern "C" int ft_attn_decode_clusters(int d, int size) {
+  if (size < 2 || size > DT_MAX_CLUSTER) return -1;
+  return d == 64 ? clusters_at_once<64>(size) : d == 128 ? clusters_at_once<128>(size) : -1;
+}
+
 // bfloat16; head_dim 64 or 128; page size a multiple of 64.  `map_kv`: the 5-D map
 // over the layer's pages (ft_attn_tc_kv_map of the prefill library).  Up to 8 splits
 // are merged inside the kernel by a cluster when part_o is null; otherwise part_o /
@@ -414,7 +449,7 @@ extern "C" int ft_attn_decode_tma(const void* map_kv, const void* q, void* out, 
                                   const int* token_seg, const int* block_table, int* status, int nq,
                                   int nkv, int d, int P, int table_width, int window, int n_rows,
                                   int splits, int split_keys, float scale, int v_plane, int chunk,
-                                  float softcap, int sink_mode, float sink_value, const float* sink,
+                                  float softcap, int sink_mode, float sink_value, const float* sink, int lets_in,
                                   cudaStream_t stream) {
   if (n_rows <= 0) return FT_OK;
   if (nkv <= 0 || nq % nkv || splits < 1 || split_keys < DT_TILE || split_keys % DT_TILE || P % DT_TILE)
@@ -424,7 +459,7 @@ extern "C" int ft_attn_decode_tma(const void* map_kv, const void* q, void* out, 
   memcpy(&mkv, map_kv, sizeof(mkv));
   DecodeTmaArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, part_o, part_ml, rows, token_pos,
                   token_seg, block_table, status, nq, nkv, P, table_width, window, n_rows, splits,
-                  split_keys, scale, ScoreOpts{chunk, softcap, sink_mode, sink_value, sink}, v_plane ? 1 : 0};
+                  split_keys, scale, ScoreOpts{chunk, softcap, sink_mode, sink_value, sink}, v_plane ? 1 : 0, lets_in};
   if (sink_mode == 2 && !sink) return FT_ERR_SHAPE;
   int rc;
   switch (d) {

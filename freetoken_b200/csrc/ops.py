@@ -1265,8 +1265,28 @@ CLUSTER_SPLITS = 8     # splits the TMA-fed decode kernel merges by itself (a th
 MERGE_COST = 24        # what the separate merge kernel costs, in 64-key tiles of a CTA's work
 
 
+# A decode attention of up to this many CTAs lets the next launch become resident beside it; of more, that launch would
+# work in the little L1 that the CTAs' stages leave an SM (one row of 4 KV heads x 1,024 keys with the projection of 2,048 x
+# 2,048 behind it: 7.7 us against 10.0; 8 rows of 8 KV heads with one of 3,072 x 6,144: 32 against 21).
+DECODE_LETS_IN = 74
+
+
+_CLUSTER_ROOM: Dict[tuple, Dict[int, int]] = {}
+
+
+def cluster_room(device, head_dim: int) -> Dict[int, int]:
+    """Size of a cluster of the decode kernel -> how many find a place on the device at once."""
+    key = (torch.device(device).index or 0, head_dim)
+    room = _CLUSTER_ROOM.get(key)
+    if room is None:
+        ask = build.load("attention_decode_tma").ft_attn_decode_clusters
+        answers = {size: ask(head_dim, size) for size in range(2, CLUSTER_SPLITS + 1)}
+        room = _CLUSTER_ROOM[key] = {size: n for size, n in answers.items() if n > 0}
+    return room
+
+
 def decode_splits(n_rows: int, num_kv_heads: int, group: int, max_kv_len: int, sms: int,
-                  cluster_merge: bool = False):
+                  cluster_merge: bool = False, room: Optional[Dict[int, int]] = None):
     """``(splits, keys per split)``, whole 64-key tiles per split.
 
     Two CTAs of the decode kernel fit an SM and a launch takes as long as its
@@ -1275,7 +1295,10 @@ def decode_splits(n_rows: int, num_kv_heads: int, group: int, max_kv_len: int, s
     the least such time is taken, the smaller one on a tie - not just "enough
     CTAs to fill the SMs", which leaves a second round nearly empty at some
     sizes.  With ``cluster_merge`` up to :data:`CLUSTER_SPLITS` splits are merged
-    inside the kernel; more need the merge kernel, whose launch is counted."""
+    inside the kernel; more need the merge kernel, whose launch is counted.  ``room``
+    (:func:`cluster_room`): a cluster's CTAs share a part of the chip, which is no multiple of
+    every size, and what does not fit waits for a whole round (8 rows x 4 KV heads x 1,024 keys,
+    with the projection behind it: eight splits 17.6 us, six 13.4)."""
     base = max(1, n_rows * num_kv_heads * (-(-group // 16)))
     tiles = max(1, -(-max_kv_len // 64))
     slots = 2 * sms
@@ -1286,6 +1309,9 @@ def decode_splits(n_rows: int, num_kv_heads: int, group: int, max_kv_len: int, s
         if splits != want:
             continue                      # the same split as a smaller request
         rounds = -(-base * splits // slots)
+        if cluster_merge and room and 1 < splits <= CLUSTER_SPLITS and splits in room:
+            # a sixteenth less: the launch in front may still hold some SMs, and then a full house is two rounds
+            rounds = max(rounds, -(-base // max(1, room[splits] * 15 // 16)))
         cost = rounds * (per + 3)
         if cluster_merge and splits > CLUSTER_SPLITS:
             cost += MERGE_COST
@@ -1313,8 +1339,14 @@ def attn_decode(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
         _need(rows, "rows", torch.int32)
     tma = DECODE_TMA and head_dim in (64, 128) and kv_pages.shape[3] % 64 == 0 \
         and kv_pages.stride(4) == 1 and kv_pages.stride(3) == head_dim
+    # what a row sees begins at the tile of its first key
+    reach = min((n for n in (int(window or 0), options.chunk if options is not None else 0) if n > 0), default=0)
+    if reach:
+        max_kv_len = min(max_kv_len, reach + 63)
+    clusters = tma and DECODE_CLUSTER
     splits, split_keys = decode_splits(n_rows, num_kv_heads, num_heads // num_kv_heads, max_kv_len,
-                                       sm_count(q.device), cluster_merge=tma and DECODE_CLUSTER)
+                                       sm_count(q.device), cluster_merge=clusters,
+                                       room=cluster_room(q.device, head_dim) if clusters else None)
     part_o = part_ml = None
     if splits > 1 and not (tma and DECODE_CLUSTER and splits <= CLUSTER_SPLITS):
         part_o = workspace.get("attn.part_o", (n_rows, num_heads, splits, head_dim), torch.float32)
@@ -1331,12 +1363,13 @@ def attn_decode(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
                       head_dim, kv_pages.stride(2), kv_pages.stride(1), kv_pages.stride(0))
         map_kv = _attn_tc_map("kv", (kv_pages.data_ptr(),) + tuple(kv_pages.shape) + tuple(kv_pages.stride()),
                               make_kv)
-        f = _fn("attention_decode_tma", "ft_attn_decode_tma", "p p p p p p p p p p i i i i i i i i i f i i f i f p")
+        f = _fn("attention_decode_tma", "ft_attn_decode_tma", "p p p p p p p p p p i i i i i i i i i f i i f i f p i")
         f(map_kv, q, out, part_o, part_ml,
           rows, token_pos, token_seg, block_table, tc_status(q.device),
           num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
           int(window or 0), n_rows, splits, split_keys, float(scale),
-          1 if kv_pages.stride(0) else 0, *extra)
+          1 if kv_pages.stride(0) else 0, *extra,
+          int(n_rows * num_kv_heads * -(-(num_heads // num_kv_heads) // 16) * splits <= DECODE_LETS_IN))
         if part_o is not None:
             fm = _fn("attention_decode", "ft_attn_merge", "p p p p i i i i")
             fm(part_o, part_ml, out, rows, n_rows, num_heads, head_dim,

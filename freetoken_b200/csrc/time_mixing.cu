@@ -69,23 +69,33 @@ struct ShiftArgs {
 // is the only one that reads the slot, and it alone replaces the slot's contents, after its read.
 template <typename AT, int VEC, int RUN>
 __global__ void __launch_bounds__(128) token_shift_kernel(ShiftArgs a) {
-  pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+  // of few tokens: the mixes' factors, cold in L2 and fetched one behind the other's store below, are near before the wait
+  if (RUN == 1 && gridDim.x <= 64 && c < a.W)
+    for (int m = 0; m < a.M; ++m) warm(a.mu + (size_t)m * a.W + c);
+  const int t0 = blockIdx.x * RUN;
+  int seg0 = 0, q0_0 = 0, end0 = 0, slot0 = 0;         // the first token's: three lookups that no launch of the step writes
+  if (RUN == 1) {
+    seg0 = a.token_seg[t0];
+    q0_0 = a.seg_q_start[seg0];
+    end0 = a.seg_q_start[seg0 + 1];
+    slot0 = a.seg_slot[seg0];
+  }
+  pdl_wait();
   if (c >= a.W) return;
   const AT* x = (const AT*)a.x;
   float cur[RUN][VEC], step[RUN][VEC];                 // x_t and x_{t-1} - x_t
-  const int t0 = blockIdx.x * RUN;
 #pragma unroll
   for (int i = 0; i < RUN; ++i) {
     const int t = t0 + i;
     if (t >= a.T) break;
-    const int seg = a.token_seg[t], q0 = a.seg_q_start[seg];
+    const int seg = RUN == 1 ? seg0 : a.token_seg[t], q0 = RUN == 1 ? q0_0 : a.seg_q_start[seg];
     load_piece(x + (size_t)t * a.ldx + c, cur[i]);
     if (t == q0) {
-      float* slot = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + c;
+      float* slot = a.state + (size_t)(RUN == 1 ? slot0 : a.seg_slot[seg]) * a.slot_stride + c;
       load_piece(slot, step[i]);
       float last[VEC];
-      load_piece(x + (size_t)(a.seg_q_start[seg + 1] - 1) * a.ldx + c, last);
+      load_piece(x + (size_t)((RUN == 1 ? end0 : a.seg_q_start[seg + 1]) - 1) * a.ldx + c, last);
       store_piece(slot, last);
     } else {
       load_piece(x + (size_t)(t - 1) * a.ldx + c, step[i]);
