@@ -149,6 +149,7 @@ class Engine:
         self._meta_generation = 0
         self._graphs: Dict[Tuple, "torch.cuda.CUDAGraph"] = {}
         self._graph_seen: Dict[Tuple, int] = {}
+        self._side_streams: List["torch.cuda.Stream"] = []
         self.graph_replays = 0
         self.steps = 0
         self.tokens_run = 0
@@ -421,6 +422,9 @@ class Engine:
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()
             before = ops.launch_count()
+            if not self._side_streams:
+                self._side_streams = [torch.cuda.Stream(self.device) for _ in range(3)]
+            ctx.side = list(self._side_streams)          # branches of the step become branches of the graph
             with torch.cuda.graph(graph):
                 self.model.forward(ctx, self.cache_views, logit_rows, logits, in_order)
             kernels = ops.launch_count() - before

@@ -161,6 +161,25 @@ class StepContext:
     # what a layer leaves for layers that run after it in the same step (values that later layers
     # blend in), by a name both know; rows in workspace buffers of their own
     shared: Dict[str, Any] = field(default_factory=dict)
+    # streams for :meth:`beside`, while a graph is captured (empty otherwise)
+    side: List[Any] = field(default_factory=list)
+
+    def beside(self, first: Callable[[], Any], second: Callable[[], Any], *scratch: Optional[Tuple[str, ...]]):
+        """``(first(), second())``, two pieces of a step that need nothing of each other; ``scratch``: the workspace names
+        of either (:meth:`Part.scratch_names`).  Where a decode step is captured they become two branches of the graph: a launch of few tokens leaves
+        most of the chip idle, and two chains of such launches pass in the time of the longer one.  Branches that
+        would write the same scratch, or whose scratch is not known, run one after the other, and so does everything outside a
+        capture (there a launch costs the host more than it costs the device)."""
+        if not self.side or None in scratch or set(scratch[0]) & set(scratch[1]) or not torch.cuda.is_current_stream_capturing():
+            return first(), second()
+        side, main = self.side.pop(), torch.cuda.current_stream(self.device)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            b = second()
+        a = first()
+        main.wait_stream(side)
+        self.side.append(side)
+        return a, b
 
     @property
     def num_segments(self) -> int:
@@ -219,6 +238,12 @@ class Part:
     # may lie further apart than H) and leaves its result there says so; a block that wants
     # the result in a place of its own copies it otherwise.
     writes_into_out = False
+    # The first words of the names of the workspace buffers a part writes (with those of its kernels' faces), or None:
+    # not stated, and then nothing runs beside the part (``StepContext.beside``).
+    scratch: Optional[Tuple[str, ...]] = None
+
+    def scratch_names(self) -> Optional[Tuple[str, ...]]:
+        return self.scratch
 
     def __init__(self, spec: PartSpec, prefix: str):
         self.spec = spec

@@ -89,14 +89,19 @@ class ParallelBlock(Block):
             return self.mixer.forward(ctx, h, cache)
         T, H = h.shape
         pair = ctx.workspace.get("block.pair", (T, 2, H), ctx.dtype)
-        if self.mixer.writes_into_out:
-            self.mixer.forward(ctx, h, cache, out=pair[:, 0])
-        else:
-            pair[:, 0].copy_(self.mixer.forward(ctx, h, cache))
-        if self.feed_forward.writes_into_out:
-            self.feed_forward.forward(ctx, h, out=pair[:, 1])
-        else:
-            pair[:, 1].copy_(plain_branch(ctx, self.feed_forward.forward(ctx, h)))
+
+        def mix():
+            if self.mixer.writes_into_out:
+                self.mixer.forward(ctx, h, cache, out=pair[:, 0])
+            else:
+                pair[:, 0].copy_(self.mixer.forward(ctx, h, cache))
+
+        def feed():
+            if self.feed_forward.writes_into_out:
+                self.feed_forward.forward(ctx, h, out=pair[:, 1])
+            else:
+                pair[:, 1].copy_(plain_branch(ctx, self.feed_forward.forward(ctx, h)))
+        ctx.beside(mix, feed, self.mixer.scratch_names(), self.feed_forward.scratch_names())
         return pair
 
 
@@ -118,8 +123,9 @@ class ParallelNormsBlock(Block):
             rows, scale = self.mixer.forward_parts(ctx, h, cache)
             return ops.RoutedRows(rows, scale=scale)
         h, g = self.norms["mixer"].forward_pair(ctx, delta, residual, self.norms["feed_forward"])
-        rows, scale = self.mixer.forward_parts(ctx, h, cache)
-        out = self.feed_forward.forward(ctx, g)
+        (rows, scale), out = ctx.beside(lambda: self.mixer.forward_parts(ctx, h, cache),
+                                        lambda: self.feed_forward.forward(ctx, g), self.mixer.scratch_names(),
+                                        self.feed_forward.scratch_names())
         if not isinstance(out, ops.RoutedRows):
             out = ops.RoutedRows(out)
         out.beside, out.beside_scale = rows, scale

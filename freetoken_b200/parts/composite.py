@@ -41,6 +41,10 @@ class MixerSum(Mixer):
     def children(self):
         return list(self.members)
 
+    def scratch_names(self):
+        names = [m.scratch_names() for m in self.members]
+        return None if None in names else ("mixer_sum", *sum(names, ()))
+
     def cache_need(self):
         return CompositeNeed(tuple(m.cache_need() for m in self.members))
 
@@ -60,11 +64,18 @@ class MixerSum(Mixer):
         """``(rows [T, members, H], scales)`` before they are added: for a consumer that adds rows anyway."""
         T, n = x.shape[0], len(self.members)
         rows = ctx.workspace.get("mixer_sum.rows", (T, n, self.hidden), ctx.dtype)
-        for j, (member, view) in enumerate(zip(self.members, cache.members)):
+
+        def run(j: int):
+            member, view = self.members[j], cache.members[j]
             if member.writes_into_out:
                 member.forward(ctx, x, view, out=rows[:, j])
             else:
                 rows[:, j].copy_(member.forward(ctx, x, view))
+        if n == 2:
+            ctx.beside(lambda: run(0), lambda: run(1), *(m.scratch_names() for m in self.members))
+        else:
+            for j in range(n):
+                run(j)
         return rows, self.scale_tensor
 
     def forward(self, ctx: StepContext, x: torch.Tensor, cache: CacheView, out=None) -> torch.Tensor:

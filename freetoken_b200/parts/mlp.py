@@ -27,6 +27,8 @@ class DenseMLP(FeedForward):
     A gated feed-forward may also take the clamped pair ``swigluoai`` with ``act_alpha`` and
     ``act_limit``: ``g = min(gate, limit)``, ``u = clamp(up, -limit, limit)``, ``g sigmoid(alpha g) (u + 1)``."""
 
+    scratch = ("mlp",)
+
     graph_capturable = True
     writes_into_out = True
 

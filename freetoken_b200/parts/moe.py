@@ -130,6 +130,12 @@ class RoutedExperts(FeedForward):
     def children(self):
         return [self.shared] if self.shared is not None else []
 
+    def scratch_names(self):
+        if self.shared is None:
+            return ("moe",)
+        names = self.shared.scratch_names()
+        return None if names is None else ("moe", *names)
+
     def tensor_specs(self) -> List[TensorSpec]:
         E, I, H = self.E, self.inter, self.hidden
         gate_up = Stack(tuple(
@@ -201,6 +207,19 @@ class RoutedExperts(FeedForward):
         return (ids, weights) if sort_into is None else (ids, weights, False)
 
     def forward(self, ctx: StepContext, x: torch.Tensor):
+        if self.shared is None:
+            return self.routed(ctx, x)
+        shared = ctx.workspace.get("moe.shared", (x.shape[0], self.hidden), ctx.dtype)
+        rows, extra = ctx.beside(lambda: self.routed(ctx, x), lambda: self.shared.forward(ctx, x, out=shared),
+                                 ("moe",), self.shared.scratch_names())
+        if isinstance(rows, ops.RoutedRows):
+            rows.extra = extra
+            return rows
+        gate = ctx.workspace.get("moe.shared_gate", (x.shape[0],), torch.float32) if self.shared_gate else None
+        return ops.RoutedRows(rows, extra=extra, extra_gate=gate)
+
+    def routed(self, ctx: StepContext, x: torch.Tensor):
+        """The routed experts alone: their rows, with the inputs handed back where there are identity experts."""
         T = x.shape[0]
         R = T * self.k
         ws = ctx.workspace
@@ -228,15 +247,7 @@ class RoutedExperts(FeedForward):
         # the k partial rows of a token are summed by whoever consumes them
         # (the next norm adds them into the residual in slot order)
         parts = parts.view(T, self.k, self.hidden)
-        if self.shared is None and not self.identity:
-            return parts
-        extra = None
-        if self.shared is not None:
-            extra = self.shared.forward(ctx, x, out=ws.get("moe.shared", (T, self.hidden), ctx.dtype))
-        if not self.identity:
-            gate = ws.get("moe.shared_gate", (T,), torch.float32) if self.shared_gate else None
-            return ops.RoutedRows(parts, extra=extra, extra_gate=gate)
-        return ops.RoutedRows(parts, ids, weights, self.E, x, extra)
+        return ops.RoutedRows(parts, ids, weights, self.E, x) if self.identity else parts
 
     def experts(self, ctx, x, mid, parts, offsets, active, sorted_route, sorted_token, route_weight, R):
         if ctx.dtype == torch.bfloat16 and R > TC_MIN_ROWS_PER_EXPERT * self.E \

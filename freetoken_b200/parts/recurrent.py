@@ -75,6 +75,8 @@ class SelectiveStateSpace(_Recurrent):
     norm_eps``, ``scope`` and ``names`` (in, conv, conv_bias, dt_bias, a_log, d, norm, o below
     the scope).  The input projection's rows are ``z | x | B | C | dt``."""
 
+    scratch = ("ssd",)
+
     kernels = ("recurrent",)
 
     def __init__(self, spec, prefix):
@@ -140,6 +142,8 @@ class GatedDelta(_Recurrent):
     beta, decay: the projections; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv:
     the merged projection and convolution the model keeps).  Query / key head ``h // (heads /
     key_heads)`` serves head ``h``; q is multiplied by ``key_dim ** -0.5`` after its unit norm."""
+
+    scratch = ("delta",)
 
     kernels = ("recurrent", "delta_scan")
 
@@ -213,6 +217,8 @@ class ChannelDelta(_Recurrent):
     of the decay's and the gate's; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv: the
     merged projection and convolution the model keeps).  ``dt_bias`` has one entry per head and key
     channel, ``norm`` one per value of a head (shared by the heads)."""
+
+    scratch = ("cdelta",)
 
     kernels = ("recurrent", "channel_delta")
 
@@ -294,6 +300,8 @@ class Retention(_Recurrent):
     ** -0.5`` after the rotation; the read-out of a head is divided by its root mean square (no
     weight), the row gated by ``silu(W_g h)``."""
 
+    scratch = ("retention",)
+
     kernels = ("retention",)
     taps = 1
     conv_channels = 0
@@ -362,6 +370,8 @@ class TimeMixing(Mixer):
     gate: projections; decay_down, decay_up: the decay's two steps; w0, u, norm, o; mu and rkvg: the merged
     mixes and projections the model keeps).  ``r, k, v`` and ``gate`` rows have one width, so ``key_dim`` must equal
     ``head_dim``; ``norm`` has one entry per value of the concatenated heads."""
+
+    scratch = ("tmix",)
 
     graph_capturable = True
     writes_into_out = True
