@@ -999,12 +999,36 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
             raise KernelError("skinny_gemm: the active list needs G + 1 entries")
     if unary is not None and (glu or unary not in ACTIVATIONS):
         raise KernelError(f"skinny_gemm: cannot apply {unary!r} (with glu: {glu})")
-    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i")
+    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i q q")
     f(a, a.stride(0), w, NW * K, c, code(c.dtype), c.stride(0),
       group_offsets, active, a_rows, c_rows, row_scale, M, N, K, G,
       int(glu), GLU_ACTS[act], float(act_alpha), float(act_limit),
       rows_per_pass, 0 if unary is None else 1 + ACTIVATIONS[unary], bias, int(group_rows),
-      int(lists_ahead))
+      int(lists_ahead), 0, 0)
+
+
+def skinny_heads_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether :func:`skinny_heads` takes these operands."""
+    return (x.dtype == w.dtype == out.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[2] % 8 == 0
+            and x.stride(2) == 1 and out.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0 and x.stride(1) > 0
+            and out.stride(1) > 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def skinny_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """``out[t, h] = w[h] @ x[t, h]`` for few tokens, one launch over the heads: ``x`` ``[T, H, K]``, ``w`` ``[H, N, K]``,
+    ``out`` ``[T, H, N]``; tokens and heads of ``x`` and ``out`` may lie any distance apart."""
+    _need(x, "x", torch.bfloat16, contiguous=False)
+    _need(w, "w", torch.bfloat16)
+    _need(out, "out", torch.bfloat16, contiguous=False)
+    T, H, K = x.shape
+    if w.shape[0] != H or w.shape[2] != K or out.shape != (T, H, w.shape[1]):
+        raise KernelError("skinny_heads: shapes do not match")
+    if not skinny_heads_takes(x, w, out):
+        raise KernelError("skinny_heads: needs bfloat16 operands, K % 8 == 0 and 16-byte aligned rows")
+    N = w.shape[1]
+    f = _fn("skinny_gemm", "ft_skinny_gemm", "p q p q p i q p p p p p i i i i i i f f i i p i i q q")
+    f(x, x.stride(0), w, N * K, out, BF16, out.stride(0), None, None, None, None, None, T * H, N, K, H, 0, 0, 0.0, 0.0,
+      pass_rows(T), 0, None, T, 0, x.stride(1), out.stride(1))
 
 
 # ------------------------------------------------ grouped GEMM on tcgen05

@@ -44,6 +44,7 @@ struct SkinnyArgs {
   int group_rows = 0;            // > 0: every group has that many rows, group g the rows g * group_rows ..
   int lists_ahead = 0;           // the lists were written before the launch right in front of this one began
   int first_round = 0;           // blocks that find a place on the chip at once
+  long long a_group = 0, c_group = 0;   // > 0 (with group_rows): group g's rows start at A + g * a_group, C + g * c_group
 };
 
 // Plain loads with a memory clobber, and a warp barrier behind a round's loads (skinny_kernel): the compiler may not
@@ -178,8 +179,8 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
       const int row = pass + 8 * j + g;
       xrow[j] = nullptr;
       if (row < row_end) {
-        const int src = a.a_rows ? a.a_rows[row] : row;
-        xrow[j] = reinterpret_cast<const uint4*>(a.A + (size_t)src * a.lda);
+        const int src = a.a_rows ? a.a_rows[row] : a.a_group ? row - row_begin : row;
+        xrow[j] = reinterpret_cast<const uint4*>(a.A + (size_t)group * a.a_group + (size_t)src * a.lda);
       }
     }
     float acc[NG][NT][4];
@@ -240,7 +241,8 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
         if (!GLU && a.bias) s += a.bias[n];
         float v = GLU ? glu_act_s(s, su, a.act, a.act_alpha, a.act_limit) : (a.unary ? unary_act_s(s, a.unary) : s);
         if (a.row_scale) v *= a.row_scale[crow];
-        C[(size_t)crow * a.ldc + n] = from_float<OT>(v);
+        if (a.c_group) C[(size_t)group * a.c_group + (size_t)(row - row_begin) * a.ldc + n] = from_float<OT>(v);
+        else C[(size_t)crow * a.ldc + n] = from_float<OT>(v);
       }
     }
     __syncthreads();
@@ -323,7 +325,8 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
                               const int* group_offsets, const int* active, const int* a_rows,
                               const int* c_rows, const float* row_scale, int M, int N, int K, int G, int glu,
                               int act, float act_alpha, float act_limit, int rows_per_pass, int unary,
-                              const float* bias, int group_rows, int lists_ahead, cudaStream_t stream) {
+                              const float* bias, int group_rows, int lists_ahead, long long a_group,
+                              long long c_group, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return FT_OK;
   if (K <= 0 || (K & 7) || (lda & 7) || G <= 0) return FT_ERR_SHAPE;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((w_group_stride * 2) & 15)) return FT_ERR_SHAPE;
@@ -336,6 +339,10 @@ extern "C" int ft_skinny_gemm(const void* A, long long lda, const void* W,
   a.bias = bias;
   a.group_rows = group_rows;
   a.lists_ahead = lists_ahead;
+  if (a_group < 0 || c_group < 0 || (a_group & 7) || (!a_group != !c_group) || (a_group && (!group_rows || c_rows || row_scale)))
+    return FT_ERR_SHAPE;
+  a.a_group = a_group;
+  a.c_group = c_group;
   // with the list of busy groups, no more groups than rows can have any
   dim3 grid((N + 15) / 16, active ? min(G, M) : G);
   const int nt = rows_per_pass / 8;

@@ -163,22 +163,26 @@ class StepContext:
     shared: Dict[str, Any] = field(default_factory=dict)
     # streams for :meth:`beside`, while a graph is captured (empty otherwise)
     side: List[Any] = field(default_factory=list)
+    minor: List[Any] = field(default_factory=list)       # of lower priority
 
-    def beside(self, first: Callable[[], Any], second: Callable[[], Any], *scratch: Optional[Tuple[str, ...]]):
+    def beside(self, first: Callable[[], Any], second: Callable[[], Any], *scratch: Optional[Tuple[str, ...]],
+               filler: bool = False):
         """``(first(), second())``, two pieces of a step that need nothing of each other; ``scratch``: the workspace names
-        of either (:meth:`Part.scratch_names`).  Where a decode step is captured they become two branches of the graph: a launch of few tokens leaves
+        of either (:meth:`Part.scratch_names`).  ``filler``: the second is the shorter one by far and takes what the first
+        leaves of the chip (shared experts beside the chain of router, selection and routed ones).  Where a decode step is captured they become two branches of the graph: a launch of few tokens leaves
         most of the chip idle, and two chains of such launches pass in the time of the longer one.  Branches that
         would write the same scratch, or whose scratch is not known, run one after the other, and so does everything outside a
         capture (there a launch costs the host more than it costs the device)."""
-        if not self.side or None in scratch or set(scratch[0]) & set(scratch[1]) or not torch.cuda.is_current_stream_capturing():
+        streams = self.minor if filler else self.side
+        if not streams or None in scratch or set(scratch[0]) & set(scratch[1]) or not torch.cuda.is_current_stream_capturing():
             return first(), second()
-        side, main = self.side.pop(), torch.cuda.current_stream(self.device)
+        side, main = streams.pop(), torch.cuda.current_stream(self.device)
         side.wait_stream(main)
         with torch.cuda.stream(side):
             b = second()
         a = first()
         main.wait_stream(side)
-        self.side.append(side)
+        streams.append(side)
         return a, b
 
     @property
@@ -241,6 +245,8 @@ class Part:
     # The first words of the names of the workspace buffers a part writes (with those of its kernels' faces), or None:
     # not stated, and then nothing runs beside the part (``StepContext.beside``).
     scratch: Optional[Tuple[str, ...]] = None
+    # whether the part runs something as a filler (``StepContext.beside``)
+    has_filler = False
 
     def scratch_names(self) -> Optional[Tuple[str, ...]]:
         return self.scratch

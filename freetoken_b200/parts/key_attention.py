@@ -142,6 +142,16 @@ class SharedKVAttention(PagedSoftmaxCore, Mixer):
         return linear.linear(o, self.w_o, out)
 
 
+def _per_head(x: torch.Tensor, rows: torch.Tensor, columns: torch.Tensor, out: torch.Tensor) -> None:
+    """``out[t, h] = W[h] x[t, h]`` in bfloat16; ``rows`` is W as ``[H, N, K]``, ``columns`` the same as ``[H, K, N]``.  Few
+    tokens take the weight-streaming kernel, whose first weights are on their way before the launch in front has ended and
+    which lets the next one in (the batched library product does neither); many the library product."""
+    if x.shape[0] <= linear.SKINNY_ROWS and ops.skinny_heads_takes(x, rows, out):
+        ops.skinny_heads(x, rows, out)
+    else:
+        torch.bmm(x.transpose(0, 1), columns, out=out.transpose(0, 1))
+
+
 @register_mixer("latent_attention")
 class LatentAttention(PagedSoftmaxCore, Mixer):
     """params: ``hidden_size, num_heads, qk_dim, v_dim, rank, sm_scale, norm_eps``,
@@ -288,8 +298,8 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         self.w_uk = self.w_up[:H * self.dq].view(H, self.dq, R)      # [head][dq, R]
         self.w_uv = self.w_up[H * self.dq:].view(H, self.dv, R)      # [head][dv, R]
         self.own_kernels, self.expands = self._takes_own_kernels(dtype), self._expands(dtype)
-        # the CUDA-core product wants [N, K] rows: Wuk^T per head
-        self.w_ukt = self.w_uk.transpose(1, 2).contiguous() if dtype == torch.float32 else None
+        # the CUDA-core product and the weight-streaming one want [N, K] rows: Wuk^T per head
+        self.w_ukt = self.w_uk.transpose(1, 2).contiguous()
         self.w_o = tensors[self.n["o"]]
         if self.q_rank:
             self.w_qnorm = tensors[self.n["q_norm"]]
@@ -318,12 +328,11 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
             # the tokens from the first to the last absorbed segment; whatever lies between is overwritten below
             t0, t1 = host["flat_tokens"]
             q_heads = q[t0:t1].unflatten(1, (H, dq + rot))[:, :, :dq]
-            torch.bmm(q_heads.transpose(0, 1), self.w_uk, out=q_abs[t0:t1, :, :R].transpose(0, 1))
+            _per_head(q_heads, self.w_ukt, self.w_uk, q_abs[t0:t1, :, :R])
             o = ws.get("lattn.o", (T, H, R), ctx.dtype)
             ops.attn_latent(q_abs, o, cache.pages, lists["flat_seg"], lists["flat_row"], ctx.seg_q_start,
                             ctx.seg_pos0, table, H, R, self.scale, self.window, host["flat_kv"], ws)
-            torch.bmm(o[t0:t1].transpose(0, 1), self.w_uv.transpose(1, 2),
-                      out=y.view(T, H, dv)[t0:t1].transpose(0, 1))
+            _per_head(o[t0:t1], self.w_uv, self.w_uv.transpose(1, 2), y.view(T, H, dv)[t0:t1])
         if host["expanded"]:
             rows = host["rows"]
             plain = ws.get("lattn.rows", (rows, d), ctx.dtype)
@@ -374,7 +383,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         if ctx.dtype == torch.float32:
             ops.gemm_heads(q_heads, self.w_ukt, q_abs[:, :, :R])
         else:
-            torch.bmm(q_heads.transpose(0, 1), self.w_uk, out=q_abs[:, :, :R].transpose(0, 1))
+            _per_head(q_heads, self.w_ukt, self.w_uk, q_abs[:, :, :R])
         o = ws.get("lattn.o", (T, H * d), ctx.dtype)
         self.attend(ctx, q_abs.view(T, H * d), o, _both_planes(cache.pages), table)
         # the first rank values of a head's result are the weighted latents: Wuv per head, then the gate
@@ -383,7 +392,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         if ctx.dtype == torch.float32:
             ops.gemm_heads(o_latent, self.w_uv, y.view(T, H, dv))
         else:
-            torch.bmm(o_latent.transpose(0, 1), self.w_uv.transpose(1, 2), out=y.view(T, H, dv).transpose(0, 1))
+            _per_head(o_latent, self.w_uv, self.w_uv.transpose(1, 2), y.view(T, H, dv))
         if self.gated:
             self._gate(y, z, at)
         if out is None:
@@ -409,7 +418,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         if ctx.dtype == torch.float32:
             ops.gemm_heads(q_heads, self.w_ukt, q.view(T, H, R))
         else:
-            torch.bmm(q_heads.transpose(0, 1), self.w_uk, out=q.view(T, H, R).transpose(0, 1))
+            _per_head(q_heads, self.w_ukt, self.w_uk, q.view(T, H, R))
         o = ws.get("lattn.o", (T, H * R), ctx.dtype)
         self.attend(ctx, q, o, _both_planes(cache.pages), table)
         # back out of the latent's space: Wuv per head, then the gate
@@ -417,8 +426,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         if ctx.dtype == torch.float32:
             ops.gemm_heads(o.view(T, H, R), self.w_uv, y.view(T, H, dv))
         else:
-            torch.bmm(o.view(T, H, R).transpose(0, 1), self.w_uv.transpose(1, 2),
-                      out=y.view(T, H, dv).transpose(0, 1))
+            _per_head(o.view(T, H, R), self.w_uv, self.w_uv.transpose(1, 2), y.view(T, H, dv))
         if self.gated:
             ops.gate_heads(y, z[:, H * dq + R:], H, dv)
         if out is None:

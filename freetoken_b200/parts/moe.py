@@ -130,6 +130,10 @@ class RoutedExperts(FeedForward):
     def children(self):
         return [self.shared] if self.shared is not None else []
 
+    @property
+    def has_filler(self) -> bool:
+        return self.shared is not None
+
     def scratch_names(self):
         if self.shared is None:
             return ("moe",)
@@ -211,7 +215,7 @@ class RoutedExperts(FeedForward):
             return self.routed(ctx, x)
         shared = ctx.workspace.get("moe.shared", (x.shape[0], self.hidden), ctx.dtype)
         rows, extra = ctx.beside(lambda: self.routed(ctx, x), lambda: self.shared.forward(ctx, x, out=shared),
-                                 ("moe",), self.shared.scratch_names())
+                                 ("moe",), self.shared.scratch_names(), filler=True)
         if isinstance(rows, ops.RoutedRows):
             rows.extra = extra
             return rows
