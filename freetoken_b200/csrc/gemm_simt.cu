@@ -230,16 +230,21 @@ constexpr size_t stream_smem() {
   return (size_t)STREAM_STAGES * ((GLU ? 2 : 1) * STREAM_COLS * (STREAM_K * sizeof(WT) + 16) + MR * STREAM_K * sizeof(AT));
 }
 
+// The first MR of a block's eight warps multiply, all of them fetch: one or two warps alone spent longer on a stage's 16 to 32
+// copies a lane than on its chain (K = 2,048: a row of 2,048 columns 26.6 -> 18.4 us, two 20.5 -> 16.4; two of 32,768 columns,
+// bound by memory, 72 -> 70).  Twelve stages instead of four were slower (two rows 20.5 -> 26.6).
+constexpr int STREAM_THREADS = 256;
+
 template <typename AT, typename WT, typename OT, int MR, bool GLU>
-__global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(GemmArgs a) {
-  constexpr int WARPS = MR < 8 ? MR : 8, R = MR / WARPS, THREADS = 32 * WARPS;
+__global__ void __launch_bounds__(STREAM_THREADS) gemm_stream_kernel(GemmArgs a) {
+  constexpr int WARPS = MR < 8 ? MR : 8, R = MR / WARPS, THREADS = STREAM_THREADS;
   constexpr int HALVES = GLU ? 2 : 1, WROWS = HALVES * STREAM_COLS;
   constexpr int WROW = STREAM_K * sizeof(WT) + 16, AROW = STREAM_K * sizeof(AT);
   constexpr int WPIECES = STREAM_K * sizeof(WT) / 16, APIECES = AROW / 16;       // 16-byte pieces of a row
   constexpr int STAGE = WROWS * WROW + MR * AROW;
   extern __shared__ __align__(16) unsigned char stream_sm[];
   __shared__ int tile_info[3];
-  pdl_wait_only();
+  if (a.group_offsets) pdl_wait_only();
   find_tile<MR>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
@@ -252,14 +257,17 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
   // Rows beyond the last repeat it; columns beyond the last repeat the first ones, spread out (hundreds of blocks that
   // all fetched one row of eight 25 times stood in each other's way: 4,096 rows of 8 columns, K = 512, 34 us); k stops at K.
   const int here = min(a.N - n0, STREAM_COLS), spread = (1 << (31 - __clz(here))) - 1;
-  auto fetch = [&](int stage, int k0) {
+  auto fetch_weights = [&](int stage, int k0) {
     unsigned char* to = stream_sm + stage * STAGE;
+#pragma unroll
     for (int i = threadIdx.x; i < WROWS * WPIECES; i += THREADS) {
       const int n = i / WPIECES, piece = i % WPIECES, k = k0 + piece * (16 / (int)sizeof(WT)), c = n % STREAM_COLS;
       const int col = n0 + (c < here ? c : c & spread) + (n / STREAM_COLS) * a.N;
       if (k < a.K) cp_async16(to + n * WROW + piece * 16, W + (size_t)col * a.K + k);
     }
-    to += WROWS * WROW;
+  };
+  auto fetch_rows = [&](int stage, int k0) {
+    unsigned char* to = stream_sm + stage * STAGE + WROWS * WROW;
     for (int i = threadIdx.x; i < MR * APIECES; i += THREADS) {
       const int r = i / APIECES, piece = i % APIECES, k = k0 + piece * (16 / (int)sizeof(AT));
       const int at = row0 + min(r, rows - 1);
@@ -273,9 +281,14 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
   for (int h = 0; h < HALVES; ++h)
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[h][r] = 0.f;
+  // Nobody writes weights: a dense product's first stages of them are fetched ahead of the wait.
+#pragma unroll
+  for (int s = 0; s < STREAM_STAGES - 1; ++s)
+    if (s * STREAM_K < a.K) fetch_weights(s, s * STREAM_K);
+  if (!a.group_offsets) pdl_wait_only();
 #pragma unroll
   for (int s = 0; s < STREAM_STAGES - 1; ++s) {
-    if (s * STREAM_K < a.K) fetch(s, s * STREAM_K);
+    if (s * STREAM_K < a.K) fetch_rows(s, s * STREAM_K);
     cp_async_commit();
   }
   int stage = 0;
@@ -283,30 +296,45 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
     cp_async_wait<STREAM_STAGES - 2>();
     __syncthreads();                           // this stage has landed for all; the one before it is free
     const int ahead = k0 + (STREAM_STAGES - 1) * STREAM_K;
-    if (ahead < a.K) fetch((stage + STREAM_STAGES - 1) % STREAM_STAGES, ahead);
+    if (ahead < a.K) {
+      fetch_weights((stage + STREAM_STAGES - 1) % STREAM_STAGES, ahead);
+      fetch_rows((stage + STREAM_STAGES - 1) % STREAM_STAGES, ahead);
+    }
     cp_async_commit();
     const unsigned char* from = stream_sm + stage * STAGE;
     const WT* ws = reinterpret_cast<const WT*>(from + lane * WROW);
     const WT* us = reinterpret_cast<const WT*>(from + (STREAM_COLS + lane) * WROW);
     const AT* as = reinterpret_cast<const AT*>(from + WROWS * WROW) + warp * R * STREAM_K;
-    auto eight = [&](int kk) {
-      float w[HALVES][8], x[8];
-      load8(ws + kk, w[0]);
-      if constexpr (GLU) load8(us + kk, w[HALVES - 1]);
+    struct Eight { float w[HALVES][8], x[R][8]; };
+    auto load = [&](int kk, Eight& e) {
+      load8(ws + kk, e.w[0]);
+      if constexpr (GLU) load8(us + kk, e.w[HALVES - 1]);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        load8(as + r * STREAM_K + kk, x);
+      for (int r = 0; r < R; ++r) load8(as + r * STREAM_K + kk, e.x[r]);
+    };
+    auto add = [&](const Eight& e) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h) acc[h][r] = fmaf(x[i], w[h][i], acc[h][r]);
-      }
+          for (int h = 0; h < HALVES; ++h) acc[h][r] = fmaf(e.x[r][i], e.w[h][i], acc[h][r]);
     };
-    if (k0 + STREAM_K <= a.K) {
+    if (warp < WARPS) {
+      Eight e[2];
+      load(0, e[0]);
+      if (k0 + STREAM_K <= a.K) {
 #pragma unroll
-      for (int kk = 0; kk < STREAM_K; kk += 8) eight(kk);
-    } else {
-      for (int kk = 0; kk < a.K - k0; kk += 8) eight(kk);
+        for (int kk = 0; kk < STREAM_K; kk += 8) {      // the next eight are read before these are added
+          if (kk + 8 < STREAM_K) load(kk + 8, e[(kk / 8 + 1) & 1]);
+          add(e[kk / 8 & 1]);
+        }
+      } else {
+        for (int kk = 0; kk < a.K - k0; kk += 8) {
+          load(kk, e[0]);
+          add(e[0]);
+        }
+      }
     }
     stage = (stage + 1) % STREAM_STAGES;
   }
@@ -316,7 +344,7 @@ __global__ void __launch_bounds__(32 * (MR < 8 ? MR : 8)) gemm_stream_kernel(Gem
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int at = warp * R + r;
-    if (at < rows && n < a.N)
+    if (warp < WARPS && at < rows && n < a.N)
       store_out<OT, GLU>(a, C, a.c_rows ? a.c_rows[row0 + at] : row0 + at, n, acc[0][r], acc[HALVES - 1][r]);
   }
 }
@@ -506,7 +534,7 @@ int launch_stream(const GemmArgs& a, cudaStream_t stream) {
   }
   const int tiles = a.group_offsets ? a.M / MR + min(a.G, a.M) : (a.M + MR - 1) / MR;
   const dim3 grid(tiles, (a.N + STREAM_COLS - 1) / STREAM_COLS, a.batch);
-  const dim3 block(32 * (MR < 8 ? MR : 8));
+  const dim3 block(STREAM_THREADS);
   const cudaError_t e = a.group_offsets ? launch_behind(kernel, grid, block, smem, stream, a)
                                         : launch_pdl(kernel, grid, block, smem, stream, a);
   return e == cudaSuccess ? FT_OK : (int)e;

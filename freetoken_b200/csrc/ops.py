@@ -891,7 +891,7 @@ def gated_norm(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: t
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
     """One product per head on CUDA cores in float32: ``c[:, h, :] = a[:, h, :] @ w[h]^T``
     with ``a`` ``[T, heads, K]``, ``w`` ``[heads, N, K]`` (dense), ``c`` ``[T, heads, N]``;
-    ``a`` and ``c`` may be views with any row stride."""
+    ``a`` and ``c`` may be views with any row stride.  ``w`` as for :func:`gemm_rows`."""
     _need(a, "a", contiguous=False)
     _need(w, "w")
     _need(c, "c", contiguous=False)
@@ -913,7 +913,8 @@ def gemm_rows(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
 
     ``w`` is ``[N_w, K]`` or ``[G, N_w, K]``; with ``glu`` the N outputs are
     ``act(w[:N] a) * (w[N:] a)``.  ``rows`` is the number of (sorted) rows when
-    ``a_rows`` / ``c_rows`` redirect them."""
+    ``a_rows`` / ``c_rows`` redirect them.  Few dense rows fetch their first weights while the launch in
+    front still runs: ``w`` is never what that launch writes."""
     _need(a, "a", contiguous=False)
     _need(w, "w")
     _need(c, "c", contiguous=False)
