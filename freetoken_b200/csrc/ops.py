@@ -1300,13 +1300,14 @@ _CLUSTER_ROOM: Dict[tuple, Dict[int, int]] = {}
 
 
 def cluster_room(device, head_dim: int) -> Dict[int, int]:
-    """Size of a cluster of the decode kernel -> how many find a place on the device at once."""
+    """Size of a cluster of the decode kernel -> how many find a place on the device at once (0: a cluster of that size is
+    refused; a size that is missing: not known)."""
     key = (torch.device(device).index or 0, head_dim)
     room = _CLUSTER_ROOM.get(key)
     if room is None:
         ask = build.load("attention_decode_tma").ft_attn_decode_clusters
         answers = {size: ask(head_dim, size) for size in range(2, CLUSTER_SPLITS + 1)}
-        room = _CLUSTER_ROOM[key] = {size: n for size, n in answers.items() if n > 0}
+        room = _CLUSTER_ROOM[key] = {size: n for size, n in answers.items() if n >= 0}
     return room
 
 
@@ -1335,6 +1336,8 @@ def decode_splits(n_rows: int, num_kv_heads: int, group: int, max_kv_len: int, s
             continue                      # the same split as a smaller request
         rounds = -(-base * splits // slots)
         if cluster_merge and room and 1 < splits <= CLUSTER_SPLITS and splits in room:
+            if room[splits] == 0:
+                continue
             # a sixteenth less: the launch in front may still hold some SMs, and then a full house is two rounds
             rounds = max(rounds, -(-base // max(1, room[splits] * 15 // 16)))
         cost = rounds * (per + 3)

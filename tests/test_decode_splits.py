@@ -20,6 +20,26 @@ def test_splits_cover_the_keys_and_fit(rows, heads, group, keys):
         assert base <= room[splits] * 15 // 16 or base > 148
 
 
+@pytest.mark.parametrize("rows,heads,group,keys", [(8, 4, 4, 1024), (1, 8, 12, 2048), (2, 1, 16, 8192), (1, 4, 4, 100)])
+def test_a_cluster_that_finds_no_place_is_not_chosen(rows, heads, group, keys):
+    def chosen(room):
+        return ops.decode_splits(rows, heads, group, keys, 148, cluster_merge=True, room=room)[0]
+    sizes = range(2, ops.CLUSTER_SPLITS + 1)
+    free = ops.decode_splits(rows, heads, group, keys, 148, cluster_merge=True)[0]
+    assert chosen({}) == chosen({size: 148 for size in sizes}) == free                # not known, and room for all
+    for none in sizes:
+        assert chosen({size: 148 * (size != none) for size in sizes}) != none
+    assert chosen(dict.fromkeys(sizes, 0)) not in sizes
+
+
+def test_sizes_that_are_refused_are_kept_apart_from_those_not_known(monkeypatch):
+    answers = {2: 74, 3: 49, 4: 36, 5: 0, 6: -1, 7: 0, 8: -1}
+    monkeypatch.setattr(ops, "_CLUSTER_ROOM", {})
+    monkeypatch.setattr(ops.build, "load", lambda name: type("Library", (), {
+        "ft_attn_decode_clusters": staticmethod(lambda d, size: answers[size])}))
+    assert ops.cluster_room("cuda:0", 128) == {2: 74, 3: 49, 4: 36, 5: 0, 7: 0}
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("window,chunk", [(None, 0), (100, 0), (128, 0), (63, 0), (None, 96), (200, 64), (1, 0)])
 @pytest.mark.parametrize("D,page", [(128, 64), (64, 128), (32, 16)])
