@@ -182,7 +182,9 @@ def host_path(folder: Optional[str] = None) -> str:
     h = hashlib.sha256()
     with open(os.path.join(HERE, HOST_SOURCE), "rb") as f:
         h.update(f.read())
-    h.update(" ".join(HOST_FLAGS + [sys.implementation.cache_tag]).encode())
+    # the object layout it is compiled against: a debug or free-threaded build of the same version has another, and so
+    # has another platform (the cache tag names neither)
+    h.update(" ".join(HOST_FLAGS + [str(sysconfig.get_config_var("SOABI"))]).encode())
     return os.path.join(folder or build_dir(), f"libft_host_{h.hexdigest()[:16]}.so")
 
 

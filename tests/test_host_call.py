@@ -108,3 +108,14 @@ def test_tensors_are_checked(host):
         host.need(t, "x", dtype=torch.float32)
     with pytest.raises(TypeError):
         host.need(t, "x", shape=1)
+
+
+def test_each_build_of_the_interpreter_has_its_own_module(monkeypatch):
+    """A debug or free-threaded interpreter of the same version, or one of another platform, lays objects out otherwise."""
+    real = build.sysconfig.get_config_var
+    paths = set()
+    for abi in ("cpython-312-x86_64-linux-gnu", "cpython-312d-x86_64-linux-gnu", "cpython-312t-x86_64-linux-gnu",
+                "cpython-312-aarch64-linux-gnu"):
+        monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name, abi=abi: abi if name == "SOABI" else real(name))
+        paths.add(build.host_path("/somewhere"))
+    assert len(paths) == 4
