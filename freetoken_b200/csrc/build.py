@@ -71,6 +71,9 @@ class BuildError(RuntimeError):
 
 
 def register_library(name: str, source: str, link: Optional[List[str]] = None) -> None:
+    """A library of one's own: ``source`` is a path (relative ones from this folder), compiled as the package's are.  Its
+    launchers are ``extern "C" int name(..., cudaStream_t)``; with ``FT_PACKED(name)`` of ``common.cuh`` behind one, it is
+    called through the compiled host module, without it through ctypes."""
     LIBRARIES[name] = source
     if link:
         EXTRA_LINK[name] = link

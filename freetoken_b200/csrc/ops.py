@@ -72,9 +72,34 @@ def _fn(lib: str, name: str, sig: str):
     key = (lib, name)
     f = _bound.get(key)
     if f is None:
-        address = ctypes.cast(getattr(build.load(lib), name + "_packed"), ctypes.c_void_p).value
-        f = _bound[key] = _host_module().Launcher(address, sig, name, _KERNELS_PER_CALL.get(name, 1))
+        library = build.load(lib)
+        kernels = _KERNELS_PER_CALL.get(name, 1)
+        packed = getattr(library, name + "_packed", None)
+        if packed is None:
+            f = _plain_launcher(getattr(library, name), name, sig, kernels)
+        else:
+            f = _host_module().Launcher(ctypes.cast(packed, ctypes.c_void_p).value, sig, name, kernels)
+        _bound[key] = f
     return f
+
+
+_C = {"p": ctypes.c_void_p, "i": ctypes.c_int, "q": ctypes.c_longlong, "f": ctypes.c_float}
+
+
+def _plain_launcher(function, name: str, sig: str, kernels: int):
+    """A launcher of a registered library that has no packed form (common.cuh, FT_PACKED): the same call through ctypes."""
+    function.argtypes = [_C[c] for c in sig.split()] + [ctypes.c_void_p]
+    function.restype = ctypes.c_int
+    label = name[3:] if name.startswith("ft_") else name
+
+    def call(*args):
+        global LAUNCHES
+        words = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+        rc = function(*words, torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+        LAUNCHES += kernels
+        if rc != 0:
+            raise KernelError(f"{label}: {_ERRORS.get(rc, f'CUDA error {rc}')}")
+    return call
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:

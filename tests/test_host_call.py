@@ -119,3 +119,33 @@ def test_each_build_of_the_interpreter_has_its_own_module(monkeypatch):
         monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name, abi=abi: abi if name == "SOABI" else real(name))
         paths.add(build.host_path("/somewhere"))
     assert len(paths) == 4
+
+
+def test_a_registered_library_without_packed_forms_is_called_too(monkeypatch, tmp_path):
+    """A launcher as a library of one's own has it: arguments, then the stream, a code back."""
+    import shutil
+    import subprocess
+    source = tmp_path / "own.c"
+    source.write_text("""long long seen[6];
+        int ft_own(const void* a, int n, long long m, float f, const void* buffer, void* stream) {
+          seen[0] = (long long)a; seen[1] = n; seen[2] = m; seen[3] = (long long)(f * 8);
+          seen[4] = (long long)buffer; seen[5] = (long long)stream;
+          return n < 0 ? -102 : n > 100 ? 9 : 0; }""")
+    subprocess.run([shutil.which("gcc") or "cc", "-shared", "-fPIC", "-o", str(tmp_path / "own.so"), str(source)], check=True)
+    library = ctypes.CDLL(str(tmp_path / "own.so"))
+    monkeypatch.setattr(build, "load", lambda name: library)
+    monkeypatch.setattr(ops, "_bound", {})
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 1000 + device, raising=False)
+    f = ops._fn("own", "ft_own", "p i q f p")
+    t, buffer, before = torch.zeros(4), ctypes.create_string_buffer(16), ops.launch_count()
+    f(t, 5, 1 << 40, 0.5, buffer)
+    assert list((ctypes.c_longlong * 6).in_dll(library, "seen")) == [t.data_ptr(), 5, 1 << 40, 4, ctypes.addressof(buffer), 1003]
+    f(None, 5, 1, 0.5, 12345)
+    assert ops.launch_count() - before == 2
+    with pytest.raises(ops.KernelError, match="own: unsupported shape"):
+        f(t, -1, 0, 0.0, None)
+    with pytest.raises(ops.KernelError, match="own: CUDA error 9"):
+        f(t, 101, 0, 0.0, None)
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        f(t)
