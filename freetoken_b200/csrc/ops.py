@@ -1033,6 +1033,11 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
       int(lists_ahead), 0, 0)
 
 
+def skinny_heads_rows(K: int, head_stride: int) -> bool:
+    """Whether :func:`skinny_heads` takes heads of ``K`` values that lie ``head_stride`` apart, placed on 16 bytes."""
+    return K % 8 == 0 and head_stride % 8 == 0
+
+
 def skinny_heads_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """Whether :func:`skinny_heads` takes these operands."""
     return (x.dtype == w.dtype == out.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[2] % 8 == 0

@@ -108,6 +108,7 @@ class Engine:
         self.tensors = tensors
         self.model.bind(tensors, self.dtype)
         self.weight_bytes = sum(t.numel() * t.element_size() for t in tensors.values())
+        self.bound_bytes = self.model.bound_bytes(tensors)       # what the parts laid out anew for their kernels
 
         needs = self.model.cache_needs()
         P = args.page_size
@@ -117,7 +118,7 @@ class Engine:
             num_pages = -(-args.max_tokens // P)
         if num_pages is None:
             per_token = max(1, kv_bytes_per_token(needs, self.dtype))
-            budget = int(args.memory_ratio * free_before) - self.weight_bytes - (4 << 30)
+            budget = int(args.memory_ratio * free_before) - self.weight_bytes - self.bound_bytes - (4 << 30)
             num_pages = max(1, budget // (per_token * P))
             cap_len = args.max_seq_len or max_pos
             num_pages = min(num_pages, args.max_running_requests * (-(-cap_len // P)))
@@ -455,6 +456,7 @@ class Engine:
             "steps": self.steps,
             "tokens": self.tokens_run,
             "weight_bytes": self.weight_bytes,
+            "bound_bytes": self.bound_bytes,
             "cache_bytes": self.storage.bytes(),
             "workspace_bytes": self.workspace.bytes(),
             "pages_total": self.cache.total_pages(),

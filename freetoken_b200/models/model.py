@@ -89,6 +89,29 @@ class Model:
         for part in self.parts():
             part.bind(tensors, dtype)
 
+    def bound_bytes(self, tensors: Dict[str, torch.Tensor]) -> int:
+        """Bytes of what the parts made for themselves when they were bound - layouts a kernel wants, filled-up heads,
+        split-up routers - beside ``tensors``."""
+        known = {t.untyped_storage().data_ptr() for t in tensors.values()}
+        total = 0
+
+        def count(value) -> None:
+            nonlocal total
+            if isinstance(value, torch.Tensor):
+                storage = value.untyped_storage()
+                if storage.data_ptr() not in known:
+                    known.add(storage.data_ptr())
+                    total += storage.nbytes()
+            elif isinstance(value, dict):
+                for v in value.values():
+                    count(v)
+            elif isinstance(value, (list, tuple)):
+                for v in value:
+                    count(v)
+        for part in self.leaf_parts():
+            count(vars(part))
+        return total
+
     def libraries(self, dtype: torch.dtype) -> List[str]:
         names: List[str] = []
         for part in self.parts():

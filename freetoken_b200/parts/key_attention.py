@@ -142,11 +142,12 @@ class SharedKVAttention(PagedSoftmaxCore, Mixer):
         return linear.linear(o, self.w_o, out)
 
 
-def _per_head(x: torch.Tensor, rows: torch.Tensor, columns: torch.Tensor, out: torch.Tensor) -> None:
-    """``out[t, h] = W[h] x[t, h]`` in bfloat16; ``rows`` is W as ``[H, N, K]``, ``columns`` the same as ``[H, K, N]``.  Few
+def _per_head(x: torch.Tensor, rows: Optional[torch.Tensor], columns: torch.Tensor, out: torch.Tensor) -> None:
+    """``out[t, h] = W[h] x[t, h]`` in bfloat16; ``rows`` is W as ``[H, N, K]`` (None: the streaming kernel does not take
+    such rows), ``columns`` the same as ``[H, K, N]``.  Few
     tokens take the weight-streaming kernel, whose first weights are on their way before the launch in front has ended and
     which lets the next one in (the batched library product does neither); many the library product."""
-    if x.shape[0] <= linear.SKINNY_ROWS and ops.skinny_heads_takes(x, rows, out):
+    if rows is not None and x.shape[0] <= linear.SKINNY_ROWS and ops.skinny_heads_takes(x, rows, out):
         ops.skinny_heads(x, rows, out)
     else:
         torch.bmm(x.transpose(0, 1), columns, out=out.transpose(0, 1))
@@ -299,7 +300,8 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         self.w_uv = self.w_up[H * self.dq:].view(H, self.dv, R)      # [head][dv, R]
         self.own_kernels, self.expands = self._takes_own_kernels(dtype), self._expands(dtype)
         # the CUDA-core product and the weight-streaming one want [N, K] rows: Wuk^T per head
-        self.w_ukt = self.w_uk.transpose(1, 2).contiguous()
+        streams = dtype == torch.bfloat16 and ops.skinny_heads_rows(self.dq, self.dq + self.rot)
+        self.w_ukt = self.w_uk.transpose(1, 2).contiguous() if streams or dtype == torch.float32 else None
         self.w_o = tensors[self.n["o"]]
         if self.q_rank:
             self.w_qnorm = tensors[self.n["q_norm"]]
