@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <utility>
 
 #define FT_DTYPE_F32 0
@@ -133,6 +134,35 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// What a device is asked once and then known for, by its ordinal; 0: not asked yet.  (Several threads may ask at once: they
+// get the same answer.)
+struct PerDevice {
+  static constexpr int MOST = 64;
+  std::atomic<int> known[MOST] = {};
+  template <typename Ask>
+  int get(Ask ask) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+      cudaGetLastError();
+      return ask(-1);
+    }
+    if (dev < 0 || dev >= MOST) return ask(dev);
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) known[dev].store(n = ask(dev), std::memory_order_relaxed);
+    return n;
+  }
+};
+// Multiprocessors of the current device (148 where there is none).
+inline int device_sms() {
+  static PerDevice sms;
+  return sms.get([](int dev) {
+    int n = 0;
+    if (dev >= 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) return n;
+    cudaGetLastError();
+    return 148;
+  });
 }
 
 // The packed form of an extern "C" launcher: the arguments in an array of 8-byte words, taken apart by the types of the

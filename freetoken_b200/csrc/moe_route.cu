@@ -600,7 +600,7 @@ int ft_route_small(const float* logits, const float* bias, int* ids, float* weig
     return FT_ERR_SHAPE;
   if (groups < 1 || groups > 256 || E % groups || keep < 1 || keep > groups || keep * (E / groups) < k)
     return FT_ERR_SHAPE;
-  const size_t smem = (size_t)T * 2 * E * sizeof(float) + ((size_t)T * k + (size_t)(T * k > 2 * E ? T * k : 2 * E)) * sizeof(int);
+  const size_t smem = (size_t)T * 2 * E * sizeof(float) + 2 * (size_t)T * k * sizeof(int);
   if (smem > 160 * 1024) return FT_ERR_SHAPE;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -1712,7 +1712,7 @@ ROUTE_SMALL_MAX_T = 8
 
 def route_small_takes(T: int, E: int, k: int) -> bool:
     """A handful of tokens: selection and route sort fit one block."""
-    return T <= ROUTE_SMALL_MAX_T and k <= 32 and (T * 2 * E + T * k + 2 * E) * 4 <= 160 * 1024
+    return T <= ROUTE_SMALL_MAX_T and k <= 32 and (T * 2 * E + 2 * T * k) * 4 <= 160 * 1024
 
 
 def route_small(logits: torch.Tensor, bias: Optional[torch.Tensor], ids: torch.Tensor,

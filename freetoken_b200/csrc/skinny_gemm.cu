@@ -255,27 +255,33 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
 // chunks (28 / ks, three at ks = 8) they lost (12,288 x 4,096 1.15, five experts of 2,048 x 2,304 1.20); beyond that they
 // won again (20,480 x 3,072 0.86).  Of experts the launch knows only the most that can be busy: there from rows on that
 // are long enough for the rounds to win by themselves (sixteen of 2,048 x 2,304 1.11, of 4,096 x 4,736 0.95).
-static bool eight_chunks(long long blocks, int ks, int K, bool experts) {
+static bool eight_chunks(long long blocks, int ks, int K, bool experts, int sms) {
   const int per = ((K + 31) / 32 + ks - 1) / ks;
   if (per <= 4) return false;
-  if (blocks <= 148 * (16 / ks)) return true;
-  return experts ? per >= 21 && blocks > 1300 : blocks > 148 * (ks == 8 ? 3 : 28 / ks);
+  if (blocks <= sms * (16 / ks)) return true;
+  return experts ? per >= 21 && blocks > 1300 : blocks > sms * (ks == 8 ? 3 : 28 / ks);
+}
+// Blocks of a kernel that an SM of the current device holds.
+template <int NT, bool GLU, typename OT, int KS, int U>
+int blocks_an_sm() {
+  static PerDevice blocks;
+  return blocks.get([](int) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, skinny_kernel<NT, GLU, OT, KS, U>, KS * 32, 0) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+  });
 }
 template <int NT, bool GLU, typename OT, int KS, int U>
 void launch_one(SkinnyArgs a, dim3 grid, cudaStream_t stream) {
-  static const int resident = [] {
-    int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, skinny_kernel<NT, GLU, OT, KS, U>, KS * 32, 0) == cudaSuccess
-               ? 148 * n : 0;
-  }();
-  a.first_round = resident;
+  a.first_round = device_sms() * blocks_an_sm<NT, GLU, OT, KS, U>();
   launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
 }
 template <int NT, bool GLU, typename OT, int KS>
 void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream) {
   constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);
   if constexpr (NT == 1 && !GLU && KS >= 4) {
-    if (eight_chunks((long long)grid.x * grid.y, KS, a.K, a.group_offsets != nullptr)) {
+    if (eight_chunks((long long)grid.x * grid.y, KS, a.K, a.group_offsets != nullptr, device_sms())) {
       launch_one<NT, GLU, OT, KS, 8>(a, grid, stream);
       return;
     }
@@ -314,7 +320,10 @@ static int dense_k_split(int N, int K) {
 using namespace ft;
 
 extern "C" int ft_skinny_eight_chunks(long long blocks, int ks, int K, int experts) {
-  return eight_chunks(blocks, ks, K, experts != 0);
+  return eight_chunks(blocks, ks, K, experts != 0, 148);
+}
+extern "C" int ft_skinny_eight_chunks_on(int sms, long long blocks, int ks, int K, int experts) {
+  return eight_chunks(blocks, ks, K, experts != 0, sms);
 }
 
 // A, W bfloat16; C bfloat16 or float32.  `rows_per_pass` in {8,16,32} picks

@@ -83,3 +83,22 @@ def test_early_fetches_of_a_stream_norm(f32, S, H, k, early):
     (512, 4, 2304, 1, 1), (640, 4, 2304, 1, 0), (4096, 4, 2304, 1, 0), (4096, 4, 2688, 1, 1), (1024, 4, 4736, 1, 0)])
 def test_chunks_a_round_of_a_weight_streaming_product(blocks, ks, K, experts, eight):
     assert build.load("skinny_gemm").ft_skinny_eight_chunks(blocks, ks, K, experts) == eight
+
+
+@pytest.mark.parametrize("sms", [74, 132, 148, 160])
+def test_rounds_are_those_of_the_device_that_runs_them(sms):
+    """Both lines of the rule lie at a whole house of blocks, whatever number of multiprocessors that is."""
+    rule = build.load("skinny_gemm").ft_skinny_eight_chunks_on
+    for ks, eight, four in ((4, 4, 7), (8, 2, 3), (16, 1, 1)):
+        assert rule(sms, sms * eight, ks, 4096, 0) == 1
+        assert rule(sms, sms * eight + 1, ks, 4096, 0) == int(eight == four)
+        assert rule(sms, sms * four + 1, ks, 4096, 0) == 1
+    assert rule(sms, 2 * sms, 4, 512, 0) == 0
+
+
+def test_nothing_that_a_device_is_asked_is_kept_for_all_devices():
+    """The streaming product's launch rule holds no device's answer in a static of its own, and no number of multiprocessors."""
+    import os
+    with open(os.path.join(build.HERE, "skinny_gemm.cu")) as f:
+        code = "\n".join(line.split("//")[0] for line in f)
+    assert "static const int" not in code and code.count("148") == 1            # the exported rule of the tests above
