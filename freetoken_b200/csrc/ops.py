@@ -1033,6 +1033,19 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
       int(lists_ahead), 0, 0)
 
 
+_SKINNY_SMS: Dict[tuple, Optional[int]] = {}
+
+
+def skinny_sms(device, rows: int, N: int, K: int, heads: int = 1) -> Optional[int]:
+    """How many SMs of ``device`` hold all blocks at once of a plain product of ``rows`` rows by :func:`skinny_gemm` (or
+    :func:`skinny_heads`, ``heads`` matrices) with ``[N, K]`` weights; None: not known."""
+    key = (torch.device(device).index or 0, pass_rows(rows), N, K, heads)
+    if key not in _SKINNY_SMS:
+        sms = build.load("skinny_gemm").ft_skinny_sms(N, K, heads, key[1])
+        _SKINNY_SMS[key] = sms if sms < 1 << 30 else None
+    return _SKINNY_SMS[key]
+
+
 def skinny_heads_rows(K: int, head_stride: int) -> bool:
     """Whether :func:`skinny_heads` takes heads of ``K`` values that lie ``head_stride`` apart, placed on 16 bytes."""
     return K % 8 == 0 and head_stride % 8 == 0
@@ -1320,10 +1333,14 @@ CLUSTER_SPLITS = 8     # splits the TMA-fed decode kernel merges by itself (a th
 MERGE_COST = 24        # what the separate merge kernel costs, in 64-key tiles of a CTA's work
 
 
-# A decode attention of up to this many CTAs lets the next launch become resident beside it; of more, that launch would
-# work in the little L1 that the CTAs' stages leave an SM (one row of 4 KV heads x 1,024 keys with the projection of 2,048 x
-# 2,048 behind it: 7.7 us against 10.0; 8 rows of 8 KV heads with one of 3,072 x 6,144: 32 against 21).
-DECODE_LETS_IN = 74
+def decode_lets_in(ctas: int, sms_behind: Optional[int], sms: int) -> bool:
+    """Whether a decode attention of ``ctas`` CTAs lets the next launch become resident beside it.  That launch then has its
+    first weights on their way when the attention ends, but a block of it on an SM where a CTA's stages have taken the
+    shared memory works in the little L1 that is left, to its end: only if the SMs without a CTA hold the whole launch
+    (``sms_behind``; None: not known).  Us a decode step of four layers, closed and open: MiniMax-M3, O projection of
+    3,072 x 6,144 on 96 SMs, one request behind 48 CTAs 512 and 503, behind 56 518 and 562, behind 64 520 and 567; O of 2,048 x 2,048
+    on 64 SMs behind 64 CTAs 235 and 228, behind 96 271 and 283; O of 4,096 x 4,096 on 128 SMs behind 48 319 and 326."""
+    return sms_behind is not None and ctas + sms_behind <= sms
 
 
 _CLUSTER_ROOM: Dict[tuple, Dict[int, int]] = {}
@@ -1383,8 +1400,10 @@ def attn_decode(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
                 rows: Optional[torch.Tensor], n_rows: int, token_pos: torch.Tensor,
                 token_seg: torch.Tensor, block_table: torch.Tensor, num_heads: int,
                 num_kv_heads: int, head_dim: int, scale: float, window: Optional[int],
-                max_kv_len: int, workspace, options: Optional[ScoreOptions] = None) -> None:
-    """Split-KV tensor-core attention for single-token rows (bfloat16)."""
+                max_kv_len: int, workspace, options: Optional[ScoreOptions] = None,
+                sms_behind: Optional[int] = None) -> None:
+    """Split-KV tensor-core attention for single-token rows (bfloat16).  ``sms_behind``: how many SMs the next launch takes
+    (:func:`decode_lets_in`)."""
     extra = (options or NO_SCORE_OPTIONS).args(num_heads)
     _need(q, "q", torch.bfloat16)
     _need(out, "out", torch.bfloat16)
@@ -1427,7 +1446,8 @@ def attn_decode(q: torch.Tensor, out: torch.Tensor, kv_pages: torch.Tensor,
           num_heads, num_kv_heads, head_dim, kv_pages.shape[3], block_table.shape[1],
           int(window or 0), n_rows, splits, split_keys, float(scale),
           1 if kv_pages.stride(0) else 0, *extra,
-          int(n_rows * num_kv_heads * -(-(num_heads // num_kv_heads) // 16) * splits <= DECODE_LETS_IN))
+          int(decode_lets_in(n_rows * num_kv_heads * -(-(num_heads // num_kv_heads) // 16) * splits,
+                             sms_behind if part_o is None else n_rows * num_heads, sm_count(q.device))))
         if part_o is not None:
             fm = _fn("attention_decode", "ft_attn_merge", "p p p p i i i i")
             fm(part_o, part_ml, out, rows, n_rows, num_heads, head_dim,

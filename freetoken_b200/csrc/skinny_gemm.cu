@@ -22,6 +22,8 @@
 // program per route, CUDA-core FMAs: an expert's weights are read once per
 // token that chose it); dense rows go through cuBLAS there
 // (python/freetoken/layers/linear.py:31-32).
+#include <limits.h>
+
 #include "common.cuh"
 
 namespace ft {
@@ -272,28 +274,34 @@ int blocks_an_sm() {
     return 0;
   });
 }
+// `sms`, where it is given: nothing is launched, it gets how many SMs hold all blocks of the launch at once.
 template <int NT, bool GLU, typename OT, int KS, int U>
-void launch_one(SkinnyArgs a, dim3 grid, cudaStream_t stream) {
-  a.first_round = device_sms() * blocks_an_sm<NT, GLU, OT, KS, U>();
+void launch_one(SkinnyArgs a, dim3 grid, cudaStream_t stream, int* sms) {
+  const int an_sm = blocks_an_sm<NT, GLU, OT, KS, U>();
+  if (sms) {
+    *sms = an_sm > 0 ? (int)(((long long)grid.x * grid.y + an_sm - 1) / an_sm) : INT_MAX;
+    return;
+  }
+  a.first_round = device_sms() * an_sm;
   launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
 }
 template <int NT, bool GLU, typename OT, int KS>
-void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream) {
+void launch_u(const SkinnyArgs& a, dim3 grid, cudaStream_t stream, int* sms) {
   constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);
   if constexpr (NT == 1 && !GLU && KS >= 4) {
     if (eight_chunks((long long)grid.x * grid.y, KS, a.K, a.group_offsets != nullptr, device_sms())) {
-      launch_one<NT, GLU, OT, KS, 8>(a, grid, stream);
+      launch_one<NT, GLU, OT, KS, 8>(a, grid, stream, sms);
       return;
     }
   }
-  launch_one<NT, GLU, OT, KS, U>(a, grid, stream);
+  launch_one<NT, GLU, OT, KS, U>(a, grid, stream, sms);
 }
 template <bool GLU, typename OT, int KS>
-int launch_nt(const SkinnyArgs& a, int nt, dim3 grid, cudaStream_t stream) {
+int launch_nt(const SkinnyArgs& a, int nt, dim3 grid, cudaStream_t stream, int* sms = nullptr) {
   switch (nt) {
-    case 1: launch_u<1, GLU, OT, KS>(a, grid, stream); break;
-    case 2: launch_u<2, GLU, OT, KS>(a, grid, stream); break;
-    case 4: launch_u<4, GLU, OT, KS>(a, grid, stream); break;
+    case 1: launch_u<1, GLU, OT, KS>(a, grid, stream, sms); break;
+    case 2: launch_u<2, GLU, OT, KS>(a, grid, stream, sms); break;
+    case 4: launch_u<4, GLU, OT, KS>(a, grid, stream, sms); break;
     default: return FT_ERR_SHAPE;
   }
   return FT_OK;
@@ -324,6 +332,22 @@ extern "C" int ft_skinny_eight_chunks(long long blocks, int ks, int K, int exper
 }
 extern "C" int ft_skinny_eight_chunks_on(int sms, long long blocks, int ks, int K, int experts) {
   return eight_chunks(blocks, ks, K, experts != 0, sms);
+}
+
+// How many SMs hold all blocks at once of a plain dense product of `groups` matrices [N, K] (1, or one a head) with a
+// bfloat16 result; INT_MAX: not known.
+extern "C" int ft_skinny_sms(int N, int K, int groups, int rows_per_pass) {
+  int sms = INT_MAX;
+  if (N <= 0 || K <= 0 || groups <= 0) return sms;
+  SkinnyArgs a{};
+  a.K = K;
+  const dim3 grid((N + 15) / 16, groups);
+  const int nt = rows_per_pass / 8, ks = dense_k_split(N * groups, K);
+  if (ks == 2) launch_nt<false, __nv_bfloat16, 2>(a, nt, grid, nullptr, &sms);
+  else if (ks == 16) launch_nt<false, __nv_bfloat16, 16>(a, nt, grid, nullptr, &sms);
+  else if (ks == 8) launch_nt<false, __nv_bfloat16, 8>(a, nt, grid, nullptr, &sms);
+  else launch_nt<false, __nv_bfloat16, 4>(a, nt, grid, nullptr, &sms);
+  return sms;
 }
 
 // A, W bfloat16; C bfloat16 or float32.  `rows_per_pass` in {8,16,32} picks

@@ -23,7 +23,7 @@ softmax).
 
 from __future__ import annotations
 
-from typing import Dict, List
+from typing import Dict, List, Optional
 
 import numpy as np
 import torch
@@ -98,11 +98,11 @@ class PagedSoftmaxCore:
             fast += ["attention_prefill_tc", "attention_decode_tma"]
         return ["attention_simt"] + fast
 
-    def attend(self, ctx: StepContext, q, o, kv_pages, table) -> None:
+    def attend(self, ctx: StepContext, q, o, kv_pages, table, sms_behind: Optional[int] = None) -> None:
         """Single-token rows go to the split-KV tensor-core kernel, rows of
         longer segments to a prefill kernel; sizes those refuse (and the
         float32 path) go to the generic kernel.  ``kv_pages`` is ``[2 (K, V),
-        pages, kv_heads, page, head_dim]``."""
+        pages, kv_heads, page, head_dim]``; ``sms_behind``: how many SMs the launch behind takes."""
         if ops.attn_decode_takes(q, self.d):
             plan = ctx.plan(self)
             n_dec, n_tiles = plan.host["num_decode_rows"], plan.host["num_prefill_tiles"]
@@ -110,7 +110,7 @@ class PagedSoftmaxCore:
                 ops.attn_decode(q, o, kv_pages, plan.tensors.get("decode_rows"), n_dec,
                                 ctx.token_pos, ctx.token_seg, table, self.nq, self.nkv, self.d,
                                 self.scale, self.window, plan.host["max_decode_kv_len"], ctx.workspace,
-                                options=self.options)
+                                options=self.options, sms_behind=sms_behind if n_tiles == 0 else None)
             if n_tiles > 0:
                 tile_seg, tile_q0 = plan.tensors["tile_seg"], plan.tensors["tile_q0"]
                 if (plan.host["prefill_scores"] >= ops.PREFILL_TC_MIN_SCORES
@@ -380,7 +380,8 @@ class PagedAttention(PagedSoftmaxCore, Mixer):
             self.position.interleaved, self.norm_eps, norm_dim=self.dk, value_first=value_source,
             value_lambda=self.w_value_mix if value_source is not None else None)
         o = ws.get("attn.o", (T, qn), ctx.dtype)
-        self.attend(ctx, q, o, cache.kv_pages, table)
+        # behind it the gate's few blocks, 2,048 values each, or the output projection
+        self.attend(ctx, q, o, cache.kv_pages, table, -(-T * qn // 2048) if self.gate else linear.sms_taken(o, self.w_o))
         if self.gate == "head":
             ops.gate_heads(o, gate, self.nq, self.d)
         elif self.gate:

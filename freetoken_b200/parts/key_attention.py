@@ -136,7 +136,7 @@ class SharedKVAttention(PagedSoftmaxCore, Mixer):
                       table, q_off=0, k_off=qn, num_heads=self.nq, q_dim=self.d, num_kv_heads=self.nkv,
                       k_dim=self.d, temp_coef=self.temp_coef, temp_every=self.temp_every)
         o = ws.get("kattn.o", (T, qn), ctx.dtype)
-        self.attend(ctx, q, o, _both_planes(cache.pages), table)
+        self.attend(ctx, q, o, _both_planes(cache.pages), table, linear.sms_taken(o, self.w_o))
         if out is None:
             out = ws.get("kattn.y", (T, self.hidden), ctx.dtype)
         return linear.linear(o, self.w_o, out)
@@ -387,7 +387,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         else:
             _per_head(q_heads, self.w_ukt, self.w_uk, q_abs[:, :, :R])
         o = ws.get("lattn.o", (T, H * d), ctx.dtype)
-        self.attend(ctx, q_abs.view(T, H * d), o, _both_planes(cache.pages), table)
+        self.attend(ctx, q_abs.view(T, H * d), o, _both_planes(cache.pages), table, linear.sms_taken(o, self.w_uv))
         # the first rank values of a head's result are the weighted latents: Wuv per head, then the gate
         y = ws.get("lattn.v", (T, H * dv), ctx.dtype)
         o_latent = o.view(T, H, d)[:, :, :R]
@@ -422,7 +422,7 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
         else:
             _per_head(q_heads, self.w_ukt, self.w_uk, q.view(T, H, R))
         o = ws.get("lattn.o", (T, H * R), ctx.dtype)
-        self.attend(ctx, q, o, _both_planes(cache.pages), table)
+        self.attend(ctx, q, o, _both_planes(cache.pages), table, linear.sms_taken(o, self.w_uv))
         # back out of the latent's space: Wuv per head, then the gate
         y = ws.get("lattn.v", (T, H * dv), ctx.dtype)
         if ctx.dtype == torch.float32:

@@ -145,6 +145,14 @@ def library_f32_out(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) ->
 SKINNY_ROWS = 32
 
 
+def sms_taken(x: torch.Tensor, weight: torch.Tensor) -> Optional[int]:
+    """How many SMs :func:`linear` of rows like ``x`` (or the product per head, ``weight`` ``[heads, N, K]``) takes with all its
+    blocks at once; None where another product than the weight-streaming one runs."""
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.shape[0] > SKINNY_ROWS:
+        return None
+    return ops.skinny_sms(x.device, x.shape[0], weight.shape[-2], weight.shape[-1], weight.shape[0] if weight.dim() == 3 else 1)
+
+
 def libraries(compute: torch.dtype, bias: bool = False) -> list:
     libs = ["gemm_simt"] if compute == torch.float32 else ["gemm_simt", "skinny_gemm"]
     return libs + (["rowwise"] if bias else [])

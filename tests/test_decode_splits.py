@@ -40,6 +40,80 @@ def test_sizes_that_are_refused_are_kept_apart_from_those_not_known(monkeypatch)
     assert ops.cluster_room("cuda:0", 128) == {2: 74, 3: 49, 4: 36, 5: 0, 7: 0}
 
 
+@pytest.mark.parametrize("ctas,behind,lets_in", [(48, 96, True), (52, 96, True), (53, 96, False), (64, 96, False), (64, 64, True),
+                                                 (96, 64, False), (48, 128, False), (1, None, False), (147, 1, True), (148, 0, True)])
+def test_what_stands_behind_decides_whether_it_is_let_in(ctas, behind, lets_in):
+    assert ops.decode_lets_in(ctas, behind, 148) is lets_in
+
+
+def test_sms_of_a_product_are_asked_once_and_kept_apart(monkeypatch):
+    asked = []
+
+    def answer(N, K, heads, rows):
+        asked.append((N, K, heads, rows))
+        return 2 ** 31 - 1 if K == 8 else N * heads // 16
+    monkeypatch.setattr(ops, "_SKINNY_SMS", {})
+    monkeypatch.setattr(ops.build, "load", lambda name: type("Library", (), {"ft_skinny_sms": staticmethod(answer)}))
+    assert [ops.skinny_sms("cuda:0", rows, 64, 64) for rows in (1, 8, 9, 16, 32)] == [4] * 5
+    assert ops.skinny_sms("cuda:1", 3, 64, 64) == 4 and ops.skinny_sms("cuda:0", 3, 64, 64, heads=4) == 16
+    assert ops.skinny_sms("cuda:0", 3, 64, 8) is None and ops.skinny_sms("cuda:0", 4, 64, 8) is None
+    assert asked == [(64, 64, 1, 8), (64, 64, 1, 16), (64, 64, 1, 32), (64, 64, 1, 8), (64, 64, 4, 8), (64, 8, 1, 8)]
+
+
+def test_a_step_says_what_stands_behind_its_attention(monkeypatch):
+    """The output projection of few rows, the gate's blocks, nothing where prompts' tiles come in between or the library takes
+    the rows."""
+    from types import SimpleNamespace
+
+    from freetoken_b200.parts import attention, linear
+    seen = []
+    monkeypatch.setattr(ops, "attn_decode", lambda *a, sms_behind=None, **k: seen.append(sms_behind))
+    monkeypatch.setattr(ops, "attn_decode_takes", lambda q, d: True)
+    monkeypatch.setattr(ops, "attn_prefill", lambda *a, **k: None)
+    monkeypatch.setattr(ops, "PREFILL_TC_MIN_SCORES", 1 << 60)
+    monkeypatch.setattr(ops, "skinny_sms", lambda device, rows, N, K, heads=1: (rows, N, K, heads))
+    core = attention.PagedSoftmaxCore()
+    core.nq, core.nkv, core.d, core.scale = 8, 2, 64, 0.1
+    q = torch.zeros(3, 512, dtype=torch.bfloat16)
+    for tiles in (0, 2):
+        plan = SimpleNamespace(host={"num_decode_rows": 3, "num_prefill_tiles": tiles, "prefill_scores": 0,
+                                     "max_decode_kv_len": 64}, tensors={"tile_seg": None, "tile_q0": None})
+        ctx = SimpleNamespace(plan=lambda part: plan, token_pos=None, token_seg=None, seg_q_start=None, seg_pos0=None,
+                              workspace=None)
+        core.attend(ctx, q, q, None, None, 40)
+    assert seen == [40, None]
+    w = torch.zeros(128, 512, dtype=torch.bfloat16)
+    assert linear.sms_taken(q, w) == (3, 128, 512, 1)
+    assert linear.sms_taken(torch.zeros(33, 512, dtype=torch.bfloat16), w) is None
+    assert linear.sms_taken(q.float(), w) is None
+    assert linear.sms_taken(q, torch.zeros(8, 16, 64, dtype=torch.bfloat16)) == (3, 16, 64, 8)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,keys", [(1, 2048), (1, 300), (4, 130)])
+def test_the_launch_behind_gives_the_same_rows_let_in_or_not(rows, keys):
+    from test_kernels_gpu import DEV, rnd
+    from freetoken_b200.parts.base import Workspace
+    H, G, D, page = 32, 4, 128, 64
+    pages = -(-keys // page)
+    kv = rnd(2, rows * pages + 1, G, page, D, dtype=torch.bfloat16, seed=1)
+    table = torch.arange(1, rows * pages + 1, dtype=torch.int32, device=DEV).view(rows, pages)
+    q, w = rnd(rows, H * D, dtype=torch.bfloat16, seed=2), rnd(2048, H * D, dtype=torch.bfloat16, seed=3, scale=0.02)
+    pos = torch.full((rows,), keys - 1, dtype=torch.int32, device=DEV)
+    seg = torch.arange(rows, dtype=torch.int32, device=DEV)
+    ws = Workspace(DEV)
+    got = []
+    for behind in (None, 0):                 # closed, and open whatever comes
+        for _ in range(10):
+            o, y = torch.zeros_like(q), torch.zeros(rows, 2048, dtype=torch.bfloat16, device=DEV)
+            ops.attn_decode(q, o, kv, None, rows, pos, seg, table, H, G, D, D ** -0.5, None, keys, ws, sms_behind=behind)
+            ops.skinny_gemm(o, w, y)
+            got.append(y)
+    assert ops.decode_lets_in(1, 0, ops.sm_count(DEV))
+    for y in got[1:]:
+        assert torch.equal(y, got[0])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("window,chunk", [(None, 0), (100, 0), (128, 0), (63, 0), (None, 96), (200, 64), (1, 0)])
 @pytest.mark.parametrize("D,page", [(128, 64), (64, 128), (32, 16)])
