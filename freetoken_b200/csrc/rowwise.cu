@@ -626,10 +626,14 @@ __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
   }
 }
 
-// The same for few tokens of several partial rows: a block of 256 KEEP threads with a piece each, so that all loads of the
-// row are one round or two, not one behind another's branch; z and the new row change hands in shared memory, and the
-// first 256 threads add the squares in the order of the kernel above.  (One token of 4,096 values, three partial rows, an
-// input handed back and a shared row: 7.8 us with four pieces a thread.)
+// The same for few tokens of several partial rows (2,049 to 4,096 values up to 64 tokens, 1,025 to 2,048 up to 8): a block of
+// 256 KEEP threads with a piece each, so that all loads of the row are one round or two, not one behind another's branch; z and
+// the new row change hands in shared memory, and the first 256 threads add the squares in the order of the kernel above.
+// (One token of 4,096 values, three partial rows, an input handed back and a shared row: 7.8 us with four pieces a thread.)
+// Between two products, us a chain of three launches of 1, 8, 32 and 64 tokens, with several pieces a thread and in this form:
+// 4,096 values, eight partial rows 19.2 -> 17.3, 20.5 -> 18.6, 34.0 -> 31.5, 56.1 -> 53.5; 3,072 values, three 13.6 -> 11.9,
+// 14.9 -> 13.0, 25.3 -> 24.2, 40.7 -> 39.5; 2,048 values, five 8.9 -> 8.1, 9.5 -> 8.7, but level from 12 to 20 tokens and then
+// 18.4 -> 18.8, 27.7 -> 29.8: two pieces a thread are two rounds of loads, which that many blocks hide from each other.
 template <typename AT, int KEEP>
 __global__ void __launch_bounds__(256 * KEEP) norm_add_few_kernel(NormAddArgs a) {
   __shared__ float4 row[256 * KEEP];
@@ -1458,6 +1462,10 @@ static bool branch_aligned(const BranchArgs& b) {
 // each, do not (4,096 values, us: one partial row 4.6 -> 3.8, three 4.6 -> 5.1, eight 5.9 -> 7.4; float32, eight: 5.7 -> 4.6).
 static bool norm_add_fetches_early(bool f32, int H, int k) { return f32 || k <= (H <= 2048 ? 4 : 2); }
 
+// Whether rows of few tokens that do not go that way take a thread a piece; both sides of the lines stand at norm_add_few_kernel.
+static bool norm_add_one_piece(int T, int H) { return H > 1024 && (H <= 2048 ? T <= 8 : H <= 4096 && T <= 64); }
+
+int ft_norm_add_one_piece(int T, int H) { return norm_add_one_piece(T, H); }
 int ft_hyper_fetches_early(int f32, int S, int H, int k) { return hyper_fetches_early(f32 != 0, S, H, k); }
 int ft_norm_add_fetches_early(int f32, int H, int k) { return norm_add_fetches_early(f32 != 0, H, k); }
 
@@ -1481,8 +1489,8 @@ int ft_norm_add(const BranchArgs* branch, const float* weight, int plus_one, flo
     if (few && H <= 1024) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 1, true>, g, th, 0, stream, a))); }
     else if (few && H <= 2048) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 2, true>, g, th, 0, stream, a))); }
     else if (few && H <= 4096) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 4, true>, g, th, 0, stream, a))); }
-    else if (T <= 64 && H > 1024 && H <= 2048) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_few_kernel<AT, 2>, g, dim3(512), 0, stream, a))); }
-    else if (T <= 64 && H > 1024 && H <= 4096) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_few_kernel<AT, 4>, g, dim3(1024), 0, stream, a))); }
+    else if (norm_add_one_piece(T, H) && H <= 2048) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_few_kernel<AT, 2>, g, dim3(512), 0, stream, a))); }
+    else if (norm_add_one_piece(T, H)) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_few_kernel<AT, 4>, g, dim3(1024), 0, stream, a))); }
     else if (H <= 1024) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 1>, g, th, 0, stream, a))); }
     else if (H <= 2048) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 2>, g, th, 0, stream, a))); }
     else if (H <= 4096) { FT_DISPATCH(dtype, AT, (launch_pdl(norm_add_kernel<AT, 4>, g, th, 0, stream, a))); }

@@ -85,6 +85,12 @@ def test_chunks_a_round_of_a_weight_streaming_product(blocks, ks, K, experts, ei
     assert build.load("skinny_gemm").ft_skinny_eight_chunks(blocks, ks, K, experts) == eight
 
 
+@pytest.mark.parametrize("T,H,one", [(1, 1024, 0), (1, 1028, 1), (8, 2048, 1), (9, 2048, 0), (64, 2048, 0), (1, 2052, 1), (64, 2052, 1),
+                                     (64, 4096, 1), (65, 4096, 0), (1, 4100, 0)])
+def test_rows_of_one_piece_a_thread(T, H, one):
+    assert build.load("rowwise").ft_norm_add_one_piece(T, H) == one
+
+
 @pytest.mark.parametrize("sms", [74, 132, 148, 160])
 def test_rounds_are_those_of_the_device_that_runs_them(sms):
     """Both lines of the rule lie at a whole house of blocks, whatever number of multiprocessors that is."""
