@@ -1045,6 +1045,18 @@ int ft_gather_rows(const void* src, const int* rows, void* dst, int dtype, int n
 
 }  // extern "C"
 
+// A stream of the caller's own on the current device, which does not wait for the default one.
+extern "C" int ft_stream_create(int priority, void** out) {
+  cudaStream_t stream = nullptr;
+  const cudaError_t e = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, priority);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return (int)e;
+  }
+  *out = stream;
+  return FT_OK;
+}
+
 FT_PACKED(ft_zero_slots)
 FT_PACKED(ft_embed_gather)
 FT_PACKED(ft_patch_tokens)

@@ -102,6 +102,17 @@ def _plain_launcher(function, name: str, sig: str, kernels: int):
     return call
 
 
+def own_stream(device, priority: int = 0) -> "torch.cuda.Stream":
+    """A stream that nobody else is given.  ``torch.cuda.Stream()`` hands out a few dozen of a pool in turn, to every thread
+    of the process; this one lives as long as the process does."""
+    handle = ctypes.c_void_p()
+    with torch.cuda.device(device):
+        rc = build.load("elementwise").ft_stream_create(ctypes.c_int(priority), ctypes.byref(handle))
+        if rc != 0:
+            raise KernelError(f"own_stream: CUDA error {rc}")
+        return torch.cuda.ExternalStream(handle.value, device=device)
+
+
 def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
     """``t`` must be a CUDA tensor, of type ``dtype`` if that is given.  (Replaced by the host module's own with the first
     call.)"""

@@ -19,6 +19,7 @@ logits are returned so that sampling stays a separate, testable step.
 
 from __future__ import annotations
 
+import weakref
 from dataclasses import dataclass
 from typing import Any, Dict, Hashable, List, Mapping, Optional, Sequence, Tuple
 
@@ -34,6 +35,7 @@ from ..parts.base import CacheView, Segment, StepContext, StepShape, Workspace
 from ..registry import Architecture, architecture_of, read_model_config
 from ..weights.loader import check_state, load_tensors
 from ..weights.random_init import RandomOptions, random_state
+from . import streams
 
 DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32,
           "fp32": torch.float32, torch.bfloat16: torch.bfloat16, torch.float32: torch.float32}
@@ -150,9 +152,7 @@ class Engine:
         self._meta_generation = 0
         self._graphs: Dict[Tuple, "torch.cuda.CUDAGraph"] = {}
         self._graph_seen: Dict[Tuple, int] = {}
-        self._capture_stream: Optional["torch.cuda.Stream"] = None
-        self._side_streams: List["torch.cuda.Stream"] = []
-        self._minor_streams: List["torch.cuda.Stream"] = []
+        self._streams: Optional[streams.CaptureStreams] = None
         self.graph_replays = 0
         self.steps = 0
         self.tokens_run = 0
@@ -425,16 +425,13 @@ class Engine:
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()
             before = ops.launch_count()
-            if not self._side_streams:
-                # A filler's blocks wait for those of everything else.  Only models that have one pay for priorities: with the
-                # same one on every launch a step of two equal branches took 2 % longer than with none.
+            if self._streams is None:
                 fills = any(part.has_filler for part in self.model.leaf_parts())
-                self._capture_stream = torch.cuda.Stream(self.device, priority=-1) if fills else None
-                self._side_streams = [torch.cuda.Stream(self.device, priority=-1 if fills else 0) for _ in range(2)]
-                self._minor_streams = [torch.cuda.Stream(self.device) for _ in range(2)] if fills else []
+                self._streams = streams.take(self.device, fills)
+                weakref.finalize(self, streams.give_back, self.device, fills, self._streams)
             # branches of the step become branches of the graph
-            ctx.side, ctx.minor = list(self._side_streams), list(self._minor_streams)
-            with torch.cuda.graph(graph, stream=self._capture_stream):
+            ctx.side, ctx.minor = list(self._streams.side), list(self._streams.minor)
+            with torch.cuda.graph(graph, stream=self._streams.main):
                 self.model.forward(ctx, self.cache_views, logit_rows, logits, in_order)
             kernels = ops.launch_count() - before
             ops.LAUNCHES -= kernels          # recorded, not run
