@@ -243,13 +243,14 @@ class Part:
     # the result in a place of its own copies it otherwise.
     writes_into_out = False
     # The first words of the names of the workspace buffers a part writes (with those of its kernels' faces), or None:
-    # not stated, and then nothing runs beside the part (``StepContext.beside``).
+    # not stated, and then nothing runs beside the part (``StepContext.beside``).  A class states its own: one that
+    # inherits another's forward may write more.
     scratch: Optional[Tuple[str, ...]] = None
     # whether the part runs something as a filler (``StepContext.beside``)
     has_filler = False
 
     def scratch_names(self) -> Optional[Tuple[str, ...]]:
-        return self.scratch
+        return vars(type(self)).get("scratch")
 
     def __init__(self, spec: PartSpec, prefix: str):
         self.spec = spec

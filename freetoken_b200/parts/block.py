@@ -101,7 +101,8 @@ class ParallelBlock(Block):
                 self.feed_forward.forward(ctx, h, out=pair[:, 1])
             else:
                 pair[:, 1].copy_(plain_branch(ctx, self.feed_forward.forward(ctx, h)))
-        ctx.beside(mix, feed, self.mixer.scratch_names(), self.feed_forward.scratch_names())
+        beside = self.feed_forward.scratch_names()
+        ctx.beside(mix, feed, self.mixer.scratch_names(), None if beside is None else beside + ("norm",))   # plain_branch
         return pair
 
 

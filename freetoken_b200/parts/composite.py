@@ -23,6 +23,8 @@ class MixerSum(Mixer):
     """params: ``hidden_size``, ``members`` (PartSpecs of mixers, built below this mixer's
     prefix) and ``scales`` (one factor per member)."""
 
+    scratch = ("mixer_sum",)
+
     writes_into_out = True
 
     def __init__(self, spec, prefix):
@@ -42,8 +44,8 @@ class MixerSum(Mixer):
         return list(self.members)
 
     def scratch_names(self):
-        names = [m.scratch_names() for m in self.members]
-        return None if None in names else ("mixer_sum", *sum(names, ()))
+        names = [super().scratch_names(), *(m.scratch_names() for m in self.members)]
+        return None if None in names else sum(names, ())
 
     def cache_need(self):
         return CompositeNeed(tuple(m.cache_need() for m in self.members))

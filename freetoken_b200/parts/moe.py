@@ -77,6 +77,8 @@ class RoutedExperts(FeedForward):
     it per token (``checkpoint_names`` then also has shared_gate, ``[1, hidden]``, and router_gate, the name
     of the merged matrix the model keeps)."""
 
+    scratch = ("moe",)
+
     graph_capturable = True
 
     def __init__(self, spec, prefix):
@@ -135,10 +137,8 @@ class RoutedExperts(FeedForward):
         return self.shared is not None
 
     def scratch_names(self):
-        if self.shared is None:
-            return ("moe",)
-        names = self.shared.scratch_names()
-        return None if names is None else ("moe", *names)
+        own, shared = super().scratch_names(), () if self.shared is None else self.shared.scratch_names()
+        return None if own is None or shared is None else own + shared
 
     def tensor_specs(self) -> List[TensorSpec]:
         E, I, H = self.E, self.inter, self.hidden
@@ -215,7 +215,7 @@ class RoutedExperts(FeedForward):
             return self.routed(ctx, x)
         shared = ctx.workspace.get("moe.shared", (x.shape[0], self.hidden), ctx.dtype)
         rows, extra = ctx.beside(lambda: self.routed(ctx, x), lambda: self.shared.forward(ctx, x, out=shared),
-                                 ("moe",), self.shared.scratch_names(), filler=True)
+                                 super().scratch_names(), self.shared.scratch_names(), filler=True)
         if isinstance(rows, ops.RoutedRows):
             rows.extra = extra
             return rows

@@ -84,3 +84,175 @@ def test_branches_of_a_graph(scratch, branches):
         assert len(streams) > streams_before
         for a, b in zip(have, want):
             assert torch.equal(a, b)
+
+
+def _written(cls, ops):
+    """First words of the workspace names in a class, the package's classes it inherits from, the functions of those modules
+    that it calls and the faces it calls; a name that comes by a variable counts with every literal the variable is given."""
+    import inspect
+    import re
+    import sys
+    source, taken = "", set()
+    for c in cls.__mro__:
+        if c.__module__.startswith("freetoken_b200.") and c.__module__ != "freetoken_b200.parts.base":
+            source += inspect.getsource(c)
+            taken.add(c.__module__)
+    seen = set()
+    while True:
+        called = {(ops.__name__, n) for n in re.findall(r"ops\.(\w+)\(", source)}
+        called |= {(m, n) for m in taken for n in re.findall(r"(?<![\w.])(\w+)\(", source)}
+        new = [(m, n) for m, n in sorted(called - seen) if inspect.isfunction(getattr(sys.modules[m], n, None))]
+        seen |= called
+        if not new:
+            break
+        source += "".join(inspect.getsource(getattr(sys.modules[m], n)) for m, n in new)
+    names = set(re.findall(r'(?:ws|workspace)\.get\(\s*"([\w.]+)"', source))
+    for variable in set(re.findall(r"(?:ws|workspace)\.get\(\s*([A-Za-z_]\w*),", source)):
+        given = re.findall(rf'\b{variable} = (.*"[\w.]+".*)', source)
+        assert given, f"{cls.__name__}: where {variable} comes from"
+        for line in given:
+            names |= set(re.findall(r'"(\w+\.\w+)"', line))
+    return {name.split(".")[0] for name in names}
+
+
+def _package_parts():
+    from freetoken_b200.parts import base
+    return [registry.get(kind) for registry in (base.MIXERS, base.FEED_FORWARDS) for kind in registry.kinds()
+            if registry.get(kind).__module__.startswith("freetoken_b200.")]
+
+
+def test_what_a_part_inherits_and_calls_is_in_its_scratch():
+    from freetoken_b200.csrc import ops
+    from freetoken_b200.parts.key_attention import SharedKVAttention
+    assert _written(SharedKVAttention, ops) == {"kattn", "attn"}          # the splits' partial results, by two steps
+    for cls in _package_parts():
+        assert "scratch" in vars(cls), cls
+        assert _written(cls, ops) <= set(cls.scratch), cls
+
+
+def test_a_class_states_its_own_scratch():
+    """One that inherits a forward may write more buffers than that: nothing runs beside it until it says which."""
+    for cls in _package_parts():
+        bare = object.__new__(type("Derived", (cls,), {}))
+        bare.members, bare.shared = [], None
+        assert bare.scratch_names() is None, cls
+        stated = object.__new__(type("Derived", (cls,), {"scratch": ("own",)}))
+        stated.members, stated.shared = [], None
+        assert stated.scratch_names() == ("own",), cls
+
+
+MODELS = [("besuzen", which) for which in "ABC"] + [("tonapel", which) for which in "ABC"] + [("mezapel", which) for which in "ABCD"]
+OTHERS = [("nirelix", which) for which in "ABC"] + [("dizatar", which) for which in "ABCD"] + [("fazinex", which) for which in "ABC"]
+SETS = {"besuzen": "BZ", "tonapel": "TN", "mezapel": "MZ", "nirelix": "NX", "dizatar": "DZ", "fazinex": "FZ"}
+
+
+def tiny_engine(folder, model, which, **more):
+    import importlib
+    from freetoken_b200.engine import Engine, EngineArgs
+    tiny = importlib.import_module(f"{model}_tiny")
+    tiny.write_tiny(folder, which)
+    engine = Engine.from_folder(folder, EngineArgs(dtype="bfloat16", page_size=tiny.PAGE[which], max_tokens=3 * 128, **more))
+    return engine, {r: tiny.tokens(90 + i, 90, getattr(tiny, SETS[model])[which]["vocab"]) for i, r in enumerate("xyz")}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model,which", MODELS + OTHERS)
+def test_branches_write_the_scratch_they_state(model, which, tmp_path, monkeypatch):
+    """Every workspace name that a branch of a decode step takes, against what its parts say of themselves."""
+    from freetoken_b200.engine import StepEntry
+    from freetoken_b200.parts.base import Workspace
+    engine, toks = tiny_engine(str(tmp_path / "m"), model, which)
+    engine.step([StepEntry(r, t[:20], []) for r, t in toks.items()])
+    open_branches, checked = [], []
+    get, beside = Workspace.get, StepContext.beside
+
+    def noted(self, name, shape, dtype):
+        for names in open_branches:
+            names.add(name.split(".")[0])
+        return get(self, name, shape, dtype)
+
+    def recorded(self, first, second, *scratch, filler=False):
+        def run(piece, stated):
+            def inner():
+                names = set()
+                open_branches.append(names)
+                out = piece()
+                open_branches.pop()
+                checked.append(stated is None or names <= set(stated))
+                assert checked[-1], (names, stated)
+                return out
+            return inner
+        return beside(self, run(first, scratch[0]), run(second, scratch[1]), *scratch, filler=filler)
+    monkeypatch.setattr(Workspace, "get", noted)
+    monkeypatch.setattr(StepContext, "beside", recorded)
+    engine.step([StepEntry(r, [t[20]], [0]) for r, t in toks.items()])
+    assert all(checked) and (checked or (model, which) not in MODELS[:3])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model,which", MODELS)
+def test_replayed_branches_give_the_rows_of_eager_steps(model, which, tmp_path):
+    """Models of parallel halves, sums of mixers and shared experts: the same tokens with and without graph replay."""
+    from freetoken_b200.engine import StepEntry
+    outs = []
+    for most in (64, 0):
+        engine, toks = tiny_engine(str(tmp_path / str(most)), model, which, cuda_graph_max_bs=most)
+        engine.step([StepEntry(r, t[:30], []) for r, t in toks.items()])
+        rows = [engine.step([StepEntry(r, [t[i]], [0]) for r, t in toks.items()]).clone() for i in range(30, 90)]
+        engine.check_status()
+        assert (engine.graph_replays > 30) == (most > 0)
+        outs.append(torch.stack(rows))
+    assert torch.equal(*outs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scratch,branches", [((("a",), ("b",)), True), ((("a",), ("a",)), False), ((("a",), None), False)])
+def test_a_filler_takes_the_minor_streams(scratch, branches):
+    """A long chain and a short one of lower priority beside it, nested once: the graph's rows are the eager ones."""
+    from test_kernels_gpu import DEV, ops, rnd
+    from freetoken_b200.csrc.ops import own_stream
+    o = ops()
+    ctx = context(DEV, [own_stream(DEV, -1), own_stream(DEV, -1)])
+    ctx.minor = [own_stream(DEV, 0), own_stream(DEV, 0)]
+    minor = {s.cuda_stream for s in ctx.minor}
+    x = rnd(3, 512, dtype=torch.bfloat16, seed=1)
+    w = [rnd(512, 512, dtype=torch.bfloat16, seed=2 + i, scale=0.05) for i in range(4)]
+    rows = [torch.empty_like(x) for _ in range(10)]
+    fillers = []
+
+    def long(source, out):
+        def run():
+            o.skinny_gemm(source, w[0], out[0])
+            o.skinny_gemm(out[0], w[1], out[1])
+            o.skinny_gemm(out[1], w[2], out[2])
+            return out[2]
+        return run
+
+    def short(source, out):
+        def run():
+            fillers.append(torch.cuda.current_stream().cuda_stream)
+            o.skinny_gemm(source, w[3], out)
+            return out
+        return run
+
+    def step():
+        a, b = ctx.beside(long(x, rows[:3]), short(x, rows[3]), *scratch, filler=True)
+        c, d = ctx.beside(lambda: ctx.beside(long(a, rows[4:7]), short(b, rows[7]), *scratch, filler=True)[1],
+                          short(a, rows[8]), *scratch)
+        o.skinny_gemm(c, w[1], rows[9])
+        return a, b, c, d, rows[9]
+
+    step()
+    assert not minor & set(fillers)
+    graph = torch.cuda.CUDAGraph()
+    del fillers[:]
+    with torch.cuda.graph(graph, stream=own_stream(DEV, -1)):
+        got = step()
+    assert len(minor & set(fillers)) == (1 if branches else 0) and len(ctx.minor) == len(ctx.side) == 2
+    assert [s in minor for s in fillers] == ([True, False, True] if branches else [False] * 3)
+    for seed in range(20):
+        x.copy_(rnd(3, 512, dtype=torch.bfloat16, seed=100 + seed))
+        graph.replay()
+        have = [t.clone() for t in got]
+        for a, b in zip(have, step()):
+            assert torch.equal(a, b)
