@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
 }
 
 // out[tok, head, :] = sum_s o_s 2^(m_s - m) / sum_s l_s 2^(m_s - m), splits ascending.
-__global__ void attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                  __nv_bfloat16* __restrict__ out, const int* __restrict__ rows,
+__global__ void attn_merge_kernel(const float* part_o, const float* part_ml,
+                                  __nv_bfloat16* __restrict__ out, const int* rows,
                                   int nq, int d, int splits) {
   pdl_wait_only();
 

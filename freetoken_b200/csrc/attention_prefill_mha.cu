@@ -343,12 +343,12 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_mha_kernel(const __grid_c
 // Cached rows of d values -> plain rows.  Eight blocks (a warp per row) copy the 64 rows of keys key0[b] .. of segment
 // seg[b] to plain rows row0[b] ..; keys the segment does not have, and keys before the first that
 // its first token sees (their pages may be another request's by now), become zeros.
-__global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ pages,
-                                                            __nv_bfloat16* __restrict__ dst, const int* __restrict__ seg,
-                                                            const int* __restrict__ key0, const int* __restrict__ row0,
-                                                            const int* __restrict__ seg_kv_len,
-                                                            const int* __restrict__ seg_pos0,
-                                                            const int* __restrict__ block_table, long long page_stride,
+__global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* pages,
+                                                            __nv_bfloat16* __restrict__ dst, const int* seg,
+                                                            const int* key0, const int* row0,
+                                                            const int* seg_kv_len,
+                                                            const int* seg_pos0,
+                                                            const int* block_table, long long page_stride,
                                                             int d, int P, int table_width, int window) {
   pdl_wait();
   const int s = seg[blockIdx.x], k0 = key0[blockIdx.x], r0 = row0[blockIdx.x];

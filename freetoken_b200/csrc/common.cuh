@@ -57,6 +57,9 @@ __device__ __forceinline__ void pdl_wait() {
   pdl_wait_only();
   pdl_release();
 }
+// Such a kernel reads global memory by plain loads: it is resident all through the launch in front, and a `const __restrict__`
+// parameter or __ldg makes a load that is defined only for what nobody writes while the kernel runs, and that the compiler
+// may move across the wait.
 // Loads for the stretch ahead of the wait: they stay where they are written.
 __device__ __forceinline__ float4 ld_ahead4(const float* p) {
   float4 v;

@@ -32,7 +32,7 @@ __device__ __forceinline__ void store4f(float* p, float4 v) { *reinterpret_cast<
 // `copies` > 1: a token's row is written that many times back to back (a model with several
 // residual streams starts them all from the embedded row).
 template <typename WT>
-__global__ void embed_gather_kernel(const int* __restrict__ ids, const WT* __restrict__ table,
+__global__ void embed_gather_kernel(const int* ids, const WT* table,
                                     float* __restrict__ residual, int H, int vocab, int copies) {
   pdl_wait();
 
@@ -75,8 +75,8 @@ constexpr int ROW_KERNEL_EAGER_TOKENS = 64;   // up to this many tokens the row 
 
 template <typename AT, bool VEC>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_kernel(const AT* __restrict__ delta, float* __restrict__ residual,
-               const float* __restrict__ weight, AT* __restrict__ out, int H, float eps,
+rmsnorm_kernel(const AT* delta, float* __restrict__ residual,
+               const float* weight, AT* __restrict__ out, int H, float eps,
                int plus_one, int k) {
   __shared__ float scratch[33];
   pdl_wait();
@@ -161,7 +161,7 @@ __device__ __forceinline__ float4 widen4(const Raw4<__nv_bfloat16>& r) {
 // SM to fall empty, 7.0 instead of 5.1 us behind eight partial rows of 3,072 values.
 template <typename AT>
 __global__ void __launch_bounds__(NORM_THREADS, 2)
-rmsnorm_few_kernel(const AT* __restrict__ delta, float* __restrict__ residual, const float* __restrict__ weight,
+rmsnorm_few_kernel(const AT* delta, float* __restrict__ residual, const float* weight,
                    AT* __restrict__ out, int H, float eps, int plus_one, int k) {
   __shared__ float scratch[33];
   for (int i = threadIdx.x * 32; i < H; i += NORM_THREADS * 32) warm(weight + i);
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(256, NPT <= 4 ? 4 : 2) qk_rope_rows_kernel(QkR
 // --------------------------------------------------------------- top-k sum
 // out[t,:] = sum_j parts[t*k+j,:] in float32, j ascending.
 template <typename AT>
-__global__ void combine_kernel(const AT* __restrict__ parts, AT* __restrict__ out, int k, int H) {
+__global__ void combine_kernel(const AT* parts, AT* __restrict__ out, int k, int H) {
   pdl_wait();
 
   const int t = blockIdx.x;
@@ -821,7 +821,7 @@ __global__ void combine_kernel(const AT* __restrict__ parts, AT* __restrict__ ou
 
 // ---------------------------------------------------------------- row gather
 template <typename AT>
-__global__ void gather_rows_kernel(const AT* __restrict__ src, const int* __restrict__ rows,
+__global__ void gather_rows_kernel(const AT* src, const int* rows,
                                    AT* __restrict__ dst, int H) {
   pdl_wait();
 
@@ -834,7 +834,7 @@ __global__ void gather_rows_kernel(const AT* __restrict__ src, const int* __rest
   if (H % PER == 0 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
     const uint4* s4 = reinterpret_cast<const uint4*>(s);
     uint4* d4 = reinterpret_cast<uint4*>(d);
-    for (int i = threadIdx.x; i < H / PER; i += blockDim.x) d4[i] = __ldg(s4 + i);
+    for (int i = threadIdx.x; i < H / PER; i += blockDim.x) d4[i] = s4[i];
     return;
   }
   for (int i = threadIdx.x; i < H; i += blockDim.x) d[i] = s[i];

@@ -15,8 +15,8 @@ __device__ __forceinline__ float gate_f(float v, int kind) {
 // square; times weight[i % weight_len]; a gate silu(z) (or sigmoid(z)) on the values before the norm
 // (gate_first) or on the result.  One warp per (token, group).
 template <typename AT>
-__global__ void __launch_bounds__(128) gated_norm_kernel(const float* __restrict__ y, const AT* __restrict__ z,
-                                                         long long ldz, const float* __restrict__ weight,
+__global__ void __launch_bounds__(128) gated_norm_kernel(const float* y, const AT* z,
+                                                         long long ldz, const float* weight,
                                                          int weight_len, AT* __restrict__ out, int T, int width,
                                                          int groups, float eps, int gate_first, int gate_kind) {
   pdl_wait();
@@ -64,8 +64,8 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, float4 v) {
 }
 
 template <typename AT, int TPI, int KEEP>
-__global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* __restrict__ y, const AT* __restrict__ z,
-                                                             long long ldz, const float* __restrict__ weight,
+__global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* y, const AT* z,
+                                                             long long ldz, const float* weight,
                                                              int weight_len, AT* __restrict__ out, int T, int width,
                                                              int groups, float eps, int gate_first, int gate_kind) {
   __shared__ float scratch[33];

@@ -16,7 +16,7 @@ namespace ft {
 // Scores and top-k of one token by one warp.  `score` and `choice` are E floats
 // of shared memory each.  With k <= 32 lane j < k returns the j-th choice in
 // (my_id, my_w); otherwise ids and weights go through `ids_out` / `weights_out`.
-__device__ __forceinline__ void select_token(const float* __restrict__ x, const float* __restrict__ bias,
+__device__ __forceinline__ void select_token(const float* x, const float* bias,
                                              float* score, float* choice, int* ids_out, float* weights_out,
                                              int E, int k, int softmax_scoring, int renormalize, float scale,
                                              int terms, int groups, int keep, int group_top, float* tail, int lane,
@@ -190,7 +190,7 @@ __device__ __forceinline__ void select_token(const float* __restrict__ x, const 
 }
 
 template <int WARPS>
-__global__ void router_select_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
+__global__ void router_select_kernel(const float* logits, const float* bias,
                                      int* __restrict__ ids, float* __restrict__ weights, int T, int E,
                                      int k, int softmax_scoring, int renormalize, float scale, int terms,
                                      int groups, int keep, int group_top, float* __restrict__ tail) {
@@ -220,7 +220,7 @@ __global__ void router_select_kernel(const float* __restrict__ logits, const flo
 constexpr int SMALL_WARPS = 8;
 
 __global__ void __launch_bounds__(SMALL_WARPS * 32) route_small_kernel(
-    const float* __restrict__ logits, const float* __restrict__ bias, int* __restrict__ ids,
+    const float* logits, const float* bias, int* __restrict__ ids,
     float* __restrict__ weights, int* __restrict__ counts, int* __restrict__ offsets,
     int* __restrict__ sorted_route, int* __restrict__ sorted_token, int* __restrict__ active, int T, int E,
     int busy_of, int k, int softmax_scoring, int renormalize, float scale, int terms, int groups, int keep,
@@ -306,8 +306,8 @@ __device__ __forceinline__ void load8f(const __nv_bfloat16* p, float (&v)[8]) {
 // EARLY (8 tokens or less, one block an expert): the first 4,096 weights of the row are fetched ahead of the wait for the
 // launch in front; with several blocks an expert the registers that takes cost more (64 tokens 17.2 -> 19.3 us).
 template <typename AT, bool EARLY>
-__global__ void __launch_bounds__(128) router_logits_kernel(const AT* __restrict__ x, long long ldx,
-                                                            const float* __restrict__ W,
+__global__ void __launch_bounds__(128) router_logits_kernel(const AT* x, long long ldx,
+                                                            const float* W,
                                                             float* __restrict__ logits, int T, int E,
                                                             int H) {
   // one block per (expert, 8 tokens); its 4 warps take a quarter of the row
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const AT* __restrict
 constexpr int SCAN = 8;  // route ids a lane reads ahead while scanning
 
 // counts[e] = number of routes that chose expert e.  One warp per expert.
-__global__ void moe_count_kernel(const int* __restrict__ ids, int* __restrict__ counts, int R, int E) {
+__global__ void moe_count_kernel(const int* ids, int* __restrict__ counts, int R, int E) {
   const int lane = threadIdx.x & 31;
   pdl_wait();
 
@@ -400,7 +400,7 @@ __global__ void moe_count_kernel(const int* __restrict__ ids, int* __restrict__ 
 // offsets[e] = sum counts[<e]; sorted_route[offsets[e] + i] = i-th route of
 // expert e in ascending route order; sorted_token = sorted_route / k;
 // active[j] = j-th expert below busy_of that has routes (ascending), active[busy_of] = how many.
-__global__ void moe_scatter_kernel(const int* __restrict__ ids, const int* __restrict__ counts,
+__global__ void moe_scatter_kernel(const int* ids, const int* counts,
                                    int* __restrict__ offsets, int* __restrict__ sorted_route,
                                    int* __restrict__ sorted_token, int* __restrict__ active,
                                    int R, int E, int busy_of, int k) {

@@ -36,8 +36,8 @@ constexpr int EMBED_KEEP = 4;      // groups of 4 elements a thread keeps betwee
 // the row is read once and stays in registers between the sum of squares and the scaling.
 template <typename WT, bool VEC>
 __global__ void __launch_bounds__(EMBED_THREADS)
-embed_norm_kernel(const int* __restrict__ ids, const WT* __restrict__ table,
-                  const float* __restrict__ weight, float* __restrict__ residual, int H, int vocab,
+embed_norm_kernel(const int* ids, const WT* table,
+                  const float* weight, float* __restrict__ residual, int H, int vocab,
                   float eps) {
   __shared__ float scratch[33];
   pdl_wait();
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(128) key_store_kernel(KeyStoreArgs a, int T, i
 // (8 bfloat16 values as one 16-byte piece when d allows it), so the gate is evaluated once a piece.
 template <typename AT, int PIECE>
 __global__ void __launch_bounds__(256)
-gate_heads_kernel(AT* __restrict__ o, const AT* __restrict__ z, long long ldz, int heads, int d, long long pieces) {
+gate_heads_kernel(AT* __restrict__ o, const AT* z, long long ldz, int heads, int d, long long pieces) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pieces) return;
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(THREADS) join_layer_norm_kernel(JoinNormArgs a
 // out[t, :] = sum_j s_j * parts[t, j, :]   (float32 sum, ascending j)
 template <typename AT>
 __global__ void __launch_bounds__(256)
-scaled_sum_kernel(const AT* __restrict__ parts, const float* __restrict__ scale, AT* __restrict__ out, int k,
+scaled_sum_kernel(const AT* parts, const float* scale, AT* __restrict__ out, int k,
                   long long n, int H) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -834,7 +834,7 @@ scaled_sum_kernel(const AT* __restrict__ parts, const float* __restrict__ scale,
 // x[t, c] += bias[c]; rows may lie further apart than their width
 template <typename AT>
 __global__ void __launch_bounds__(256)
-bias_add_kernel(AT* __restrict__ x, long long ld, const float* __restrict__ bias, long long n, int width) {
+bias_add_kernel(AT* __restrict__ x, long long ld, const float* bias, long long n, int width) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -848,7 +848,7 @@ bias_add_kernel(AT* __restrict__ x, long long ld, const float* __restrict__ bias
 // kind 3: the clamped pair  g = min(gate, limit), u = clamp(up, -limit, limit),  g sigmoid(alpha g) (u + 1)
 template <typename AT>
 __global__ void __launch_bounds__(256)
-glu_rows_kernel(const AT* __restrict__ gu, AT* __restrict__ mid, long long n, int I, int kind, float alpha,
+glu_rows_kernel(const AT* gu, AT* __restrict__ mid, long long n, int I, int kind, float alpha,
                 float limit) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -869,7 +869,7 @@ glu_rows_kernel(const AT* __restrict__ gu, AT* __restrict__ mid, long long n, in
 
 // the same in 16-byte pieces (bfloat16, I a multiple of 8)
 __global__ void __launch_bounds__(256)
-glu_rows8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ mid, long long n8, int I8, int kind,
+glu_rows8_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ mid, long long n8, int I8, int kind,
                  float alpha, float limit) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -903,9 +903,9 @@ glu_rows8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict
 constexpr int HYPER_MAX_STREAMS = 8;
 template <typename AT>
 __global__ void __launch_bounds__(256)
-hyper_norm_kernel(float* __restrict__ streams, const AT* __restrict__ branch, int k, const float* __restrict__ mix,
-                  const float* __restrict__ out_w, const float* __restrict__ read, const float* __restrict__ weight,
-                  const float* __restrict__ bias, float eps, int center, AT* __restrict__ normed, int S, int H) {
+hyper_norm_kernel(float* __restrict__ streams, const AT* branch, int k, const float* mix,
+                  const float* out_w, const float* read, const float* weight,
+                  const float* bias, float eps, int center, AT* __restrict__ normed, int S, int H) {
   extern __shared__ float u_row[];
   __shared__ float scratch[33];
   __shared__ float s_mix[HYPER_MAX_STREAMS * HYPER_MAX_STREAMS], s_out[HYPER_MAX_STREAMS], s_read[HYPER_MAX_STREAMS];
@@ -974,9 +974,9 @@ hyper_norm_kernel(float* __restrict__ streams, const AT* __restrict__ branch, in
 // 4.4 -> 3.7).  With every SM full of rows those registers would cost occupancy.
 template <typename AT, int S, int KEEP, bool EAGER>
 __global__ void __launch_bounds__(256)
-hyper_norm_vec_kernel(float* __restrict__ streams, const AT* __restrict__ branch, int k, const float* __restrict__ mix,
-                      const float* __restrict__ out_w, const float* __restrict__ read,
-                      const float* __restrict__ weight, const float* __restrict__ bias, float eps, int center,
+hyper_norm_vec_kernel(float* __restrict__ streams, const AT* branch, int k, const float* mix,
+                      const float* out_w, const float* read,
+                      const float* weight, const float* bias, float eps, int center,
                       AT* __restrict__ normed, int H) {
   __shared__ float scratch[33];
   const int t = blockIdx.x, groups = H >> 2;
@@ -1136,7 +1136,7 @@ static cudaError_t launch_hyper_vec(cudaStream_t stream, int T, int H, float* st
 constexpr int RMS_KEEP = 16;
 template <typename AT>
 __global__ void __launch_bounds__(128)
-rms_rows_kernel(const AT* __restrict__ x, long long ldx, const float* __restrict__ w, AT* __restrict__ out,
+rms_rows_kernel(const AT* x, long long ldx, const float* w, AT* __restrict__ out,
                 long long ldo, int n, float eps) {
   __shared__ float scratch[33];
   for (int c = threadIdx.x * 32; c < n; c += blockDim.x * 32) warm(w + c);
@@ -1314,7 +1314,7 @@ __global__ void __launch_bounds__(256) embed_pair_kernel(EmbedPairArgs a) {
 // o[t, i] *= sigmoid(z[t, i]): a gate per value, 16-byte pieces of eight bfloat16 values (the sigmoid from the
 // fast exponential and division: float32 arithmetic whose error lies far below the bfloat16 result's rounding)
 __global__ void __launch_bounds__(256)
-gate_values_bf16x8_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ z, long long ldz, int n8,
+gate_values_bf16x8_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* z, long long ldz, int n8,
                           long long pieces) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

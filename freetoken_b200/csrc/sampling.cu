@@ -45,9 +45,9 @@ __device__ __forceinline__ void kept_mass(const float* p, int V, float thr, floa
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const float* __restrict__ uniform, int* __restrict__ out, float* __restrict__ probs,
+sample_kernel(const float* logits, const float* temperature,
+              const int* top_k, const float* top_p,
+              const float* uniform, int* __restrict__ out, float* __restrict__ probs,
               int V) {
   __shared__ float scratch[33];
   __shared__ float prefix[SAMPLE_THREADS];

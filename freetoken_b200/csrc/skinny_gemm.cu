@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(KS * 32) skinny_kernel(SkinnyArgs a) {
         const bool kin = (c + u) < c_end && (k8 << 3) < K;
 #pragma unroll
         for (int j = 0; j < NT; ++j)
-          xv[u][j] = (kin && xrow[j]) ? (U >= 4 ? ld_rows(xrow[j] + k8) : __ldg(xrow[j] + k8)) : zero;
+          xv[u][j] = (kin && xrow[j]) ? ld_rows(xrow[j] + k8) : zero;
       }
       if constexpr (U >= 4) __syncwarp();
 #pragma unroll
