@@ -73,12 +73,16 @@ __device__ __forceinline__ void store4f(__nv_bfloat16* p, float4 v) {
 
 constexpr int ROW_KERNEL_EAGER_TOKENS = 64;   // up to this many tokens the row kernels fetch eagerly
 
-template <typename AT, bool VEC>
+// EAGER (up to ROW_KERNEL_EAGER_TOKENS tokens, rows that rmsnorm_few_kernel is not taken for): the partial rows of a piece are
+// fetched four at a time before they are added, in the same order, and the weight is asked for ahead of the wait.
+template <typename AT, bool VEC, bool EAGER = false>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_kernel(const AT* delta, float* __restrict__ residual,
                const float* weight, AT* __restrict__ out, int H, float eps,
                int plus_one, int k) {
   __shared__ float scratch[33];
+  if (EAGER)
+    for (int i = threadIdx.x * 32; i < H; i += NORM_THREADS * 32) warm(weight + i);
   pdl_wait();
   const int t = blockIdx.x;
   float* r = residual + (size_t)t * H;
@@ -96,9 +100,15 @@ rmsnorm_kernel(const AT* delta, float* __restrict__ residual,
         float4 z = load4f(r + 4 * gi);
         if (d) {
           float4 add = load4f(d + 4 * gi);
-          for (int q = 1; q < k; ++q) {
-            const float4 more = load4f(d + (size_t)q * H + 4 * gi);
-            add.x += more.x; add.y += more.y; add.z += more.z; add.w += more.w;
+          constexpr int ROUND = EAGER ? 4 : 1;
+          for (int q0 = 1; q0 < k; q0 += ROUND) {
+            float4 more[ROUND];
+#pragma unroll
+            for (int u = 0; u < ROUND; ++u)
+              more[u] = q0 + u < k ? load4f(d + (size_t)(q0 + u) * H + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < ROUND; ++u)
+              if (q0 + u < k) { add.x += more[u].x; add.y += more[u].y; add.z += more[u].z; add.w += more[u].w; }
           }
           z.x += add.x; z.y += add.y; z.z += add.z; z.w += add.w;
           store4f(r + 4 * gi, z);
@@ -153,12 +163,17 @@ __device__ __forceinline__ float4 widen4(const Raw4<__nv_bfloat16>& r) {
 }
 
 // For a step of few tokens, where a launch is a chain of waits for L2 rather than a
-// stream: the k partial rows are fetched four at a time, of two pieces together, before they are
+// stream: the partial rows are fetched four at a time, of two pieces together, before they are
 // added, in the same order, and the weight - cold in L2 after a step's worth of others - is asked
 // for ahead of the wait.  With every SM full of such blocks the extra loads in flight cost more
 // than they save (25 -> 29 us at 2,048 tokens), so many tokens keep the one-by-one loop.  Of 64 registers
 // a thread, so that a block finds a place beside those of the launch in front: with 128 it waited for an
 // SM to fall empty, 7.0 instead of 5.1 us behind eight partial rows of 3,072 values.
+// Two pieces together pay where a thread has two and their partial rows are one round (rmsnorm_two_pieces): between two
+// products, us a chain of three launches of 1, 8 and 64 tokens, piece by piece (rmsnorm_kernel, EAGER) and two together: one
+// row of 3,072 values 12.3 -> 11.9, 13.4 -> 13.0, 16.7 -> 16.3, three 12.15 -> 12.1, 13.5 -> 13.4, 17.1 -> 17.0; but four
+// 12.15 and 12.2, 13.6 and 13.6, 17.1 and 17.1, four of 4,096 values 16.3 and 16.3, 17.6 and 17.5, 23.8 and 24.0, eight
+// 17.2 -> 17.7, 18.5 -> 19.0, 25.2 -> 26.6, and of 2,048 values, a piece a thread, two 7.6 -> 7.9, eight 8.0 -> 8.9.
 template <typename AT>
 __global__ void __launch_bounds__(NORM_THREADS, 2)
 rmsnorm_few_kernel(const AT* delta, float* __restrict__ residual, const float* weight,
@@ -930,6 +945,10 @@ int ft_embed_gather(const int* ids, const void* table, int table_dtype, float* r
   return FT_OK;
 }
 
+// Whether a row of few tokens is fetched two pieces at a time; both sides of the lines stand at rmsnorm_few_kernel.
+static bool rmsnorm_two_pieces(int H, int k) { return k == 1 || (H > 4 * NORM_THREADS && k <= 3); }
+int ft_rmsnorm_two_pieces(int H, int k) { return rmsnorm_two_pieces(H, k); }
+
 int ft_rmsnorm(const void* delta, float* residual, const float* weight, void* out, int dtype,
                int T, int H, float eps, int plus_one, int k, cudaStream_t stream) {
   if (T <= 0) return FT_OK;
@@ -938,9 +957,15 @@ int ft_rmsnorm(const void* delta, float* residual, const float* weight, void* ou
   const bool vec = !(H & 3) && H <= 4 * NORM_THREADS * NORM_KEEP && !((uintptr_t)delta & 15) &&
                    !((uintptr_t)residual & 15) && !((uintptr_t)weight & 15) && !((uintptr_t)out & 15);
   if (vec && T <= ROW_KERNEL_EAGER_TOKENS) {
-    FT_DISPATCH(dtype, AT,
-                (launch_pdl(rmsnorm_few_kernel<AT>, dim3(T), dim3(NORM_THREADS), 0, stream,
-                            (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
+    if (!delta || rmsnorm_two_pieces(H, k)) {
+      FT_DISPATCH(dtype, AT,
+                  (launch_pdl(rmsnorm_few_kernel<AT>, dim3(T), dim3(NORM_THREADS), 0, stream,
+                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
+    } else {
+      FT_DISPATCH(dtype, AT,
+                  (launch_pdl(rmsnorm_kernel<AT, true, true>, dim3(T), dim3(NORM_THREADS), 0, stream,
+                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
+    }
   } else if (vec) {
     FT_DISPATCH(dtype, AT,
                 launch_pdl(rmsnorm_kernel<AT, true>, dim3(T), dim3(NORM_THREADS), 0, stream,

@@ -108,3 +108,26 @@ def test_nothing_that_a_device_is_asked_is_kept_for_all_devices():
     with open(os.path.join(build.HERE, "skinny_gemm.cu")) as f:
         code = "\n".join(line.split("//")[0] for line in f)
     assert "static const int" not in code and code.count("148") == 1            # the exported rule of the tests above
+
+
+@pytest.mark.parametrize("H,k,two", [(2048, 1, 1), (2048, 2, 0), (2052, 2, 1), (3072, 3, 1), (3072, 4, 0), (8192, 8, 0), (512, 1, 1)])
+def test_pieces_of_a_norm_of_few_tokens(H, k, two):
+    assert build.load("elementwise").ft_rmsnorm_two_pieces(H, k) == two
+
+
+# both forms of few tokens and the form of many: a token's row has the same bits
+@pytest.mark.gpu
+@pytest.mark.parametrize("H", [128, 2048, 2052, 3072, 8192])
+@pytest.mark.parametrize("k", [0, 1, 2, 3, 4, 5, 9])
+def test_norms_of_few_and_many_tokens_agree(H, k):
+    import torch
+    from test_kernels_gpu import DEV, ops, rnd
+    delta = rnd(65, max(k, 1), H, dtype=torch.bfloat16, seed=1) if k else None
+    residual, weight = rnd(65, H, seed=2), rnd(H, seed=3)
+    got = []
+    for T in (65, 64, 1):
+        r, out = residual[:T].clone(), torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+        ops().rmsnorm(delta[:T].contiguous() if k else None, r, weight, out, 1e-5, False)
+        got.append((r, out))
+    for r, out in got[1:]:
+        assert torch.equal(r, got[0][0][:len(r)]) and torch.equal(out, got[0][1][:len(r)])
