@@ -52,6 +52,7 @@ struct DecodeTmaArgs {
   ScoreOpts opt;             // chunks, cap, sink (the sink joins the partial of split 0)
   int v_plane = 1;           // which plane of the cache holds the values (0: the keys are the values)
   int lets_in = 0;           // the next launch becomes resident beside this one
+  bool ahead = false;        // promised_ahead
 };
 
 constexpr int DT_TILE = 64;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(160) attn_decode_tma_kernel(const __grid_const
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (!a.ahead) pdl_wait_only();
   const int G = a.nq / a.nkv;
   const int gtiles = (G + 15) / 16;
   const int kvh = blockIdx.y / gtiles, gt = blockIdx.y % gtiles;
@@ -459,7 +461,8 @@ extern "C" int ft_attn_decode_tma(const void* map_kv, const void* q, void* out, 
   memcpy(&mkv, map_kv, sizeof(mkv));
   DecodeTmaArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, part_o, part_ml, rows, token_pos,
                   token_seg, block_table, status, nq, nkv, P, table_width, window, n_rows, splits,
-                  split_keys, scale, ScoreOpts{chunk, softcap, sink_mode, sink_value, sink}, v_plane ? 1 : 0, lets_in};
+                  split_keys, scale, ScoreOpts{chunk, softcap, sink_mode, sink_value, sink}, v_plane ? 1 : 0, lets_in,
+                  promised_ahead};
   if (sink_mode == 2 && !sink) return FT_ERR_SHAPE;
   int rc;
   switch (d) {

@@ -45,6 +45,7 @@ struct LatentAttnArgs {
   long long page_stride, ldo;
   int nq, d, rank, P, table_width, window, splits, split_keys, stages;
   float scale_log2;
+  bool ahead;                   // promised_ahead
 };
 
 constexpr int LT_KEYS = 64, LT_PLD = LT_KEYS + 8, LT_SLD = LT_KEYS + 8, LT_STAGES = 3, LT_THREADS = 384, LT_PRODUCERS = 128;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
       *reinterpret_cast<uint4*>((r < RT ? sQ + r * ld : sK + (size_t)(r - RT) * ld) + c * 8) = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
 
+  if (!a.ahead) pdl_wait();
   const int seg = a.tile_seg[blockIdx.x], row0 = a.tile_row[blockIdx.x];
   const int split = blockIdx.y;
   const int seg_begin = a.seg_q_start[seg];
@@ -350,6 +352,7 @@ __global__ void __launch_bounds__(LT_THREADS) attn_latent_kernel(LatentAttnArgs 
 // asks for more); further ones follow in rounds of as many.
 constexpr int MERGE_AHEAD = 8, MERGE_SPLITS = 1024, MERGE_THREADS = 128;
 __global__ void __launch_bounds__(MERGE_THREADS) latent_merge_kernel(LatentAttnArgs a, int rt) {
+  if (!a.ahead) pdl_wait();
   const int tile = blockIdx.x, r = blockIdx.y;
   const int seg = a.tile_seg[tile], row0 = a.tile_row[tile];
   const int seg_begin = a.seg_q_start[seg];
@@ -497,7 +500,7 @@ int ft_attn_latent(const void* q, void* out, long long ldo, float* part_o, float
   if (stages == 0) return FT_ERR_SHAPE;
   LatentAttnArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, part_o, part_ml, (const __nv_bfloat16*)pages,
                    tile_seg, tile_row, seg_q_start, seg_pos0, block_table, status, page_stride, ldo, nq, d, rank, P,
-                   table_width, window, splits, split_keys, stages, scale * 1.4426950408889634f};
+                   table_width, window, splits, split_keys, stages, scale * 1.4426950408889634f, promised_ahead};
   const int rc = mt == 1 ? launch_latent_by_size<1>(a, tiles, stream) : launch_latent_by_size<2>(a, tiles, stream);
   if (rc != FT_OK) return rc;
   if (splits > 1)

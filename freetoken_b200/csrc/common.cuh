@@ -40,8 +40,8 @@ namespace ft {
 // visible, and only then lets the kernel behind it in.  So no more than one
 // launch waits beside the one that works, and what a kernel does ahead of its
 // wait may read whatever the launch right in front of it does not write:
-// weights, tables and the step's metadata always, a request's state where the
-// caller says so.  Everything else is touched behind the wait, and a kernel
+// weights, tables and the step's metadata where the caller promises it
+// (promised_ahead), a request's state where it says so of that.  Everything else is touched behind the wait, and a kernel
 // whose blocks all leave must have waited in one of them.  Kernels that fill the
 // chip with large blocks (float32 tiles, prompt scans and attention) let the
 // next one in only as they leave (pdl_wait_only): resident beside them it works
@@ -168,8 +168,14 @@ inline int device_sms() {
   });
 }
 
-// The packed form of an extern "C" launcher: the arguments in an array of 8-byte words, taken apart by the types of the
-// launcher's own parameters.  FT_PACKED(name), behind the launcher, defines `name_packed`, which the host side calls.
+// Whether the caller of a launcher promises that the launch right in front of it writes nothing of what the kernel reads
+// ahead of its wait: weights, tables, the step's metadata.  Without that a kernel waits before it reads anything
+// (`if (!ahead) pdl_wait();`, the later wait is then passed at once).  The packed form hands it on for the length of its call;
+// who calls a launcher directly promises nothing.
+inline thread_local bool promised_ahead = false;
+
+// The packed form of an extern "C" launcher: the arguments in an array of 8-byte words (and behind them the promise),
+// taken apart by the types of the launcher's own parameters.  FT_PACKED(name), behind the launcher, defines `name_packed`, which the host side calls.
 union PackedArg {
   void* p;
   long long i;
@@ -184,7 +190,10 @@ inline int call_packed(int (*f)(P...), const PackedArg* a, std::index_sequence<I
 }
 template <typename... P>
 inline int call_packed(int (*f)(P...), const PackedArg* a) {
-  return call_packed(f, a, std::index_sequence_for<P...>());
+  promised_ahead = a[sizeof...(P)].i != 0;
+  const int rc = call_packed(f, a, std::index_sequence_for<P...>());
+  promised_ahead = false;
+  return rc;
 }
 #define FT_PACKED(NAME) \
   extern "C" int NAME##_packed(const ft::PackedArg* a) { return ft::call_packed(NAME, a); }

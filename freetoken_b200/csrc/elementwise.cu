@@ -79,9 +79,9 @@ template <typename AT, bool VEC, bool EAGER = false>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_kernel(const AT* delta, float* __restrict__ residual,
                const float* weight, AT* __restrict__ out, int H, float eps,
-               int plus_one, int k) {
+               int plus_one, int k, bool ahead) {
   __shared__ float scratch[33];
-  if (EAGER)
+  if (EAGER && ahead)
     for (int i = threadIdx.x * 32; i < H; i += NORM_THREADS * 32) warm(weight + i);
   pdl_wait();
   const int t = blockIdx.x;
@@ -177,9 +177,9 @@ __device__ __forceinline__ float4 widen4(const Raw4<__nv_bfloat16>& r) {
 template <typename AT>
 __global__ void __launch_bounds__(NORM_THREADS, 2)
 rmsnorm_few_kernel(const AT* delta, float* __restrict__ residual, const float* weight,
-                   AT* __restrict__ out, int H, float eps, int plus_one, int k) {
+                   AT* __restrict__ out, int H, float eps, int plus_one, int k, bool ahead) {
   __shared__ float scratch[33];
-  for (int i = threadIdx.x * 32; i < H; i += NORM_THREADS * 32) warm(weight + i);
+  for (int i = threadIdx.x * 32; ahead && i < H; i += NORM_THREADS * 32) warm(weight + i);
   pdl_wait();
   const int t = blockIdx.x, groups = H >> 2;
   float* r = residual + (size_t)t * H;
@@ -270,6 +270,7 @@ struct QkRopeArgs {
   const float* v_lambda;  // l, one number
   long long ld_first;
   int d_first;
+  bool ahead = false;     // promised_ahead
 };
 
 // value i of KV head h of the earlier layer's row (zero where only this layer's heads are filled up)
@@ -499,6 +500,7 @@ template <bool EAGER>
 __global__ void __launch_bounds__(256) qk_rope_store_vec_kernel(QkRopeArgs a) {
   extern __shared__ float head_inv[];
   __shared__ float scratch[66];
+  if (!a.ahead) pdl_wait();
   const int t = blockIdx.x;
   const int pos = a.token_pos[t];
   size_t page_base = 0;
@@ -960,20 +962,20 @@ int ft_rmsnorm(const void* delta, float* residual, const float* weight, void* ou
     if (!delta || rmsnorm_two_pieces(H, k)) {
       FT_DISPATCH(dtype, AT,
                   (launch_pdl(rmsnorm_few_kernel<AT>, dim3(T), dim3(NORM_THREADS), 0, stream,
-                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
+                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k, promised_ahead)));
     } else {
       FT_DISPATCH(dtype, AT,
                   (launch_pdl(rmsnorm_kernel<AT, true, true>, dim3(T), dim3(NORM_THREADS), 0, stream,
-                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k)));
+                              (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k, promised_ahead)));
     }
   } else if (vec) {
     FT_DISPATCH(dtype, AT,
                 launch_pdl(rmsnorm_kernel<AT, true>, dim3(T), dim3(NORM_THREADS), 0, stream,
-                           (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k));
+                           (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k, false));
   } else {
     FT_DISPATCH(dtype, AT,
                 launch_pdl(rmsnorm_kernel<AT, false>, dim3(T), dim3(NORM_THREADS), 0, stream,
-                           (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k));
+                           (const AT*)delta, residual, weight, (AT*)out, H, eps, plus_one, k, false));
   }
   FT_LAUNCH_CHECK();
   return FT_OK;
@@ -992,7 +994,7 @@ int ft_qk_rope_store(const void* qkv, void* q_out, void* kv_pages, const float* 
   if (norm_dim <= 0 || norm_dim > d) norm_dim = d;
   QkRopeArgs a{qkv, q_out, kv_pages, q_weight, k_weight, cos_sin, token_pos, token_seg,
                block_table, ld, page_stride, kv_stride, nq, nkv, d, R, P, table_width,
-               norm_mode, plus_one, interleaved, eps, norm_dim, v_first, v_lambda, ld_first, d_first};
+               norm_mode, plus_one, interleaved, eps, norm_dim, v_first, v_lambda, ld_first, d_first, promised_ahead};
   const size_t smem = (size_t)(nq + nkv) * sizeof(float);
   const bool aligned = !((uintptr_t)qkv & 15) && !((uintptr_t)q_out & 15) &&
                        !((uintptr_t)kv_pages & 15) && !(ld & 7) && !(page_stride & 7) &&

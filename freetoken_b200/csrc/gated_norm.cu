@@ -67,7 +67,8 @@ template <typename AT, int TPI, int KEEP>
 __global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* y, const AT* z,
                                                              long long ldz, const float* weight,
                                                              int weight_len, AT* __restrict__ out, int T, int width,
-                                                             int groups, float eps, int gate_first, int gate_kind) {
+                                                             int groups, float eps, int gate_first, int gate_kind,
+                                                             bool ahead) {
   __shared__ float scratch[33];
   const int sub = threadIdx.x % TPI;
   // 32 bits (the host sees to it): a division of 64 took as long as the load behind it
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* y, con
   const bool live = item < (unsigned)T * (unsigned)groups;
   const int t = live ? (int)(item / (unsigned)groups) : 0, grp = live ? (int)(item - (unsigned)t * (unsigned)groups) : 0;
   const int size = width / groups, base = grp * size, pieces = live ? size >> 2 : 0;
-  for (int i = sub * 32; i < (live ? size : 0); i += TPI * 32) warm(weight + (base + i) % weight_len);
+  for (int i = sub * 32; ahead && i < (live ? size : 0); i += TPI * 32) warm(weight + (base + i) % weight_len);
   pdl_wait();
   if (TPI >= 32 && !live) return;                     // a warp (TPI 32) or the whole block (TPI 128) leaves
   const float* row = y + (size_t)t * width + base;
@@ -141,28 +142,28 @@ int ft_gated_norm(const float* y, const void* z, long long ldz, const float* wei
   if (vec && size <= 16 * 8) {
     FT_DISPATCH(dtype, AT, launch_pdl(gated_norm_vec_kernel<AT, 8, 4>, dim3((unsigned)((items + 15) / 16)), dim3(128), 0, stream,
                                       y, (const AT*)z, ldz, weight, weight_len, (AT*)out, T, width, groups, eps,
-                                      gate_first, gate_kind));
+                                      gate_first, gate_kind, promised_ahead));
     FT_LAUNCH_CHECK();
     return FT_OK;
   }
   if (vec && size <= 16 * 32) {
     FT_DISPATCH(dtype, AT, launch_pdl(gated_norm_vec_kernel<AT, 32, 4>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream,
                                       y, (const AT*)z, ldz, weight, weight_len, (AT*)out, T, width, groups, eps,
-                                      gate_first, gate_kind));
+                                      gate_first, gate_kind, promised_ahead));
     FT_LAUNCH_CHECK();
     return FT_OK;
   }
   if (vec && size <= 16 * 128) {
     FT_DISPATCH(dtype, AT, launch_pdl(gated_norm_vec_kernel<AT, 128, 4>, dim3((unsigned)items), dim3(128), 0, stream, y,
                                       (const AT*)z, ldz, weight, weight_len, (AT*)out, T, width, groups, eps,
-                                      gate_first, gate_kind));
+                                      gate_first, gate_kind, promised_ahead));
     FT_LAUNCH_CHECK();
     return FT_OK;
   }
   if (vec && size <= 64 * 128) {
     FT_DISPATCH(dtype, AT, launch_pdl(gated_norm_vec_kernel<AT, 128, 16>, dim3((unsigned)items), dim3(128), 0, stream, y,
                                       (const AT*)z, ldz, weight, weight_len, (AT*)out, T, width, groups, eps,
-                                      gate_first, gate_kind));
+                                      gate_first, gate_kind, promised_ahead));
     FT_LAUNCH_CHECK();
     return FT_OK;
   }

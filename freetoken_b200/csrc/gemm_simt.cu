@@ -39,6 +39,7 @@ struct GemmArgs {
   // A, W and C start this many elements further on
   long long a_batch_stride = 0, w_batch_stride = 0, c_batch_stride = 0;
   int batch = 1;
+  bool ahead = false;        // promised_ahead
 };
 
 __device__ __forceinline__ float glu_act(float g, float u, int act, float alpha, float limit) {
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(STREAM_THREADS) gemm_stream_kernel(GemmArgs a)
   constexpr int STAGE = WROWS * WROW + MR * AROW;
   extern __shared__ __align__(16) unsigned char stream_sm[];
   __shared__ int tile_info[3];
-  if (a.group_offsets) pdl_wait_only();
+  if (a.group_offsets || !a.ahead) pdl_wait_only();
   find_tile<MR>(a, tile_info);
   __syncthreads();
   const int group = tile_info[0], row0 = tile_info[1], rows = tile_info[2];
@@ -654,6 +655,7 @@ extern "C" int ft_gemm_rows(const void* A, int a_dtype, long long lda, const voi
   if (K <= 0 || G <= 0) return FT_ERR_SHAPE;
   GemmArgs a{A, W, C, group_offsets, a_rows, c_rows, row_scale, lda, ldc, w_group_stride,
              M, N, K, G, act, act_alpha, act_limit};
+  a.ahead = promised_ahead;
   const int key = a_dtype * 100 + w_dtype * 10 + c_dtype;
   int rc;
   switch (key) {
@@ -679,6 +681,7 @@ extern "C" int ft_gemm_heads(const void* A, int a_dtype, long long lda, long lon
   a.w_batch_stride = w_batch_stride;
   a.c_batch_stride = c_batch_stride;
   a.batch = batch;
+  a.ahead = promised_ahead;
   const int key = a_dtype * 100 + w_dtype * 10 + c_dtype;
   int rc;
   switch (key) {

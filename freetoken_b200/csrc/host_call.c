@@ -31,6 +31,7 @@ typedef struct {
 static PyObject *tensor_type, *get_device, *get_stream, *kernel_error, *error_names;
 static PyObject *s_data_ptr, *s_is_cuda, *s_dtype, *s_is_contiguous;
 static long long launches;
+static _Thread_local int promised_ahead;      // handed on behind the arguments (common.cuh)
 
 static int address_of(PyObject* o, void** out) {
   if (o == Py_None) {
@@ -61,7 +62,7 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
   if (n != l->n || (kwnames && PyTuple_GET_SIZE(kwnames)))
     return PyErr_Format(PyExc_TypeError, "%s takes %d arguments, not %zd", l->name, l->n, n);
-  Arg a[MOST_ARGS + 1];
+  Arg a[MOST_ARGS + 2];
   for (int k = 0; k < l->n; ++k) {
     PyObject* o = args[k];
     switch (l->kinds[k]) {
@@ -86,6 +87,7 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
   Py_DECREF(device);
   if (!stream) return NULL;
   a[l->n].p = PyLong_AsVoidPtr(stream);
+  a[l->n + 1].i = promised_ahead;
   Py_DECREF(stream);
   if (PyErr_Occurred()) return NULL;
   int rc;
@@ -178,6 +180,14 @@ static PyObject* need(PyObject* self, PyObject* const* args, Py_ssize_t n, PyObj
 
 static PyObject* count(PyObject* self, PyObject* unused) { return PyLong_FromLongLong(launches); }
 
+// ahead(promise) -> what was promised before; this thread's launches from here on
+static PyObject* ahead(PyObject* self, PyObject* promise) {
+  const int now = PyObject_IsTrue(promise), before = promised_ahead;
+  if (now < 0) return NULL;
+  promised_ahead = now;
+  return PyBool_FromLong(before);
+}
+
 // setup(tensor type, current device, current raw stream of a device, error type, {code: what it means})
 static PyObject* setup(PyObject* self, PyObject* args) {
   PyObject* o[5];
@@ -192,6 +202,7 @@ static PyObject* setup(PyObject* self, PyObject* args) {
 
 static PyMethodDef methods[] = {
     {"need", (PyCFunction)(void (*)(void))need, METH_FASTCALL | METH_KEYWORDS, "a CUDA tensor of that type, contiguous"},
+    {"ahead", ahead, METH_O, "whether this thread's launches may read weights, tables and metadata ahead of their wait"},
     {"count", count, METH_NOARGS, "kernels launched so far"},
     {"setup", setup, METH_VARARGS, "what the module asks Python for"},
     {NULL, NULL, 0, NULL},

@@ -224,13 +224,13 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32) route_small_kernel(
     float* __restrict__ weights, int* __restrict__ counts, int* __restrict__ offsets,
     int* __restrict__ sorted_route, int* __restrict__ sorted_token, int* __restrict__ active, int T, int E,
     int busy_of, int k, int softmax_scoring, int renormalize, float scale, int terms, int groups, int keep,
-    int group_top, float* __restrict__ tail) {
+    int group_top, float* __restrict__ tail, bool ahead) {
   extern __shared__ float smem[];  // [T][2][E] scores and choices, then ints: ids [T*k], first routes' experts [T*k]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int R = T * k;
   int* s_ids = reinterpret_cast<int*>(smem + (size_t)T * 2 * E);
   int* s_first = s_ids + R;
-  if (bias)
+  if (bias && ahead)
     for (int e = threadIdx.x * 32; e < E; e += blockDim.x * 32) warm(bias + e);
   pdl_wait();
 
@@ -309,7 +309,8 @@ template <typename AT, bool EARLY>
 __global__ void __launch_bounds__(128) router_logits_kernel(const AT* x, long long ldx,
                                                             const float* W,
                                                             float* __restrict__ logits, int T, int E,
-                                                            int H) {
+                                                            int H, bool ahead) {
+  if (!ahead) pdl_wait();
   // one block per (expert, 8 tokens); its 4 warps take a quarter of the row
   // each (pieces p = warp, warp+4, ... of 256 values) and their partial sums are
   // added in warp order
@@ -606,7 +607,7 @@ int ft_route_small(const float* logits, const float* bias, int* ids, float* weig
     cudaFuncSetAttribute(route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   launch_pdl(route_small_kernel, dim3(1), dim3(SMALL_WARPS * 32), smem, stream, logits, bias, ids, weights,
              counts, offsets, sorted_route, sorted_token, active, T, E, busy_of, k, softmax_scoring, renormalize, scale,
-             terms, groups, keep, group_top, tail);
+             terms, groups, keep, group_top, tail, promised_ahead);
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
@@ -618,7 +619,7 @@ int ft_router_logits(const void* x, int x_dtype, long long ldx, const float* W, 
   dim3 grid(E, (T + 7) / 8);
   FT_DISPATCH(x_dtype, AT,
               launch_pdl(T <= 8 ? router_logits_kernel<AT, true> : router_logits_kernel<AT, false>, grid, dim3(128), 0, stream,
-                         (const AT*)x, ldx, W, logits, T, E, H));
+                         (const AT*)x, ldx, W, logits, T, E, H, promised_ahead));
   FT_LAUNCH_CHECK();
   return FT_OK;
 }

@@ -65,6 +65,18 @@ def _host_module():
     return _host
 
 
+def read_ahead(promise: bool) -> bool:
+    """What this thread's launches may read ahead of their wait for the launch in front of them, from here on; returns what
+    held before (off at first).  With the promise that the package's launch right in front of another one never writes what
+    that one takes as a weight, a norm's or connection's weights, a bias, a table, positions, segment lists or block tables,
+    faces of few tokens fetch those while it still runs: :func:`rmsnorm`, :func:`qk_rope_store`, :func:`norm_add`,
+    :func:`join_layer_norm`, :func:`hyper_norm`, :func:`rms_rows`, :func:`latent_store`, :func:`gated_norm`,
+    :func:`token_shift`, :func:`router_logits`, :func:`route_small`, :func:`attn_decode`, :func:`attn_latent`,
+    :func:`skinny_gemm`, :func:`skinny_heads`, :func:`gemm_rows` and :func:`gemm_heads`.  A model's step promises it if
+    all its parts do (``Part.reads_ahead``).  Without the promise they wait first and may follow whatever wrote those."""
+    return _host_module().ahead(promise)
+
+
 def _fn(lib: str, name: str, sig: str):
     """The launcher ``name``: called with its arguments as ``sig`` lists them (p: a tensor, None, a buffer or an address; i,
     q: whole numbers of 32 and 64 bits; f: a float32), without the stream, which is the current one.  Raises
@@ -691,8 +703,8 @@ def latent_store(down: torch.Tensor, q: torch.Tensor, q_abs: Optional[torch.Tens
 
 
 # ------------------------------------------------------- mixers with a carried state
-# STATE_AHEAD.  A scan's or convolution's ``state_ahead`` promises that the launch right in front of this one does not write
-# ``state``: a step of one token a request then fetches it while that launch still runs.  So it is where a mixer's own
+# STATE_AHEAD.  A scan's or convolution's ``state_ahead`` promises that the launch right in front of this one writes neither
+# ``state`` nor the weights nor the segments' lists: a step of one token a request then fetches them while that launch still runs.  So it is where a mixer's own
 # projection comes in between; two scans of one state back to back leave it out.
 def conv_silu(x: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
               state: torch.Tensor, token_seg: torch.Tensor, seg_slot: torch.Tensor,
@@ -927,7 +939,7 @@ def gated_norm(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: t
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
     """One product per head on CUDA cores in float32: ``c[:, h, :] = a[:, h, :] @ w[h]^T``
     with ``a`` ``[T, heads, K]``, ``w`` ``[heads, N, K]`` (dense), ``c`` ``[T, heads, N]``;
-    ``a`` and ``c`` may be views with any row stride.  ``w`` as for :func:`gemm_rows`."""
+    ``a`` and ``c`` may be views with any row stride."""
     _need(a, "a", contiguous=False)
     _need(w, "w")
     _need(c, "c", contiguous=False)
@@ -949,8 +961,7 @@ def gemm_rows(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
 
     ``w`` is ``[N_w, K]`` or ``[G, N_w, K]``; with ``glu`` the N outputs are
     ``act(w[:N] a) * (w[N:] a)``.  ``rows`` is the number of (sorted) rows when
-    ``a_rows`` / ``c_rows`` redirect them.  Few dense rows fetch their first weights while the launch in
-    front still runs: ``w`` is never what that launch writes."""
+    ``a_rows`` / ``c_rows`` redirect them."""
     _need(a, "a", contiguous=False)
     _need(w, "w")
     _need(c, "c", contiguous=False)
@@ -1002,9 +1013,9 @@ def skinny_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *,
     :data:`ACTIVATIONS`, without ``glu``): that function of the float32 accumulator is stored; ``bias``
     (float32 ``[N]``, without ``glu``) is added to the accumulator first.  ``group_rows``: ``w`` is ``[G, N, K]``
     and rows ``g * group_rows ..`` of ``a`` and ``c`` belong to matrix g.  With ``glu``, ``act`` may be
-    ``silu``, ``swigluoai`` or ``gelu_tanh``.  The kernel fetches its first weights while the launch in front of it
-    still runs: ``w`` is never what that launch writes.  ``lists_ahead`` promises the same of ``group_offsets``, ``active``,
-    ``a_rows`` and ``c_rows``, and lets a grouped product do so too."""
+    ``silu``, ``swigluoai`` or ``gelu_tanh``.  ``lists_ahead`` promises that the launch in front writes neither ``w`` nor
+    ``group_offsets`` nor ``active``: a grouped product then fetches its first weights while that launch
+    still runs (an ungrouped one does so by :func:`read_ahead`)."""
     _need(a, "a", torch.bfloat16, contiguous=False)
     _need(w, "w", torch.bfloat16)
     _need(c, "c", contiguous=False)

@@ -517,6 +517,7 @@ struct NormAddArgs {
   long long copy_ld;
   int plus_one, next_plus_one, H;
   float eps, next_eps, mult;
+  bool ahead;              // promised_ahead
 };
 
 // KEEP > 0: rows of up to 4 * 256 * KEEP elements, a multiple of 4, every row 16-byte (bfloat16: 8-byte)
@@ -529,6 +530,7 @@ template <typename AT, int KEEP, bool EAGER = false>
 __global__ void __launch_bounds__(256) norm_add_kernel(NormAddArgs a) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
+  if (!a.ahead) pdl_wait();
   const int t = blockIdx.x, H = a.H;
   float4 w[KEEP > 0 ? KEEP : 1], w_next[EAGER ? KEEP : 1];
   if constexpr (EAGER) {
@@ -638,6 +640,7 @@ template <typename AT, int KEEP>
 __global__ void __launch_bounds__(256 * KEEP) norm_add_few_kernel(NormAddArgs a) {
   __shared__ float4 row[256 * KEEP];
   __shared__ float part[2][8];
+  if (!a.ahead) pdl_wait();
   const int t = blockIdx.x, H = a.H, gi = threadIdx.x, groups = H >> 2;
   const bool in = gi < groups;
   float4 w = make_float4(0.f, 0.f, 0.f, 0.f), w_next = w, x = w;
@@ -703,6 +706,7 @@ struct JoinNormArgs {
   void *out1, *out2;
   int H;
   float eps1, eps2;
+  bool ahead;              // promised_ahead
 };
 
 // EAGER (few tokens): the weights are fetched ahead of the wait for the launch in front.
@@ -710,6 +714,7 @@ template <typename AT, int KEEP, int THREADS, bool EAGER = false>
 __global__ void __launch_bounds__(THREADS) join_layer_norm_kernel(JoinNormArgs a) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
+  if (!a.ahead) pdl_wait();
   const int t = blockIdx.x, H = a.H;
   float4 e1[EAGER ? KEEP : 1], e2[EAGER ? KEEP : 1];
   if constexpr (EAGER) {
@@ -977,8 +982,9 @@ __global__ void __launch_bounds__(256)
 hyper_norm_vec_kernel(float* __restrict__ streams, const AT* branch, int k, const float* mix,
                       const float* out_w, const float* read,
                       const float* weight, const float* bias, float eps, int center,
-                      AT* __restrict__ normed, int H) {
+                      AT* __restrict__ normed, int H, bool ahead) {
   __shared__ float scratch[33];
+  if (!ahead) pdl_wait();
   const int t = blockIdx.x, groups = H >> 2;
   float m[S * S], ow[S], rd[S];
   float4 w_early[EAGER ? KEEP : 1], b_early[EAGER ? KEEP : 1];
@@ -1115,9 +1121,9 @@ static cudaError_t launch_hyper_keep(cudaStream_t stream, int T, int H, float* s
                                      const float* bias, float eps, int center, AT* normed) {
   const bool eager = T <= 64 && hyper_fetches_early(sizeof(AT) == 4, S, H, k);
   return eager   ? launch_pdl(hyper_norm_vec_kernel<AT, S, KEEP, true>, dim3(T), dim3(256), 0, stream, streams, branch, k,
-                              mix, out_w, read, weight, bias, eps, center, normed, H)
+                              mix, out_w, read, weight, bias, eps, center, normed, H, promised_ahead)
                  : launch_pdl(hyper_norm_vec_kernel<AT, S, KEEP, false>, dim3(T), dim3(256), 0, stream, streams, branch, k,
-                              mix, out_w, read, weight, bias, eps, center, normed, H);
+                              mix, out_w, read, weight, bias, eps, center, normed, H, promised_ahead);
 }
 template <typename AT, int S>
 static cudaError_t launch_hyper_vec(cudaStream_t stream, int T, int H, float* streams, const AT* branch, int k,
@@ -1137,9 +1143,9 @@ constexpr int RMS_KEEP = 16;
 template <typename AT>
 __global__ void __launch_bounds__(128)
 rms_rows_kernel(const AT* x, long long ldx, const float* w, AT* __restrict__ out,
-                long long ldo, int n, float eps) {
+                long long ldo, int n, float eps, bool ahead) {
   __shared__ float scratch[33];
-  for (int c = threadIdx.x * 32; c < n; c += blockDim.x * 32) warm(w + c);
+  for (int c = threadIdx.x * 32; ahead && c < n; c += blockDim.x * 32) warm(w + c);
   pdl_wait();
   const AT* row = x + (size_t)blockIdx.x * ldx;
   float sq = 0.f;
@@ -1189,6 +1195,7 @@ struct LatentStoreArgs {
   long long ld_down, ld_q, page_stride;
   int heads, dq, rank, rot, P, table_width, interleaved, turn_q;
   float eps;
+  bool ahead;              // promised_ahead
 };
 
 // A block a token; of few tokens (gridDim.y > 1) block 0 stores the row and the others share the heads' pairs, which
@@ -1196,6 +1203,7 @@ struct LatentStoreArgs {
 template <typename AT>
 __global__ void __launch_bounds__(128) latent_store_kernel(LatentStoreArgs a) {
   __shared__ float scratch[33];
+  if (!a.ahead) pdl_wait();
   const int t = blockIdx.x;
   const int pos = a.token_pos[t];
   const int half = a.rot >> 1;
@@ -1480,6 +1488,7 @@ int ft_norm_add(const BranchArgs* branch, const float* weight, int plus_one, flo
   a.weight = weight; a.residual = residual; a.next_weight = next_weight; a.next_out = next_out;
   a.copy_out = copy_out; a.copy_ld = copy_ld; a.plus_one = plus_one; a.next_plus_one = next_plus_one; a.H = H;
   a.eps = eps; a.next_eps = next_eps; a.mult = mult;
+  a.ahead = promised_ahead;
   const bool vec = !(H & 3) && H <= 4 * 256 * NORM_ADD_KEEP && branch_aligned(a.b) && !((uintptr_t)weight & 15) &&
                    !((uintptr_t)residual & 15) && !((uintptr_t)next_weight & 15) && !((uintptr_t)next_out & 15) &&
                    !((uintptr_t)copy_out & 15) && !(copy_ld & 3);
@@ -1517,6 +1526,7 @@ int ft_join_layer_norm(const BranchArgs* branch, float* residual, const float* w
   if (H <= 0 || H > 12288 || !residual || !w1 || !out1 || (w2 && !out2)) return FT_ERR_SHAPE;
   a.residual = residual; a.w1 = w1; a.b1 = b1; a.w2 = w2; a.b2 = b2; a.out1 = out1; a.out2 = out2; a.H = H;
   a.eps1 = eps1; a.eps2 = eps2;
+  a.ahead = promised_ahead;
   const bool vec = !(H & 3) && H <= 8192 && branch_aligned(a.b) && a.b.k <= 32 && !((uintptr_t)residual & 15) &&
                    !((uintptr_t)w1 & 15) && !((uintptr_t)b1 & 15) && !((uintptr_t)w2 & 15) && !((uintptr_t)b2 & 15) &&
                    !((uintptr_t)out1 & 15) && !((uintptr_t)out2 & 15);
@@ -1650,7 +1660,7 @@ int ft_rms_rows(const void* x, long long ldx, const float* w, void* out, long lo
   if (n <= 0) return FT_ERR_SHAPE;
   FT_DISPATCH(dtype, AT,
               (launch_pdl(rms_rows_kernel<AT>, dim3(T), dim3(128), 0, stream, (const AT*)x, ldx, w, (AT*)out, ldo, n,
-                          eps)));
+                          eps, promised_ahead)));
   FT_LAUNCH_CHECK();
   return FT_OK;
 }
@@ -1662,7 +1672,7 @@ int ft_latent_store(const void* down, long long ld_down, void* q, long long ld_q
   if (T <= 0) return FT_OK;
   if (heads <= 0 || dq < 0 || rank <= 0 || rot < 0 || (rot & 1) || P <= 0) return FT_ERR_SHAPE;
   LatentStoreArgs a{down, q, q_abs, pages, weight, cos_sin, token_pos, token_seg, block_table, ld_down, ld_q,
-                    page_stride, heads, dq, rank, rot, P, table_width, interleaved, turn_q, eps};
+                    page_stride, heads, dq, rank, rot, P, table_width, interleaved, turn_q, eps, promised_ahead};
   const int rounds = (heads * (rot / 2) + 127) / 128;
   const dim3 grid(T, T <= 64 && rounds > 1 ? 1 + (rounds < 16 ? rounds : 16) : 1);
   FT_DISPATCH(dtype, AT, (launch_pdl(latent_store_kernel<AT>, grid, dim3(128), 0, stream, a)));

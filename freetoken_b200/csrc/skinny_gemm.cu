@@ -45,7 +45,7 @@ struct SkinnyArgs {
   const float* bias = nullptr;   // [N], added to the accumulator (not with GLU)
   int group_rows = 0;            // > 0: every group has that many rows, group g the rows g * group_rows ..
   int lists_ahead = 0;           // the lists were written before the launch right in front of this one began
-  int first_round = 0;           // blocks that find a place on the chip at once
+  int first_round = 0;           // blocks that find a place on the chip at once (0: nothing is promised, all wait first)
   long long a_group = 0, c_group = 0;   // > 0 (with group_rows): group g's rows start at A + g * a_group, C + g * c_group
 };
 
@@ -282,7 +282,7 @@ void launch_one(SkinnyArgs a, dim3 grid, cudaStream_t stream, int* sms) {
     *sms = an_sm > 0 ? (int)(((long long)grid.x * grid.y + an_sm - 1) / an_sm) : INT_MAX;
     return;
   }
-  a.first_round = device_sms() * an_sm;
+  a.first_round = promised_ahead || a.lists_ahead ? device_sms() * an_sm : 0;
   launch_pdl(skinny_kernel<NT, GLU, OT, KS, U>, grid, dim3(KS * 32), 0, stream, a);
 }
 template <int NT, bool GLU, typename OT, int KS>

@@ -62,6 +62,7 @@ struct ShiftArgs {
   const int* seg_q_start;  // [S + 1]
   long long ldx, slot_stride;
   int T, W, M;
+  bool ahead;              // promised_ahead
 };
 
 // A thread owns VEC neighbouring columns of RUN consecutive tokens: their inputs stay in registers while the
@@ -69,6 +70,7 @@ struct ShiftArgs {
 // is the only one that reads the slot, and it alone replaces the slot's contents, after its read.
 template <typename AT, int VEC, int RUN>
 __global__ void __launch_bounds__(128) token_shift_kernel(ShiftArgs a) {
+  if (!a.ahead) pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   // of few tokens: the mixes' factors, cold in L2 and fetched one behind the other's store below, are near before the wait
   if (RUN == 1 && gridDim.x <= 64 && c < a.W)
@@ -529,7 +531,7 @@ int ft_token_shift(const void* x, long long ldx, const float* mu, void* out, flo
                    cudaStream_t stream) {
   if (T <= 0) return FT_OK;
   if (W <= 0 || M <= 0) return FT_ERR_SHAPE;
-  ShiftArgs a{x, mu, out, state, token_seg, seg_slot, seg_q_start, ldx, slot_stride, T, W, M};
+  ShiftArgs a{x, mu, out, state, token_seg, seg_slot, seg_q_start, ldx, slot_stride, T, W, M, promised_ahead};
   const bool aligned = !((uintptr_t)x & 15) && !((uintptr_t)mu & 15) && !((uintptr_t)out & 15) &&
                        !((uintptr_t)state & 15) && !(slot_stride & 3);
   const bool many = T >= 1024;

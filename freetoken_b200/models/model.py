@@ -60,6 +60,8 @@ class Model:
                                              for spec in plan.stream_maps]
         self.final_norm = NORMS.get(plan.final_norm.kind)(plan.final_norm, _prefix(plan.final_norm, ""))
         self.head = HEADS.get(plan.head.kind)(plan.head, _prefix(plan.head, ""))
+        # nobody writes weights, tables or metadata during a step: launches may read them ahead of their wait
+        self.reads_ahead = all(part.keeps_ahead() for part in self.leaf_parts())
         if nvtx:
             for i, block in enumerate(self.blocks):
                 _with_nvtx_range(block, f"layer_{i}")
@@ -168,6 +170,13 @@ class Model:
         ``logits`` ``[len(logit_rows), vocab]``.  ``all_rows_in_order`` says
         that ``logit_rows`` is ``0..T-1``, which saves the row gather.  ``caches`` holds a view
         per stop and, behind them, the embedding's if it has a cache need."""
+        before = ops.read_ahead(self.reads_ahead)
+        try:
+            return self._forward(ctx, caches, logit_rows, logits, all_rows_in_order)
+        finally:
+            ops.read_ahead(before)
+
+    def _forward(self, ctx, caches, logit_rows, logits, all_rows_in_order):
         T = ctx.num_tokens
         H = self.plan.hidden_size
         streams = self.plan.residual_streams

@@ -162,6 +162,8 @@ class PagedAttention(PagedSoftmaxCore, Mixer):
     runs its prompts and decoded tokens on the tensor-core kernels with heads of 128, at the price
     of a seventh more cache and arithmetic in the mixer.  float32 keeps the sizes as they are."""
 
+    reads_ahead = True
+
     scratch = ("attn",)
 
     graph_capturable = True

@@ -246,8 +246,15 @@ class Part:
     # not stated, and then nothing runs beside the part (``StepContext.beside``).  A class states its own: one that
     # inherits another's forward may write more.
     scratch: Optional[Tuple[str, ...]] = None
+    # Whether the part keeps to this: no launch of its own writes what the package's launch right behind it takes as a weight, a
+    # table or step metadata (positions, lists, block tables).  Then that launch may fetch them while the one in front still
+    # runs (``ops.read_ahead``); a model does so if all its parts say it.  Each class states it for itself, as above.
+    reads_ahead = False
     # whether the part runs something as a filler (``StepContext.beside``)
     has_filler = False
+
+    def keeps_ahead(self) -> bool:
+        return bool(vars(type(self)).get("reads_ahead"))
 
     def scratch_names(self) -> Optional[Tuple[str, ...]]:
         return vars(type(self)).get("scratch")

@@ -62,6 +62,7 @@ from .norm import NormedBranch, plain_branch
 
 @register_block("prenorm")
 class PreNormBlock(Block):
+    reads_ahead = True
     NORM_NAMES = ("mixer", "feed_forward")
     HAS_FEED_FORWARD = True
 
@@ -74,6 +75,7 @@ class PreNormBlock(Block):
 
 @register_block("parallel")
 class ParallelBlock(Block):
+    reads_ahead = True
     NORM_NAMES = ("mixer",)
     HAS_FEED_FORWARD = True          # or none: see check_parts
 
@@ -108,6 +110,7 @@ class ParallelBlock(Block):
 
 @register_block("parallel_norms")
 class ParallelNormsBlock(Block):
+    reads_ahead = True
     NORM_NAMES = ("mixer", "feed_forward")
     HAS_FEED_FORWARD = True          # or none: then only the mixer's norm
 
@@ -137,6 +140,8 @@ class ParallelNormsBlock(Block):
 class SandwichBlock(Block):
     """params: ``residual_mult`` (default 1): the factor on every normed sublayer output."""
 
+    reads_ahead = True
+
     NORM_NAMES = ("mixer", "mixer_out", "feed_forward", "feed_forward_out")
     HAS_FEED_FORWARD = True          # or none: then only the mixer's two norms
 
@@ -162,6 +167,7 @@ class SandwichBlock(Block):
 
 @register_block("hyper")
 class HyperBlock(Block):
+    reads_ahead = True
     NORM_NAMES = ("mixer", "feed_forward")
     HAS_FEED_FORWARD = True          # or none: then only the mixer's norm
 

@@ -23,6 +23,8 @@ class MixerSum(Mixer):
     """params: ``hidden_size``, ``members`` (PartSpecs of mixers, built below this mixer's
     prefix) and ``scales`` (one factor per member)."""
 
+    reads_ahead = True
+
     scratch = ("mixer_sum",)
 
     writes_into_out = True

@@ -35,6 +35,8 @@ class TokenEmbedding(Embedding):
     a factor on the embedded row.  ``pair_tensor`` with ``buckets, mul_prev, mul_cur``: a second
     table of ``buckets + 1`` rows, added by the hash of (previous token, token)."""
 
+    reads_ahead = True
+
     graph_capturable = True
 
     def __init__(self, spec, prefix):
@@ -96,6 +98,8 @@ class LMHead(Head):
     (its whole name), ``tied_to`` (full name of
     the embedding table, or None; a tied head with no ``scope`` has no tensor of its own,
     not even an optional one), ``softcap`` (None or 0: no cap on the logits)."""
+
+    reads_ahead = True
 
     graph_capturable = True
 

@@ -79,6 +79,8 @@ class SharedKVAttention(PagedSoftmaxCore, Mixer):
     ``q_temp_coef`` (0: no temperature), ``q_temp_every``, ``sliding_window`` (None: all
     keys), ``scope`` and ``names`` (q, k, o and the merged qk tensor below the scope)."""
 
+    reads_ahead = True
+
     scratch = ("kattn", "attn",)
 
     graph_capturable = True
@@ -164,6 +166,8 @@ class LatentAttention(PagedSoftmaxCore, Mixer):
     that size; ``names`` then also has q_down, q_norm, q_up), ``rot_dim`` with ``position`` (a PartSpec;
     the rotated key part and the rotated tail of every head's query), ``sliding_window``, ``gate_per``
     (``"head"``, the default, or ``"element"``: one gate per output value)."""
+
+    reads_ahead = True
 
     scratch = ("lattn", "attn",)
 

@@ -27,6 +27,8 @@ class DenseMLP(FeedForward):
     A gated feed-forward may also take the clamped pair ``swigluoai`` with ``act_alpha`` and
     ``act_limit``: ``g = min(gate, limit)``, ``u = clamp(up, -limit, limit)``, ``g sigmoid(alpha g) (u + 1)``."""
 
+    reads_ahead = True
+
     scratch = ("mlp",)
 
     graph_capturable = True

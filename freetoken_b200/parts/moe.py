@@ -77,6 +77,8 @@ class RoutedExperts(FeedForward):
     it per token (``checkpoint_names`` then also has shared_gate, ``[1, hidden]``, and router_gate, the name
     of the merged matrix the model keeps)."""
 
+    reads_ahead = True
+
     scratch = ("moe",)
 
     graph_capturable = True

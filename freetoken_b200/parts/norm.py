@@ -25,6 +25,8 @@ class RMSNorm(Norm):
     a second vector the normed values are multiplied by element by element (a layer scale behind a
     sublayer's output norm); the product of both vectors is formed once, in float32, at binding."""
 
+    reads_ahead = True
+
     graph_capturable = True
 
     def __init__(self, spec, prefix):
@@ -128,6 +130,8 @@ class LayerNorm(Norm):
     constant on the result - in front of a head, a factor on the logits that costs no pass over them; it is
     multiplied into weight and bias at binding, in float32."""
 
+    reads_ahead = True
+
     graph_capturable = True
 
     def __init__(self, spec, prefix):
@@ -193,6 +197,8 @@ class HyperNorm(Norm):
     of the ``in``, ``out`` and ``mix`` tensors below the layer's; None: the norm reads the plain sum
     of the streams and no branch leaves through it - the model's last norm; ``"identity"``: no
     tensors, every weight is one - with one stream the plain pre-norm residual ``x <- x + y``)."""
+
+    reads_ahead = True
 
     graph_capturable = True
 

@@ -117,16 +117,19 @@ class _Rotary(Position):
 
 @register_position("rotary_neox")
 class RotaryNeox(_Rotary):
+    reads_ahead = True
     interleaved = False
 
 
 @register_position("rotary_interleaved")
 class RotaryInterleaved(_Rotary):
+    reads_ahead = True
     interleaved = True
 
 
 @register_position("none")
 class NoPosition(Position):
+    reads_ahead = True
     graph_capturable = True
     interleaved = False
     rotary_dim = 0

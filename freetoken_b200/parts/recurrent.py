@@ -75,6 +75,8 @@ class SelectiveStateSpace(_Recurrent):
     norm_eps``, ``scope`` and ``names`` (in, conv, conv_bias, dt_bias, a_log, d, norm, o below
     the scope).  The input projection's rows are ``z | x | B | C | dt``."""
 
+    reads_ahead = True
+
     scratch = ("ssd",)
 
     kernels = ("recurrent",)
@@ -142,6 +144,8 @@ class GatedDelta(_Recurrent):
     beta, decay: the projections; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv:
     the merged projection and convolution the model keeps).  Query / key head ``h // (heads /
     key_heads)`` serves head ``h``; q is multiplied by ``key_dim ** -0.5`` after its unit norm."""
+
+    reads_ahead = True
 
     scratch = ("delta",)
 
@@ -217,6 +221,8 @@ class ChannelDelta(_Recurrent):
     of the decay's and the gate's; q_conv, k_conv, v_conv; a_log, dt_bias, norm, o; in and conv: the
     merged projection and convolution the model keeps).  ``dt_bias`` has one entry per head and key
     channel, ``norm`` one per value of a head (shared by the heads)."""
+
+    reads_ahead = True
 
     scratch = ("cdelta",)
 
@@ -300,6 +306,8 @@ class Retention(_Recurrent):
     ** -0.5`` after the rotation; the read-out of a head is divided by its root mean square (no
     weight), the row gated by ``silu(W_g h)``."""
 
+    reads_ahead = True
+
     scratch = ("retention",)
 
     kernels = ("retention",)
@@ -370,6 +378,8 @@ class TimeMixing(Mixer):
     gate: projections; decay_down, decay_up: the decay's two steps; w0, u, norm, o; mu and rkvg: the merged
     mixes and projections the model keeps).  ``r, k, v`` and ``gate`` rows have one width, so ``key_dim`` must equal
     ``head_dim``; ``norm`` has one entry per value of the concatenated heads."""
+
+    reads_ahead = True
 
     scratch = ("tmix",)
 

@@ -30,6 +30,8 @@ from .norm import add_pending
 class EmbeddingMix(StreamMap):
     """params: ``hidden_size``, ``tensor`` (the matrix ``[H, 2 H]``, the stream's columns first)."""
 
+    reads_ahead = True
+
     graph_capturable = True
 
     def __init__(self, spec, prefix):
