@@ -169,20 +169,24 @@ class StepContext:
                filler: bool = False):
         """``(first(), second())``, two pieces of a step that need nothing of each other; ``scratch``: the workspace names
         of either (:meth:`Part.scratch_names`).  ``filler``: the second is the shorter one by far and takes what the first
-        leaves of the chip (shared experts beside the chain of router, selection and routed ones).  Where a decode step is captured they become two branches of the graph: a launch of few tokens leaves
-        most of the chip idle, and two chains of such launches pass in the time of the longer one.  Branches that
-        would write the same scratch, or whose scratch is not known, run one after the other, and so does everything outside a
-        capture (there a launch costs the host more than it costs the device)."""
+        leaves of the chip (shared experts beside the chain of router, selection and routed ones).  Where a decode step is captured
+        they become two branches of the graph: a launch of few tokens leaves most of the chip idle, and two chains of such launches
+        pass in the time of the longer one.  Branches that would write the same scratch, or whose scratch is not known, run one
+        after the other, and so does everything outside a capture (there a launch costs the host more than it costs the device)."""
         streams = self.minor if filler else self.side
         if not streams or None in scratch or set(scratch[0]) & set(scratch[1]) or not torch.cuda.is_current_stream_capturing():
             return first(), second()
         side, main = streams.pop(), torch.cuda.current_stream(self.device)
         side.wait_stream(main)
-        with torch.cuda.stream(side):
-            b = second()
-        a = first()
-        main.wait_stream(side)
-        streams.append(side)
+        try:
+            with torch.cuda.stream(side):
+                b = second()
+            a = first()
+        finally:
+            # joined whatever happens: a capture that ends with a branch left open fails with an error of its own, in the place
+            # of the one that a piece raised
+            main.wait_stream(side)
+            streams.append(side)
         return a, b
 
     @property

@@ -20,6 +20,34 @@ def test_outside_a_capture_one_follows_the_other():
     assert order == [1, 2]
 
 
+@pytest.mark.parametrize("failing", ["first", "second", None])
+def test_a_branch_is_joined_whatever_a_piece_raises(failing, monkeypatch):
+    """A capture left with an open branch would end in an error of its own, in the place of the piece's."""
+    import contextlib
+    calls = []
+
+    class Stream:
+        def __init__(self, name):
+            self.name = name
+
+        def wait_stream(self, other):
+            calls.append((self.name, other.name))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream("main"))
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    ctx = context(side=[Stream("side")])
+
+    def piece(name):
+        def run():
+            if name == failing:
+                raise KeyError(name)
+            return name
+        return run
+    with contextlib.nullcontext() if failing is None else pytest.raises(KeyError):
+        assert ctx.beside(piece("first"), piece("second"), ("x",), ("y",)) == ("first", "second")
+    assert calls == [("side", "main"), ("main", "side")] and [s.name for s in ctx.side] == ["side"]
+
+
 def test_parts_name_every_buffer_they_write():
     """The scratch a part states covers the workspace names in its class and in the faces it calls."""
     import inspect
